@@ -134,7 +134,7 @@ hdbf_status potrf_db_impl(hdbf_context* ctx, T* A, int lda, int n, int nb, int b
                     HDBF_TRY(dbtrsm_impl(ctx, Aii, lda, at(A, lda, ps, inner), lda, rows, isz,
                                          isz, std::min(kPotrfDbTrsmMicroBlock, isz)));
                 } else {
-                    HDBF_TRY(trsm_rlt(ctx, rows, isz, Aii, lda, at(A, lda, ps, inner), lda));
+                    HDBF_TRY(trsm_rlt_ready(ctx, rows, isz, Aii, lda, at(A, lda, ps, inner), lda));
                 }
             }
             if (ps < oend) {  // update_next_inner_panel (:210-249)
@@ -200,7 +200,7 @@ hdbf_status potrf_blocked_rl_impl(hdbf_context* ctx, T* A, int lda, int n, int n
         HDBF_TRY(potrf_diag(ctx, psz, Akk, lda, info, k));
         if (tr <= 0) continue;
         T* A21 = at(A, lda, k + psz, k);
-        HDBF_TRY(trsm_rlt(ctx, tr, psz, Akk, lda, A21, lda));
+        HDBF_TRY(trsm_rlt_ready(ctx, tr, psz, Akk, lda, A21, lda));
         HDBF_TRY(syrk_lower(ctx, tr, psz, A21, lda, at(A, lda, k + psz, k + psz), lda));
     }
     return last_cuda(ctx);

@@ -24,14 +24,15 @@ hdbf_status potrf_diag(hdbf_context* ctx, int n, float* A, long long lda, int* i
                        int info_base)
 {
     if (n <= 0) return HDBF_STATUS_SUCCESS;
-    if (n <= kDiagLeaf) return potf2_small(ctx, n, A, lda, info, info_base);
+    HDBF_TRY(ensure_ws(ctx, n));
+    if (n <= kDiagLeaf) return potf2_small(ctx, n, A, lda, info, info_base, ws_inv(ctx));
     if (n <= potrf_block_max_n()) return potrf_block(ctx, n, A, lda, info, info_base, nullptr, 0);
     const int n1 = split_at(n, kDiagLeaf);
     const int n2 = n - n1;
     float* A21 = A + n1;
     float* A22 = A + (long long)n1 * lda + n1;
     HDBF_TRY(potrf_diag(ctx, n1, A, lda, info, info_base));
-    HDBF_TRY(trsm_rlt(ctx, n2, n1, A, lda, A21, lda));
+    HDBF_TRY(trsm_rlt_ready(ctx, n2, n1, A, lda, A21, lda));
     HDBF_TRY(syrk_lower(ctx, n2, n1, A21, lda, A22, lda));
     return potrf_diag(ctx, n2, A22, lda, info, info_base + n1);
 }
@@ -80,6 +81,15 @@ hdbf_status trsm_rlt(hdbf_context* ctx, int rows, int cols, const float* L, long
     float* inv = ws_inv(ctx);
     HDBF_TRY(tri_inv64(ctx, cols, L, ldl, false, inv));
     return trsm_rlt_rec(ctx, rows, cols, L, ldl, B, ldb, inv);
+}
+
+hdbf_status trsm_rlt_ready(hdbf_context* ctx, int rows, int cols, const float* L, long long ldl,
+                           float* B, long long ldb)
+{
+    if (rows <= 0 || cols <= 0) return HDBF_STATUS_SUCCESS;
+    // The recursion of a larger diagonal block reuses the inverse table.
+    if (cols > potrf_block_max_n()) return trsm_rlt(ctx, rows, cols, L, ldl, B, ldb);
+    return trsm_rlt_rec(ctx, rows, cols, L, ldl, B, ldb, ws_inv(ctx));
 }
 
 // B(rows x cols) <- L^{-1} B, L unit lower, same scheme on row halves.

@@ -311,9 +311,10 @@ size_t skinny_partial_floats(int n);
 hdbf_status sgemm_sub_tn(hdbf_context* ctx, int M, int N, int K, const float* A, long long lda,
                          const float* B, long long ldb, float* C, long long ldc);
 
-// Unblocked-in-shared-memory Cholesky of an n x n (n <= 64) diagonal block.
+// Cholesky of an n x n (n <= 64) diagonal block; with inv also the inverse of
+// its factor (one tri_inv64 block).
 hdbf_status potf2_small(hdbf_context* ctx, int n, float* A, long long lda, int* info,
-                        int info_base);
+                        int info_base, float* inv = nullptr);
 
 // Inverses of the 64x64 diagonal blocks of lower-triangular L (order n) into
 // out[b*4096 ...] (column-major blocks); unit selects an implicit unit diagonal.
@@ -451,10 +452,15 @@ hdbf_status add_damping(cudaStream_t s, float* A, int n, long long lda, float la
 hdbf_status potrf_block(hdbf_context* ctx, int n, float* A, long long lda, int* info,
                         int info_base, float* W, long long ldw);
 int potrf_block_max_n();
+// Orders up to potrf_block_max_n() also leave the 64x64 diagonal-block
+// inverses of the factor in ws_inv, for a trsm_rlt_ready with the same block.
 hdbf_status potrf_diag(hdbf_context* ctx, int n, float* A, long long lda, int* info,
                        int info_base);
 hdbf_status trsm_rlt(hdbf_context* ctx, int rows, int cols, const float* L, long long ldl,
                      float* B, long long ldb);
+// trsm_rlt against the block that potrf_diag has just factored on this stream.
+hdbf_status trsm_rlt_ready(hdbf_context* ctx, int rows, int cols, const float* L, long long ldl,
+                           float* B, long long ldb);
 hdbf_status trsm_llu(hdbf_context* ctx, int rows, int cols, const float* L, long long ldl,
                      float* B, long long ldb);
 // Create the look-ahead stream and events (outside stream capture).
@@ -492,6 +498,11 @@ hdbf_status potf2_small(hdbf_context* ctx, int n, double* A, long long lda, int*
                         int info_base);
 hdbf_status trsm_rlt(hdbf_context* ctx, int rows, int cols, const double* L, long long ldl,
                      double* B, long long ldb);
+inline hdbf_status trsm_rlt_ready(hdbf_context* ctx, int rows, int cols, const double* L,
+                                  long long ldl, double* B, long long ldb)
+{
+    return trsm_rlt(ctx, rows, cols, L, ldl, B, ldb);
+}
 hdbf_status trsm_llu(hdbf_context* ctx, int rows, int cols, const double* L, long long ldl,
                      double* B, long long ldb);
 hdbf_status syrk_lower(hdbf_context* ctx, int n, int k, const double* A, long long lda,

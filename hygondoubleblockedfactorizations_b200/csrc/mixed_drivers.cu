@@ -319,7 +319,7 @@ hdbf_status potrf_mixed_body(hdbf_context* ctx, int prec, float* A, long long ld
         // pair's panels side by side, rows counted from the pair's first column
         char* sh = pair ? hi + ((size_t)(k + psz - k0) * lds + (k - k0)) * 2 : hi;
         if (!inv_tc) {
-            HDBF_TRY(trsm_rlt(ctx, tr, psz, Akk, lda, A21, lda));
+            HDBF_TRY(trsm_rlt_ready(ctx, tr, psz, Akk, lda, A21, lda));
         } else {
             // L21 = A21 L11^{-T} as one tensor-core GEMM with W = L11^{-1}
             // from the diagonal-block kernel; A21 is rounded into the scratch

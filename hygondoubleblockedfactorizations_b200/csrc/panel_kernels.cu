@@ -8,124 +8,59 @@
 #include <cfloat>
 
 #include "internal.h"
+#include "tile64.cuh"
 
 namespace hdbf {
 namespace {
 
 constexpr int kLeaf = 64;
 
-// Right-looking Cholesky of an n x n (n <= 64) lower block, register
-// resident: thread (r, g) = (tid % 64, tid / 64) holds A(r, g + 4i), i < 16.
-// Per column j the owner group publishes the scaled column to shared memory
-// and every thread applies the rank-1 update to its own 16 entries (two
-// barriers per column, no shared-memory read-modify-write chains).
+// Cholesky of an n x n (n <= 64) lower block, one CTA (chol64), and, with inv,
+// the inverse of its factor in tri_inv64's layout, so that the panel solve
+// which follows needs no launch of its own for it.
 // Pivot test and info follow LAPACK xPOTRF: the first column whose updated
 // diagonal is not > 0 (or is NaN) stops the factorization, its value is left
 // in place, and info = info_base + j + 1 (first failure wins).  A block whose
 // info is already non-zero is left untouched.
-__global__ void __launch_bounds__(256) potf2_kernel(int n, float* A, long long lda, int* info,
-                                                    int info_base)
+__global__ void __launch_bounds__(tile64::kThreads)
+potf2_kernel(int n, float* A, long long lda, int* info, int info_base, float* inv)
 {
-    __shared__ float lcol[kLeaf];
-    __shared__ float s_d;
-    const int tid = threadIdx.x;
-    const int r = tid & 63;
-    const int g = tid >> 6;
+    __shared__ __align__(16) float S[kLeaf * tile64::kLd];
+    __shared__ __align__(16) float W[kLeaf * tile64::kLd];
+    __shared__ __align__(16) float X[tile64::kScratch];
+    __shared__ float rd[kLeaf];
+    __shared__ int s_fail;
     if (info && *reinterpret_cast<volatile int*>(info) != 0) return;
-
-    float a[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const int c = g + 4 * i;
-        a[i] = (r < n && c < n && r >= c) ? A[(long long)c * lda + r] : 0.f;
+    tile64::load_lower<false>(S, A, lda, n, false);
+    __syncthreads();
+    const int fail = tile64::chol64(S, n, &s_fail);
+    tile64::store_lower(A, S, lda, n);
+    if (fail >= 0 && threadIdx.x == 0 && info) atomicCAS(info, 0, info_base + fail + 1);
+    if (inv) {
+        tile64::inv64(S, W, X, rd, false);
+        tile64::store_inv(inv, W, false);
     }
-
-    int failed_at = -1;
-    for (int j = 0; j < n; ++j) {
-        const int gj = j & 3, ij = j >> 2;
-        float own = 0.f;
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-            if (i == ij) own = a[i];
-        if (g == gj && r == j) s_d = own;
-        __syncthreads();
-        const float d = s_d;
-        if (!(d > 0.f)) {  // uniform: every thread read the same value
-            failed_at = j;
-            break;
-        }
-        const float sd = sqrtf(d);
-        const float rcp = 1.0f / sd;
-        if (g == gj) {
-            const float v = (r == j) ? sd : (r > j ? own * rcp : own);
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-                if (i == ij) a[i] = v;
-            if (r > j) lcol[r] = v;
-        }
-        __syncthreads();
-        if (r > j) {
-            const float lr = lcol[r];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int c = g + 4 * i;
-                if (c > j && c <= r) a[i] = fmaf(-lr, lcol[c], a[i]);
-            }
-        }
-    }
-
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const int c = g + 4 * i;
-        if (r < n && c < n && r >= c) A[(long long)c * lda + r] = a[i];
-    }
-    if (failed_at >= 0 && tid == 0 && info) atomicCAS(info, 0, info_base + failed_at + 1);
 }
 
-
 // Inverses of the 64x64 diagonal blocks of a lower-triangular n x n matrix
-// (unit or non-unit diagonal), one CTA per block, thread t solving
-// L_bb x = e_t by forward substitution (right-looking, so every L read is a
-// shared-memory broadcast).  out[b*4096 + c*64 + r] = inv(L_bb)(r, c); a
-// partial last block is padded with the identity.
+// (unit or non-unit diagonal), one CTA per block (inv64).
+// out[b*4096 + c*64 + r] = inv(L_bb)(r, c); a partial last block is padded
+// with the identity.
 // mode 0: lower non-unit, 1: lower unit, 2: upper non-unit (the upper block
 // U is inverted as (U^T)^{-1} and stored transposed).
-__global__ void __launch_bounds__(kLeaf) tri_inv64_kernel(int n, const float* __restrict__ L,
-                                                          long long ldl, int mode, float* out)
+__global__ void __launch_bounds__(tile64::kThreads)
+tri_inv64_kernel(int n, const float* __restrict__ L, long long ldl, int mode, float* out)
 {
-    __shared__ float Ls[kLeaf][kLeaf + 1];  // Ls[r][c] = T(base + r, base + c), T lower
+    __shared__ __align__(16) float S[kLeaf * tile64::kLd];
+    __shared__ __align__(16) float W[kLeaf * tile64::kLd];
+    __shared__ __align__(16) float X[tile64::kScratch];
+    __shared__ float rd[kLeaf];
     const int base = blockIdx.x * kLeaf;
-    const int nb = min(kLeaf, n - base);
-    const int t = threadIdx.x;
-    const int unit = mode == 1;
-    for (int idx = t; idx < kLeaf * kLeaf; idx += kLeaf) {
-        const int c = idx / kLeaf, r = idx - c * kLeaf;
-        float v = 0.f;
-        if (r < nb && c < nb && r >= c)
-            v = mode == 2 ? L[(long long)(base + r) * ldl + base + c]
-                          : L[(long long)(base + c) * ldl + base + r];
-        Ls[r][c] = v;
-    }
+    tile64::load_lower<false>(S, L + (long long)base * ldl + base, ldl, min(kLeaf, n - base),
+                              mode == 2);
     __syncthreads();
-    float x[kLeaf];
-#pragma unroll
-    for (int i = 0; i < kLeaf; ++i) x[i] = (i == t) ? 1.f : 0.f;
-#pragma unroll
-    for (int k = 0; k < kLeaf; ++k) {
-        if (k < nb) {
-            if (!unit) x[k] = x[k] / Ls[k][k];
-#pragma unroll
-            for (int i = k + 1; i < kLeaf; ++i) x[i] = fmaf(-Ls[i][k], x[k], x[i]);
-        }
-    }
-    float* ob = out + (long long)blockIdx.x * kLeaf * kLeaf;
-    if (mode == 2) {
-#pragma unroll
-        for (int i = 0; i < kLeaf; ++i) ob[(long long)i * kLeaf + t] = x[i];  // row t of U^{-1}
-    } else {
-#pragma unroll
-        for (int i = 0; i < kLeaf; ++i) ob[(long long)t * kLeaf + i] = x[i];  // column t
-    }
+    tile64::inv64(S, W, X, rd, mode == 1);
+    tile64::store_inv(out + (long long)blockIdx.x * kLeaf * kLeaf, W, mode == 2);
 }
 
 // B(rows x cols) <- inv * B for rows <= 64 (inv = L^{-1} of the leaf block):
@@ -215,12 +150,12 @@ __global__ void __launch_bounds__(256) rlt_apply_kernel(int rows, int cols,
 }  // namespace
 
 hdbf_status potf2_small(hdbf_context* ctx, int n, float* A, long long lda, int* info,
-                        int info_base)
+                        int info_base, float* inv)
 {
     if (n <= 0) return HDBF_STATUS_SUCCESS;
     if (n > kLeaf) return HDBF_STATUS_INVALID_VALUE;
     ProfScope prof(ctx, kClsPotf2, (double)n * n * n / 3.0, 8.0 * n * n);
-    potf2_kernel<<<1, 256, 0, ctx->stream>>>(n, A, lda, info, info_base);
+    potf2_kernel<<<1, tile64::kThreads, 0, ctx->stream>>>(n, A, lda, info, info_base, inv);
     ctx->launches++;
     return last_cuda(ctx);
 }
@@ -238,7 +173,7 @@ hdbf_status tri_inv64_mode(hdbf_context* ctx, int n, const float* L, long long l
     const int blocks = (n + kLeaf - 1) / kLeaf;
     ProfScope prof(ctx, kClsTrsmInv, (double)blocks * kLeaf * kLeaf * kLeaf / 3.0,
                    8.0 * blocks * kLeaf * kLeaf);
-    tri_inv64_kernel<<<blocks, kLeaf, 0, ctx->stream>>>(n, L, ldl, mode, out);
+    tri_inv64_kernel<<<blocks, tile64::kThreads, 0, ctx->stream>>>(n, L, ldl, mode, out);
     ctx->launches++;
     return last_cuda(ctx);
 }

@@ -7,8 +7,8 @@
 // for every tile column k the CTAs solve the tiles below the diagonal against
 // the inverse D_k of the factored diagonal tile, then apply the rank-64 update
 // to the trailing tiles; with look-ahead, CTA 0 updates tile (k+1, k+1) first
-// and factors and inverts it (register-resident potf2) while the other CTAs
-// finish the update -- two bounded grid barriers per tile column.  With the
+// and factors and inverts it (tile64.cuh) while the other CTAs finish the
+// update -- two bounded grid barriers per tile column.  With the
 // inverse requested, W = L^{-1} (lower, the strictly upper tiles zeroed) is
 // formed by recursive doubling over tile blocks: for siblings A and C,
 // W(C,A) = -W(C,C) (L(C,A) W(A,A)), two GEMM phases per level.
@@ -22,6 +22,7 @@
 #include <algorithm>
 
 #include "internal.h"
+#include "tile64.cuh"
 
 namespace hdbf {
 namespace {
@@ -29,7 +30,7 @@ namespace {
 constexpr int kT = 64;        // tile
 constexpr int kThreads = 256;
 constexpr int kMaxNT = 16;    // n <= 1024
-constexpr int kLdS = 68;      // padded shared row (float4-aligned)
+constexpr int kLdS = tile64::kLd;  // padded shared row (float4-aligned)
 
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p)
 {
@@ -120,98 +121,6 @@ __device__ __forceinline__ void tile_mma(float acc[4][4], const float* As, const
     }
 }
 
-// Register-resident Cholesky of the nb x nb (nb <= 64) lower tile at T
-// (thread (r, g) holds T(r, g + 4i), i < 16).  Returns the first failing
-// column or -1 (uniform over the CTA).
-__device__ int potf2_tile(float* T, long long ld, int nb, float* lcol, float* s_d)
-{
-    const int tid = threadIdx.x, r = tid & 63, g = tid >> 6;
-    float a[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const int c = g + 4 * i;
-        a[i] = (r < nb && c < nb && r >= c) ? __ldcg(T + (long long)c * ld + r) : 0.f;
-    }
-    int failed_at = -1;
-    for (int j = 0; j < nb; ++j) {
-        const int gj = j & 3, ij = j >> 2;
-        float own = 0.f;
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-            if (i == ij) own = a[i];
-        if (g == gj && r == j) *s_d = own;
-        __syncthreads();
-        const float d = *s_d;
-        if (!(d > 0.f)) {
-            failed_at = j;
-            break;
-        }
-        const float sd = sqrtf(d);
-        const float rcp = 1.0f / sd;
-        if (g == gj) {
-            const float v = (r == j) ? sd : (r > j ? own * rcp : own);
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-                if (i == ij) a[i] = v;
-            if (r > j) lcol[r] = v;
-        }
-        __syncthreads();
-        if (r > j) {
-            const float lr = lcol[r];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int c = g + 4 * i;
-                if (c > j && c <= r) a[i] = fmaf(-lr, lcol[c], a[i]);
-            }
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const int c = g + 4 * i;
-        if (r < nb && c < nb && r >= c) T[(long long)c * ld + r] = a[i];
-    }
-    return failed_at;
-}
-
-// D = L^{-1} for the nb x nb lower tile L (padded with the identity to 64):
-// thread t < 64 solves L x = e_t by forward substitution over a shared copy.
-// D is written column-major with leading dimension 64 (D[c * 64 + r]).
-__device__ void tri_inv_tile(const float* L, long long ld, int nb, float* Ls /*64 x 65*/,
-                             float* D)
-{
-    {
-        float v[kT * kT / kThreads];  // all loads in flight before the first store
-#pragma unroll
-        for (int u = 0; u < kT * kT / kThreads; ++u) {
-            const int q = threadIdx.x + u * kThreads, c = q >> 6, r = q & 63;
-            v[u] = (r < nb && c < nb && r >= c) ? __ldcg(L + (long long)c * ld + r) : 0.f;
-        }
-#pragma unroll
-        for (int u = 0; u < kT * kT / kThreads; ++u) {
-            const int q = threadIdx.x + u * kThreads, c = q >> 6, r = q & 63;
-            Ls[r * 65 + c] = v[u];
-        }
-    }
-    __syncthreads();
-    const int t = threadIdx.x;
-    if (t < kT) {
-        float x[kT];
-#pragma unroll
-        for (int i = 0; i < kT; ++i) x[i] = (i == t) ? 1.f : 0.f;
-#pragma unroll
-        for (int k = 0; k < kT; ++k) {
-            if (k < nb) {
-                x[k] = x[k] / Ls[k * 65 + k];
-#pragma unroll
-                for (int i = k + 1; i < kT; ++i) x[i] = fmaf(-Ls[i * 65 + k], x[k], x[i]);
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < kT; ++i) D[t * kT + i] = x[i];  // column t
-    }
-    __syncthreads();
-}
-
 __global__ void __launch_bounds__(kThreads, 1)
 potrf_block_kernel(int n, float* A, long long lda, int* info, int info_base, float* W,
                    long long ldw, float* dinv, float* Tsc, unsigned* ctr, int* fail,
@@ -219,8 +128,9 @@ potrf_block_kernel(int n, float* A, long long lda, int* info, int info_base, flo
 {
     __shared__ __align__(16) float As[kT * kLdS];
     __shared__ __align__(16) float Bs[kT * kLdS];
-    __shared__ float lcol[kT];
-    __shared__ float s_d;
+    __shared__ __align__(16) float Xs[tile64::kScratch];
+    __shared__ float rd[kT];
+    __shared__ int s_fail;
     __shared__ int s_flag;
     const int NT = (n + kT - 1) / kT;
     const int cta = blockIdx.x;
@@ -240,19 +150,20 @@ potrf_block_kernel(int n, float* A, long long lda, int* info, int info_base, flo
     grid_barrier(sy);
     if (skip) return;
 
-    // Factor (and invert) diagonal tile k on this CTA; false on a bad pivot.
-    auto factor_diag = [&](int k) -> bool {
-        const int f = potf2_tile(tile(k, k), lda, ext(k), lcol, &s_d);
-        if (f >= 0) {
-            if (tid == 0) {
-                if (info) atomicCAS(info, 0, info_base + k * kT + f + 1);
-                atomicExch(fail, 1);
-            }
-            return false;
-        }
+    // Factor and invert diagonal tile k on this CTA.  The inverse is also
+    // formed when the tile fails: the columns before the failing one are valid.
+    auto factor_diag = [&](int k) {
+        tile64::load_lower<true>(As, tile(k, k), lda, ext(k), false);
         __syncthreads();
-        tri_inv_tile(tile(k, k), lda, ext(k), As, dinv + (long long)k * kT * kT);
-        return true;
+        const int f = tile64::chol64(As, ext(k), &s_fail);
+        tile64::store_lower(tile(k, k), As, lda, ext(k));
+        if (f >= 0 && tid == 0) {
+            if (info) atomicCAS(info, 0, info_base + k * kT + f + 1);
+            atomicExch(fail, 1);
+        }
+        tile64::inv64(As, Bs, Xs, rd, false);
+        tile64::store_inv(dinv + (long long)k * kT * kT, Bs, false);
+        __syncthreads();
     };
     // A(i,j) -= L(i,k) L(j,k)^T (lower part only on the diagonal)
     auto update_tile = [&](int k, int i, int j) {

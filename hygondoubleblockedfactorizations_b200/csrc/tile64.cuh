@@ -1,0 +1,335 @@
+// Cholesky factor and triangular inverse of one 64 x 64 tile in shared memory,
+// by a block of 256 threads.  Both sit on the serial chain of every diagonal
+// block, so what counts is latency, not rate.
+//
+// chol64 works in panels whose diagonal block fits in a thread's registers
+// (chol_panel_fast), with look-ahead between the panels.
+// inv64 inverts the four 16 x 16 diagonal blocks (one warp each, a lane per
+// column) and joins them by doubling: W21 = -W22 (L21 W11), first 16, then 32.
+// One tile in one launch (load, factor, inverse, stores): 9.9 us; 62 us before,
+// with two barriers, an IEEE square root and a division per column of the
+// factor and one thread per column of the inverse, a division per row.
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace hdbf {
+namespace tile64 {
+
+constexpr int kN = 64;
+constexpr int kLd = 68;        // shared row pitch: float4 / double2 aligned
+constexpr int kThreads = 256;
+constexpr int kScratch = 32 * 36;
+
+template <class T>
+struct alignas(16) Vec4 {
+    T x[4];
+};
+
+// 1 / d, and 1 / sqrt(d) with sqrt(d), each to about an ulp: one Newton step
+// on the hardware estimate (and one residual correction of the root).  For d
+// in fast_range, where no intermediate product over- or underflows.
+__device__ __forceinline__ bool fast_range(float d) { return d > 1e-30f && d < 1e30f; }
+__device__ __forceinline__ bool fast_range(double d) { return d > 1e-250 && d < 1e250; }
+__device__ __forceinline__ float fast_rcp(float d)
+{
+    const float r = __fdividef(1.f, d);
+    return fmaf(r, fmaf(-d, r, 1.f), r);
+}
+__device__ __forceinline__ double fast_rcp(double d) { return 1.0 / d; }
+__device__ __forceinline__ void rsqrt_pair(float d, float& r, float& s)
+{
+    r = rsqrtf(d);
+    r = fmaf(0.5f * r, fmaf(-d * r, r, 1.f), r);
+    s = d * r;
+    s = fmaf(fmaf(-s, s, d), 0.5f * r, s);
+}
+__device__ __forceinline__ void rsqrt_pair(double d, double& r, double& s)
+{
+    s = sqrt(d);
+    r = 1.0 / s;
+}
+__device__ __forceinline__ float sqrt_t(float d) { return sqrtf(d); }
+__device__ __forceinline__ double sqrt_t(double d) { return sqrt(d); }
+__device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
+
+// S[c * kLd + r] <- src(r, c) = src[c * ld + r] for r >= c, identity beyond nb,
+// zero above the diagonal; every load of the thread in flight before the first
+// store.  trans reads src(c, r) instead (a lower tile from an upper matrix).
+template <bool CG, class T>
+__device__ __forceinline__ void load_lower(T* S, const T* src, long long ld, int nb, bool trans)
+{
+    constexpr int kPer = kN * kN / kThreads;
+    T v[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        const int q = threadIdx.x + u * kThreads, hi = q >> 6, lo = q & 63;
+        const int r = trans ? hi : lo, c = trans ? lo : hi;  // memory (lo, hi) of src
+        const T* p = src + (long long)hi * ld + lo;
+        v[u] = (r < nb && c <= r) ? (CG ? __ldcg(p) : *p) : (r == c ? T(1) : T(0));
+    }
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        const int q = threadIdx.x + u * kThreads, hi = q >> 6, lo = q & 63;
+        S[(trans ? lo : hi) * kLd + (trans ? hi : lo)] = v[u];
+    }
+}
+
+// Panel width.  Its diagonal block sits in every panel thread's registers; 8
+// beats 16 (11.0K against 13.7K cycles a tile), whose panel is bound by the FMA
+// issue of its two warps.
+constexpr int PW = 8;
+
+// One panel of chol64 on the first two warps: every thread factors its own
+// register copy of the PW x PW diagonal block and carries one row below it
+// along, so a column costs a reciprocal square root, a multiply and FMAs with
+// no exchange between lanes at all (a shuffle per multiplier measured 2.5x
+// slower: 180 cycles a column).  Returns false, with nothing written, when a
+// pivot is outside the fast range (failed, tiny, huge or NaN).
+template <class T>
+__device__ bool chol_panel_fast(T* S, int kb)
+{
+    const int tid = threadIdx.x;
+    const int row = kb + PW + tid;
+    T D[PW][PW], x[PW];  // D[c][r], r >= c
+#pragma unroll
+    for (int c = 0; c < PW; ++c) {
+#pragma unroll
+        for (int g = c / 4; g < PW / 4; ++g) {
+            const Vec4<T> v = *reinterpret_cast<const Vec4<T>*>(S + (kb + c) * kLd + kb + 4 * g);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) D[c][4 * g + i] = v.x[i];
+        }
+        x[c] = row < kN ? S[(kb + c) * kLd + row] : T(0);
+    }
+    asm volatile("bar.sync 1, 64;" ::: "memory");  // both warps hold the block: it may be written
+    bool ok = true;
+#pragma unroll
+    for (int j = 0; j < PW; ++j) {
+        ok = ok & fast_range(D[j][j]);
+        T r;
+        rsqrt_pair(D[j][j], r, D[j][j]);
+        x[j] *= r;
+#pragma unroll
+        for (int i = j + 1; i < PW; ++i) D[j][i] *= r;
+#pragma unroll
+        for (int c = j + 1; c < PW; ++c) {
+#pragma unroll
+            for (int i = c; i < PW; ++i) D[c][i] = fma_t(-D[j][i], D[j][c], D[c][i]);
+            x[c] = fma_t(-x[j], D[j][c], x[c]);
+        }
+    }
+    if (!ok) return false;
+    if (row < kN) {
+#pragma unroll
+        for (int c = 0; c < PW; ++c) S[(kb + c) * kLd + row] = x[c];
+    }
+    if (tid == 63) {  // the diagonal block; above its diagonal the input stays
+#pragma unroll
+        for (int c = 0; c < PW; ++c)
+#pragma unroll
+            for (int i = c; i < PW; ++i) S[(kb + c) * kLd + kb + i] = D[c][i];
+    }
+    return true;
+}
+
+// The same panel for pivots outside the fast range: IEEE operations, the pivot
+// tested before each column.  One warp.  Returns the failing column of the
+// panel or -1.
+template <class T>
+__device__ __noinline__ int chol_panel_careful(T* S, int kb)
+{
+    const int lane = threadIdx.x & 31;
+    for (int j = kb; j < kb + PW; ++j) {
+        const T d = S[j * kLd + j];
+        __syncwarp();
+        if (!(d > T(0))) return j - kb;
+        const T s = sqrt_t(d), r = T(1) / s;
+        for (int i = j + lane; i < kN; i += 32)
+            S[j * kLd + i] = i == j ? s : S[j * kLd + i] * r;
+        __syncwarp();
+        for (int c = j + 1; c < kb + PW; ++c) {
+            const T lc = S[j * kLd + c];
+            for (int i = c + lane; i < kN; i += 32)
+                S[c * kLd + i] = fma_t(-S[j * kLd + i], lc, S[c * kLd + i]);
+        }
+        __syncwarp();
+    }
+    return -1;
+}
+
+// Columns [c0, c1) of the tile, rows c0 .. 63 on or below the diagonal, minus
+// the product of panel columns [kb, kb + kmax): thread t of nthr takes four
+// rows of one column at a time.
+template <int CW, class T>
+__device__ __forceinline__ void chol_update(T* S, int kb, int kmax, int c0, int c1, int t, int nthr)
+{
+    for (int c = c0 + t % CW; c < c1; c += CW)
+    for (int r = c0 + 4 * (t / CW); r < kN; r += 4 * (nthr / CW)) {
+        if (r + 3 < c) continue;
+        Vec4<T> acc = {};
+        const T* p = S + kb * kLd;
+#pragma unroll 8
+        for (int k = 0; k < kmax; ++k, p += kLd) {
+            const Vec4<T> a = *reinterpret_cast<const Vec4<T>*>(p + r);
+            const T b = p[c];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc.x[i] = fma_t(a.x[i], b, acc.x[i]);
+        }
+        Vec4<T>* o = reinterpret_cast<Vec4<T>*>(S + c * kLd + r);
+        Vec4<T> v = *o;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v.x[i] -= acc.x[i];
+        *o = v;
+    }
+}
+
+// Cholesky of the lower tile in S (identity beyond nb); S is complete on entry
+// (barrier before) and on return (barrier inside).  Returns the first column
+// whose updated diagonal is not > 0 (or is NaN), or -1, the same in every
+// thread.  On failure the columns before it are factored and applied to the
+// rest, the failing diagonal holds its updated value.
+// Look-ahead: after a panel all warps update only the next panel's columns;
+// the rest of that update runs on warps 2..7 beside the next panel.
+template <class T>
+__device__ int chol64(T* S, int nb, int* s_fail)
+{
+    const int tid = threadIdx.x;
+    for (int kb = 0; kb < nb; kb += PW) {
+        if (tid == 0) *s_fail = -1;
+        bool ok = true;
+        if (tid < 64) ok = chol_panel_fast(S, kb);
+        else if (kb > 0) chol_update<16>(S, kb - PW, PW, kb + PW, kN, tid - 64, kThreads - 64);
+        if (__syncthreads_or(!ok)) {
+            if (tid < 32) {
+                const int f = chol_panel_careful(S, kb);
+                if (tid == 0) *s_fail = f < 0 ? -1 : kb + f;
+            }
+            __syncthreads();
+            const int fail = *s_fail;
+            if (fail >= 0) {
+                chol_update<16>(S, kb, fail - kb, kb + PW, kN, tid, kThreads);
+                __syncthreads();
+                return fail;
+            }
+        }
+        if (kb + PW < kN) {
+            chol_update<PW>(S, kb, PW, kb + PW, kb + 2 * PW, tid, kThreads);
+            __syncthreads();
+        }
+    }
+    return -1;
+}
+
+// The lower part (nb x nb) of S to dst(r, c) = dst[c * ld + r].
+template <class T>
+__device__ __forceinline__ void store_lower(T* dst, const T* S, long long ld, int nb)
+{
+#pragma unroll
+    for (int u = 0; u < kN * kN / kThreads; ++u) {
+        const int q = threadIdx.x + u * kThreads, c = q >> 6, r = q & 63;
+        if (r < nb && c <= r) dst[(long long)c * ld + r] = S[c * kLd + r];
+    }
+}
+
+// All of W, packed: dst[c * 64 + r] (trans: dst[r * 64 + c]) = W(r, c).
+template <class T>
+__device__ __forceinline__ void store_inv(T* dst, const T* W, bool trans)
+{
+#pragma unroll
+    for (int u = 0; u < kN * kN / kThreads; ++u) {
+        const int q = threadIdx.x + u * kThreads, hi = q >> 6, lo = q & 63;
+        dst[q] = trans ? W[lo * kLd + hi] : W[hi * kLd + lo];
+    }
+}
+
+// W <- inverse of the lower tile in S (upper part of S ignored; unit: implicit
+// ones on the diagonal), W[c * kLd + r], zero above the diagonal.  X: kScratch
+// entries, rd: 64.  S complete on entry; W complete on return.
+template <class T>
+__device__ void inv64(const T* S, T* W, T* X, T* rd, bool unit)
+{
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int q = tid; q < kN * kLd; q += kThreads) W[q] = T(0);
+    if (tid < kN) rd[tid] = unit ? T(1) : T(1) / S[tid * kLd + tid];
+    __syncthreads();
+    if (warp < 4 && lane < 16) {
+        const int b = warp * 16;
+        T x[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) x[i] = i == lane ? T(1) : T(0);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            const T* col = S + (b + k) * kLd + b;
+            x[k] *= rd[b + k];
+#pragma unroll
+            for (int i = k + 1; i < 16; ++i) x[i] = fma_t(-col[i], x[k], x[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) W[(b + lane) * kLd + b + i] = x[i];
+    }
+    __syncthreads();
+    {  // two pairs of 16 x 16 blocks, two rows of one column per thread
+        const int b = (tid >> 7) * 32, c = (tid & 127) >> 3, r = (tid & 7) * 2;
+        T* Xp = X + (tid >> 7) * 256;
+        T t0 = T(0), t1 = T(0);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            const T w = W[(b + c) * kLd + b + k];
+            const T* l = S + (b + k) * kLd + b + 16 + r;
+            t0 = fma_t(l[0], w, t0);
+            t1 = fma_t(l[1], w, t1);
+        }
+        Xp[c * 16 + r] = t0;
+        Xp[c * 16 + r + 1] = t1;
+        __syncthreads();
+        t0 = t1 = T(0);
+        // only k <= row: a NaN in a later row of the tile must not reach this one
+#pragma unroll 4
+        for (int k = 0; k <= r; ++k) {
+            const T x = Xp[c * 16 + k];
+            const T* w = W + (b + 16 + k) * kLd + b + 16 + r;
+            t0 = fma_t(w[0], x, t0);
+            t1 = fma_t(w[1], x, t1);
+        }
+        t1 = fma_t(W[(b + 17 + r) * kLd + b + 17 + r], Xp[c * 16 + r + 1], t1);
+        W[(b + c) * kLd + b + 16 + r] = -t0;
+        W[(b + c) * kLd + b + 16 + r + 1] = -t1;
+    }
+    __syncthreads();
+    {  // the pair of 32 x 32 blocks, four rows of one column per thread
+        const int c = tid >> 3, r = (tid & 7) * 4;
+        Vec4<T> t = {};
+#pragma unroll
+        for (int k = 0; k < 32; ++k) {
+            const T w = W[c * kLd + k];
+            const Vec4<T> l = *reinterpret_cast<const Vec4<T>*>(S + k * kLd + 32 + r);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) t.x[i] = fma_t(l.x[i], w, t.x[i]);
+        }
+        *reinterpret_cast<Vec4<T>*>(X + c * 36 + r) = t;
+        __syncthreads();
+        Vec4<T> v = {};
+#pragma unroll 4
+        for (int k = 0; k < r; ++k) {
+            const T x = X[c * 36 + k];
+            const Vec4<T> w = *reinterpret_cast<const Vec4<T>*>(W + (32 + k) * kLd + 32 + r);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v.x[i] = fma_t(w.x[i], x, v.x[i]);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const T x = X[c * 36 + r + k];
+            const Vec4<T> w = *reinterpret_cast<const Vec4<T>*>(W + (32 + r + k) * kLd + 32 + r);
+#pragma unroll
+            for (int i = k; i < 4; ++i) v.x[i] = fma_t(w.x[i], x, v.x[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) W[c * kLd + 32 + r + i] = -v.x[i];
+    }
+    __syncthreads();
+}
+
+}  // namespace tile64
+}  // namespace hdbf

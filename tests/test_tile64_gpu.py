@@ -1,0 +1,50 @@
+"""Diagonal-tile Cholesky (64 x 64, one launch) at its panel edges, on failing
+tiles and outside the range of its fast pivots."""
+import numpy as np
+import pytest
+
+from tests.common import dev, host2d, info_tensor, ptr
+
+pytestmark = pytest.mark.gpu
+
+
+def spd(n, scale=1.0, seed=0):
+    rng = np.random.default_rng(seed + n)
+    G = rng.uniform(-1, 1, (n, n))
+    return ((G @ G.T / n + np.eye(n)) * scale).astype(np.float32)
+
+
+def factor(torch, hd, handle, A, n):
+    d, info = dev(torch, A), info_tensor(torch)
+    hd.call("double_blocked_potrf", handle.ptr, ptr(d), n, n, 64, 64, ptr(info))
+    torch.cuda.synchronize()
+    return host2d(d, n, n, n), int(info.item())
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 16, 23, 56, 57, 63, 64, 65, 72, 130])
+@pytest.mark.parametrize("scale", [1.0, 1e-36, 1e33])
+def test_tile_factor(torch_cuda, hd, handle, n, scale):
+    A = spd(n, scale)
+    F, info = factor(torch_cuda, hd, handle, A, n)
+    assert info == 0
+    L = np.tril(F).astype(np.float64)
+    # backward error of a Cholesky factor: (n + 1) u |L||L^T|, u = 2^-24, twice
+    # for the reciprocal square roots
+    bound = 2 * (n + 1) * 2.0 ** -24 * (np.abs(L) @ np.abs(L).T)
+    assert (np.abs(np.tril(L @ L.T - A)) <= bound).all()
+
+
+@pytest.mark.parametrize("col", [0, 1, 7, 8, 9, 31, 40, 63])
+@pytest.mark.parametrize("value", [-1.0, 0.0, np.nan])
+def test_tile_failure(torch_cuda, hd, handle, col, value):
+    n = 96
+    A = spd(n)
+    A[col, col] = value
+    F, info = factor(torch_cuda, hd, handle, A, n)
+    assert info == col + 1
+    # the leading columns are factored, rows below the tile included
+    k = col
+    L = np.tril(F)[:, :k].astype(np.float64)
+    R = np.tril(L @ L[:k].T - A[:, :k].astype(np.float64))
+    bound = 4 * (n + 1) * 2.0 ** -24 * (np.abs(L) @ np.abs(L[:k]).T)
+    assert (np.abs(R) <= bound)[~np.isnan(R)].all() and not np.isnan(R[:col]).any()
