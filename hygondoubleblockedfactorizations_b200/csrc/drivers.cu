@@ -9,7 +9,7 @@ namespace hdbf {
 
 namespace {
 constexpr int kDiagLeaf = 64;   // potf2_small / trsm_*_small leaf order
-constexpr int kClusterLeaf = 32;  // widest block of the cluster panel kernel
+constexpr int kClusterLeaf = 32;  // leaf width when the cluster panel kernel is forced
 
 // Split point for a recursion on `n` columns with `leaf`-aligned halves.
 inline int split_at(int n, int leaf)
@@ -121,22 +121,33 @@ hdbf_status getrf_workspace(hdbf_context* ctx, int n, GetrfWs* ws)
     return HDBF_STATUS_SUCCESS;
 }
 
-// Recursive (Toledo/Gustavson) LU of an m x w panel.  Leaves are column
-// blocks of the handle's panel-leaf width (default 128; 32 when the cluster
-// kernel is forced) and go to the cluster kernel when they fit in one cluster
-// (w <= 32), otherwise to the grid-wide kernel.  ipiv receives (local row + 1
-// + ipiv_add) for the panel's w columns.
+// Leaf width for the cluster panel kernel at height m, 0 for the grid-wide one.
+// A cluster holds 64 or more columns up to m = 13300 (FP32): there a column
+// costs 1.7-2.0 us against 4.1-4.5 us.  Taller panels would need leaves of 32
+// or 16 columns (2.4 and 4.6 us a column at m = 16384 and 30000), and the extra
+// merges between them (compose, moves, TRSM, GEMM: ~130 us each) cost more than
+// the grid-wide kernel's 128-column leaf (5-6.5 us a column).
+int panel_cluster_leaf(hdbf_context* ctx, int m, int elem)
+{
+    if (ctx->panel_mode == 1) return 0;
+    const int leaf = getf2_cluster_leaf(ctx, m, elem);
+    return ctx->panel_mode == 2 || leaf * elem >= 256 ? leaf : 0;
+}
+
+// Recursive (Toledo/Gustavson) LU of an m x w panel.  A leaf is as wide as one
+// cluster can hold at this height, at most the handle's panel-leaf width (32
+// when the cluster kernel is forced); heights beyond a cluster, and the forced
+// grid-wide kernel, take leaves of the panel-leaf width on getf2_coop.  ipiv
+// receives (local row + 1 + ipiv_add) for the panel's w columns.
 hdbf_status getrf_panel(hdbf_context* ctx, int m, int w, float* A, long long lda, int* ipiv,
                         int ipiv_add, int* info, int info_base, bool pivot, const GetrfWs& ws)
 {
     if (m <= 0 || w <= 0) return HDBF_STATUS_SUCCESS;
-    const int leaf = ctx->panel_mode == 2 ? kClusterLeaf : ctx->panel_leaf;
+    const int held = panel_cluster_leaf(ctx, m, (int)sizeof(float));
+    const int widest = ctx->panel_mode == 2 ? kClusterLeaf : ctx->panel_leaf;
+    const int leaf = held > 0 ? std::min(held, widest) : widest;
     if (w <= leaf) {
-        if (ctx->panel_mode != 1 && w <= kClusterLeaf) {
-            const hdbf_status st =
-                getf2_cluster(ctx, m, w, A, lda, ipiv, ipiv_add, info, info_base, pivot);
-            if (st != HDBF_STATUS_NOT_SUPPORTED) return st;
-        }
+        if (held > 0) return getf2_cluster(ctx, m, w, A, lda, ipiv, ipiv_add, info, info_base, pivot);
         return getf2_coop(ctx, m, w, A, lda, ipiv, ipiv_add, info, info_base, pivot);
     }
     const int w1 = split_at(w, leaf);

@@ -878,15 +878,20 @@ hdbf_status apply_moves(hdbf_context* ctx, double* A, long long lda, int ncols, 
     return last_cuda(ctx);
 }
 
-// Recursive (Toledo/Gustavson) LU of an m x w FP64 panel down to 64-column
-// leaves on the grid-wide kernel; ipiv receives (local row + 1 + ipiv_add).
+// Recursive (Toledo/Gustavson) LU of an m x w FP64 panel; leaves as in the FP32
+// panel (64 columns on the grid-wide kernel).
 hdbf_status getrf_panel(hdbf_context* ctx, int m, int w, double* A, long long lda, int* ipiv,
                         int ipiv_add, int* info, int info_base, bool pivot, const GetrfWs& ws)
 {
     if (m <= 0 || w <= 0) return HDBF_STATUS_SUCCESS;
-    if (w <= kPMaxW) return getf2_coop64(ctx, m, w, A, lda, ipiv, ipiv_add, info, info_base, pivot);
+    const int held = panel_cluster_leaf(ctx, m, (int)sizeof(double));
+    const int leaf = held > 0 ? held : kPMaxW;
+    if (w <= leaf) {
+        if (held > 0) return getf2_cluster(ctx, m, w, A, lda, ipiv, ipiv_add, info, info_base, pivot);
+        return getf2_coop64(ctx, m, w, A, lda, ipiv, ipiv_add, info, info_base, pivot);
+    }
     double* temp = reinterpret_cast<double*>(ws.temp);
-    const int w1 = split64(w);
+    const int w1 = std::max(leaf, w / 2 / leaf * leaf);
     const int w2 = w - w1;
     HDBF_TRY(getrf_panel(ctx, m, w1, A, lda, ipiv, ipiv_add, info, info_base, pivot, ws));
     double* A12 = A + (long long)w1 * lda;

@@ -1,273 +1,629 @@
 // GETRF panel leaf on one thread-block cluster: partially pivoted LU of an
-// m x w (w <= 32) column block, replacing rocsolver_sgetrf's unblocked leaf on
-// the tall panel (src/getrf/getrf_pivot_internal.h:17-39) whenever the block
-// fits in the shared memory of one cluster (up to 16 CTAs).
+// m x w (w <= 128, m <= 32768) column block, FP32 and FP64, replacing
+// rocsolver_sgetrf's unblocked leaf on the tall panel
+// (src/getrf/getrf_pivot_internal.h:17-39).
 //
-// Each CTA of the cluster keeps a contiguous slice of rows resident in shared
-// memory (column-major tile[c * ldt + r], ldt = rpc rounded up to odd); thread t
-// owns local rows t, t + T,
-// ...  Per column j:
-//   1. every CTA finds its candidate (largest |a| over owned rows >= j, lowest
-//      row on ties -- LAPACK ISAMAX) and writes it, the candidate row and (on
-//      the CTA owning row j) the diagonal row into its own slot (two parities);
-//   2. one cluster barrier (release / acquire);
-//   3. warp 0 of every CTA reads the cluster's candidates through distributed
-//      shared memory, reduces them identically, and copies the winning row and
-//      the diagonal row from their slots (copies, so owners may overwrite their
-//      live rows at once) into local shared memory for the other warps;
-//   4. the owners swap rows j and p, every thread scales its rows below j by
-//      the reciprocal pivot (division when |pivot| < FLT_MIN, as xGETF2) and
-//      applies the rank-1 update to its own rows.
-// A slot of parity j & 1 is rewritten at column j + 2 only after the barrier
-// of column j + 1, which every CTA reaches after its reads of column j, so two
-// parities suffice.  All CTAs run the same loop, so every cluster barrier is
-// met; there are no spin-waits.
+// What bounds it is the serial chain of one pivot per column, so the whole
+// block stays on chip and the exchange of each column stays inside a cluster
+// (<= 16 CTAs, <= 16 SMs), where a message takes a fraction of an L2 round
+// trip.  The block sits in the cluster's shared memory, a contiguous slice of
+// rows per CTA (tile[c * ldt + r], ldt odd).  It is factored in sub-panels of
+// NB columns (64 bytes of a row: 16 FP32, 8 FP64) that live in registers,
+// thread t owning local rows t, t + TH, ...  Per column:
+//   1. every warp finds its candidate (largest |a| over owned rows >= J, lowest
+//      row on ties -- LAPACK ISAMAX) with integer warp reductions; its owner
+//      lane writes the candidate's sub-panel row to shared memory;
+//   2. after one block barrier a few warps reduce the warps' candidates and
+//      push the CTA's one (magnitude, row, NB values) and, from the CTA that
+//      owns it, the diagonal row to every CTA of the cluster with st.async,
+//      counted in bytes on the receiver's mbarrier: data and flag arrive in
+//      one trip, and nothing needs a fence;
+//   3. every warp reduces the CTAs' candidates from its own shared memory; the
+//      owners replace their rows in registers, and every thread scales and
+//      applies the rank-1 update.  The registers rotate by one column per step
+//      (the column just finished goes to the back), so that the loop is rolled
+//      and a row swap carries the multipliers already computed.
+// Two message buffers (column parity) suffice: a CTA sends column J + 1 only
+// after a block barrier that follows all its reads of column J, and nobody can
+// send column J + 2 without it.
+// After a sub-panel, the rest of the block (other columns of the tile) takes
+// the sub-panel's interchanges as at most 2 NB composed row moves through
+// distributed shared memory; every CTA reads the new diagonal rows and solves
+// U12 = L11^{-1} A12 for itself (L11 came with the candidates), and every thread
+// applies the rank-NB update to its own rows, in column order: the result is
+// bit-identical to column-by-column elimination (getf2_coop).
+// Measured per column, against the grid-wide kernel's 4.1-6.5 us: 1.7 us at
+// m = 1001, 1.8 at 4096, 2.0 at 8192 (FP32).  The rest is issue: about 400
+// mostly dependent instructions per warp and column, two warps per scheduler.
+// Waits on an mbarrier are bounded by the handle's poll limit; an expired wait
+// records a timeout and the CTA runs on without waiting, so that every cluster
+// barrier is still met.
 #include <cfloat>
 #include <climits>
-#include <cooperative_groups.h>
 
 #include "internal.h"
-
-namespace cg = cooperative_groups;
 
 namespace hdbf {
 namespace {
 
-constexpr int kClThreads = 256;
-constexpr int kClMaxW = 32;
-constexpr int kClSlot = 4 + 2 * kClMaxW;  // [|v|, row, -, - | candidate row | diagonal row]
+constexpr int kClMaxW = 128;
 constexpr int kClMaxCluster = 16;
+constexpr int kClMaxRows = 2048;  // per CTA: 4 register rows for each of 512 threads
 
-__device__ __forceinline__ bool better(float v, int i, float bv, int bi)
+__device__ __forceinline__ uint32_t smem_addr(const void* p)
 {
-    if (i == INT_MAX) return false;
-    if (bi == INT_MAX) return true;
-    return v > bv || (v == bv && i < bi);
+    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+__device__ __forceinline__ uint32_t peer_addr(uint32_t addr, int rank)
+{
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void cluster_arrive()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait()
+{
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void push16(uint32_t dst, uint32_t bar, uint4 v)
+{
+    asm volatile(
+        "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, "
+        "[%5];" ::"r"(dst),
+        "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(bar)
+        : "memory");
+}
+__device__ __forceinline__ float peer_load(uint32_t addr, float)
+{
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ double peer_load(uint32_t addr, double)
+{
+    double v;
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(addr) : "memory");
+    return v;
 }
 
-// Copy an nr x w column block between global memory (leading dimension lda)
-// and the shared tile (leading dimension ldt), eight independent loads in
-// flight per thread.
-template <bool TO_SMEM>
-__device__ __forceinline__ void move_block(float* A, long long lda, float* tile, int ldt, int nr,
-                                           int w)
+template <class T>
+struct Bits;
+template <>
+struct Bits<float> {
+    using Mag = unsigned;
+    static __device__ __forceinline__ Mag of(float v) { return __float_as_uint(v); }
+    static __device__ __forceinline__ float val(Mag m) { return __uint_as_float(m); }
+    static __device__ __forceinline__ float rcp(float v) { return __frcp_rn(v); }
+};
+template <>
+struct Bits<double> {
+    using Mag = unsigned long long;
+    static __device__ __forceinline__ Mag of(double v)
+    {
+        return (unsigned long long)__double_as_longlong(v);
+    }
+    static __device__ __forceinline__ double val(Mag m) { return __longlong_as_double((long long)m); }
+    static __device__ __forceinline__ double rcp(double v) { return 1.0 / v; }
+};
+template <class T>
+using Mag = typename Bits<T>::Mag;
+
+// |v| as bits that order like the values; a NaN loses to everything else.
+template <class T>
+__device__ __forceinline__ Mag<T> mag_bits(T v)
 {
-    const int total = nr * w;
-    int e = threadIdx.x;
-    for (; e + 7 * kClThreads < total; e += 8 * kClThreads) {
-        float v[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int q = e + u * kClThreads, c = q / nr, r = q - c * nr;
-            v[u] = TO_SMEM ? A[(long long)c * lda + r] : tile[c * ldt + r];
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int q = e + u * kClThreads, c = q / nr, r = q - c * nr;
-            if (TO_SMEM) tile[c * ldt + r] = v[u];
-            else A[(long long)c * lda + r] = v[u];
-        }
-    }
-    for (; e < total; e += kClThreads) {
-        const int c = e / nr, r = e - c * nr;
-        if (TO_SMEM) tile[c * ldt + r] = A[(long long)c * lda + r];
-        else A[(long long)c * lda + r] = tile[c * ldt + r];
-    }
+    return v == v ? Bits<T>::of(v < T(0) ? -v : v) & (~(Mag<T>)0 >> 1) : (Mag<T>)0;
+}
+// Largest magnitude over the warp and the lowest row that has it (INT_MAX: no
+// candidate).
+__device__ __forceinline__ void warp_argmax(unsigned vb, int row, unsigned& mv, int& mrow)
+{
+    mv = __reduce_max_sync(0xffffffffu, vb);
+    mrow = __reduce_min_sync(0xffffffffu, vb == mv ? row : INT_MAX);
+}
+__device__ __forceinline__ void warp_argmax(unsigned long long vb, int row, unsigned long long& mv,
+                                            int& mrow)
+{
+    const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(vb >> 32));
+    const unsigned lo = __reduce_max_sync(
+        0xffffffffu, (unsigned)(vb >> 32) == hi ? (unsigned)(vb & 0xffffffffu) : 0u);
+    mv = ((unsigned long long)hi << 32) | lo;
+    mrow = __reduce_min_sync(0xffffffffu, vb == mv ? row : INT_MAX);
 }
 
-__global__ void __launch_bounds__(kClThreads, 1)
-getf2_cluster_kernel(int m, int w, float* A, long long lda, int rpc, int ldt, int* ipiv,
-                     int ipiv_add, int* info, int info_base, int pivot)
-{
-    extern __shared__ __align__(16) float smem[];
-    float* slots = smem;               // [2][kClSlot]
-    float* tile = smem + 2 * kClSlot;  // tile[c * ldt + r], ldt odd (no bank conflicts)
-    __shared__ float red_v[kClThreads / 32];
-    __shared__ int red_i[kClThreads / 32];
-    __shared__ float s_prow[kClMaxW], s_orow[kClMaxW];
-    __shared__ int s_p;
+__device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float min_normal(float) { return FLT_MIN; }
+__device__ __forceinline__ double min_normal(double) { return DBL_MIN; }
+__device__ __forceinline__ float abs_t(float v) { return fabsf(v); }
+__device__ __forceinline__ double abs_t(double v) { return fabs(v); }
 
-    cg::cluster_group cluster = cg::this_cluster();
-    const int C = (int)cluster.num_blocks();
-    const int rank = (int)cluster.block_rank();
+template <class T>
+struct alignas(16) Vec4 {
+    T x[4];
+};
+
+template <class T>
+constexpr int kNB = 64 / (int)sizeof(T);
+
+// A candidate as it travels: five 16-byte chunks.
+template <class T>
+struct Cand;
+template <>
+struct alignas(16) Cand<float> {
+    unsigned mag;
+    int row;
+    int pad[2];
+    float x[16];
+};
+template <>
+struct alignas(16) Cand<double> {
+    unsigned long long mag;
+    int row;
+    int pad;
+    double x[8];
+};
+
+// Magnitude and row of a candidate in one 16-byte load.
+__device__ __forceinline__ void load_key(const Cand<float>& c, unsigned& mag, int& row)
+{
+    const uint2 v = *reinterpret_cast<const uint2*>(&c);
+    mag = v.x;
+    row = (int)v.y;
+}
+__device__ __forceinline__ void load_key(const Cand<double>& c, unsigned long long& mag, int& row)
+{
+    const uint4 v = *reinterpret_cast<const uint4*>(&c);
+    mag = ((unsigned long long)v.y << 32) | v.x;
+    row = (int)v.z;
+}
+
+template <class T>
+struct ClusterSmem {
+    Cand<T> in[2][kClMaxCluster];  // the cluster's candidates
+    T diag[2][kNB<T>];             // the diagonal row
+    Cand<T> own[2][16];            // this CTA's warps' candidates
+    T own_diag[2][kNB<T>];
+    T U[kClMaxW / 2][kNB<T>][2];  // U12 of the sub-panel, columns in pairs: U[c / 2][k][c & 1]
+    T L[kNB<T>][kNB<T> + 1];      // L11 rows as they arrived (rotated, see the kernel)
+    int mv_pos[32], mv_src[32];   // composed interchanges of the sub-panel
+    unsigned long long bar[2];
+};
+
+// acc(c), acc(c + 1) -= l * (u(c), u(c + 1)): one packed FMA in FP32.
+struct Pair32 {
+    unsigned long long v;
+    __device__ __forceinline__ Pair32(float x, float y)
+    {
+        asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(x), "f"(y));
+    }
+    __device__ __forceinline__ void fma(Pair32 l, Pair32 u)
+    {
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(v) : "l"(l.v), "l"(u.v));
+    }
+    __device__ __forceinline__ void get(float& x, float& y) const
+    {
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
+    }
+};
+struct Pair64 {
+    double x, y;
+    __device__ __forceinline__ Pair64(double a, double b) : x(a), y(b) {}
+    __device__ __forceinline__ void fma(Pair64 l, Pair64 u)
+    {
+        x = ::fma(l.x, u.x, x);
+        y = ::fma(l.y, u.y, y);
+    }
+    __device__ __forceinline__ void get(double& a, double& b) const
+    {
+        a = x;
+        b = y;
+    }
+};
+template <class T>
+struct PairOf {
+    using type = Pair32;
+};
+template <>
+struct PairOf<double> {
+    using type = Pair64;
+};
+
+__device__ __forceinline__ void copy_async(float* dst, const float* src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_async(double* dst, const double* src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(dst)), "l"(src)
+                 : "memory");
+}
+
+template <class T, int TH, int R>
+__global__ void __launch_bounds__(TH, 1)
+getf2_cluster_kernel(int m, int w, T* A, long long lda, int rpc, int* ipiv, int ipiv_add, int* info,
+                     int info_base, int pivot, int* err)
+{
+    constexpr int NB = kNB<T>;
+    constexpr int NW = TH / 32;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    ClusterSmem<T>& sm = *reinterpret_cast<ClusterSmem<T>*>(smem_raw);
+    T* tile = reinterpret_cast<T*>(smem_raw + sizeof(ClusterSmem<T>));
+    const int ldt = rpc | 1;
+
+    int C, rank;
+    asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(C));
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int r0 = rank * rpc;
     const int nr = max(0, min(m, r0 + rpc) - r0);
+    const unsigned limit = spin_limit_of(err);
+    const uint32_t base = smem_addr(smem_raw);
+    auto off_of = [&](const void* q) { return smem_addr(q) - base; };
+    auto peer_base = [&](int q) { return peer_addr(base, q); };
+    bool dead = false;  // an expired wait: run on without waiting
 
-    move_block<true>(A + r0, lda, tile, ldt, nr, w);
-    cluster.sync();  // every CTA of the cluster is running before any DSMEM access
+    if (tid == 0) {
+        for (int b = 0; b < 2; ++b)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&sm.bar[b])));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    for (int c = 0; c < w; ++c) {  // the whole slice in flight at once
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int r = tid + TH * i;
+            if (r < nr) copy_async(tile + c * ldt + r, A + (long long)c * lda + r0 + r);
+        }
+    }
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    cluster_arrive();
+    cluster_wait();  // every CTA runs and its barriers are initialised
 
     const int steps = min(m, w);
-    for (int j = 0; j < steps; ++j) {
-        const int par = j & 1;
-        float* my_slot = slots + par * kClSlot;
-        const int owner = j / rpc;
+    const bool others = w > NB;
+    for (int jb = 0; jb < steps; jb += NB) {
+        const int nbc = min(NB, w - jb);     // columns of this sub-panel
+        const int sb = min(nbc, steps - jb);  // pivots in it
+        cluster_arrive();  // releases the updates of the previous sub-panel
+        const int owner = jb / rpc;  // rpc is a multiple of NB: it owns all diagonal rows
+        T a[R][NB];
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int r = tid + TH * i;
+#pragma unroll
+            for (int c = 0; c < NB; ++c)
+                a[i][c] = (r < nr && c < nbc) ? tile[(jb + c) * ldt + r] : T(0);
+        }
+        // Composed interchanges, one position per lane of the last warp:
+        // position mv_pos takes the row that was at mv_src before the
+        // sub-panel.  Lanes < NB are the diagonal positions, later ones the
+        // pivot rows met so far.
+        int mv_pos = lane < NB ? jb + lane : -1, mv_src = mv_pos, mv_cnt = NB;
+        const bool own_j = rank == owner;
+        const int dst = lane & 15, ch = tid >> 4;  // sender roles: peer, 16-byte chunk
 
-        // 1. local candidate
-        float bv = -1.f;
-        int bi = INT_MAX;
-        if (pivot) {
-            for (int r = tid; r < nr; r += kClThreads) {
-                if (r0 + r >= j) {
-                    const float v = fabsf(tile[j * ldt + r]);
-                    if (bi == INT_MAX || v > bv) { bv = v; bi = r0 + r; }
+#pragma unroll 1
+        for (int j = 0; j < sb; ++j) {
+            const int J = jb + j, par = J & 1;
+            // 1. this CTA's candidates for column J
+            Mag<T> vb = 0;
+            int row = INT_MAX;
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const int r = tid + TH * i, g = r0 + r;
+                const bool can = r < nr && (pivot ? g >= J : g == J);
+                const Mag<T> b = mag_bits(a[i][0]);
+                if (can && (row == INT_MAX || b > vb)) {
+                    vb = b;
+                    row = g;
                 }
             }
+            Mag<T> mv;
+            int mrow;
+            warp_argmax(vb, row, mv, mrow);
+            Cand<T>& mine_c = sm.own[par][warp];
+            if (row == mrow && (row != INT_MAX || lane == 0)) {
+                mine_c.mag = mv;
+                mine_c.row = mrow;
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                const float ov = __shfl_down_sync(0xffffffffu, bv, off);
-                const int oi = __shfl_down_sync(0xffffffffu, bi, off);
-                if (better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
+                for (int i = 0; i < R; ++i)
+                    if (R == 1 || r0 + tid + TH * i == mrow) {
+#pragma unroll
+                        for (int c = 0; c < NB; ++c) mine_c.x[c] = a[i][c];
+                    }
             }
-            if (lane == 0) { red_v[warp] = bv; red_i[warp] = bi; }
+            if (own_j) {
+#pragma unroll
+                for (int i = 0; i < R; ++i)
+                    if (r0 + tid + TH * i == J) {
+#pragma unroll
+                        for (int c = 0; c < NB; ++c) sm.own_diag[par][c] = a[i][c];
+                    }
+            }
+            if (tid == 0 && C > 1)  // every candidate (80 bytes) and the diagonal row
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
+                                 smem_addr(&sm.bar[par])),
+                             "r"(C * 80 + 64)
+                             : "memory");
+            __syncthreads();
+            // 2. the CTA's candidate to every CTA: 16 peers per 16-byte chunk
+            int from = 0;
+            if (C == 1 || warp < 3) {
+                Mag<T> k = 0;
+                int kr = INT_MAX;
+                if (lane < NW) load_key(sm.own[par][lane], k, kr);
+                warp_argmax(k, kr, mv, mrow);
+                from = __ffs(__ballot_sync(0xffffffffu, lane < NW && kr == mrow)) - 1;
+                if (C > 1 && dst < C && ch < 5)
+                    push16(peer_base(dst) + off_of(&sm.in[par][rank]) + 16 * ch,
+                           peer_base(dst) + off_of(&sm.bar[par]),
+                           reinterpret_cast<const uint4*>(&sm.own[par][from])[ch]);
+            } else if (own_j && warp < 5) {  // warps 3, 4: the diagonal row
+                if (dst < C)
+                    push16(peer_base(dst) + off_of(sm.diag[par]) + 16 * (ch - 6),
+                           peer_base(dst) + off_of(&sm.bar[par]),
+                           reinterpret_cast<const uint4*>(sm.own_diag[par])[ch - 6]);
+            }
+            // 3. the cluster's candidate
+            const T* urow;
+            const T* drow;
+            T rcp;
+            if (C > 1) {
+                if (!dead) {
+                    const uint32_t bar = smem_addr(&sm.bar[par]);
+                    const uint32_t phase = (J >> 1) & 1;
+                    unsigned polls = 0;
+                    for (;;) {
+                        uint32_t ok;
+                        asm volatile(
+                            "{\n\t.reg .pred q;\n\t"
+                            "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 q, [%1], %2;\n\t"
+                            "selp.u32 %0, 1, 0, q;\n\t}"
+                            : "=r"(ok)
+                            : "r"(bar), "r"(phase)
+                            : "memory");
+                        if (ok) break;
+                        if (++polls > limit) {
+                            atomicCAS(err, 0, kErrTimeout);
+                            dead = true;
+                            break;
+                        }
+                    }
+                    dead = __any_sync(0xffffffffu, dead);
+                }
+                Mag<T> k = 0;
+                int kr = INT_MAX;
+                if (lane < C) load_key(sm.in[par][lane], k, kr);
+                rcp = Bits<T>::rcp(Bits<T>::val(k));  // every candidate's, beside the reductions
+                warp_argmax(k, kr, mv, mrow);
+                const unsigned who = __ballot_sync(0xffffffffu, lane < C && kr == mrow);
+                from = who ? __ffs(who) - 1 : 0;
+                rcp = __shfl_sync(0xffffffffu, rcp, from);
+                urow = sm.in[par][from].x;
+                drow = sm.diag[par];
+            } else {
+                urow = sm.own[par][from].x;
+                drow = sm.own_diag[par];
+                rcp = Bits<T>::rcp(Bits<T>::val(mv));
+            }
+            const int p = mrow >= J && mrow < m ? mrow : J;
+            T u[NB];
+#pragma unroll
+            for (int c = 0; c < NB; ++c) u[c] = urow[c];
+            const T piv = u[0];
+            const bool nz = piv != T(0);
+            rcp = piv < T(0) ? -rcp : (piv == piv ? rcp : piv);
+            const bool recip = abs_t(piv) >= min_normal(piv) || piv != piv;
+            bool touched = false;
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const int g = r0 + tid + TH * i;
+                touched = touched || g == J || g == p;
+            }
+            if (__any_sync(0xffffffffu, touched)) {  // the interchange, in the two rows' warps
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    const int g = r0 + tid + TH * i;
+                    if (g == J) {
+#pragma unroll
+                        for (int c = 0; c < NB; ++c) a[i][c] = u[c];
+                    } else if (g == p) {
+#pragma unroll
+                        for (int c = 0; c < NB; ++c) a[i][c] = drow[c];
+                    }
+                }
+            }
+            T l[R];
+#pragma unroll
+            for (int i = 0; i < R; ++i) l[i] = a[i][0] * rcp;
+            if (!(nz && recip)) {  // a zero or subnormal pivot
+#pragma unroll
+                for (int i = 0; i < R; ++i) l[i] = nz ? a[i][0] / piv : a[i][0];
+            }
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const bool below = r0 + tid + TH * i > J;
+                l[i] = below ? l[i] : a[i][0];
+                const int top = below ? NB - j : 0;  // columns still in the update
+#pragma unroll
+                for (int c = 1; c < NB; ++c) {
+                    const T x = fma_t(-l[i], u[c], a[i][c]);
+                    a[i][c - 1] = c < top ? x : a[i][c];
+                }
+                a[i][NB - 1] = l[i];
+            }
+            if (warp == NW - 1) {  // off the chain: bookkeeping
+                if (rank == 0 && lane == 0) {
+                    if (pivot) ipiv[J] = p + 1 + ipiv_add;
+                    if (!nz && info) atomicCAS(info, 0, info_base + J + 1);
+                }
+                if (others) {
+                    // the pivot row carries L11's row j in its last j places
+                    if (lane < NB) sm.L[j][lane] = urow[lane];
+                    if (p != J) {
+                        const unsigned hit = __ballot_sync(0xffffffffu, mv_pos == p);
+                        const int x = hit ? __ffs(hit) - 1 : mv_cnt;
+                        if (!hit) {
+                            if (lane == x) mv_pos = mv_src = p;
+                            ++mv_cnt;
+                        }
+                        const int st = __shfl_sync(0xffffffffu, mv_src, j);
+                        const int sx = __shfl_sync(0xffffffffu, mv_src, x);
+                        if (lane == j) mv_src = sx;
+                        if (lane == x) mv_src = st;
+                    }
+                }
+            }
+        }
+        // a short last sub-panel: rotate the rest of the way
+        for (int j = sb; j < NB; ++j) {
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const T l = a[i][0];
+#pragma unroll
+                for (int c = 1; c < NB; ++c) a[i][c - 1] = a[i][c];
+                a[i][NB - 1] = l;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int r = tid + TH * i;
+#pragma unroll
+            for (int c = 0; c < NB; ++c)
+                if (r < nr && c < nbc) tile[(jb + c) * ldt + r] = a[i][c];
+        }
+        if (others && warp == NW - 1) {
+            sm.mv_pos[lane] = mv_pos;
+            sm.mv_src[lane] = mv_src;
+        }
+        cluster_wait();
+        if (!others) continue;
+        __syncthreads();
+        // The interchanges on the other columns.  Lane = move, warp = columns:
+        // the moves into this CTA's rows, and on every CTA the new diagonal
+        // rows right of the sub-panel, from which each solves U12 itself.
+        constexpr int kOther = kClMaxW * 4 / (int)sizeof(T) - NB;
+        constexpr int kIt = (kOther + NW - 1) / NW;
+        const int c1 = jb + nbc, nother = w - nbc;
+        mv_pos = sm.mv_pos[lane];
+        mv_src = sm.mv_src[lane];
+        const bool top_row = lane < NB;
+        const bool here = mv_pos >= r0 && mv_pos < r0 + nr;
+        T v[kIt];
+        {
+            const int q_src = mv_src >= 0 ? mv_src / rpc : 0;
+            const uint32_t src = peer_base(q_src) + off_of(tile + (mv_src - q_src * rpc));
+#pragma unroll
+            for (int k = 0; k < kIt; ++k) {
+                const int q = warp + NW * k, c = q < jb ? q : q + nbc;
+                const bool want = mv_src >= 0 && q < nother &&
+                                  ((top_row && c >= c1 && lane < sb) || (here && mv_src != mv_pos));
+                v[k] = want ? peer_load(src + (uint32_t)(c * ldt * (int)sizeof(T)), T(0)) : T(0);
+            }
+        }
+        cluster_arrive();
+        if (top_row) {
+#pragma unroll
+            for (int k = 0; k < kIt; ++k) {
+                const int q = warp + NW * k, c = q < jb ? q : q + nbc;
+                if (q < nother && c >= c1) sm.U[(c - c1) >> 1][lane][(c - c1) & 1] = v[k];
+            }
         }
         __syncthreads();
-        if (warp == 0) {
-            if (pivot) {
-                bv = lane < kClThreads / 32 ? red_v[lane] : -1.f;
-                bi = lane < kClThreads / 32 ? red_i[lane] : INT_MAX;
+        T x[NB];  // U12 = L11^{-1} A12, a column per thread
+        if (c1 + tid < w) {
+            T* up = &sm.U[tid >> 1][0][tid & 1];
 #pragma unroll
-                for (int off = 16; off > 0; off >>= 1) {
-                    const float ov = __shfl_down_sync(0xffffffffu, bv, off);
-                    const int oi = __shfl_down_sync(0xffffffffu, bi, off);
-                    if (better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
+            for (int k = 0; k < NB; ++k) x[k] = up[2 * k];
+#pragma unroll
+            for (int r = 1; r < NB; ++r) {
+                if (r < sb) {
+#pragma unroll
+                    for (int k = 0; k < r; ++k) x[r] = fma_t(-sm.L[r][NB - r + k], x[k], x[r]);
                 }
-                bv = __shfl_sync(0xffffffffu, bv, 0);
-                bi = __shfl_sync(0xffffffffu, bi, 0);
-            }
-            if (lane == 0) {
-                my_slot[0] = bv;
-                my_slot[1] = __int_as_float(bi);
-            }
-            if (lane < w) {
-                if (bi != INT_MAX) my_slot[4 + lane] = tile[lane * ldt + (bi - r0)];
-                if (rank == owner) my_slot[4 + kClMaxW + lane] = tile[lane * ldt + (j - r0)];
+                up[2 * r] = x[r];
             }
         }
-        // 2. publish to the cluster
-        cluster.sync();
-
-        // 3. warp 0 gathers the cluster's candidates and the two rows
-        if (warp == 0) {
-            float gv = -1.f;
-            int gi = INT_MAX, gc = -1;
-            if (pivot) {
-                if (lane < C) {
-                    const float* rs = cluster.map_shared_rank(slots, lane) + par * kClSlot;
-                    gv = rs[0];
-                    gi = __float_as_int(rs[1]);
-                    gc = lane;
-                }
+        cluster_wait();  // everybody has read: rows may change
 #pragma unroll
-                for (int off = 16; off > 0; off >>= 1) {
-                    const float ov = __shfl_down_sync(0xffffffffu, gv, off);
-                    const int oi = __shfl_down_sync(0xffffffffu, gi, off);
-                    const int oc = __shfl_down_sync(0xffffffffu, gc, off);
-                    if (better(ov, oi, gv, gi)) { gv = ov; gi = oi; gc = oc; }
-                }
-                gi = __shfl_sync(0xffffffffu, gi, 0);
-                gc = __shfl_sync(0xffffffffu, gc, 0);
-            }
-            if (lane < w) {
-                const float* os = cluster.map_shared_rank(slots, owner) + par * kClSlot;
-                const float ov = os[4 + kClMaxW + lane];
-                s_orow[lane] = ov;
-                if (pivot) {
-                    const float* ws = cluster.map_shared_rank(slots, gc) + par * kClSlot;
-                    s_prow[lane] = ws[4 + lane];
-                } else {
-                    s_prow[lane] = ov;
-                }
-            }
-            if (lane == 0) {
-                s_p = pivot ? gi : j;
-                if (pivot && rank == 0) ipiv[j] = (pivot ? gi : j) + 1 + ipiv_add;
-            }
+        for (int k = 0; k < kIt; ++k) {
+            const int q = warp + NW * k, c = q < jb ? q : q + nbc;
+            if (here && mv_src != mv_pos && q < nother && !(top_row && c >= c1))
+                tile[c * ldt + mv_pos - r0] = v[k];
+        }
+        if (own_j && c1 + tid < w) {
+#pragma unroll
+            for (int k = 0; k < NB; ++k)
+                if (k < sb) tile[(c1 + tid) * ldt + jb - r0 + k] = x[k];
         }
         __syncthreads();
-
-        // 4. swap, scale, rank-1 update (each thread on its own rows)
-        const int p = s_p;
-        const float piv = s_prow[j];
-        const bool nz = piv != 0.f;
-        const bool recip = fabsf(piv) >= FLT_MIN;
-        const float rcp = 1.0f / piv;
-        if (!nz && rank == 0 && tid == 0 && info) atomicCAS(info, 0, info_base + j + 1);
-        if (j >= r0 && j < r0 + nr && ((j - r0) % kClThreads) == tid)
-            for (int c = 0; c < w; ++c) tile[c * ldt + (j - r0)] = s_prow[c];
-        if (p != j && p >= r0 && p < r0 + nr && ((p - r0) % kClThreads) == tid)
-            for (int c = 0; c < w; ++c) tile[c * ldt + (p - r0)] = s_orow[c];
-        for (int r = tid; r < nr; r += kClThreads) {
-            if (r0 + r > j) {
-                float l = tile[j * ldt + r];
-                if (nz) {
-                    l = recip ? l * rcp : l / piv;
-                    tile[j * ldt + r] = l;
+        if (c1 >= w) continue;
+        // the rank-NB update of this thread's rows, two columns at a time
+        if (jb + sb < m) {
+            using P = typename PairOf<T>::type;
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const int r = tid + TH * i;
+                if (r >= nr || r0 + r < jb + sb) continue;
+                T* xp = tile + c1 * ldt + r;
+                for (int c = 0; c + c1 < w; c += 2, xp += 2 * ldt) {
+                    const bool two = c + 1 + c1 < w;
+                    P acc(xp[0], two ? xp[ldt] : T(0));
+                    const Vec4<T>* up = reinterpret_cast<const Vec4<T>*>(sm.U[c >> 1]);
+#pragma unroll
+                    for (int k = 0; k < NB; k += 2) {
+                        const Vec4<T> u = up[k >> 1];
+                        acc.fma(P(-a[i][k], -a[i][k]), P(u.x[0], u.x[1]));
+                        acc.fma(P(-a[i][k + 1], -a[i][k + 1]), P(u.x[2], u.x[3]));
+                    }
+                    T x0, x1;
+                    acc.get(x0, x1);
+                    xp[0] = x0;
+                    if (two) xp[ldt] = x1;
                 }
-                for (int c = j + 1; c < w; ++c)
-                    tile[c * ldt + r] = fmaf(-l, s_prow[c], tile[c * ldt + r]);
             }
         }
     }
     __syncthreads();
-    move_block<false>(A + r0, lda, tile, ldt, nr, w);
-    cluster.sync();  // no CTA leaves while another may still read its slots
+    for (int c0 = 0; c0 < w; c0 += 8) {
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int r = tid + TH * i;
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+                if (r < nr && c0 + c < w)
+                    A[(long long)(c0 + c) * lda + r0 + r] = tile[(c0 + c) * ldt + r];
+        }
+    }
+    if (dead) __nanosleep(200000);  // messages nobody waited for land before the exit
+    cluster_arrive();
+    cluster_wait();  // no CTA leaves while another may still reach its shared memory
 }
 
-int cluster_ldt(int rpc) { return rpc | 1; }
+// Rows per CTA: a multiple of 16 so that a sub-panel's diagonal rows sit in one CTA.
+int cluster_rpc(int m, int C) { return ((m + C - 1) / C + 15) / 16 * 16; }
+template <class T>
 size_t cluster_smem(int rpc, int w)
 {
-    return sizeof(float) * (2 * (size_t)kClSlot + (size_t)cluster_ldt(rpc) * w);
+    return sizeof(ClusterSmem<T>) + sizeof(T) * (size_t)(rpc | 1) * w;
+}
+size_t cluster_cap(const hdbf_context* ctx)
+{
+    return ctx->max_smem_optin > 1024 ? ctx->max_smem_optin - 1024 : 0;
 }
 
-}  // namespace
-
-int configure_cluster_panel(hdbf_context* ctx)
+template <class T, int TH, int R>
+cudaError_t launch_cluster(hdbf_context* ctx, int C, size_t smem, int m, int w, T* A, long long lda,
+                           int rpc, int* ipiv, int ipiv_add, int* info, int info_base, int pivot)
 {
-    const size_t cap = ctx->max_smem_optin > 4096 ? ctx->max_smem_optin - 4096 : 0;
-    cudaFuncSetAttribute(getf2_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap);
-    cudaFuncSetAttribute(getf2_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    cudaGetLastError();
-    int best = 0;
-    for (int C = kClMaxCluster; C >= 1 && best == 0; C /= 2) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(C);
-        cfg.blockDim = dim3(kClThreads);
-        cfg.dynamicSmemBytes = cap;
-        cudaLaunchAttribute at;
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = C;
-        at.val.clusterDim.y = 1;
-        at.val.clusterDim.z = 1;
-        cfg.attrs = &at;
-        cfg.numAttrs = 1;
-        int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, getf2_cluster_kernel, &cfg) == cudaSuccess &&
-            clusters >= 1)
-            best = C;
-        cudaGetLastError();
-    }
-    return best;
-}
-
-hdbf_status getf2_cluster(hdbf_context* ctx, int m, int w, float* A, long long lda, int* ipiv,
-                          int ipiv_add, int* info, int info_base, bool pivot)
-{
-    if (m <= 0 || w <= 0) return HDBF_STATUS_SUCCESS;
-    if (w > kClMaxW || ctx->cluster_max < 1) return HDBF_STATUS_NOT_SUPPORTED;
-    const size_t cap = ctx->max_smem_optin > 4096 ? ctx->max_smem_optin - 4096 : 0;
-    // Fewest CTAs whose slices fit, but at most 8 rows per thread.
-    int C = 1;
-    while (C < ctx->cluster_max &&
-           (cluster_smem((m + C - 1) / C, w) > cap || (m + C - 1) / C > 8 * kClThreads))
-        C *= 2;
-    const int rpc = (m + C - 1) / C;
-    const int ldt = cluster_ldt(rpc);
-    const size_t smem = cluster_smem(rpc, w);
-    if (smem > cap) return HDBF_STATUS_NOT_SUPPORTED;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(C);
-    cfg.blockDim = dim3(kClThreads);
+    cfg.blockDim = dim3(TH);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
     cudaLaunchAttribute at;
@@ -277,16 +633,121 @@ hdbf_status getf2_cluster(hdbf_context* ctx, int m, int w, float* A, long long l
     at.val.clusterDim.z = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    const int piv_flag = pivot ? 1 : 0;
-    ProfScope prof(ctx, kClsPanel, (double)m * w * w - (double)w * w * w / 3.0, 8.0 * m * w);
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, getf2_cluster_kernel, m, w, A, lda, rpc, ldt,
-                                             ipiv, ipiv_add, info, info_base, piv_flag);
+    int* err = ctx->dev_small + kSmallErr;
+    return cudaLaunchKernelEx(&cfg, getf2_cluster_kernel<T, TH, R>, m, w, A, lda, rpc, ipiv, ipiv_add,
+                              info, info_base, pivot, err);
+}
+
+template <class T>
+hdbf_status getf2_cluster_t(hdbf_context* ctx, int m, int w, T* A, long long lda, int* ipiv,
+                            int ipiv_add, int* info, int info_base, bool pivot)
+{
+    if (m <= 0 || w <= 0) return HDBF_STATUS_SUCCESS;
+    if (w > getf2_cluster_leaf(ctx, m, (int)sizeof(T))) return HDBF_STATUS_NOT_SUPPORTED;
+    // One row per thread of 256 where the cluster is large enough for that.
+    int C = 1;
+    while (C < ctx->cluster_max &&
+           (cluster_rpc(m, C) > 256 || cluster_smem<T>(cluster_rpc(m, C), w) > cluster_cap(ctx)))
+        C *= 2;
+    const int rpc = cluster_rpc(m, C);
+    const size_t smem = cluster_smem<T>(rpc, w);
+    const int piv = pivot ? 1 : 0;
+    ProfScope prof(ctx, kClsPanel, (double)m * w * w - (double)w * w * w / 3.0,
+                   2.0 * sizeof(T) * m * w, m, w, C);
+    cudaError_t e;
+    if (rpc <= 256)
+        e = launch_cluster<T, 256, 1>(ctx, C, smem, m, w, A, lda, rpc, ipiv, ipiv_add, info,
+                                      info_base, piv);
+    else if (rpc <= 512)
+        e = launch_cluster<T, 512, 1>(ctx, C, smem, m, w, A, lda, rpc, ipiv, ipiv_add, info,
+                                      info_base, piv);
+    else if (rpc <= 1024)
+        e = launch_cluster<T, 512, 2>(ctx, C, smem, m, w, A, lda, rpc, ipiv, ipiv_add, info,
+                                      info_base, piv);
+    else
+        e = launch_cluster<T, 512, 4>(ctx, C, smem, m, w, A, lda, rpc, ipiv, ipiv_add, info,
+                                      info_base, piv);
     ctx->launches++;
     if (e != cudaSuccess) {
         cudaGetLastError();
         return HDBF_STATUS_CUDA_ERROR;
     }
     return HDBF_STATUS_SUCCESS;
+}
+
+template <class T, int TH, int R>
+int configure_one(hdbf_context* ctx, int best)
+{
+    auto* k = getf2_cluster_kernel<T, TH, R>;
+    const int cap = (int)cluster_cap(ctx);
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, cap) != cudaSuccess ||
+        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    for (; best >= 1; best /= 2) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(best);
+        cfg.blockDim = dim3(TH);
+        cfg.dynamicSmemBytes = cap;
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = best;
+        at.val.clusterDim.y = 1;
+        at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        const bool ok = cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) == cudaSuccess &&
+                        clusters >= 1;
+        cudaGetLastError();
+        if (ok) break;
+    }
+    return best;
+}
+
+}  // namespace
+
+// Largest cluster that every instance can launch with the full shared memory.
+int configure_cluster_panel(hdbf_context* ctx)
+{
+    int best = kClMaxCluster;
+    best = configure_one<float, 256, 1>(ctx, best);
+    best = configure_one<float, 512, 1>(ctx, best);
+    best = configure_one<float, 512, 2>(ctx, best);
+    best = configure_one<float, 512, 4>(ctx, best);
+    best = configure_one<double, 256, 1>(ctx, best);
+    best = configure_one<double, 512, 1>(ctx, best);
+    best = configure_one<double, 512, 2>(ctx, best);
+    best = configure_one<double, 512, 4>(ctx, best);
+    return best;
+}
+
+// Widest leaf (a power of two, <= 128 FP32 or 64 FP64 columns) that one cluster
+// holds at height m; 0 when not even one sub-panel fits.
+int getf2_cluster_leaf(hdbf_context* ctx, int m, int elem)
+{
+    if (ctx->cluster_max < 1) return 0;
+    const int rpc = cluster_rpc(m, ctx->cluster_max);
+    if (rpc > kClMaxRows) return 0;
+    const int widest = kClMaxW * 4 / elem;
+    for (int w = widest; w >= 64 / elem; w /= 2) {
+        const size_t need = elem == 4 ? cluster_smem<float>(rpc, w) : cluster_smem<double>(rpc, w);
+        if (need <= cluster_cap(ctx)) return w;
+    }
+    return 0;
+}
+
+hdbf_status getf2_cluster(hdbf_context* ctx, int m, int w, float* A, long long lda, int* ipiv,
+                          int ipiv_add, int* info, int info_base, bool pivot)
+{
+    return getf2_cluster_t(ctx, m, w, A, lda, ipiv, ipiv_add, info, info_base, pivot);
+}
+
+hdbf_status getf2_cluster(hdbf_context* ctx, int m, int w, double* A, long long lda, int* ipiv,
+                          int ipiv_add, int* info, int info_base, bool pivot)
+{
+    return getf2_cluster_t(ctx, m, w, A, lda, ipiv, ipiv_add, info, info_base, pivot);
 }
 
 }  // namespace hdbf

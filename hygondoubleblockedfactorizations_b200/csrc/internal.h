@@ -371,10 +371,16 @@ hdbf_status getf2_coop(hdbf_context* ctx, int m, int w, float* A, long long lda,
 size_t getf2_coop_scratch_bytes();
 void configure_getrf_kernels(hdbf_context* ctx);
 // Same contract on one thread-block cluster with the block in distributed
-// shared memory; NOT_SUPPORTED when the block does not fit (caller falls
-// back to getf2_coop).
+// shared memory (getf2_cluster.cu), FP32 and FP64; NOT_SUPPORTED when w is above
+// getf2_cluster_leaf(m).
 hdbf_status getf2_cluster(hdbf_context* ctx, int m, int w, float* A, long long lda, int* ipiv,
                           int ipiv_add, int* info, int info_base, bool pivot);
+hdbf_status getf2_cluster(hdbf_context* ctx, int m, int w, double* A, long long lda, int* ipiv,
+                          int ipiv_add, int* info, int info_base, bool pivot);
+// Widest leaf one cluster holds at height m for elements of `elem` bytes (0: none).
+int getf2_cluster_leaf(hdbf_context* ctx, int m, int elem);
+// The leaf the panel recursion takes on the cluster kernel (0: the grid-wide one).
+int panel_cluster_leaf(hdbf_context* ctx, int m, int elem);
 int configure_cluster_panel(hdbf_context* ctx);
 
 // Compose LAPACK swaps  row (i) <-> row (ipiv[i]-1-ipiv_minus), i in [0,k),

@@ -100,10 +100,11 @@ hdbf_status hdbf_set_graph_mode(hdbf_handle handle, int enabled);
  * column block fits in one cluster's shared memory, otherwise the
  * grid-wide publish-and-poll kernel), 1 = always the grid-wide kernel,
  * 2 = cluster only (blocks that do not fit still take the grid-wide kernel).
- * Both produce identical pivots and factors.  A new handle starts in the mode
- * named by the environment variable HDBF_PANEL_KERNEL (0, 1 or 2), else 0.
- * The panel recursion stops at leaves of 128 columns (the grid-wide kernel
- * takes up to 128; the cluster kernel up to 32, so mode 2 recurses to 32);
+ * On the same leaf both produce identical pivots and factors.  A new handle
+ * starts in the mode named by the environment variable HDBF_PANEL_KERNEL (0, 1
+ * or 2), else 0.  The panel recursion stops at leaves of 128 columns, or, where
+ * one cluster cannot hold that many at the panel's height, at 64; above that
+ * height automatic mode takes the grid-wide kernel.  Mode 2 recurses to 32;
  * HDBF_PANEL_LEAF (32, 64 or 128) sets a new handle's leaf width, and
  * HDBF_PANEL_ROWS (64..4096, default 256) the rows each CTA of the grid-wide
  * kernel aims to hold. */
