@@ -98,6 +98,11 @@ struct hdbf_context {
     // Tensor-core GEMM kernel: 0 persistent 128 x 256 tiles with two TMEM
     // accumulators (default), 1 one 128 x 128 tile per CTA (HDBF_TC_KERNEL).
     int tc_kernel = 0;
+    // FP32 updates on the tensor cores (three BF16 words, tc_sgemm.cu): 1 by
+    // size, 0 never, 2 at any size (HDBF_TC_SGEMM).  tc_plan fixes the K
+    // chunk for the parts of one GEMM, as split_kc does (-1: decide per launch).
+    int tc_sgemm = 1;
+    int tc_plan = -1;
     unsigned spin_limit = 0; // hdbf_set_wait_limit (0: default)
     // Conditional launches (RunIf): while set, the FP32 GEMM and the
     // diagonal-block kernel run only when *run_if != 0 (read on the device).
@@ -177,6 +182,20 @@ __device__ __forceinline__ float pow2f_exact(int k)
     return __uint_as_float((unsigned)(127 + k) << 23);
 }
 
+// Whether an operand pair is outside the range of the three-word BF16 split:
+// range[0], range[1] hold the bits of max |x| of A and of B (0: all zero, or B
+// is part of A).
+__device__ __forceinline__ bool split_range_bad(const unsigned* range)
+{
+    bool bad = false;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const unsigned m = __ldcg(range + i);
+        bad = bad || m > (253u << 23) || (m != 0u && m < (37u << 23));  // 2^126, 2^-90
+    }
+    return bad;
+}
+
 // The handle's poll limit, read at kernel start from the small device block
 // whose error word `err` points at (hdbf_set_wait_limit).
 __device__ __forceinline__ unsigned spin_limit_of(const int* err)
@@ -249,8 +268,10 @@ void* mixed_arena(hdbf_context* ctx, size_t bytes, hdbf_status* st);
 //   temp  column-tiled swap buffer, 64*n floats
 //   skinny  split-K partial sums of the skinny GEMM, 256*n floats
 //   wave  wavefront-solve row-major x copy (32 columns) and its flags
+//   words BF16 words of the operands of an FP32 update on the tensor cores, one
+//         half per stream (handle's, look-ahead)
 struct WsLayout {
-    size_t coop, inv, perm, coop64, src, tgt, gperm, temp, skinny, wave, split, total;
+    size_t coop, inv, perm, coop64, src, tgt, gperm, temp, skinny, wave, split, words, total;
 };
 // Split-K partial sums of under-filled FP32 GEMM launches: two halves of
 // kSplitFloats each, one for the handle's stream and one for its look-ahead
@@ -271,6 +292,9 @@ float* ws_skinny(hdbf_context* ctx);
 // Split-K scratch half for GEMMs enqueued on ctx->stream.
 float* ws_split(hdbf_context* ctx);
 float* ws_wave(hdbf_context* ctx);
+// This stream's half of the words region, and its size in bytes (less the range slots).
+void* ws_words(hdbf_context* ctx);
+size_t ws_words_half(const hdbf_context* ctx);
 
 hdbf_status last_cuda(hdbf_context* ctx);
 
@@ -287,17 +311,32 @@ hdbf_status sgemm_sub(hdbf_context* ctx, bool nn, bool lower_only, int M, int N,
 // K split of the FP32 GEMM of shape M x N x K (tri: lower-triangle mode):
 // the number of chunks (1 = no split) and, in *kc, their length.
 int split_count(const hdbf_context* ctx, int M, int N, int K, bool tri, int* kc);
+// FP32 update on the tensor cores (tc_sgemm.cu): the K chunk for this shape, 0
+// where the FP32 kernel is taken; one chunk of it (a_kc / b_kc: the operand's K
+// is contiguous), whose operand range, in *range, tells the FP32 kernel behind it
+// whether it has to do the update (split_range_bad).
+int tc_sgemm_chunk(const hdbf_context* ctx, int M, int N, int K, bool tri);
+hdbf_status tc_sgemm_chunk_run(hdbf_context* ctx, bool a_kc, bool b_kc, bool lower, int M, int N,
+                               int K, const float* A, long long lda, const float* B, long long ldb,
+                               float* C, long long ldc, unsigned** range);
+void configure_tc_sgemm(hdbf_context* ctx);
 // While alive, every FP32 GEMM splits K as the GEMM of the given shape does.
 struct SplitPlan {
     hdbf_context* ctx;
-    int saved;
-    SplitPlan(hdbf_context* c, int M, int N, int K) : ctx(c), saved(c->split_kc)
+    int saved, saved_tc;
+    SplitPlan(hdbf_context* c, int M, int N, int K)
+        : ctx(c), saved(c->split_kc), saved_tc(c->tc_plan)
     {
         int kc = 0;
+        c->tc_plan = tc_sgemm_chunk(c, M, N, K, false);
         const int S = split_count(c, M, N, K, false, &kc);
         c->split_kc = S > 1 ? kc : 0;
     }
-    ~SplitPlan() { ctx->split_kc = saved; }
+    ~SplitPlan()
+    {
+        ctx->split_kc = saved;
+        ctx->tc_plan = saved_tc;
+    }
 };
 
 // Skinny update (N <= 32): mode 0 C -= A * B^T, 1 C -= A * B, 2 C -= A^T * B,

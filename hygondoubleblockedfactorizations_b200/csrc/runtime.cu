@@ -80,6 +80,13 @@ void* mixed_arena(hdbf_context* ctx, size_t bytes, hdbf_status* st)
     return ctx->mix;
 }
 
+// Operand words of an update of order n: M + N <= 2 n rows, up to 2048 of K at a
+// time, 6 bytes an element, plus the range slots.
+static size_t words_half(int n)
+{
+    return align_up((size_t)12 * n * (n < 2048 ? n : 2048), 256) + 256;
+}
+
 WsLayout ws_layout(int n)
 {
     if (n < 64) n = 64;
@@ -107,6 +114,8 @@ WsLayout ws_layout(int n)
     off += wave_scratch_bytes(n);
     L.split = off;
     off += align_up(2 * kSplitFloats * sizeof(float), 256);
+    L.words = off;
+    off += 2 * words_half(n);
     L.total = off;
     return L;
 }
@@ -202,6 +211,13 @@ float* ws_split(hdbf_context* ctx)
         reinterpret_cast<float*>(static_cast<char*>(ctx->ws) + ws_layout(ctx->ws_n).split);
     return (ctx->la_stream && ctx->stream == ctx->la_stream) ? base + kSplitFloats : base;
 }
+
+void* ws_words(hdbf_context* ctx)
+{
+    char* base = static_cast<char*>(ctx->ws) + ws_layout(ctx->ws_n).words;
+    return (ctx->la_stream && ctx->stream == ctx->la_stream) ? base + words_half(ctx->ws_n) : base;
+}
+size_t ws_words_half(const hdbf_context* ctx) { return words_half(ctx->ws_n) - 256; }
 
 ProfScope::ProfScope(hdbf_context* ctx, int cls, double flops, double bytes, int m, int n,
                      int k)
@@ -396,7 +412,12 @@ hdbf_status hdbf_create(hdbf_handle* handle)
     }
     if (const char* la = std::getenv("HDBF_LOOKAHEAD")) ctx->lookahead = std::atoi(la) != 0;
     if (const char* tk = std::getenv("HDBF_TC_KERNEL")) ctx->tc_kernel = std::atoi(tk) != 0;
+    if (const char* ts = std::getenv("HDBF_TC_SGEMM")) {  // FP32 updates on the tensor cores
+        const int v = std::atoi(ts);
+        if (v >= 0 && v <= 2) ctx->tc_sgemm = v;
+    }
     configure_tc_kernels(ctx);
+    configure_tc_sgemm(ctx);
     configure_trsm_block_kernels(ctx);
     configure_solve_kernels(ctx);
     configure_batched_kernels(ctx);

@@ -48,9 +48,10 @@ __global__ void __launch_bounds__(NTHR, 2)
 sgemm_sub_kernel(int M, int N, int K, const float* __restrict__ A, long long lda,
                  const float* __restrict__ B, long long ldb, float* __restrict__ C,
                  long long ldc, int tiles_m, const int* __restrict__ run_if,
-                 float* __restrict__ part, int kc, int tiles)
+                 float* __restrict__ part, int kc, int tiles, const unsigned* range)
 {
     if (run_if && *run_if == 0) return;  // conditional launch (RunIf) not taken
+    if (range && !split_range_bad(range)) return;  // done on the tensor cores
     constexpr bool AT = MODE == kTN;  // A read k-contiguous (transposed load)
     constexpr bool BT = MODE != kNT;  // B read k-contiguous (transposed load)
     // Split K (part != nullptr): CTA blockIdx.x handles K chunk s of tile
@@ -293,17 +294,17 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 template <int MODE, bool VEC, bool TRI>
 void launch_sub(cudaStream_t s, int M, int N, int K, const float* A, long long lda,
                 const float* B, long long ldb, float* C, long long ldc, const int* run_if,
-                float* part = nullptr, int splits = 1, int kc = 0)
+                float* part, int splits, int kc, const unsigned* range)
 {
     const int tiles_m = (M + BM - 1) / BM;
     const int tiles_n = (N + BN - 1) / BN;
     const long long tiles = (long long)tiles_m * tiles_n;
     if (!part) {
         sgemm_sub_kernel<MODE, VEC, TRI, false><<<(unsigned)tiles, NTHR, 0, s>>>(
-            M, N, K, A, lda, B, ldb, C, ldc, tiles_m, run_if, nullptr, 0, (int)tiles);
+            M, N, K, A, lda, B, ldb, C, ldc, tiles_m, run_if, nullptr, 0, (int)tiles, range);
     } else {
         sgemm_sub_kernel<MODE, VEC, TRI, true><<<(unsigned)(tiles * splits), NTHR, 0, s>>>(
-            M, N, K, A, lda, B, ldb, C, ldc, tiles_m, run_if, part, kc, (int)tiles);
+            M, N, K, A, lda, B, ldb, C, ldc, tiles_m, run_if, part, kc, (int)tiles, nullptr);
         const long long total = (long long)M * N;
         const int g = (int)std::min<long long>((total + 255) / 256, 1184);
         split_reduce_kernel<TRI><<<g, 256, 0, s>>>(M, N, splits, part, C, ldc);
@@ -364,14 +365,30 @@ namespace {
 
 hdbf_status sgemm_launch(hdbf_context* ctx, int mode, bool lower_only, int M, int N, int K,
                          const float* A, long long lda, const float* B, long long ldb, float* C,
-                         long long ldc)
+                         long long ldc, const unsigned* range = nullptr)
 {
     if (M <= 0 || N <= 0 || K <= 0) return HDBF_STATUS_SUCCESS;
     if (!A || !B || !C) return HDBF_STATUS_INVALID_VALUE;
     if (lower_only && mode != kNT) return HDBF_STATUS_INVALID_VALUE;
-    if (!lower_only && !ctx->no_skinny && !ctx->run_if && N <= 32 && M >= 4 * N && M >= 256)
+    if (!range && !lower_only && !ctx->no_skinny && !ctx->run_if && N <= 32 && M >= 4 * N && M >= 256)
         return sgemm_skinny(ctx, mode == kNT ? 0 : mode == kNN ? 1 : 2, M, N, K, A, lda, B, ldb,
                             C, ldc);
+    const int tc = range              ? 0
+                   : ctx->tc_plan >= 0 ? ctx->tc_plan
+                                       : tc_sgemm_chunk(ctx, M, N, K, lower_only);
+    if (tc > 0) {
+        const bool a_kc = mode == kTN, b_kc = mode != kNT;  // K contiguous in memory
+        for (int k0 = 0; k0 < K; k0 += tc) {
+            const int kk = std::min(tc, K - k0);
+            const float* Ak = a_kc ? A + k0 : A + (long long)k0 * lda;
+            const float* Bk = b_kc ? B + k0 : B + (long long)k0 * ldb;
+            unsigned* r = nullptr;
+            HDBF_TRY(tc_sgemm_chunk_run(ctx, a_kc, b_kc, lower_only, M, N, kk, Ak, lda, Bk, ldb, C,
+                                        ldc, &r));
+            HDBF_TRY(sgemm_launch(ctx, mode, lower_only, M, N, kk, Ak, lda, Bk, ldb, C, ldc, r));
+        }
+        return HDBF_STATUS_SUCCESS;
+    }
     const long long tiles = (long long)((M + BM - 1) / BM) * ((N + BN - 1) / BN);
     if (tiles > 0x7fffffffLL) return HDBF_STATUS_NOT_SUPPORTED;
     const bool vec = aligned16(A) && aligned16(B) && aligned16(C) && (lda % 4 == 0) &&
@@ -384,12 +401,13 @@ hdbf_status sgemm_launch(hdbf_context* ctx, int mode, bool lower_only, int M, in
         const double d = (double)(M < N ? M : N);
         flops = 2.0 * (double)K * (d * (double)M - d * (d - 1.0) / 2.0);
     }
+    if (range) flops = 0.0;  // counted by the tensor-core launch it stands behind
     ProfScope prof(ctx, kClsGemm, flops, 4.0 * ((double)M * K + (double)N * K + 2.0 * M * N), M,
                    N, K);
     int kc = 0;
-    const int S = split_count(ctx, M, N, K, lower_only, &kc);
+    const int S = range ? 1 : split_count(ctx, M, N, K, lower_only, &kc);
     float* part = S > 1 ? ws_split(ctx) : nullptr;
-#define HDBF_SUB(MD, V, T) launch_sub<MD, V, T>(s, M, N, K, A, lda, B, ldb, C, ldc, ri, part, S, kc)
+#define HDBF_SUB(MD, V, T) launch_sub<MD, V, T>(s, M, N, K, A, lda, B, ldb, C, ldc, ri, part, S, kc, range)
     if (mode == kNT) {
         if (vec) {
             if (lower_only) HDBF_SUB(kNT, true, true);
