@@ -103,6 +103,7 @@ struct hdbf_context {
     // chunk for the parts of one GEMM, as split_kc does (-1: decide per launch).
     int tc_sgemm = 1;
     int tc_plan = -1;
+    int small_plan = -1;  // the same for sgemm_small_split (0: the 128 x 128 kernel)
     unsigned spin_limit = 0; // hdbf_set_wait_limit (0: default)
     // Conditional launches (RunIf): while set, the FP32 GEMM and the
     // diagonal-block kernel run only when *run_if != 0 (read on the device).
@@ -311,6 +312,13 @@ hdbf_status sgemm_sub(hdbf_context* ctx, bool nn, bool lower_only, int M, int N,
 // K split of the FP32 GEMM of shape M x N x K (tri: lower-triangle mode):
 // the number of chunks (1 = no split) and, in *kc, their length.
 int split_count(const hdbf_context* ctx, int M, int N, int K, bool tri, int* kc);
+// Updates below one wave of 128 x 128 tiles (sgemm_small.cu): the CTAs that share
+// a tile's K (0: not taken), and the launch.
+int sgemm_small_split(const hdbf_context* ctx, int M, int N, int K);
+hdbf_status sgemm_small(hdbf_context* ctx, bool nn, bool lower, int S, int M, int N, int K,
+                        const float* A, long long lda, const float* B, long long ldb, float* C,
+                        long long ldc);
+void configure_sgemm_small(hdbf_context* ctx);
 // FP32 update on the tensor cores (tc_sgemm.cu): the K chunk for this shape, 0
 // where the FP32 kernel is taken; one chunk of it (a_kc / b_kc: the operand's K
 // is contiguous), whose operand range, in *range, tells the FP32 kernel behind it
@@ -323,17 +331,19 @@ void configure_tc_sgemm(hdbf_context* ctx);
 // While alive, every FP32 GEMM splits K as the GEMM of the given shape does.
 struct SplitPlan {
     hdbf_context* ctx;
-    int saved, saved_tc;
+    int saved, saved_tc, saved_small;
     SplitPlan(hdbf_context* c, int M, int N, int K)
-        : ctx(c), saved(c->split_kc), saved_tc(c->tc_plan)
+        : ctx(c), saved(c->split_kc), saved_tc(c->tc_plan), saved_small(c->small_plan)
     {
         int kc = 0;
         c->tc_plan = tc_sgemm_chunk(c, M, N, K, false);
         const int S = split_count(c, M, N, K, false, &kc);
         c->split_kc = S > 1 ? kc : 0;
+        c->small_plan = sgemm_small_split(c, M, N, K);
     }
     ~SplitPlan()
     {
+        ctx->small_plan = saved_small;
         ctx->split_kc = saved;
         ctx->tc_plan = saved_tc;
     }

@@ -418,6 +418,7 @@ hdbf_status hdbf_create(hdbf_handle* handle)
     }
     configure_tc_kernels(ctx);
     configure_tc_sgemm(ctx);
+    configure_sgemm_small(ctx);
     configure_trsm_block_kernels(ctx);
     configure_solve_kernels(ctx);
     configure_batched_kernels(ctx);
