@@ -369,13 +369,6 @@ hdbf_status potf2_small(hdbf_context* ctx, int n, float* A, long long lda, int* 
 // out[b*4096 ...] (column-major blocks); unit selects an implicit unit diagonal.
 hdbf_status tri_inv64(hdbf_context* ctx, int n, const float* L, long long ldl, bool unit,
                       float* out);
-// Leaf applications of a precomputed block inverse (in place):
-// B(rows<=64 x cols) <- inv * B  and  B(rows x cols<=64) <- B * inv^T.
-hdbf_status llu_apply(hdbf_context* ctx, int rows, int cols, const float* inv, float* B,
-                      long long ldb);
-hdbf_status rlt_apply(hdbf_context* ctx, int rows, int cols, const float* inv, float* B,
-                      long long ldb);
-
 // Inverse modes: 0 lower non-unit, 1 lower unit, 2 upper non-unit.
 hdbf_status tri_inv64_mode(hdbf_context* ctx, int n, const float* L, long long ldl, int mode,
                            float* out);

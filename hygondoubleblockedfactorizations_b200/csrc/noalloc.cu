@@ -62,7 +62,7 @@ inline int split_at(int n)
 hdbf_status rlt_recurse(hdbf_context* ctx, int rows, int cols, const float* L, long long ldl,
                         float* B, long long ldb, const float* inv)
 {
-    if (cols <= kDiagLeaf) return rlt_apply(ctx, rows, cols, inv, B, ldb);
+    if (cols <= kDiagLeaf) return rlt_block(ctx, rows, cols, L, ldl, inv, B, ldb);
     const int c1 = split_at(cols);
     const int c2 = cols - c1;
     HDBF_TRY(rlt_recurse(ctx, rows, c1, L, ldl, B, ldb, inv));

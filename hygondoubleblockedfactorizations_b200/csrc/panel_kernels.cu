@@ -2,9 +2,8 @@
 //
 // potf2_small replaces rocsolver_spotrf on the diagonal block
 // (src/potrf/double_blocked_potrf.cpp:34-56, call :334) at the leaf of this
-// library's recursive diagonal factorization; tri_inv64 + {llu,rlt}_apply
-// replace rocblas_strsm at the leaves of the recursive TRSMs
-// (src/trsm/right_lower_trsm.cpp:24-37, src/getrf/getrf_npvt_internal.h:57-70).
+// library's recursive diagonal factorization; tri_inv64 inverts the
+// diagonal blocks for the TRSM leaves (trsm_block.cu) and the solves.
 #include <cfloat>
 
 #include "internal.h"
@@ -105,48 +104,6 @@ __global__ void __launch_bounds__(256) llu_apply_kernel(int rows, int cols,
     }
 }
 
-// B(rows x cols) <- B * inv^T for cols <= 64 (inv = L^{-1} of the leaf
-// block): CTA = 128 x 64 tile of B, thread = 8 rows x 4 columns, in place.
-__global__ void __launch_bounds__(256) rlt_apply_kernel(int rows, int cols,
-                                                        const float* __restrict__ inv, float* B,
-                                                        long long ldb)
-{
-    __shared__ __align__(16) float Bs[kLeaf][128];   // Bs[k][r] = B(r0 + r, k)
-    __shared__ __align__(16) float Is[kLeaf][kLeaf];  // Is[k][c] = inv(c, k)
-    const int tid = threadIdx.x;
-    const long long r0 = (long long)blockIdx.x * 128;
-    for (int idx = tid; idx < kLeaf * kLeaf; idx += 256) Is[idx >> 6][idx & 63] = inv[idx];
-    for (int idx = tid; idx < kLeaf * 128; idx += 256) {
-        const int k = idx >> 7, r = idx & 127;
-        Bs[k][r] = (k < cols && r0 + r < rows) ? B[(long long)k * ldb + r0 + r] : 0.f;
-    }
-    __syncthreads();
-    const int ty = tid >> 4, tx = tid & 15;
-    float acc[8][4] = {};
-#pragma unroll 8
-    for (int k = 0; k < kLeaf; ++k) {
-        const float4 a0 = *reinterpret_cast<const float4*>(&Bs[k][ty * 8]);
-        const float4 a1 = *reinterpret_cast<const float4*>(&Bs[k][ty * 8 + 4]);
-        const float4 b = *reinterpret_cast<const float4*>(&Is[k][tx * 4]);
-        const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-        const float bv[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int c = tx * 4 + j;
-        if (c >= cols) continue;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const long long r = r0 + ty * 8 + i;
-            if (r < rows) B[(long long)c * ldb + r] = acc[i][j];
-        }
-    }
-}
-
 }  // namespace
 
 hdbf_status potf2_small(hdbf_context* ctx, int n, float* A, long long lda, int* info,
@@ -178,12 +135,6 @@ hdbf_status tri_inv64_mode(hdbf_context* ctx, int n, const float* L, long long l
     return last_cuda(ctx);
 }
 
-hdbf_status llu_apply(hdbf_context* ctx, int rows, int cols, const float* inv, float* B,
-                      long long ldb)
-{
-    return llu_apply_t(ctx, rows, cols, inv, B, ldb, false);
-}
-
 hdbf_status llu_apply_t(hdbf_context* ctx, int rows, int cols, const float* inv, float* B,
                         long long ldb, bool trans)
 {
@@ -193,18 +144,6 @@ hdbf_status llu_apply_t(hdbf_context* ctx, int rows, int cols, const float* inv,
     ProfScope prof(ctx, kClsTrsmL, 2.0 * kLeaf * kLeaf * (double)cols, 8.0 * rows * cols);
     llu_apply_kernel<<<(unsigned)grid, 256, 0, ctx->stream>>>(rows, cols, inv, B, ldb,
                                                                trans ? 1 : 0);
-    ctx->launches++;
-    return last_cuda(ctx);
-}
-
-hdbf_status rlt_apply(hdbf_context* ctx, int rows, int cols, const float* inv, float* B,
-                      long long ldb)
-{
-    if (rows <= 0 || cols <= 0) return HDBF_STATUS_SUCCESS;
-    if (cols > kLeaf) return HDBF_STATUS_INVALID_VALUE;
-    const long long grid = ((long long)rows + 127) / 128;
-    ProfScope prof(ctx, kClsTrsmR, 2.0 * kLeaf * kLeaf * (double)rows, 8.0 * rows * cols);
-    rlt_apply_kernel<<<(unsigned)grid, 256, 0, ctx->stream>>>(rows, cols, inv, B, ldb);
     ctx->launches++;
     return last_cuda(ctx);
 }

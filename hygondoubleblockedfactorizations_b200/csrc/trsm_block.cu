@@ -1,236 +1,391 @@
-// Coarse leaves of the recursive TRSMs: left/lower/unit B <- L^{-1} B
-// (rows <= 256) and right/lower/transposed B <- B L^{-T} (cols <= 256).
+// Leaves of the recursive TRSMs, up to four 64 x 64 diagonal blocks at once:
+// left/lower/unit B <- L^{-1} B (rows <= 256) and right/lower/transposed
+// B <- B L^{-T} (cols <= 256).  They replace the reference's trsm_left_lower_unit
+// (src/getrf/getrf_npvt_internal.h:42-88) and rocblas_strsm at the leaves of its
+// right-side TRSM (src/trsm/right_lower_trsm.cpp:24-37).
 //
-// The recursive TRSM (trsm_llu in drivers.cu, replacing the reference's
-// trsm_left_lower_unit, src/getrf/getrf_npvt_internal.h:42-88) used to
-// recurse down to 64-row leaves, which produced GEMMs with M = K = 64 -- each a
-// latency-bound launch.  This kernel solves up to four 64-row blocks at once:
-// a CTA keeps 64 columns of B (all rows) in shared memory and runs the block
-// forward substitution
-//     X_i = D_i (B_i - sum_{j<i} L_ij X_j),   D_i = L_ii^{-1}
-// with 64 x 64 tile products (D_i from tri_inv64, unit diagonal).
+// A CTA keeps a slice of B (all rows, or all columns) in shared memory and runs
+// the block forward substitution with the inverted diagonal blocks D_i:
+//     X_i = D_i (B_i - sum_{j<i} L_ij X_j)       (and its transpose on the right).
+// The order of the L and D tiles is known from the start, so they come through
+// a three-deep cp.async ring while earlier ones are multiplied (4 x 4 or smaller
+// register tiles, packed FP32 FMAs); before, each of the ten tile products of a
+// 256-wide block waited for its own loads (57 us at 7500 x 256, now 33; 19 us
+// at 2000 x 64, now 7.5).  The slice width falls when wider slices would not give
+// every SM a CTA.
 #include "internal.h"
 
 namespace hdbf {
 namespace {
 
 constexpr int kT = 64;
-constexpr int kThreads = 256;
-constexpr int kMaxRows = 256;
-constexpr int kLdS = 68;
+constexpr int kThr = 256;
+constexpr int kMaxW = 256;   // rows (left) / columns (right) of the solved block
+constexpr int kRing = 3;
+constexpr int kTile = kT * kT;
+constexpr int kLdL = kMaxW + 4;  // left: pitch of a column of X
 
-__device__ __forceinline__ void tile_mma(float acc[4][4], const float* As, const float* Bs)
+__device__ __forceinline__ uint32_t smem_addr(const void* p)
 {
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-#pragma unroll 8
-    for (int k = 0; k < kT; ++k) {
-        const float4 a = *reinterpret_cast<const float4*>(As + k * kLdS + ty * 4);
-        const float4 b = *reinterpret_cast<const float4*>(Bs + k * kLdS + tx * 4);
-        const float av[4] = {a.x, a.y, a.z, a.w};
-        const float bv[4] = {b.x, b.y, b.z, b.w};
+    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+__device__ __forceinline__ void copy16(float* dst, const float* src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void copy4(float* dst, const float* src, bool have)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_addr(dst)), "l"(src),
+                 "r"(have ? 4 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+
+// 64 columns of 64 contiguous floats: dst[c * pitch + r] = src[c * ld + r], zero
+// outside rows x cols.
+__device__ __forceinline__ void copy_tile(float* dst, int pitch, const float* src, long long ld,
+                                          int rows, int cols)
+{
+    const bool vec = rows == kT && cols == kT && ld % 4 == 0 &&
+                     (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
+    if (vec) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int u = 0; u < kTile / 4 / kThr; ++u) {
+            const int q = threadIdx.x + u * kThr, c = q >> 4, r = (q & 15) * 4;
+            copy16(dst + c * pitch + r, src + (long long)c * ld + r);
+        }
+    } else {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+        for (int u = 0; u < kTile / kThr; ++u) {
+            const int q = threadIdx.x + u * kThr, c = q >> 6, r = q & 63;
+            const bool have = r < rows && c < cols;
+            copy4(dst + c * pitch + r, have ? src + (long long)c * ld + r : src, have);
+        }
     }
 }
 
-// As[k][m] = src(m, k) = src[k * ld + m] for m < rows, k < cols (else 0)
-__device__ __forceinline__ void load_kmajor(float* As, const float* src, long long ld, int rows,
-                                            int cols)
+// Tile t of the substitution: (i, j) with j < i the block L_ij, j == i the
+// inverse D_i; i = 0, 1, ... and within it j = 0 .. i.
+__device__ __forceinline__ void tile_at(int t, int& i, int& j)
 {
-    for (int q = threadIdx.x; q < kT * kT; q += kThreads) {
-        const int k = q >> 6, m = q & 63;
-        As[k * kLdS + m] = (m < rows && k < cols) ? src[(long long)k * ld + m] : 0.f;
-    }
+    i = 0;
+    while (t > i) t -= ++i;
+    j = t;
 }
 
-// 64 x 64 tile into shared memory, k-major (As[k][m] = src(m, k) =
-// src[k * ld + m], zero outside rows x cols), every load of the thread in
-// flight before the first store.
-__device__ __forceinline__ void load_kmajor_batched(float* As, const float* src, long long ld,
-                                                    int rows, int cols)
+__device__ __forceinline__ unsigned long long pack2(float x, float y)
 {
-    float v[kT * kT / kThreads];
-#pragma unroll
-    for (int u = 0; u < kT * kT / kThreads; ++u) {
-        const int q = threadIdx.x + u * kThreads, k = q >> 6, m = q & 63;
-        v[u] = (m < rows && k < cols) ? src[(long long)k * ld + m] : 0.f;
-    }
-#pragma unroll
-    for (int u = 0; u < kT * kT / kThreads; ++u) {
-        const int q = threadIdx.x + u * kThreads, k = q >> 6, m = q & 63;
-        As[k * kLdS + m] = v[u];
-    }
+    unsigned long long v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(x), "f"(y));
+    return v;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a,
+                                     unsigned long long b)
+{
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
 
-// acc[a][b] += sum_k As[k][ty*4+a] * Xs[k][tx*CW+b] (64 rows x 16*CW columns)
-template <int CW>
-__device__ __forceinline__ void tile_mma_cw(float acc[4][CW], const float* As, const float* Xs,
-                                            int ldx)
+// ------------------------------------------------------------------- right
+// CTA: 16 RP rows of B, all columns.  X[c * 16 RP + r].  Thread: RP rows
+// (RP * (tid & 15)) x 4 columns (4 * (tid >> 4)) of a 64-column block.
+template <int RP>
+__global__ void __launch_bounds__(kThr) rlt_block_kernel(int rows, int cols,
+                                                         const float* __restrict__ L, long long ldl,
+                                                         const float* __restrict__ inv, float* B,
+                                                         long long ldb)
 {
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-#pragma unroll 8
-    for (int k = 0; k < kT; ++k) {
-        const float4 a = *reinterpret_cast<const float4*>(As + k * kLdS + ty * 4);
-        const float av[4] = {a.x, a.y, a.z, a.w};
-        float bv[CW];
-#pragma unroll
-        for (int b = 0; b < CW; ++b) bv[b] = Xs[k * ldx + tx * CW + b];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < CW; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
-    }
-}
-
-// B <- L^{-1} B for a column slice of CT = 16 * CW columns per CTA (all
-// rows <= 256 in shared memory): narrow right-hand sides get more CTAs.
-template <int CW>
-__global__ void __launch_bounds__(kThreads) llu_block_kernel(int rows, int cols,
-                                                             const float* __restrict__ L,
-                                                             long long ldl,
-                                                             const float* __restrict__ inv,
-                                                             float* B, long long ldb)
-{
-    constexpr int CT = 16 * CW;
-    constexpr int LDX = CT + 4;
+    constexpr int RT = 16 * RP;  // rows of the slice
     extern __shared__ __align__(16) float sm[];
-    float* Xs = sm;                       // kMaxRows x LDX: Xs[r][c] = B(r, c0 + c)
-    float* As = Xs + kMaxRows * LDX;      // left operand tile (k-major)
-    float* Ts = As + kT * kLdS;           // right operand staging (64 x LDX)
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int nb = (cols + kT - 1) / kT, nt = nb * (nb + 1) / 2;
+    const int ring = min(nt, kRing);
+    float* tiles = sm;
+    float* X = sm + ring * kTile;
+    const int tid = threadIdx.x, ty = tid & 15, tx = tid >> 4;
+    const long long r0 = (long long)blockIdx.x * RT;
+    const int nr = (int)min((long long)RT, (long long)rows - r0);
+    auto fetch = [&](int t) {
+        if (t < nt) {
+            int i, j;
+            tile_at(t, i, j);
+            float* dst = tiles + (t % ring) * kTile;
+            if (i == j) copy_tile(dst, kT, inv + (long long)i * kTile, kT, kT, kT);
+            else  // [k][c] = L(64 i + c, 64 j + k)
+                copy_tile(dst, kT, L + (long long)(j * kT) * ldl + i * kT, ldl,
+                          min(kT, cols - i * kT), kT);
+        }
+        commit();
+    };
+    {
+        const bool vec = nr == RT && ldb % 4 == 0 && (reinterpret_cast<uintptr_t>(B + r0) & 15u) == 0;
+        const int total = nb * kT * RT;
+        if (vec) {
+            for (int q = tid * 4; q < total; q += kThr * 4) {
+                const int c = q / RT, r = q % RT;
+                if (c < cols) copy16(X + q, B + (long long)c * ldb + r0 + r);
+                else *reinterpret_cast<float4*>(X + q) = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        } else {
+            for (int q = tid; q < total; q += kThr) {
+                const int c = q / RT, r = q % RT;
+                const bool have = r < nr && c < cols;
+                copy4(X + q, have ? B + (long long)c * ldb + r0 + r : B, have);
+            }
+        }
+    }
+    fetch(0);
+    if (ring > 1) fetch(1); else commit();
+    int t = 0;
+    for (int i = 0; i < nb; ++i) {
+        unsigned long long acc[4][(RP + 1) / 2];
+        float a1[4];  // RP == 1
+        for (int j = 0; j <= i; ++j, ++t) {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncthreads();  // tile t and X are there; tile t - 1 and X_i's old reads are done
+            if (ring > 2) fetch(t + 2); else commit();
+            if (j == 0) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const float* x = X + (i * kT + tx * 4 + c) * RT + ty * RP;
+                    if (RP == 1) a1[c] = i == 0 ? 0.f : x[0];
+#pragma unroll
+                    for (int h = 0; h < RP / 2; ++h)
+                        acc[c][h] = i == 0 ? 0ull : *reinterpret_cast<const unsigned long long*>(x + 2 * h);
+                }
+            }
+            const float* b = tiles + (t % ring) * kTile + tx * 4;
+            const float* x = X + j * kT * RT + ty * RP;
+            if (j == i && i > 0) {  // B_i - sum back into X_i, then times D_i
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    float* o = X + (i * kT + tx * 4 + c) * RT + ty * RP;
+                    if (RP == 1) o[0] = a1[c], a1[c] = 0.f;
+#pragma unroll
+                    for (int h = 0; h < RP / 2; ++h) {
+                        *reinterpret_cast<unsigned long long*>(o + 2 * h) = acc[c][h];
+                        acc[c][h] = 0ull;
+                    }
+                }
+                __syncthreads();
+            }
+            const float sign = j == i ? 1.f : -1.f;
+#pragma unroll 8
+            for (int k = 0; k < kT; ++k) {
+                const float4 bv = *reinterpret_cast<const float4*>(b + k * kT);
+                const float bb[4] = {sign * bv.x, sign * bv.y, sign * bv.z, sign * bv.w};
+                if (RP == 1) {
+                    const float xv = x[k * RT];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) a1[c] = fmaf(xv, bb[c], a1[c]);
+                }
+#pragma unroll
+                for (int h = 0; h < RP / 2; ++h) {
+                    const unsigned long long xv =
+                        *reinterpret_cast<const unsigned long long*>(x + k * RT + 2 * h);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) fma2(acc[c][h], xv, pack2(bb[c], bb[c]));
+                }
+            }
+            if (j == i) {
+                if (i + 1 < nb) __syncthreads();  // X_i is still being read
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const int col = i * kT + tx * 4 + c;
+                    float v[RP];
+                    if (RP == 1) v[0] = a1[c];
+#pragma unroll
+                    for (int h = 0; h < RP / 2; ++h) {
+                        const float2 p = unpack2(acc[c][h]);
+                        v[2 * h] = p.x;
+                        v[(2 * h + 1) % RP] = p.y;
+                    }
+#pragma unroll
+                    for (int e = 0; e < RP; ++e) {
+                        if (i + 1 < nb) X[col * RT + ty * RP + e] = col < cols ? v[e] : 0.f;
+                        if (col < cols && ty * RP + e < nr)
+                            B[(long long)col * ldb + r0 + ty * RP + e] = v[e];
+                    }
+                }
+            }
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+// -------------------------------------------------------------------- left
+// CTA: 16 CP columns of B, all rows.  X[n * kLdL + k].  Thread: 4 rows
+// (4 * (tid & 15)) of a 64-row block x CP columns (CP * (tid >> 4)).
+template <int CP>
+__global__ void __launch_bounds__(kThr) llu_block_kernel(int rows, int cols,
+                                                         const float* __restrict__ L, long long ldl,
+                                                         const float* __restrict__ inv, float* B,
+                                                         long long ldb)
+{
+    constexpr int CT = 16 * CP;
+    extern __shared__ __align__(16) float sm[];
+    const int nb = (rows + kT - 1) / kT, nt = nb * (nb + 1) / 2;
+    const int ring = min(nt, kRing);
+    float* tiles = sm;
+    float* X = sm + ring * kTile;
+    const int tid = threadIdx.x, ty = tid & 15, tx = tid >> 4;
     const long long c0 = (long long)blockIdx.x * CT;
     const int nc = (int)min((long long)CT, (long long)cols - c0);
-    const int nb = (rows + kT - 1) / kT;
-
-    for (int q = tid; q < kMaxRows * CT; q += kThreads) {
-        const int c = q / kMaxRows, r = q - c * kMaxRows;
-        Xs[r * LDX + c] = (r < rows && c < nc) ? B[(c0 + c) * ldb + r] : 0.f;
+    auto fetch = [&](int t) {
+        if (t < nt) {
+            int i, j;
+            tile_at(t, i, j);
+            float* dst = tiles + (t % ring) * kTile;
+            if (i == j) copy_tile(dst, kT, inv + (long long)i * kTile, kT, kT, kT);
+            else  // [k][m] = L(64 i + m, 64 j + k)
+                copy_tile(dst, kT, L + (long long)(j * kT) * ldl + i * kT, ldl,
+                          min(kT, rows - i * kT), kT);
+        }
+        commit();
+    };
+    {
+        const int len = nb * kT;
+        const bool vec = rows == len && ldb % 4 == 0 && (reinterpret_cast<uintptr_t>(B) & 15u) == 0;
+        if (vec) {
+            for (int q = tid * 4; q < CT * len; q += kThr * 4) {
+                const int n = q / len, k = q - n * len;
+                if (n < nc) copy16(X + n * kLdL + k, B + (c0 + n) * ldb + k);
+                else *reinterpret_cast<float4*>(X + n * kLdL + k) = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        } else {
+            for (int q = tid; q < CT * len; q += kThr) {
+                const int n = q / len, k = q - n * len;
+                const bool have = n < nc && k < rows;
+                copy4(X + n * kLdL + k, have ? B + (c0 + n) * ldb + k : B, have);
+            }
+        }
     }
-    __syncthreads();
+    fetch(0);
+    if (ring > 1) fetch(1); else commit();
+    int t = 0;
     for (int i = 0; i < nb; ++i) {
-        const int ri = min(kT, rows - i * kT);
-        float acc[4][CW];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < CW; ++b) acc[a][b] = Xs[(i * kT + ty * 4 + a) * LDX + tx * CW + b];
-        for (int j = 0; j < i; ++j) {
-            load_kmajor_batched(As, L + (long long)(j * kT) * ldl + i * kT, ldl, ri, kT);
+        unsigned long long acc[CP][2];  // [column][row pair]
+        for (int j = 0; j <= i; ++j, ++t) {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
             __syncthreads();
-            float p[4][CW] = {};
-            tile_mma_cw<CW>(p, As, Xs + j * kT * LDX, LDX);
+            if (ring > 2) fetch(t + 2); else commit();
+            if (j == 0) {
 #pragma unroll
-            for (int a = 0; a < 4; ++a)
+                for (int c = 0; c < CP; ++c) {
+                    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(
+                        X + (tx * CP + c) * kLdL + i * kT + ty * 4);
+                    acc[c][0] = i == 0 ? 0ull : v.x;
+                    acc[c][1] = i == 0 ? 0ull : v.y;
+                }
+            }
+            const float* a = tiles + (t % ring) * kTile + ty * 4;
+            if (j == i && i > 0) {
 #pragma unroll
-                for (int b = 0; b < CW; ++b) acc[a][b] -= p[a][b];
-            __syncthreads();
+                for (int c = 0; c < CP; ++c) {
+                    ulonglong2 v;
+                    v.x = acc[c][0];
+                    v.y = acc[c][1];
+                    *reinterpret_cast<ulonglong2*>(X + (tx * CP + c) * kLdL + i * kT + ty * 4) = v;
+                    acc[c][0] = acc[c][1] = 0ull;
+                }
+                __syncthreads();
+            }
+            const float sign = j == i ? 1.f : -1.f;
+            const float* x = X + tx * CP * kLdL + j * kT;
+#pragma unroll 4
+            for (int k = 0; k < kT; k += 4) {
+                float4 xv[CP];
+#pragma unroll
+                for (int c = 0; c < CP; ++c)
+                    xv[c] = *reinterpret_cast<const float4*>(x + c * kLdL + k);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const ulonglong2 av = *reinterpret_cast<const ulonglong2*>(a + (k + q) * kT);
+#pragma unroll
+                    for (int c = 0; c < CP; ++c) {
+                        const float e = sign * (q == 0 ? xv[c].x : q == 1 ? xv[c].y
+                                                       : q == 2 ? xv[c].z : xv[c].w);
+                        fma2(acc[c][0], av.x, pack2(e, e));
+                        fma2(acc[c][1], av.y, pack2(e, e));
+                    }
+                }
+            }
+            if (j == i) {
+                if (i + 1 < nb) __syncthreads();
+#pragma unroll
+                for (int c = 0; c < CP; ++c) {
+                    const int n = tx * CP + c;
+                    const float2 p = unpack2(acc[c][0]), q = unpack2(acc[c][1]);
+                    const float v[4] = {p.x, p.y, q.x, q.y};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int r = i * kT + ty * 4 + e;
+                        if (i + 1 < nb) X[n * kLdL + r] = r < rows ? v[e] : 0.f;
+                        if (r < rows && n < nc) B[(c0 + n) * ldb + r] = v[e];
+                    }
+                }
+            }
         }
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < CW; ++b) Ts[(ty * 4 + a) * LDX + tx * CW + b] = acc[a][b];
-        load_kmajor_batched(As, inv + (long long)i * kT * kT, kT, kT, kT);
-        __syncthreads();
-        float x[4][CW] = {};
-        tile_mma_cw<CW>(x, As, Ts, LDX);
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < CW; ++b)
-                Xs[(i * kT + ty * 4 + a) * LDX + tx * CW + b] = (ty * 4 + a < ri) ? x[a][b] : 0.f;
-        __syncthreads();
     }
-    for (int q = tid; q < kMaxRows * CT; q += kThreads) {
-        const int c = q / kMaxRows, r = q - c * kMaxRows;
-        if (r < rows && c < nc) B[(c0 + c) * ldb + r] = Xs[r * LDX + c];
-    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-// B(rows x cols <= 256) <- B L^{-T}, L lower non-unit: a CTA keeps 64 rows of
-// B (all columns) in shared memory, column-major (Xs[c][r]), and runs
-//     X_j = (B_j - sum_{i<j} X_i L_ji^T) D_j^T,   D_j = L_jj^{-1}.
-__global__ void __launch_bounds__(kThreads) rlt_block_kernel(int rows, int cols,
-                                                             const float* __restrict__ L,
-                                                             long long ldl,
-                                                             const float* __restrict__ inv,
-                                                             float* B, long long ldb)
+// Dynamic shared memory for nb diagonal blocks; one block needs no more than the
+// default limit, so a launch without a configured handle may take it.
+template <int RP>
+size_t rlt_smem(int nb)
 {
-    extern __shared__ __align__(16) float sm[];
-    float* Xs = sm;                       // kMaxRows (columns) x kLdS: Xs[c][r] = B(r0 + r, c)
-    float* Bs = Xs + kMaxRows * kLdS;     // right operand tile
-    float* Ts = Bs + kT * kLdS;           // left operand staging
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const long long r0 = (long long)blockIdx.x * kT;
-    const int nr = (int)min((long long)kT, (long long)rows - r0);
-    const int nb = (cols + kT - 1) / kT;
-
-    for (int q = tid; q < kMaxRows * kT; q += kThreads) {
-        const int c = q >> 6, r = q & 63;
-        Xs[c * kLdS + r] = (r < nr && c < cols) ? B[(long long)c * ldb + r0 + r] : 0.f;
-    }
-    __syncthreads();
-    for (int j = 0; j < nb; ++j) {
-        const int cj = min(kT, cols - j * kT);
-        float acc[4][4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < 4; ++b) acc[a][b] = Xs[(j * kT + tx * 4 + b) * kLdS + ty * 4 + a];
-        for (int i = 0; i < j; ++i) {
-            // Bs[k][c] = L_ji(c, k) = L(j*64 + c, i*64 + k)
-            load_kmajor(Bs, L + (long long)(i * kT) * ldl + j * kT, ldl, cj, kT);
-            __syncthreads();
-            float p[4][4] = {};
-            tile_mma(p, Xs + i * kT * kLdS, Bs);
-#pragma unroll
-            for (int a = 0; a < 4; ++a)
-#pragma unroll
-                for (int b = 0; b < 4; ++b) acc[a][b] -= p[a][b];
-            __syncthreads();
-        }
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < 4; ++b) Ts[(tx * 4 + b) * kLdS + ty * 4 + a] = acc[a][b];
-        load_kmajor(Bs, inv + (long long)j * kT * kT, kT, kT, kT);  // Bs[k][c] = D_j(c, k)
-        __syncthreads();
-        float x[4][4] = {};
-        tile_mma(x, Ts, Bs);
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < 4; ++b)
-                Xs[(j * kT + tx * 4 + b) * kLdS + ty * 4 + a] = (tx * 4 + b < cj) ? x[a][b] : 0.f;
-        __syncthreads();
-    }
-    for (int q = tid; q < kMaxRows * kT; q += kThreads) {
-        const int c = q >> 6, r = q & 63;
-        if (r < nr && c < cols) B[(long long)c * ldb + r0 + r] = Xs[c * kLdS + r];
-    }
+    const int nt = nb * (nb + 1) / 2;
+    return sizeof(float) * ((size_t)(nt < kRing ? nt : kRing) * kTile + (size_t)nb * kT * 16 * RP);
+}
+template <int CP>
+size_t llu_smem(int nb)
+{
+    const int nt = nb * (nb + 1) / 2;
+    return sizeof(float) * ((size_t)(nt < kRing ? nt : kRing) * kTile + (size_t)16 * CP * kLdL);
 }
 
-constexpr size_t kSmem = sizeof(float) * ((size_t)kMaxRows * kLdS + 2 * (size_t)kT * kLdS);
-// llu_block_kernel<CW>: Xs (kMaxRows x (16 CW + 4)), As (64 x kLdS), Ts (64 x (16 CW + 4))
-template <int CW>
-constexpr size_t llu_smem()
+template <int RP>
+void rlt_launch(hdbf_context* ctx, int rows, int cols, const float* L, long long ldl,
+                const float* inv, float* B, long long ldb)
 {
-    return sizeof(float) * ((size_t)kMaxRows * (16 * CW + 4) + (size_t)kT * kLdS +
-                            (size_t)kT * (16 * CW + 4));
+    const unsigned grid = (unsigned)(((long long)rows + 16 * RP - 1) / (16 * RP));
+    rlt_block_kernel<RP><<<grid, kThr, rlt_smem<RP>((cols + kT - 1) / kT), ctx->stream>>>(
+        rows, cols, L, ldl, inv, B, ldb);
+}
+template <int CP>
+void llu_launch(hdbf_context* ctx, int rows, int cols, const float* L, long long ldl,
+                const float* inv, float* B, long long ldb)
+{
+    const unsigned grid = (unsigned)(((long long)cols + 16 * CP - 1) / (16 * CP));
+    llu_block_kernel<CP><<<grid, kThr, llu_smem<CP>((rows + kT - 1) / kT), ctx->stream>>>(
+        rows, cols, L, ldl, inv, B, ldb);
 }
 
 }  // namespace
 
-int llu_block_max_rows() { return kMaxRows; }
+int llu_block_max_rows() { return kMaxW; }
 
 void configure_trsm_block_kernels(hdbf_context*)
 {
+    const int nb = kMaxW / kT;
+    cudaFuncSetAttribute(rlt_block_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)rlt_smem<4>(nb));
+    cudaFuncSetAttribute(rlt_block_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)rlt_smem<2>(nb));
+    cudaFuncSetAttribute(rlt_block_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)rlt_smem<1>(nb));
     cudaFuncSetAttribute(llu_block_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)llu_smem<4>());
+                         (int)llu_smem<4>(nb));
+    cudaFuncSetAttribute(llu_block_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)llu_smem<2>(nb));
     cudaFuncSetAttribute(llu_block_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)llu_smem<1>());
-    cudaFuncSetAttribute(rlt_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+                         (int)llu_smem<1>(nb));
     cudaGetLastError();
 }
 
@@ -240,12 +395,14 @@ hdbf_status rlt_block(hdbf_context* ctx, int rows, int cols, const float* L, lon
                       const float* inv, float* B, long long ldb)
 {
     if (rows <= 0 || cols <= 0) return HDBF_STATUS_SUCCESS;
-    if (cols > kMaxRows) return HDBF_STATUS_INVALID_VALUE;
-    const long long grid = ((long long)rows + kT - 1) / kT;
+    if (cols > kMaxW) return HDBF_STATUS_INVALID_VALUE;
     ProfScope prof(ctx, kClsTrsmR, (double)cols * cols * rows, 8.0 * (double)rows * cols, rows,
                    cols, (cols + kT - 1) / kT);
-    rlt_block_kernel<<<(unsigned)grid, kThreads, kSmem, ctx->stream>>>(rows, cols, L, ldl, inv, B,
-                                                                      ldb);
+    // 64 rows per CTA when that gives two thirds of the SMs one, else 32, else 16
+    const long long full = 2LL * ctx->sm_count / 3 * 64;
+    if (rows >= full) rlt_launch<4>(ctx, rows, cols, L, ldl, inv, B, ldb);
+    else if (2LL * rows >= full) rlt_launch<2>(ctx, rows, cols, L, ldl, inv, B, ldb);
+    else rlt_launch<1>(ctx, rows, cols, L, ldl, inv, B, ldb);
     ctx->launches++;
     return last_cuda(ctx);
 }
@@ -256,20 +413,13 @@ hdbf_status llu_block(hdbf_context* ctx, int rows, int cols, const float* L, lon
                       const float* inv, float* B, long long ldb)
 {
     if (rows <= 0 || cols <= 0) return HDBF_STATUS_SUCCESS;
-    if (rows > kMaxRows) return HDBF_STATUS_INVALID_VALUE;
-    const int nb = (rows + kT - 1) / kT;
+    if (rows > kMaxW) return HDBF_STATUS_INVALID_VALUE;
     ProfScope prof(ctx, kClsTrsmL, (double)rows * rows * cols, 8.0 * (double)rows * cols, rows,
-                   cols, nb);
-    // 64 columns per CTA when that fills the SMs, else 16 (four times the CTAs)
-    if ((cols + kT - 1) / kT >= ctx->sm_count) {
-        const long long grid = ((long long)cols + 63) / 64;
-        llu_block_kernel<4><<<(unsigned)grid, kThreads, llu_smem<4>(), ctx->stream>>>(
-            rows, cols, L, ldl, inv, B, ldb);
-    } else {
-        const long long grid = ((long long)cols + 15) / 16;
-        llu_block_kernel<1><<<(unsigned)grid, kThreads, llu_smem<1>(), ctx->stream>>>(
-            rows, cols, L, ldl, inv, B, ldb);
-    }
+                   cols, (rows + kT - 1) / kT);
+    const long long full = 2LL * ctx->sm_count / 3 * 64;  // as rlt_block
+    if (cols >= full) llu_launch<4>(ctx, rows, cols, L, ldl, inv, B, ldb);
+    else if (2LL * cols >= full) llu_launch<2>(ctx, rows, cols, L, ldl, inv, B, ldb);
+    else llu_launch<1>(ctx, rows, cols, L, ldl, inv, B, ldb);
     ctx->launches++;
     return last_cuda(ctx);
 }
