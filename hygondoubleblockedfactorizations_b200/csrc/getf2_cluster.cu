@@ -10,34 +10,35 @@
 // rows per CTA (tile[c * ldt + r], ldt odd).  It is factored in sub-panels of
 // NB columns (64 bytes of a row: 16 FP32, 8 FP64) that live in registers,
 // thread t owning local rows t, t + TH, ...  Per column:
-//   1. every warp finds its candidate (largest |a| over owned rows >= J, lowest
-//      row on ties -- LAPACK ISAMAX) with integer warp reductions; its owner
-//      lane writes the candidate's sub-panel row to shared memory;
+//   1. every warp finds its candidate (largest |a| over rows at position >= J,
+//      lowest position on ties -- LAPACK ISAMAX) with integer warp reductions;
+//      its owner lane writes the candidate's row to shared memory;
 //   2. after one block barrier a few warps reduce the warps' candidates and
-//      push the CTA's one (magnitude, row, NB values) and, from the CTA that
-//      owns it, the diagonal row to every CTA of the cluster with st.async,
-//      counted in bytes on the receiver's mbarrier: data and flag arrive in
-//      one trip, and nothing needs a fence;
-//   3. every warp reduces the CTAs' candidates from its own shared memory; the
-//      owners replace their rows in registers, and every thread scales and
-//      applies the rank-1 update.  The registers rotate by one column per step
-//      (the column just finished goes to the back), so that the loop is rolled
-//      and a row swap carries the multipliers already computed.
+//      push the CTA's one (magnitude, position, NB values) to every CTA of the
+//      cluster with st.async, counted in bytes on the receiver's mbarrier: data
+//      and flag arrive in one trip, and nothing needs a fence;
+//   3. every warp reduces the CTAs' candidates from its own shared memory, and
+//      every thread scales and applies the rank-1 update.
+// No row moves inside a sub-panel: a row keeps its place and carries its
+// position (what LAPACK's swaps so far would have made it), the chosen row
+// stores its U entries and the others their multiplier where they are.  The
+// registers shift by one column per step, so the loop is rolled and needs no
+// selects.
 // Two message buffers (column parity) suffice: a CTA sends column J + 1 only
 // after a block barrier that follows all its reads of column J, and nobody can
 // send column J + 2 without it.
-// After a sub-panel, the rest of the block (other columns of the tile) takes
-// the sub-panel's interchanges as at most 2 NB composed row moves through
-// distributed shared memory; every CTA reads the new diagonal rows and solves
-// U12 = L11^{-1} A12 for itself (L11 came with the candidates), and every thread
+// After a sub-panel, all columns of the tile take its interchanges as at most 2
+// NB composed row moves through distributed shared memory; every CTA reads the
+// new diagonal rows and solves U12 = L11^{-1} A12 for itself, and every thread
 // applies the rank-NB update to its own rows, in column order: the result is
 // bit-identical to column-by-column elimination (getf2_coop).
-// Measured per column, against the grid-wide kernel's 4.1-6.5 us: 1.7 us at
-// m = 1001, 1.8 at 4096, 2.0 at 8192 (FP32).  The rest is issue: about 400
-// mostly dependent instructions per warp and column, two warps per scheduler.
+// Measured per column, against the grid-wide kernel's 4.1-6.5 us: 1.3 us at m =
+// 1001, 1.5 at 4096, 1.8 at 8192, 2.1 at 16384 (FP32).  The rest is issue and
+// fixed latencies: ~300 dependent instructions per warp and column.
 // Waits on an mbarrier are bounded by the handle's poll limit; an expired wait
-// records a timeout and the CTA runs on without waiting, so that every cluster
-// barrier is still met.
+// records a timeout and the CTA runs on without waiting or arriving (a second
+// arrival in an incomplete phase is an error), so that every cluster barrier is
+// still met.
 #include <cfloat>
 #include <climits>
 
@@ -184,12 +185,10 @@ __device__ __forceinline__ void load_key(const Cand<double>& c, unsigned long lo
 template <class T>
 struct ClusterSmem {
     Cand<T> in[2][kClMaxCluster];  // the cluster's candidates
-    T diag[2][kNB<T>];             // the diagonal row
     Cand<T> own[2][16];            // this CTA's warps' candidates
-    T own_diag[2][kNB<T>];
     T U[kClMaxW / 2][kNB<T>][2];  // U12 of the sub-panel, columns in pairs: U[c / 2][k][c & 1]
-    T L[kNB<T>][kNB<T> + 1];      // L11 rows as they arrived (rotated, see the kernel)
-    int mv_pos[32], mv_src[32];   // composed interchanges of the sub-panel
+    T L[kNB<T>][kNB<T> + 1];      // L11, L[r][k]
+    int piv[kNB<T>];              // pivot positions of the sub-panel
     unsigned long long bar[2];
 };
 
@@ -285,26 +284,20 @@ getf2_cluster_kernel(int m, int w, T* A, long long lda, int rpc, int* ipiv, int 
     cluster_wait();  // every CTA runs and its barriers are initialised
 
     const int steps = min(m, w);
-    const bool others = w > NB;
     for (int jb = 0; jb < steps; jb += NB) {
-        const int nbc = min(NB, w - jb);     // columns of this sub-panel
+        const int nbc = min(NB, w - jb);      // columns of this sub-panel
         const int sb = min(nbc, steps - jb);  // pivots in it
-        cluster_arrive();  // releases the updates of the previous sub-panel
         const int owner = jb / rpc;  // rpc is a multiple of NB: it owns all diagonal rows
         T a[R][NB];
+        int pos[R];  // the row's position; below J once it has been a pivot row
 #pragma unroll
         for (int i = 0; i < R; ++i) {
             const int r = tid + TH * i;
+            pos[i] = r < nr ? r0 + r : -1;
 #pragma unroll
             for (int c = 0; c < NB; ++c)
                 a[i][c] = (r < nr && c < nbc) ? tile[(jb + c) * ldt + r] : T(0);
         }
-        // Composed interchanges, one position per lane of the last warp:
-        // position mv_pos takes the row that was at mv_src before the
-        // sub-panel.  Lanes < NB are the diagonal positions, later ones the
-        // pivot rows met so far.
-        int mv_pos = lane < NB ? jb + lane : -1, mv_src = mv_pos, mv_cnt = NB;
-        const bool own_j = rank == owner;
         const int dst = lane & 15, ch = tid >> 4;  // sender roles: peer, 16-byte chunk
 
 #pragma unroll 1
@@ -315,40 +308,31 @@ getf2_cluster_kernel(int m, int w, T* A, long long lda, int rpc, int* ipiv, int 
             int row = INT_MAX;
 #pragma unroll
             for (int i = 0; i < R; ++i) {
-                const int r = tid + TH * i, g = r0 + r;
-                const bool can = r < nr && (pivot ? g >= J : g == J);
                 const Mag<T> b = mag_bits(a[i][0]);
-                if (can && (row == INT_MAX || b > vb)) {
+                if ((pivot ? pos[i] >= J : pos[i] == J) &&
+                    (row == INT_MAX || b > vb || (b == vb && pos[i] < row))) {
                     vb = b;
-                    row = g;
+                    row = pos[i];
                 }
             }
             Mag<T> mv;
             int mrow;
             warp_argmax(vb, row, mv, mrow);
-            Cand<T>& mine_c = sm.own[par][warp];
             if (row == mrow && (row != INT_MAX || lane == 0)) {
-                mine_c.mag = mv;
-                mine_c.row = mrow;
+                Cand<T>& c = sm.own[par][warp];
+                c.mag = mv;
+                c.row = mrow;
 #pragma unroll
                 for (int i = 0; i < R; ++i)
-                    if (R == 1 || r0 + tid + TH * i == mrow) {
+                    if (R == 1 || pos[i] == mrow) {
 #pragma unroll
-                        for (int c = 0; c < NB; ++c) mine_c.x[c] = a[i][c];
+                        for (int q = 0; q < NB; ++q) c.x[q] = a[i][q];
                     }
             }
-            if (own_j) {
-#pragma unroll
-                for (int i = 0; i < R; ++i)
-                    if (r0 + tid + TH * i == J) {
-#pragma unroll
-                        for (int c = 0; c < NB; ++c) sm.own_diag[par][c] = a[i][c];
-                    }
-            }
-            if (tid == 0 && C > 1)  // every candidate (80 bytes) and the diagonal row
+            if (tid == 0 && C > 1 && !dead)  // every candidate, 80 bytes
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
                                  smem_addr(&sm.bar[par])),
-                             "r"(C * 80 + 64)
+                             "r"(C * 80)
                              : "memory");
             __syncthreads();
             // 2. the CTA's candidate to every CTA: 16 peers per 16-byte chunk
@@ -363,15 +347,9 @@ getf2_cluster_kernel(int m, int w, T* A, long long lda, int rpc, int* ipiv, int 
                     push16(peer_base(dst) + off_of(&sm.in[par][rank]) + 16 * ch,
                            peer_base(dst) + off_of(&sm.bar[par]),
                            reinterpret_cast<const uint4*>(&sm.own[par][from])[ch]);
-            } else if (own_j && warp < 5) {  // warps 3, 4: the diagonal row
-                if (dst < C)
-                    push16(peer_base(dst) + off_of(sm.diag[par]) + 16 * (ch - 6),
-                           peer_base(dst) + off_of(&sm.bar[par]),
-                           reinterpret_cast<const uint4*>(sm.own_diag[par])[ch - 6]);
             }
             // 3. the cluster's candidate
             const T* urow;
-            const T* drow;
             T rcp;
             if (C > 1) {
                 if (!dead) {
@@ -382,7 +360,7 @@ getf2_cluster_kernel(int m, int w, T* A, long long lda, int rpc, int* ipiv, int 
                         uint32_t ok;
                         asm volatile(
                             "{\n\t.reg .pred q;\n\t"
-                            "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 q, [%1], %2;\n\t"
+                            "mbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\n\t"
                             "selp.u32 %0, 1, 0, q;\n\t}"
                             : "=r"(ok)
                             : "r"(bar), "r"(phase)
@@ -405,10 +383,8 @@ getf2_cluster_kernel(int m, int w, T* A, long long lda, int rpc, int* ipiv, int 
                 from = who ? __ffs(who) - 1 : 0;
                 rcp = __shfl_sync(0xffffffffu, rcp, from);
                 urow = sm.in[par][from].x;
-                drow = sm.diag[par];
             } else {
                 urow = sm.own[par][from].x;
-                drow = sm.own_diag[par];
                 rcp = Bits<T>::rcp(Bits<T>::val(mv));
             }
             const int p = mrow >= J && mrow < m ? mrow : J;
@@ -419,25 +395,6 @@ getf2_cluster_kernel(int m, int w, T* A, long long lda, int rpc, int* ipiv, int 
             const bool nz = piv != T(0);
             rcp = piv < T(0) ? -rcp : (piv == piv ? rcp : piv);
             const bool recip = abs_t(piv) >= min_normal(piv) || piv != piv;
-            bool touched = false;
-#pragma unroll
-            for (int i = 0; i < R; ++i) {
-                const int g = r0 + tid + TH * i;
-                touched = touched || g == J || g == p;
-            }
-            if (__any_sync(0xffffffffu, touched)) {  // the interchange, in the two rows' warps
-#pragma unroll
-                for (int i = 0; i < R; ++i) {
-                    const int g = r0 + tid + TH * i;
-                    if (g == J) {
-#pragma unroll
-                        for (int c = 0; c < NB; ++c) a[i][c] = u[c];
-                    } else if (g == p) {
-#pragma unroll
-                        for (int c = 0; c < NB; ++c) a[i][c] = drow[c];
-                    }
-                }
-            }
             T l[R];
 #pragma unroll
             for (int i = 0; i < R; ++i) l[i] = a[i][0] * rcp;
@@ -447,82 +404,58 @@ getf2_cluster_kernel(int m, int w, T* A, long long lda, int rpc, int* ipiv, int 
             }
 #pragma unroll
             for (int i = 0; i < R; ++i) {
-                const bool below = r0 + tid + TH * i > J;
-                l[i] = below ? l[i] : a[i][0];
-                const int top = below ? NB - j : 0;  // columns still in the update
+                T* x = tile + J * ldt + tid + TH * i;
+                if (pos[i] == p) {  // the pivot row: its U entries, in place
 #pragma unroll
-                for (int c = 1; c < NB; ++c) {
-                    const T x = fma_t(-l[i], u[c], a[i][c]);
-                    a[i][c - 1] = c < top ? x : a[i][c];
+                    for (int c = 0; c < NB; ++c)
+                        if (c < nbc - j) x[c * ldt] = u[c];
+                    pos[i] = J;
+                } else if (pos[i] == J) {
+                    pos[i] = p;
                 }
-                a[i][NB - 1] = l[i];
+                if (pos[i] > J) x[0] = l[i];
+#pragma unroll
+                for (int c = 1; c < NB; ++c) a[i][c - 1] = fma_t(-l[i], u[c], a[i][c]);
+                a[i][NB - 1] = T(0);
             }
-            if (warp == NW - 1) {  // off the chain: bookkeeping
-                if (rank == 0 && lane == 0) {
+            if (tid == TH - 1) {
+                sm.piv[j] = p;
+                if (rank == 0) {
                     if (pivot) ipiv[J] = p + 1 + ipiv_add;
                     if (!nz && info) atomicCAS(info, 0, info_base + J + 1);
                 }
-                if (others) {
-                    // the pivot row carries L11's row j in its last j places
-                    if (lane < NB) sm.L[j][lane] = urow[lane];
-                    if (p != J) {
-                        const unsigned hit = __ballot_sync(0xffffffffu, mv_pos == p);
-                        const int x = hit ? __ffs(hit) - 1 : mv_cnt;
-                        if (!hit) {
-                            if (lane == x) mv_pos = mv_src = p;
-                            ++mv_cnt;
-                        }
-                        const int st = __shfl_sync(0xffffffffu, mv_src, j);
-                        const int sx = __shfl_sync(0xffffffffu, mv_src, x);
-                        if (lane == j) mv_src = sx;
-                        if (lane == x) mv_src = st;
-                    }
-                }
             }
         }
-        // a short last sub-panel: rotate the rest of the way
-        for (int j = sb; j < NB; ++j) {
-#pragma unroll
-            for (int i = 0; i < R; ++i) {
-                const T l = a[i][0];
-#pragma unroll
-                for (int c = 1; c < NB; ++c) a[i][c - 1] = a[i][c];
-                a[i][NB - 1] = l;
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < R; ++i) {
-            const int r = tid + TH * i;
-#pragma unroll
-            for (int c = 0; c < NB; ++c)
-                if (r < nr && c < nbc) tile[(jb + c) * ldt + r] = a[i][c];
-        }
-        if (others && warp == NW - 1) {
-            sm.mv_pos[lane] = mv_pos;
-            sm.mv_src[lane] = mv_src;
-        }
-        cluster_wait();
-        if (!others) continue;
         __syncthreads();
-        // The interchanges on the other columns.  Lane = move, warp = columns:
-        // the moves into this CTA's rows, and on every CTA the new diagonal
-        // rows right of the sub-panel, from which each solves U12 itself.
-        constexpr int kOther = kClMaxW * 4 / (int)sizeof(T) - NB;
-        constexpr int kIt = (kOther + NW - 1) / NW;
-        const int c1 = jb + nbc, nother = w - nbc;
-        mv_pos = sm.mv_pos[lane];
-        mv_src = sm.mv_src[lane];
+        cluster_arrive();
+        cluster_wait();  // every CTA's rows are in its tile
+        // The interchanges, composed: lanes < NB are the diagonal positions, the
+        // others the pivot positions; the row that ends up at mv_pos is found
+        // by undoing the swaps from the last one on (a position that appears
+        // twice gets the same row twice).
+        int mv_pos = lane < NB ? jb + lane : (lane < NB + sb ? sm.piv[lane - NB] : -1);
+        if (lane >= NB && mv_pos < jb + NB) mv_pos = -1;  // a diagonal position: lanes < NB have it
+        int mv_src = mv_pos;
+        for (int t = sb - 1; t >= 0; --t) {
+            const int q = sm.piv[t];
+            mv_src = mv_src == jb + t ? q : (mv_src == q ? jb + t : mv_src);
+        }
+        // Lane = move, warp = columns: the moves into this
+        // CTA's rows, and on every CTA the new diagonal rows from the sub-panel
+        // on, from which each takes L11 and solves U12 itself.
+        constexpr int kIt = (kClMaxW * 4 / (int)sizeof(T) + NW - 1) / NW;
+        const int c1 = jb + nbc;
         const bool top_row = lane < NB;
-        const bool here = mv_pos >= r0 && mv_pos < r0 + nr;
+        const bool moved = mv_pos >= r0 && mv_pos < r0 + nr && mv_src != mv_pos;
         T v[kIt];
         {
             const int q_src = mv_src >= 0 ? mv_src / rpc : 0;
             const uint32_t src = peer_base(q_src) + off_of(tile + (mv_src - q_src * rpc));
 #pragma unroll
             for (int k = 0; k < kIt; ++k) {
-                const int q = warp + NW * k, c = q < jb ? q : q + nbc;
-                const bool want = mv_src >= 0 && q < nother &&
-                                  ((top_row && c >= c1 && lane < sb) || (here && mv_src != mv_pos));
+                const int c = warp + NW * k;
+                const bool want =
+                    mv_src >= 0 && c < w && ((top_row && c >= jb && lane < sb) || moved);
                 v[k] = want ? peer_load(src + (uint32_t)(c * ldt * (int)sizeof(T)), T(0)) : T(0);
             }
         }
@@ -530,8 +463,9 @@ getf2_cluster_kernel(int m, int w, T* A, long long lda, int rpc, int* ipiv, int 
         if (top_row) {
 #pragma unroll
             for (int k = 0; k < kIt; ++k) {
-                const int q = warp + NW * k, c = q < jb ? q : q + nbc;
-                if (q < nother && c >= c1) sm.U[(c - c1) >> 1][lane][(c - c1) & 1] = v[k];
+                const int c = warp + NW * k;
+                if (c >= c1 && c < w) sm.U[(c - c1) >> 1][lane][(c - c1) & 1] = v[k];
+                else if (c >= jb && c < c1) sm.L[lane][c - jb] = v[k];
             }
         }
         __syncthreads();
@@ -544,7 +478,7 @@ getf2_cluster_kernel(int m, int w, T* A, long long lda, int rpc, int* ipiv, int 
             for (int r = 1; r < NB; ++r) {
                 if (r < sb) {
 #pragma unroll
-                    for (int k = 0; k < r; ++k) x[r] = fma_t(-sm.L[r][NB - r + k], x[k], x[r]);
+                    for (int k = 0; k < r; ++k) x[r] = fma_t(-sm.L[r][k], x[k], x[r]);
                 }
                 up[2 * r] = x[r];
             }
@@ -552,11 +486,10 @@ getf2_cluster_kernel(int m, int w, T* A, long long lda, int rpc, int* ipiv, int 
         cluster_wait();  // everybody has read: rows may change
 #pragma unroll
         for (int k = 0; k < kIt; ++k) {
-            const int q = warp + NW * k, c = q < jb ? q : q + nbc;
-            if (here && mv_src != mv_pos && q < nother && !(top_row && c >= c1))
-                tile[c * ldt + mv_pos - r0] = v[k];
+            const int c = warp + NW * k;
+            if (moved && c < w && !(top_row && c >= c1)) tile[c * ldt + mv_pos - r0] = v[k];
         }
-        if (own_j && c1 + tid < w) {
+        if (rank == owner && c1 + tid < w) {
 #pragma unroll
             for (int k = 0; k < NB; ++k)
                 if (k < sb) tile[(c1 + tid) * ldt + jb - r0 + k] = x[k];
@@ -570,6 +503,9 @@ getf2_cluster_kernel(int m, int w, T* A, long long lda, int rpc, int* ipiv, int 
             for (int i = 0; i < R; ++i) {
                 const int r = tid + TH * i;
                 if (r >= nr || r0 + r < jb + sb) continue;
+                T nl[NB];
+#pragma unroll
+                for (int k = 0; k < NB; ++k) nl[k] = -tile[(jb + k) * ldt + r];
                 T* xp = tile + c1 * ldt + r;
                 for (int c = 0; c + c1 < w; c += 2, xp += 2 * ldt) {
                     const bool two = c + 1 + c1 < w;
@@ -578,8 +514,8 @@ getf2_cluster_kernel(int m, int w, T* A, long long lda, int rpc, int* ipiv, int 
 #pragma unroll
                     for (int k = 0; k < NB; k += 2) {
                         const Vec4<T> u = up[k >> 1];
-                        acc.fma(P(-a[i][k], -a[i][k]), P(u.x[0], u.x[1]));
-                        acc.fma(P(-a[i][k + 1], -a[i][k + 1]), P(u.x[2], u.x[3]));
+                        acc.fma(P(nl[k], nl[k]), P(u.x[0], u.x[1]));
+                        acc.fma(P(nl[k + 1], nl[k + 1]), P(u.x[2], u.x[3]));
                     }
                     T x0, x1;
                     acc.get(x0, x1);

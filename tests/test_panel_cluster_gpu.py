@@ -84,3 +84,25 @@ def test_cluster_special_values(hd, handle, torch_cuda, case):
     np.testing.assert_array_equal(out[0][1], out[1][1])
     same = (out[0][0] == out[1][0]) | (torch_cuda.isnan(out[0][0]) & torch_cuda.isnan(out[1][0]))
     assert bool(same.all())
+
+
+def test_cluster_wait_limit(hd, handle, torch_cuda):
+    """With a limit of one poll the cluster's waits may run out; the call then
+    reports a timeout, and either way the handle factors correctly afterwards."""
+    A = clear_pivots(2048, 1, np.float32)
+    d, info = dev(torch_cuda, A), info_tensor(torch_cuda)
+    ipiv = torch_cuda.zeros(2048, dtype=torch_cuda.int32, device="cuda")
+    try:
+        handle.set_wait_limit(1)
+        hd.call("double_blocked_getrf", handle.ptr, ptr(d), 2048, 2048, 128, 128, 0, 0, ptr(ipiv),
+                ptr(info))
+        torch_cuda.cuda.synchronize()
+        assert handle.device_errors() in (0, 6)  # 6: timeout
+    finally:
+        handle.set_wait_limit(0)
+    got = factor(torch_cuda, hd, handle, A, 128)
+    handle.set_panel_kernel(1)
+    want = factor(torch_cuda, hd, handle, A, 128)
+    handle.set_panel_kernel(0)
+    np.testing.assert_array_equal(got[1], want[1])
+    assert torch_cuda.equal(got[0], want[0])
