@@ -6,17 +6,25 @@
 // work queue (largest work first, so the tail is short).  Each CTA factors its
 // matrix in place, right-looking with panels of PW columns:
 //   * the panel (all rows below the diagonal, PW columns) is copied into
-//     shared memory and factored there with two barriers per column -- the
-//     pivot search of column j+1 is fused into the rank-1 update of column j;
+//     shared memory and factored there.  Cholesky: sub-panels of 8 columns, whose
+//     diagonal block every thread factors in its own registers while it carries
+//     its rows along -- three barriers per 8 columns.  LU: sub-panels of 16
+//     columns in registers, one barrier per column; no row moves inside a
+//     sub-panel (a row carries its position), the interchanges follow as at most
+//     32 composed row moves;
 //   * LU: the panel's row interchanges are composed into at most 2 PW row
 //     moves and applied to the other columns with one gather / scatter per
-//     column (every load of a column before its first store);
-//   * the trailing update runs over 64-column chunks: the chunk's U12 block
-//     (LU: a unit-lower triangular solve against the panel's diagonal block,
-//     one thread per column) and then A22 -= L21 U12 (Cholesky: L21 L21^T,
-//     lower part only) with 8 x 4 register tiles fed by 128-bit shared loads;
-// then solves its right-hand side with blocked substitutions (one warp per
-// diagonal block, all threads on the off-diagonal block rows).
+//     column (every load of a column before its first store); U12 by one thread
+//     per column (unit-lower solve against the panel's diagonal block);
+//   * the trailing update A22 -= L21 U12 (Cholesky: L21 L21^T, lower part) in
+//     items of 128 rows x 8 columns per warp, packed FP32 FMAs, lanes on
+//     consecutive rows, so that C moves in whole 128-byte lines and no block
+//     barrier is needed (the earlier 8 x 4 tiles per thread scattered every
+//     access over 16 columns: 41% of the kernel's time at 13% of the FMA rate);
+//   * the right-hand side goes along as one more column (moves, solve against
+//     the diagonal block, update), so only the backward substitution is left:
+//     32-row blocks, one warp on the diagonal block with reciprocals ready, the
+//     other rows' entries loaded while it works.
 // The launch shape is a variant: threads per CTA and panel width; the
 // shared-memory footprint of the panel width sets the CTAs per SM.
 // No reference counterpart (the reference factors one matrix per call); the
@@ -29,6 +37,7 @@
 #include <vector>
 
 #include "internal.h"
+#include "tile64.cuh"
 #include "hdbf/batched.h"
 
 namespace hdbf {
@@ -37,8 +46,8 @@ namespace {
 constexpr int kMaxChol = 512;  // largest Cholesky order
 constexpr int kMaxLu = 768;    // largest LU order
 constexpr int kLdp = kMaxLu + 8;  // panel rows (padding for 8-row register tiles)
-constexpr int kChunk = 64;        // trailing-update columns per pass
-constexpr int kUbLd = kChunk + 4;
+constexpr int kNB = 16;           // LU sub-panel
+constexpr int kWC = 8;            // columns of a trailing-update item
 
 struct BatchArgs {
     int count;
@@ -53,127 +62,214 @@ struct BatchArgs {
     unsigned* queue;
 };
 
-// Shared-memory footprint (floats) for panel width PW.
-template <int PW>
-constexpr size_t smem_floats()
-{
-    return (size_t)kLdp * PW          // panel
-           + (size_t)PW * kUbLd       // U12 chunk
-           + (size_t)kMaxLu           // row map (factor) / solution (solve)
-           + (size_t)2 * PW * 2       // move list
-           + 2 * PW + 64;             // column scratch, reductions
-}
+// A warp's pivot candidate: magnitude bits, position, its sub-panel row.
+struct alignas(16) Cand {
+    unsigned mag;
+    int pos;
+    int pad[2];
+    float x[kNB];
+};
 
 template <int T, int PW>
 struct Smem {
-    float* P;      // panel P[c * kLdp + r], r relative to the panel's first row
-    float* Ub;     // U12 chunk Ub[q * kUbLd + c]
-    int* rowmap;   // LU: composed swaps of the panel (aliases x)
-    float* x;      // solve vector
-    int* mv;       // moves: mv[i] = source row, mv[2 PW + i] = target row
-    float* col;    // scaled column entries / dot products (2 PW)
-    float* rv;     // reductions (T / 32)
-    int* ri;
-    __device__ explicit Smem(float* sm)
-    {
-        P = sm;
-        Ub = P + (size_t)kLdp * PW;
-        x = Ub + (size_t)PW * kUbLd;
-        rowmap = reinterpret_cast<int*>(x);
-        mv = reinterpret_cast<int*>(x + kMaxLu);
-        col = reinterpret_cast<float*>(mv + 4 * PW);
-        rv = col + 2 * PW;
-        ri = reinterpret_cast<int*>(rv + 32);
-    }
+    static constexpr int kW = T / 32;
+    float P[(size_t)PW * kLdp];   // panel P[c * kLdp + r], r relative to the panel's first row
+    float Ub[kW * PW * kWC];      // a warp's columns of U12: [warp][q][c]
+    float x[kMaxLu];              // right-hand side / solution
+    Cand cand[2][kW];             // LU: the warps' candidates, by column parity
+    float U[kNB][kNB + 1];        // LU: U12 of the sub-panel inside the panel, U[c][k]
+    float dots[32];
+    int piv[PW];                  // LU: swap rows of the panel's columns
+    int item;
 };
 
-// (v, i) beats (bv, bi): a real row beats none, then larger |a|, then the
-// lower row (LAPACK ISAMAX returns the first maximum).
-__device__ __forceinline__ bool better(float v, int i, float bv, int bi)
+// Largest magnitude over the warp and the lowest position that has it.
+__device__ __forceinline__ void warp_argmax(unsigned vb, int pos, unsigned& mv, int& mp)
 {
-    if (i == INT_MAX) return false;
-    if (bi == INT_MAX) return true;
-    return v > bv || (v == bv && i < bi);
+    mv = __reduce_max_sync(0xffffffffu, vb);
+    mp = __reduce_min_sync(0xffffffffu, vb == mv ? pos : INT_MAX);
 }
-
-// Block-wide argmax of the per-thread candidates; every thread gets the row.
-template <int T>
-__device__ __forceinline__ int block_argmax(float v, int i, float* rv, int* ri)
+__device__ __forceinline__ unsigned long long pack2(float x, float y)
 {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, v, off);
-        const int oi = __shfl_xor_sync(0xffffffffu, i, off);
-        if (better(ov, oi, v, i)) { v = ov; i = oi; }
-    }
-    if ((threadIdx.x & 31) == 0) { rv[threadIdx.x >> 5] = v; ri[threadIdx.x >> 5] = i; }
-    __syncthreads();
-    v = rv[0];
-    i = ri[0];
-#pragma unroll
-    for (int w = 1; w < T / 32; ++w)
-        if (better(rv[w], ri[w], v, i)) { v = rv[w]; i = ri[w]; }
-    return i;
+    unsigned long long v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(x), "f"(y));
+    return v;
+}
+__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a,
+                                     unsigned long long b)
+{
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
 
 // ------------------------------------------------------------ panel kernels
-// Pivoted LU of the m x kb panel P (m rows from the diagonal down).  piv[j]
-// receives the panel row swapped with row j.  Returns the first zero-pivot
-// column + 1 (0: none); the factorization continues past it, as xGETF2.
-template <int T, int PW>
-__device__ int lu_panel(Smem<T, PW>& s, int m, int kb, int* piv)
+// Pivoted LU of the m x kb panel P (m rows from the diagonal down), kb a multiple
+// of kNB or the last panel.  piv[j] receives the panel row swapped with row j.
+// Returns the first zero-pivot column + 1 (0: none); the factorization continues
+// past it, as xGETF2.  P complete on entry and on return.  R rows per thread.
+template <int T, int PW, int R>
+__device__ __noinline__ int lu_panel_rows(Smem<T, PW>& s, int m, int kb)
 {
-    const int tid = threadIdx.x;
+    constexpr int NW = T / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int zero = 0;
-    // candidates of column 0
-    float bv = -1.f;
-    int bi = INT_MAX;
-    for (int r = tid; r < m; r += T) {
-        const float a = fabsf(s.P[r]);
-        if (bi == INT_MAX || a > bv) { bv = a; bi = r; }
-    }
-    for (int j = 0; j < kb; ++j) {
-        const int p = block_argmax<T>(bv, bi, s.rv, s.ri);  // barrier: column j final
-        if (tid == 0) piv[j] = p;
-        if (p != j && tid < kb) {
-            const float t = s.P[tid * kLdp + j];
-            s.P[tid * kLdp + j] = s.P[tid * kLdp + p];
-            s.P[tid * kLdp + p] = t;
+    const int steps = min(m, kb);
+    for (int jb = 0; jb < steps; jb += kNB) {
+        const int nbc = min(kNB, kb - jb), sb = min(nbc, steps - jb);
+        float a[R][kNB];
+        int pos[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int r = tid + T * i;
+            pos[i] = r < m ? r : -1;
+#pragma unroll
+            for (int c = 0; c < kNB; ++c)
+                a[i][c] = (r < m && c < nbc) ? s.P[(jb + c) * kLdp + r] : 0.f;
+        }
+#pragma unroll 1
+        for (int j = 0; j < sb; ++j) {
+            const int J = jb + j, par = J & 1;
+            unsigned vb = 0;
+            int best = INT_MAX;
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const float v = fabsf(a[i][0]);
+                const unsigned b = v == v ? __float_as_uint(v) : 0u;  // a NaN loses
+                if (pos[i] >= J &&
+                    (best == INT_MAX || b > vb || (b == vb && pos[i] < best))) {
+                    vb = b;
+                    best = pos[i];
+                }
+            }
+            unsigned mv;
+            int mp;
+            warp_argmax(vb, best, mv, mp);
+            if (best == mp && (best != INT_MAX || lane == 0)) {
+                Cand& c = s.cand[par][warp];
+                c.mag = mv;
+                c.pos = mp;
+#pragma unroll
+                for (int i = 0; i < R; ++i)
+                    if (R == 1 || pos[i] == mp) {
+#pragma unroll
+                        for (int q = 0; q < kNB; ++q) c.x[q] = a[i][q];
+                    }
+            }
+            __syncthreads();
+            unsigned k = 0;
+            int kp = INT_MAX;
+            if (lane < NW) {
+                const uint2 key = *reinterpret_cast<const uint2*>(&s.cand[par][lane]);
+                k = key.x;
+                kp = (int)key.y;
+            }
+            warp_argmax(k, kp, mv, mp);
+            const int from = __ffs(__ballot_sync(0xffffffffu, lane < NW && kp == mp)) - 1;
+            const float* urow = s.cand[par][from].x;
+            float u[kNB];
+#pragma unroll
+            for (int c = 0; c < kNB; ++c) u[c] = urow[c];
+            const float pv = u[0];
+            if (pv == 0.f && zero == 0) zero = J + 1;
+            const float rcp = 1.0f / pv;
+            const bool plain = fabsf(pv) >= FLT_MIN || pv != pv;
+            if (tid == T - 1) s.piv[J] = mp;
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                float l = a[i][0] * rcp;
+                if (!plain) l = pv != 0.f ? a[i][0] / pv : a[i][0];
+                float* x = s.P + J * kLdp + tid + T * i;
+                if (pos[i] == mp) {  // the pivot row: its U entries, in place
+#pragma unroll
+                    for (int c = 0; c < kNB; ++c)
+                        if (c < nbc - j) x[c * kLdp] = u[c];
+                    pos[i] = J;
+                } else if (pos[i] == J) {
+                    pos[i] = mp;
+                }
+                if (pos[i] > J) x[0] = l;
+#pragma unroll
+                for (int c = 1; c < kNB; ++c) a[i][c - 1] = fmaf(-l, u[c], a[i][c]);
+                a[i][kNB - 1] = 0.f;
+            }
         }
         __syncthreads();
-        const float pv = s.P[j * kLdp + j];
-        if (pv == 0.f && zero == 0) zero = j + 1;
-        const bool recip = fabsf(pv) >= FLT_MIN;
-        const float rcp = 1.0f / pv;
-        // scale column j, update columns j+1.. of the own rows, candidates of
-        // column j+1 on the way
-        bv = -1.f;
-        bi = INT_MAX;
-        for (int r = j + 1 + tid; r < m; r += T) {
-            float l = s.P[j * kLdp + r];
-            if (pv != 0.f) {
-                l = recip ? l * rcp : l / pv;
-                s.P[j * kLdp + r] = l;
-            }
-            for (int c = j + 1; c < kb; ++c)
-                s.P[c * kLdp + r] = fmaf(-l, s.P[c * kLdp + j], s.P[c * kLdp + r]);
-            if (j + 1 < kb) {
-                const float a = fabsf(s.P[(j + 1) * kLdp + r]);
-                if (bi == INT_MAX || a > bv) { bv = a; bi = r; }
+        // The sub-panel's interchanges on all panel columns, composed: lanes <
+        // kNB are its diagonal positions, the others the pivot positions; the
+        // row that ends up at mv_pos is found by undoing the swaps.
+        int mv_pos = lane < kNB ? jb + lane : (lane < kNB + sb ? s.piv[jb + lane - kNB] : -1);
+        if (lane < kNB ? lane >= sb : mv_pos < jb + kNB) mv_pos = -1;
+        int mv_src = mv_pos;
+        for (int t = sb - 1; t >= 0; --t) {
+            const int q = s.piv[jb + t];
+            mv_src = mv_src == jb + t ? q : (mv_src == q ? jb + t : mv_src);
+        }
+        constexpr int kIt = (PW + NW - 1) / NW;
+        float v[kIt];
+#pragma unroll
+        for (int q = 0; q < kIt; ++q) {
+            const int c = warp + NW * q;
+            v[q] = (c < kb && mv_pos >= 0) ? s.P[c * kLdp + mv_src] : 0.f;
+        }
+        __syncwarp();  // a column's rows belong to one warp
+#pragma unroll
+        for (int q = 0; q < kIt; ++q) {
+            const int c = warp + NW * q;
+            if (c < kb && mv_pos >= 0) s.P[c * kLdp + mv_pos] = v[q];
+        }
+        __syncthreads();
+        const int c1 = jb + nbc;
+        if (c1 >= kb || jb + sb >= m) continue;
+        // U12 of the panel's remaining columns (at most kNB), a thread each
+        if (c1 + tid < kb) {
+            float x[kNB];
+            float* col = s.P + (c1 + tid) * kLdp + jb;
+#pragma unroll
+            for (int k = 0; k < kNB; ++k) x[k] = col[k];
+#pragma unroll
+            for (int k = 0; k < kNB; ++k)
+#pragma unroll
+                for (int r = k + 1; r < kNB; ++r)
+                    x[r] = fmaf(-s.P[(jb + k) * kLdp + jb + r], x[k], x[r]);
+#pragma unroll
+            for (int k = 0; k < kNB; ++k) s.U[tid][k] = col[k] = x[k];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int r = tid + T * i;
+            if (r >= m || r < jb + kNB) continue;
+            float l[kNB];
+#pragma unroll
+            for (int k = 0; k < kNB; ++k) l[k] = -s.P[(jb + k) * kLdp + r];
+            for (int c = 0; c < kb - c1; ++c) {
+                float x = s.P[(c1 + c) * kLdp + r];
+#pragma unroll
+                for (int k = 0; k < kNB; ++k) x = fmaf(l[k], s.U[c][k], x);
+                s.P[(c1 + c) * kLdp + r] = x;
             }
         }
+        __syncthreads();
     }
-    __syncthreads();
     return zero;
 }
 
-// Cholesky of the m x kb panel P (diagonal block on top): the first failing
-// column + 1, or 0.  Columns past a failure are left as they are.
 template <int T, int PW>
-__device__ int chol_panel(Smem<T, PW>& s, int m, int kb)
+__device__ __forceinline__ int lu_panel(Smem<T, PW>& s, int m, int kb)
+{
+    constexpr int kAll = (kMaxLu + T - 1) / T;
+    if (m <= T) return lu_panel_rows<T, PW, 1>(s, m, kb);
+    if (kAll > 2 && m <= 2 * T) return lu_panel_rows<T, PW, 2>(s, m, kb);
+    return lu_panel_rows<T, PW, kAll>(s, m, kb);
+}
+
+// Cholesky of the m x kb panel P (diagonal block on top) from column j0 on, a
+// column at a time with IEEE operations: the first failing column + 1, or 0.
+// Columns past a failure are left as they are.
+template <int T, int PW>
+__device__ __noinline__ int chol_panel_careful(Smem<T, PW>& s, int m, int kb, int j0)
 {
     const int tid = threadIdx.x;
-    for (int j = 0; j < kb; ++j) {
+    for (int j = j0; j < kb; ++j) {
         const float d = s.P[j * kLdp + j];  // final: updated before the last barrier
         if (!(d > 0.f)) return j + 1;       // uniform: every thread read the same value
         const float sd = sqrtf(d);
@@ -181,7 +277,7 @@ __device__ int chol_panel(Smem<T, PW>& s, int m, int kb)
         for (int r = j + 1 + tid; r < m; r += T) {
             const float l = s.P[j * kLdp + r] * rcp;
             s.P[j * kLdp + r] = l;
-            if (r < kb) s.col[r] = l;
+            if (r < kb) s.dots[r] = l;
         }
         __syncthreads();
         if (tid == 0) s.P[j * kLdp + j] = sd;
@@ -189,170 +285,320 @@ __device__ int chol_panel(Smem<T, PW>& s, int m, int kb)
             const float l = s.P[j * kLdp + r];
             const int cmax = min(kb - 1, r);
             for (int c = j + 1; c <= cmax; ++c)
-                s.P[c * kLdp + r] = fmaf(-l, s.col[c], s.P[c * kLdp + r]);
+                s.P[c * kLdp + r] = fmaf(-l, s.dots[c], s.P[c * kLdp + r]);
         }
         __syncthreads();
     }
     return 0;
 }
 
-// P (m x kb) <-> global A at the panel's top-left corner (element e is row
-// e % m of column e / m: coalesced), eight loads in flight per thread.
-template <int T, int PW, bool TO_SMEM>
-__device__ __forceinline__ void move_panel(Smem<T, PW>& s, float* A, long long lda, int m, int kb)
+// The same in sub-panels of 8 columns: every thread factors the 8 x 8 diagonal
+// block in registers and solves its own rows against it, then updates the panel's
+// remaining columns of those rows.  A sub-panel with a pivot outside the fast
+// range (failed, tiny, huge, NaN) and the rest of the panel go the careful way.
+// P complete on entry and on return; a last panel that is no multiple of 8 is
+// padded with the identity.
+template <int T, int PW>
+__device__ int chol_panel(Smem<T, PW>& s, int m, int kb)
 {
-    const int total = m * kb;
-    int e = threadIdx.x;
-    for (; e + 7 * T < total; e += 8 * T) {
-        float v[8];
+    constexpr int W = 8;
+    constexpr int R = (kMaxChol + T - 1) / T;
+    const int tid = threadIdx.x;
+    for (int jb = 0; jb < kb; jb += W) {
+        float D[W][W];  // D[c][r], r >= c
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int q = e + u * T, c = q / m, r = q - c * m;
-            v[u] = TO_SMEM ? A[(long long)c * lda + r] : s.P[c * kLdp + r];
+        for (int c = 0; c < W; ++c)
+#pragma unroll
+            for (int r = c; r < W; ++r)
+                D[c][r] = (jb + r < kb) ? s.P[(jb + c) * kLdp + jb + r] : (r == c ? 1.f : 0.f);
+        bool ok = true;
+        float rs[W];
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+            ok = ok & tile64::fast_range(D[j][j]);
+            tile64::rsqrt_pair(D[j][j], rs[j], D[j][j]);
+#pragma unroll
+            for (int r = j + 1; r < W; ++r) D[j][r] *= rs[j];
+#pragma unroll
+            for (int c = j + 1; c < W; ++c)
+#pragma unroll
+                for (int r = c; r < W; ++r) D[c][r] = fmaf(-D[j][r], D[j][c], D[c][r]);
         }
+        if (__syncthreads_or(!ok)) return chol_panel_careful<T, PW>(s, m, kb, jb);
+        if (tid == T - 1) {
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int q = e + u * T, c = q / m, r = q - c * m;
-            if (TO_SMEM) s.P[c * kLdp + r] = v[u];
-            else A[(long long)c * lda + r] = v[u];
+            for (int c = 0; c < W; ++c)
+#pragma unroll
+                for (int r = c; r < W; ++r)
+                    if (jb + r < kb) s.P[(jb + c) * kLdp + jb + r] = D[c][r];
+        }
+        if (jb + W >= m) break;
+        float x[R][W];
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int r = jb + W + tid + T * i;
+            if (r >= m) continue;
+#pragma unroll
+            for (int c = 0; c < W; ++c) x[i][c] = s.P[(jb + c) * kLdp + r];
+#pragma unroll
+            for (int j = 0; j < W; ++j) {
+                x[i][j] *= rs[j];
+#pragma unroll
+                for (int c = j + 1; c < W; ++c) x[i][c] = fmaf(-x[i][j], D[j][c], x[i][c]);
+            }
+#pragma unroll
+            for (int c = 0; c < W; ++c) s.P[(jb + c) * kLdp + r] = x[i][c];
+        }
+        __syncthreads();
+        if (jb + W < kb) {
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const int r = jb + W + tid + T * i;
+                if (r >= m) continue;
+                for (int c = jb + W; c < kb; c += 4) {  // four columns (rows of L) at a time
+                    if (c > r) break;
+                    float y[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) y[e] = c + e < kb ? s.P[(c + e) * kLdp + r] : 0.f;
+#pragma unroll
+                    for (int k = 0; k < W; ++k) {
+                        const float4 l = *reinterpret_cast<const float4*>(s.P + (jb + k) * kLdp + c);
+                        y[0] = fmaf(-x[i][k], l.x, y[0]);
+                        y[1] = fmaf(-x[i][k], l.y, y[1]);
+                        y[2] = fmaf(-x[i][k], l.z, y[2]);
+                        y[3] = fmaf(-x[i][k], l.w, y[3]);
+                    }
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (c + e < kb && c + e <= r) s.P[(c + e) * kLdp + r] = y[e];
+                }
+            }
+            __syncthreads();
         }
     }
-    for (; e < total; e += T) {
-        const int c = e / m, r = e - c * m;
-        if (TO_SMEM) s.P[c * kLdp + r] = A[(long long)c * lda + r];
-        else A[(long long)c * lda + r] = s.P[c * kLdp + r];
+    __syncthreads();
+    return 0;
+}
+
+// P (m x kb) <-> global A at the panel's top-left corner, a warp per column,
+// eight loads in flight per lane; lower: only rows r >= c are stored.
+template <int T, int PW, bool TO_SMEM>
+__device__ __forceinline__ void move_panel(Smem<T, PW>& s, float* A, long long lda, int m, int kb,
+                                           bool lower)
+{
+    const int lane = threadIdx.x & 31;
+    for (int c = threadIdx.x >> 5; c < kb; c += T / 32) {
+        float* g = A + (long long)c * lda;
+        float* p = s.P + c * kLdp;
+        for (int r0 = lower ? c / 32 * 32 : 0; r0 < m; r0 += 256) {
+            float v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int r = r0 + lane + 32 * u;
+                v[u] = r < m ? (TO_SMEM ? g[r] : p[r]) : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int r = r0 + lane + 32 * u;
+                if (r < m && (!lower || r >= c)) (TO_SMEM ? p[r] : g[r]) = v[u];
+            }
+        }
     }
 }
 
 // --------------------------------------------------------- trailing update
-// C(rows x cw) -= Aop(rows x kb) * Bop(kb x cw): Aop(r, q) = P[q * kLdp + a0 + r],
-// Bop(q, c) = bsrc[q * bld + c], C(r, c) = C[c * ldc + r] in global memory.
-// 8 x 4 register tiles: T/16 row groups x 16 column groups of 4 (64 columns);
-// with `lower` only entries with r + diag >= c are written (diag: the offset
-// of C's rows against its columns).  a0, bld and kb are multiples of 4.
-template <int T, int PW>
-__device__ __forceinline__ void update_chunk(const Smem<T, PW>& s, int a0, int rows, int kb,
-                                             const float* bsrc, int bld, int cw, float* C,
-                                             long long ldc, bool lower, int diag)
+// One item: rows r0 + lane + 32 i (i < RI) x 8 columns, C -= A B with A(r, q) =
+// a[q * kLdp + r] (shared) and B(q, c) = b[q * ldb + c] (shared, 16-byte aligned
+// rows).  lower: only entries with r >= c0 + column are touched.
+template <int RI, int PW>
+__device__ __forceinline__ void update_item(const float* a, const float* b, int ldb, int kb, float* C,
+                                            long long ldc, int r0, int rows, int c0, int cols,
+                                            bool lower)
 {
-    constexpr int TY = T / 16;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int first = lower ? max(0, ((0 - diag) / 8) * 8) : 0;
-    for (int rb = first; rb < rows; rb += TY * 8) {
-        const int r = rb + ty * 8;
-        if (r >= rows) continue;
-        if (lower && r + 7 + diag < tx * 4) continue;  // tile wholly above the diagonal
-        float acc[8][4] = {};
-        const float* ap = s.P + a0 + r;
-        for (int q = 0; q < kb; ++q) {
-            const float4 x0 = *reinterpret_cast<const float4*>(ap + q * kLdp);
-            const float4 x1 = *reinterpret_cast<const float4*>(ap + q * kLdp + 4);
-            const float4 y = *reinterpret_cast<const float4*>(bsrc + q * bld + tx * 4);
-            const float av[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-            const float bv[4] = {y.x, y.y, y.z, y.w};
+    const int lane = threadIdx.x & 31;
+    float old[RI][kWC];
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
+    for (int c = 0; c < kWC; ++c)
 #pragma unroll
-                for (int v = 0; v < 4; ++v) acc[u][v] = fmaf(av[u], bv[v], acc[u][v]);
+        for (int i = 0; i < RI; ++i) {
+            const int r = r0 + lane + 32 * i;
+            old[i][c] = (c0 + c < cols && r < rows && (!lower || r >= c0 + c))
+                            ? C[(long long)(c0 + c) * ldc + r]
+                            : 0.f;
         }
-        float old[8][4];  // every load of the tile before its first store
+    unsigned long long acc[RI][kWC / 2];
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const int c = tx * 4 + v;
+    for (int i = 0; i < RI; ++i)
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int rr = r + u;
-                const bool ok = c < cw && rr < rows && (!lower || rr + diag >= c);
-                old[u][v] = ok ? C[(long long)c * ldc + rr] : 0.f;
-            }
-        }
+        for (int c = 0; c < kWC / 2; ++c) acc[i][c] = 0ull;
+    a += r0 + lane;
+#pragma unroll 4
+    for (int q = 0; q < kb; ++q) {
+        const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(b + q * ldb);
+        const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(b + q * ldb + 4);
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const int c = tx * 4 + v;
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int rr = r + u;
-                if (c < cw && rr < rows && (!lower || rr + diag >= c))
-                    C[(long long)c * ldc + rr] = old[u][v] - acc[u][v];
-            }
+        for (int i = 0; i < RI; ++i) {
+            const float x = a[q * kLdp + 32 * i];
+            const unsigned long long xx = pack2(x, x);
+            fma2(acc[i][0], xx, b0.x);
+            fma2(acc[i][1], xx, b0.y);
+            fma2(acc[i][2], xx, b1.x);
+            fma2(acc[i][3], xx, b1.y);
         }
     }
+#pragma unroll
+    for (int c = 0; c < kWC; ++c)
+#pragma unroll
+        for (int i = 0; i < RI; ++i) {
+            const int r = r0 + lane + 32 * i;
+            float lo, hi;
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[i][c >> 1]));
+            if (c0 + c < cols && r < rows && (!lower || r >= c0 + c))
+                C[(long long)(c0 + c) * ldc + r] = old[i][c] - ((c & 1) ? hi : lo);
+        }
+}
+
+// C (n2 x n2) -= L21 B over all items, warps in turn.  LU: B = U12 in global
+// memory (kb rows above C), copied to the warp's own buffer per item; Cholesky: B
+// = L21^T from the panel, lower part only.
+template <int T, int PW>
+__device__ __forceinline__ void trailing_update(Smem<T, PW>& s, int kb, int n2, float* C,
+                                                long long ldc, bool lower)
+{
+    constexpr int NW = T / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int groups = (n2 + kWC - 1) / kWC, blocks = (n2 + 127) / 128;
+    float* ub = s.Ub + warp * PW * kWC;
+    for (int it = warp; it < groups * blocks; it += NW) {
+        const int g = it % groups, blk = it / groups;
+        const int c0 = g * kWC, end = min(n2, 128 * blk + 128);
+        int r0 = 128 * blk;
+        if (lower) r0 = max(r0, c0 / 32 * 32);
+        if (r0 >= end) continue;
+        const float* b = s.P + kb + c0;
+        int ldb = kLdp;
+        if (!lower) {
+            float v[PW * kWC / 32];
+#pragma unroll
+            for (int u = 0; u < PW * kWC / 32; ++u) {
+                const int e = lane + 32 * u, c = e / PW, q = e % PW;
+                v[u] = (c0 + c < n2 && q < kb) ? C[(long long)(c0 + c) * ldc - kb + q] : 0.f;
+            }
+            __syncwarp();  // the previous item's reads are done
+#pragma unroll
+            for (int u = 0; u < PW * kWC / 32; ++u) {
+                const int e = lane + 32 * u, c = e / PW, q = e % PW;
+                ub[q * kWC + c] = v[u];
+            }
+            __syncwarp();
+            b = ub;
+            ldb = kWC;
+        }
+        const float* a = s.P + kb;
+        const int left = end - r0;
+        if (left > 64) update_item<4, PW>(a, b, ldb, kb, C, ldc, r0, end, c0, n2, lower);
+        else if (left > 32) update_item<2, PW>(a, b, ldb, kb, C, ldc, r0, end, c0, n2, lower);
+        else update_item<1, PW>(a, b, ldb, kb, C, ldc, r0, end, c0, n2, lower);
+    }
+}
+
+// x2 -= L21 x1 for the right-hand side (x1 the panel's kb entries, solved).
+template <int T, int PW>
+__device__ __forceinline__ void rhs_update(Smem<T, PW>& s, int k, int kb, int m)
+{
+    for (int r = kb + threadIdx.x; r < m; r += T) {
+        float acc = s.x[k + r];
+#pragma unroll 8
+        for (int q = 0; q < kb; ++q) acc = fmaf(-s.P[q * kLdp + r], s.x[k + q], acc);
+        s.x[k + r] = acc;
+    }
+}
+
+// x1 <- L11^{-1} x1 on one warp (unit: implicit ones on the diagonal).
+template <int T, int PW>
+__device__ __forceinline__ void rhs_solve(Smem<T, PW>& s, int k, int kb, bool unit)
+{
+    const int i = threadIdx.x & 31;
+    float li[PW];
+#pragma unroll
+    for (int q = 0; q < PW; ++q) li[q] = (i < kb && q < i) ? s.P[q * kLdp + i] : 0.f;
+    const float rd = (i < kb && !unit) ? 1.f / s.P[i * kLdp + i] : 1.f;
+    float xi = i < kb ? s.x[k + i] : 0.f;
+#pragma unroll
+    for (int q = 0; q < PW; ++q) {
+        const float xq = __shfl_sync(0xffffffffu, xi * rd, q);
+        xi = i > q ? fmaf(-li[q], xq, xi) : xi;
+    }
+    if (i < kb) s.x[k + i] = xi * rd;
 }
 
 // ------------------------------------------------------------------ LU
 template <int T, int PW>
 __device__ int lu_factor(Smem<T, PW>& s, float* A, int n, long long lda, int* ipiv)
 {
-    const int tid = threadIdx.x;
-    const int lane = tid & 31, warp = tid >> 5;
-    __shared__ int s_piv[PW];
-    __shared__ int s_nm;
+    constexpr int NW = T / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int info = 0;
     for (int k = 0; k < n; k += PW) {
         const int kb = min(PW, n - k), m = n - k;
         float* Ak = A + (long long)k * lda + k;  // panel's top-left corner
-        move_panel<T, PW, true>(s, Ak, lda, m, kb);
+        move_panel<T, PW, true>(s, Ak, lda, m, kb, false);
         __syncthreads();
-        const int z = lu_panel<T, PW>(s, m, kb, s_piv);
+        const int z = lu_panel<T, PW>(s, m, kb);
         if (z && !info) info = k + z;
-        move_panel<T, PW, false>(s, Ak, lda, m, kb);
-        // compose the panel's interchanges into moves (panel rows)
-        for (int r = tid; r < m; r += T) s.rowmap[r] = r;
-        if (tid == 0) s_nm = 0;
-        __syncthreads();
-        if (tid == 0)
-            for (int j = 0; j < kb; ++j) {
-                const int p = s_piv[j];
-                ipiv[k + j] = k + p + 1;
-                const int t = s.rowmap[j];
-                s.rowmap[j] = s.rowmap[p];
-                s.rowmap[p] = t;
-            }
-        __syncthreads();
-        if (tid < 2 * kb) {  // candidate rows j and piv[j]; the first occurrence adds its move
-            const int t = tid < kb ? tid : s_piv[tid - kb];
-            bool first = true;
-            for (int q = 0; q < tid; ++q)
-                if ((q < kb ? q : s_piv[q - kb]) == t) first = false;
-            if (first && s.rowmap[t] != t) {
-                const int q = atomicAdd(&s_nm, 1);
-                s.mv[q] = s.rowmap[t];
-                s.mv[2 * PW + q] = t;
-            }
+        move_panel<T, PW, false>(s, Ak, lda, m, kb, false);
+        if (tid < kb) ipiv[k + tid] = k + s.piv[tid] + 1;
+        // The panel's interchanges as row moves: two per lane, into diagonal
+        // position `lane` and into the pivot position of column `lane`; the
+        // source is found by undoing the swaps (a position that appears twice
+        // gets the same row twice).
+        int t0 = lane < kb ? lane : -1, t1 = lane < kb ? s.piv[lane] : -1;
+        if (t1 < kb) t1 = -1;
+        int s0 = t0, s1 = t1;
+        for (int t = kb - 1; t >= 0; --t) {
+            const int q = s.piv[t];
+            s0 = s0 == t ? q : (s0 == q ? t : s0);
+            s1 = s1 == t ? q : (s1 == q ? t : s1);
         }
-        __syncthreads();
-        const int nm = s_nm;
-        // apply the moves to the columns left and right of the panel: one warp
-        // per column, four columns per pass, every source of a column read
-        // before any of its targets is written
-        const int src0 = lane < nm ? s.mv[lane] : 0, src1 = lane + 32 < nm ? s.mv[lane + 32] : 0;
-        const int tgt0 = lane < nm ? s.mv[2 * PW + lane] : 0;
-        const int tgt1 = lane + 32 < nm ? s.mv[2 * PW + lane + 32] : 0;
-        for (int c = warp; c < n - kb; c += 4 * (T / 32)) {
-            float v0[4], v1[4];
+        const bool m0 = t0 != s0, m1 = t1 != s1;
+        // apply them to the columns left and right of the panel: one warp per
+        // column, eight columns per pass, every source of a column read before
+        // any of its targets is written
+        constexpr int kPass = 8;
+        for (int c = warp; c < n - kb; c += kPass * NW) {
+            float v0[kPass], v1[kPass];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int cu = c + u * (T / 32);
+            for (int u = 0; u < kPass; ++u) {
+                const int cu = c + u * NW;
                 v0[u] = v1[u] = 0.f;
                 if (cu < n - kb) {
                     const float* Ac = A + (long long)(cu < k ? cu : cu + kb) * lda + k;
-                    if (lane < nm) v0[u] = Ac[src0];
-                    if (lane + 32 < nm) v1[u] = Ac[src1];
+                    if (m0) v0[u] = Ac[s0];
+                    if (m1) v1[u] = Ac[s1];
                 }
             }
             __syncwarp();
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int cu = c + u * (T / 32);
+            for (int u = 0; u < kPass; ++u) {
+                const int cu = c + u * NW;
                 if (cu < n - kb) {
                     float* Ac = A + (long long)(cu < k ? cu : cu + kb) * lda + k;
-                    if (lane < nm) Ac[tgt0] = v0[u];
-                    if (lane + 32 < nm) Ac[tgt1] = v1[u];
+                    if (m0) Ac[t0] = v0[u];
+                    if (m1) Ac[t1] = v1[u];
                 }
             }
         }
+        if (warp == NW - 1) {  // and to the right-hand side, then L11^{-1} on it
+            const float v0 = m0 ? s.x[k + s0] : 0.f, v1 = m1 ? s.x[k + s1] : 0.f;
+            __syncwarp();
+            if (m0) s.x[k + t0] = v0;
+            if (m1) s.x[k + t1] = v1;
+            __syncwarp();
+            rhs_solve<T, PW>(s, k, kb, true);
+        }
         __syncthreads();
         const int m2 = m - kb;  // trailing rows / columns
+        rhs_update<T, PW>(s, k, kb, m);
         // U12 = L11^{-1} A12 (unit lower) for every trailing column at once,
         // one thread per column
         for (int c = tid; c < m2; c += T) {
@@ -369,28 +615,8 @@ __device__ int lu_factor(Smem<T, PW>& s, float* A, int n, long long lda, int* ip
                 if (q < kb) colp[q] = xv[q];
         }
         __syncthreads();
-        for (int c0 = 0; c0 < m2; c0 += kChunk) {
-            const int cw = min(kChunk, m2 - c0);
-            // the chunk's U12 block into shared memory, all loads in flight
-            constexpr int kPer = (PW * kChunk + T - 1) / T;
-            float v[kPer];
-#pragma unroll
-            for (int u = 0; u < kPer; ++u) {
-                const int e = threadIdx.x + u * T, c = e / PW, q = e - c * PW;
-                v[u] = (e < PW * kChunk && c < cw && q < kb)
-                           ? A[(long long)(k + kb + c0 + c) * lda + k + q]
-                           : 0.f;
-            }
-#pragma unroll
-            for (int u = 0; u < kPer; ++u) {
-                const int e = threadIdx.x + u * T, c = e / PW, q = e - c * PW;
-                if (e < PW * kChunk) s.Ub[q * kUbLd + c] = v[u];
-            }
-            __syncthreads();
-            update_chunk<T, PW>(s, kb, m2, kb, s.Ub, kUbLd, cw,
-                                A + (long long)(k + kb + c0) * lda + k + kb, lda, false, 0);
-            __syncthreads();
-        }
+        trailing_update<T, PW>(s, kb, m2, A + (long long)(k + kb) * lda + k + kb, lda, false);
+        __syncthreads();
     }
     return info;
 }
@@ -402,114 +628,88 @@ __device__ int chol_factor(Smem<T, PW>& s, float* A, int n, long long lda)
     for (int k = 0; k < n; k += PW) {
         const int kb = min(PW, n - k), m = n - k;
         float* Ak = A + (long long)k * lda + k;
-        move_panel<T, PW, true>(s, Ak, lda, m, kb);
+        move_panel<T, PW, true>(s, Ak, lda, m, kb, false);
         __syncthreads();
         const int f = chol_panel<T, PW>(s, m, kb);
-        // write back the lower part (the strictly upper part of the diagonal
-        // block keeps its input values)
-        for (int c = 0; c < kb; ++c)
-            for (int r = c + threadIdx.x; r < m; r += T) Ak[(long long)c * lda + r] = s.P[c * kLdp + r];
+        // the strictly upper part of the diagonal block keeps its input values
+        move_panel<T, PW, false>(s, Ak, lda, m, kb, true);
         if (f) {
-            if (threadIdx.x == 0) {
-                // the failing column's diagonal keeps the updated value, as xPOTRF
-                Ak[(long long)(f - 1) * lda + f - 1] = s.P[(f - 1) * kLdp + f - 1];
-            }
             __syncthreads();
             return k + f;
         }
+        if (threadIdx.x >= T - 32) rhs_solve<T, PW>(s, k, kb, false);
         __syncthreads();
-        const int m2 = m - kb;
-        for (int c0 = 0; c0 < m2; c0 += kChunk) {
-            const int cw = min(kChunk, m2 - c0);
-            // rows c0.. of the trailing block, columns c0 .. c0+cw, lower part
-            update_chunk<T, PW>(s, kb + c0, m2 - c0, kb, s.P + kb + c0, kLdp, cw,
-                                A + (long long)(k + kb + c0) * lda + k + kb + c0, lda, true, 0);
-        }
+        rhs_update<T, PW>(s, k, kb, m);
+        trailing_update<T, PW>(s, kb, m - kb, A + (long long)(k + kb) * lda + k + kb, lda, true);
         __syncthreads();
     }
     return 0;
 }
 
 // ------------------------------------------------------------------ solves
-// Blocked substitutions on x (shared memory): warp 0 solves each PW x PW
-// diagonal block with shuffles (the block's entries prefetched into
-// registers), then all threads update the remaining rows with the block's
-// columns (coalesced column reads).
+// Backward substitutions on x (shared memory), 32 rows at a time.  The panel's
+// shared memory holds the diagonal blocks D[r * 33 + c] of the current and the
+// next step.
+constexpr int kBk = 32;
 
-// x <- L^{-1} x, L lower (unit diagonal when `unit`), column-major in A.
-template <int T, int PW>
-__device__ void forward_lower(const float* A, int n, long long lda, float* x, bool unit)
+// The diagonal block at k (kb rows) into D by all threads; entries outside the
+// triangle are not used.
+template <int T>
+__device__ __forceinline__ void load_block(float* D, const float* A, long long lda, int k, int kb)
 {
-    const int tid = threadIdx.x, lane = tid & 31;
-    for (int k = 0; k < n; k += PW) {
-        const int kb = min(PW, n - k);
-        if (tid < 32) {
-            for (int h = 0; h < PW; h += 32) {  // PW <= 32: one pass
-                const int i = h + lane;
-                float li[PW];
-#pragma unroll
-                for (int q = 0; q < PW; ++q)
-                    li[q] = (i < kb && q <= i && q < kb) ? A[(long long)(k + q) * lda + k + i] : 0.f;
-                float xi = i < kb ? x[k + i] : 0.f;
-#pragma unroll
-                for (int q = 0; q < PW; ++q) {
-                    if (q < kb) {
-                        if (!unit && i == q) xi = xi / li[q];
-                        const float xq = __shfl_sync(0xffffffffu, xi, q);
-                        if (i > q) xi = fmaf(-li[q], xq, xi);
-                    }
-                }
-                if (i < kb) x[k + i] = xi;
-            }
-        }
-        __syncthreads();
-        for (int r = k + kb + tid; r < n; r += T) {
-            float a[PW];  // the row's block entries, all loads in flight together
-#pragma unroll
-            for (int q = 0; q < PW; ++q) a[q] = q < kb ? A[(long long)(k + q) * lda + r] : 0.f;
-            float acc = x[r];
-#pragma unroll
-            for (int q = 0; q < PW; ++q)
-                if (q < kb) acc = fmaf(-a[q], x[k + q], acc);
-            x[r] = acc;
-        }
-        __syncthreads();
+    for (int q = threadIdx.x; q < kBk * kBk; q += T) {
+        const int c = q >> 5, r = q & 31;
+        if (r < kb && c < kb) D[r * 33 + c] = A[(long long)(k + c) * lda + k + r];
     }
 }
 
-// x <- U^{-1} x, U the upper triangle of A (non-unit).
-template <int T, int PW>
-__device__ void backward_upper(const float* A, int n, long long lda, float* x)
+// x1 <- D^{-1} x1 on one warp, D upper, or lower and transposed.
+template <bool TRANS>
+__device__ __forceinline__ void block_back(const float* D, float* x, int kb, const float* sub)
 {
-    const int tid = threadIdx.x, lane = tid & 31;
-    const int nblk = (n + PW - 1) / PW;
+    const int i = threadIdx.x & 31;
+    float d[kBk];
+#pragma unroll
+    for (int q = 0; q < kBk; ++q)
+        d[q] = (i < kb && q > i && q < kb) ? (TRANS ? D[q * 33 + i] : D[i * 33 + q]) : 0.f;
+    const float rd = i < kb ? 1.f / D[i * 33 + i] : 1.f;
+    float xi = i < kb ? x[i] - (sub ? sub[i] : 0.f) : 0.f;
+#pragma unroll
+    for (int q = kBk - 1; q >= 0; --q) {
+        const float xq = __shfl_sync(0xffffffffu, xi * rd, q);
+        xi = i < q ? fmaf(-d[q], xq, xi) : xi;
+    }
+    if (i < kb) x[i] = xi * rd;
+}
+
+// x <- U^{-1} x, U the upper triangle of A (non-unit): the block's columns of the
+// rows above are loaded while one warp solves the diagonal block.
+template <int T>
+__device__ void backward_upper(const float* A, int n, long long lda, float* x, float* D)
+{
+    const int tid = threadIdx.x;
+    const int nblk = (n + kBk - 1) / kBk;
+    load_block<T>(D + ((nblk - 1) & 1) * kBk * 33, A, lda, (nblk - 1) * kBk,
+                  n - (nblk - 1) * kBk);
+    __syncthreads();
     for (int bi = nblk - 1; bi >= 0; --bi) {
-        const int k = bi * PW, kb = min(PW, n - k);
-        if (tid < 32) {
-            const int i = lane;
-            float ui[PW];
+        const int k = bi * kBk, kb = min(kBk, n - k);
+        float a[kBk];
+        if (tid < k) {
 #pragma unroll
-            for (int q = 0; q < PW; ++q)
-                ui[q] = (i < kb && q >= i && q < kb) ? A[(long long)(k + q) * lda + k + i] : 0.f;
-            float xi = i < kb ? x[k + i] : 0.f;
-#pragma unroll
-            for (int q = PW - 1; q >= 0; --q) {
-                if (q < kb) {
-                    if (i == q) xi = xi / ui[q];
-                    const float xq = __shfl_sync(0xffffffffu, xi, q);
-                    if (i < q) xi = fmaf(-ui[q], xq, xi);
-                }
-            }
-            if (i < kb) x[k + i] = xi;
+            for (int q = 0; q < kBk; ++q) a[q] = q < kb ? A[(long long)(k + q) * lda + tid] : 0.f;
         }
+        if (bi > 0) load_block<T>(D + ((bi - 1) & 1) * kBk * 33, A, lda, k - kBk, kBk);
+        if (tid >= T - 32) block_back<false>(D + (bi & 1) * kBk * 33, x + k, kb, nullptr);
         __syncthreads();
         for (int r = tid; r < k; r += T) {
-            float a[PW];  // the row's block entries, all loads in flight together
+            if (r != tid) {
 #pragma unroll
-            for (int q = 0; q < PW; ++q) a[q] = q < kb ? A[(long long)(k + q) * lda + r] : 0.f;
+                for (int q = 0; q < kBk; ++q) a[q] = q < kb ? A[(long long)(k + q) * lda + r] : 0.f;
+            }
             float acc = x[r];
 #pragma unroll
-            for (int q = 0; q < PW; ++q)
+            for (int q = 0; q < kBk; ++q)
                 if (q < kb) acc = fmaf(-a[q], x[k + q], acc);
             x[r] = acc;
         }
@@ -517,43 +717,36 @@ __device__ void backward_upper(const float* A, int n, long long lda, float* x)
     }
 }
 
-// x <- L^{-T} x, L lower (non-unit): per block, the dot products of the
-// block's columns with the already solved rows below (one warp per column),
-// then the block backward on warp 0.
-template <int T, int PW>
-__device__ void backward_lower_t(const float* A, int n, long long lda, float* x, float* dots)
+// x <- L^{-T} x, L lower (non-unit): per block, the dot products of its columns
+// with the solved rows below (a warp per column), then the block on one warp.
+template <int T>
+__device__ void backward_lower_t(const float* A, int n, long long lda, float* x, float* dots,
+                                 float* D)
 {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nblk = (n + PW - 1) / PW;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nblk = (n + kBk - 1) / kBk;
     for (int bi = nblk - 1; bi >= 0; --bi) {
-        const int k = bi * PW, kb = min(PW, n - k);
-        for (int j = warp; j < kb; j += T / 32) {
-            const float* cj = A + (long long)(k + j) * lda;
+        const int k = bi * kBk, kb = min(kBk, n - k);
+        load_block<T>(D, A, lda, k, kb);
+        for (int j = warp; j < kBk; j += T / 32) {
             float sum = 0.f;
-#pragma unroll 4
-            for (int r = k + kb + lane; r < n; r += 32) sum = fmaf(cj[r], x[r], sum);
+            if (j < kb) {
+                const float* cj = A + (long long)(k + j) * lda;
+                for (int r = k + kb + lane; r < n; r += 128) {  // four loads in flight
+                    float v[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) v[u] = r + 32 * u < n ? cj[r + 32 * u] : 0.f;
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (r + 32 * u < n) sum = fmaf(v[u], x[r + 32 * u], sum);
+                }
+            }
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
             if (lane == 0) dots[j] = sum;
         }
         __syncthreads();
-        if (tid < 32) {
-            const int i = lane;
-            float li[PW];  // L(k + q, k + i), q >= i: column k + i of the block
-#pragma unroll
-            for (int q = 0; q < PW; ++q)
-                li[q] = (i < kb && q >= i && q < kb) ? A[(long long)(k + i) * lda + k + q] : 0.f;
-            float xi = i < kb ? x[k + i] - dots[i] : 0.f;
-#pragma unroll
-            for (int q = PW - 1; q >= 0; --q) {
-                if (q < kb) {
-                    if (i == q) xi = xi / li[q];
-                    const float xq = __shfl_sync(0xffffffffu, xi, q);
-                    if (i < q) xi = fmaf(-li[q], xq, xi);
-                }
-            }
-            if (i < kb) x[k + i] = xi;
-        }
+        if (warp == T / 32 - 1) block_back<true>(D, x + k, kb, dots);
         __syncthreads();
     }
 }
@@ -568,14 +761,13 @@ constexpr int min_ctas() { return T >= 512 ? 1 : (T >= 256 ? 2 : 3); }
 template <int T, int PW>
 __global__ void __launch_bounds__(T, min_ctas<T>()) batched_factor_solve_kernel(BatchArgs a)
 {
-    extern __shared__ __align__(16) float sm[];
-    Smem<T, PW> s(sm);
-    __shared__ int s_item;
+    extern __shared__ __align__(16) unsigned char sm_raw[];
+    Smem<T, PW>& s = *reinterpret_cast<Smem<T, PW>*>(sm_raw);
     const int tid = threadIdx.x;
     for (;;) {
-        if (tid == 0) s_item = (int)atomicAdd(a.queue, 1u);
+        if (tid == 0) s.item = (int)atomicAdd(a.queue, 1u);
         __syncthreads();
-        const int it = s_item;
+        const int it = s.item;
         __syncthreads();
         if (it >= a.count) break;
         const int idx = a.order[it];
@@ -585,33 +777,14 @@ __global__ void __launch_bounds__(T, min_ctas<T>()) batched_factor_solve_kernel(
         float* A = a.A[idx];
         const long long lda = a.lda[idx];
         float* b = a.b[idx];
+        for (int r = tid; r < n; r += T) s.x[r] = b[r];
         int info;
         if (op == 0) info = chol_factor<T, PW>(s, A, n, lda);
         else info = lu_factor<T, PW>(s, A, n, lda, a.ipiv[idx]);
         if (tid == 0) a.info[idx] = info;
-        if (info) continue;
-        // solve: x = b (LU: with the row interchanges applied in order)
-        for (int r = tid; r < n; r += T) s.x[r] = b[r];
-        __syncthreads();
-        if (op != 0) {
-            if (tid == 0) {
-                const int* ip = a.ipiv[idx];
-                for (int i = 0; i < n; ++i) {
-                    const int p = ip[i] - 1;
-                    if (p != i) {
-                        const float t = s.x[i];
-                        s.x[i] = s.x[p];
-                        s.x[p] = t;
-                    }
-                }
-            }
-            __syncthreads();
-            forward_lower<T, PW>(A, n, lda, s.x, true);
-            backward_upper<T, PW>(A, n, lda, s.x);
-        } else {
-            forward_lower<T, PW>(A, n, lda, s.x, false);
-            backward_lower_t<T, PW>(A, n, lda, s.x, s.col);
-        }
+        if (info) continue;  // b keeps its input
+        if (op != 0) backward_upper<T>(A, n, lda, s.x, s.P);
+        else backward_lower_t<T>(A, n, lda, s.x, s.dots, s.P);
         for (int r = tid; r < n; r += T) b[r] = s.x[r];
         __syncthreads();
     }
@@ -627,7 +800,7 @@ constexpr int kNumVariants = (int)(sizeof(kVariants) / sizeof(kVariants[0]));
 template <int T, int PW>
 hdbf_status launch_batched(hdbf_context* ctx, const BatchArgs& a)
 {
-    const size_t smem = smem_floats<PW>() * sizeof(float);
+    const size_t smem = sizeof(Smem<T, PW>);
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batched_factor_solve_kernel<T, PW>,
                                                       T, smem) != cudaSuccess || per_sm < 1) {
@@ -645,7 +818,7 @@ void configure_one()
 {
     cudaFuncSetAttribute(batched_factor_solve_kernel<T, PW>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(smem_floats<PW>() * sizeof(float)));
+                         (int)sizeof(Smem<T, PW>));
 }
 
 }  // namespace
