@@ -48,6 +48,10 @@ hdbf_status permute_cols(hdbf_context* ctx, const GetrfWs& ws, T* A, long long l
     bool any = false;
     for (int r = 0; r < ranges; ++r) any = any || col_count[r] > 0;
     if (!any) return HDBF_STATUS_SUCCESS;
+    const hdbf_status st =
+        swap_rows(ctx, at(A, lda, row0, 0), lda, ipiv, k, minus, m, col_begin[0], col_count[0],
+                  ranges > 1 ? col_begin[1] : 0, ranges > 1 ? col_count[1] : 0, info);
+    if (st != HDBF_STATUS_NOT_SUPPORTED) return st;
     HDBF_TRY(compose_swaps(ctx, ipiv, k, minus, m, ws.src, ws.tgt, ws.count, ws.gperm, info));
     const int max_moves = std::min(m, 2 * k);
     for (int r = 0; r < ranges; ++r)

@@ -119,6 +119,28 @@ hdbf_status getrf_workspace(hdbf_context* ctx, int n, GetrfWs* ws)
     return HDBF_STATUS_SUCCESS;
 }
 
+// A part's interchanges on columns [c0, c0 + nc) of its rows.
+template <class T>
+static hdbf_status panel_swaps_t(hdbf_context* ctx, T* A, long long lda, const int* ipiv, int k,
+                                 int ipiv_add, int m, int c0, int nc, int* info, const GetrfWs& ws)
+{
+    const hdbf_status st = swap_rows(ctx, A, lda, ipiv, k, ipiv_add, m, c0, nc, 0, 0, info);
+    if (st != HDBF_STATUS_NOT_SUPPORTED) return st;
+    HDBF_TRY(compose_swaps(ctx, ipiv, k, ipiv_add, m, ws.src, ws.tgt, ws.count, ws.gperm, info));
+    return apply_moves(ctx, A + (long long)c0 * lda, lda, nc, ws.src, ws.tgt, ws.count,
+                       std::min(m, 2 * k), reinterpret_cast<T*>(ws.temp), ws.temp_cols);
+}
+hdbf_status panel_swaps(hdbf_context* ctx, float* A, long long lda, const int* ipiv, int k,
+                        int ipiv_add, int m, int c0, int nc, int* info, const GetrfWs& ws)
+{
+    return panel_swaps_t(ctx, A, lda, ipiv, k, ipiv_add, m, c0, nc, info, ws);
+}
+hdbf_status panel_swaps(hdbf_context* ctx, double* A, long long lda, const int* ipiv, int k,
+                        int ipiv_add, int m, int c0, int nc, int* info, const GetrfWs& ws)
+{
+    return panel_swaps_t(ctx, A, lda, ipiv, k, ipiv_add, m, c0, nc, info, ws);
+}
+
 // Leaf width for the cluster panel kernel at height m, 0 for the grid-wide one.
 // A cluster holds 64 or more columns up to m = 13300 (FP32): there a column
 // costs 1.7-2.0 us against 4.1-4.5 us.  Taller panels would need leaves of 32
@@ -152,22 +174,14 @@ hdbf_status getrf_panel(hdbf_context* ctx, int m, int w, float* A, long long lda
     const int w2 = w - w1;
     HDBF_TRY(getrf_panel(ctx, m, w1, A, lda, ipiv, ipiv_add, info, info_base, pivot, ws));
     float* A12 = A + (long long)w1 * lda;
-    if (pivot) {
-        HDBF_TRY(compose_swaps(ctx, ipiv, w1, ipiv_add, m, ws.src, ws.tgt, ws.count, ws.gperm,
-                               info));
-        HDBF_TRY(apply_moves(ctx, A12, lda, w2, ws.src, ws.tgt, ws.count,
-                             std::min(m, 2 * w1), ws.temp, ws.temp_cols));
-    }
+    if (pivot)
+        HDBF_TRY(panel_swaps(ctx, A, lda, ipiv, w1, ipiv_add, m, w1, w2, info, ws));
     HDBF_TRY(trsm_llu(ctx, w1, w2, A, lda, A12, lda));
     HDBF_TRY(sgemm_sub(ctx, true, false, m - w1, w2, w1, A + w1, lda, A12, lda, A12 + w1, lda));
     HDBF_TRY(getrf_panel(ctx, m - w1, w2, A12 + w1, lda, pivot ? ipiv + w1 : nullptr,
                          ipiv_add + w1, info, info_base + w1, pivot, ws));
-    if (pivot) {
-        HDBF_TRY(compose_swaps(ctx, ipiv + w1, w2, ipiv_add + w1, m - w1, ws.src, ws.tgt,
-                               ws.count, ws.gperm, info));
-        HDBF_TRY(apply_moves(ctx, A + w1, lda, w1, ws.src, ws.tgt, ws.count,
-                             std::min(m - w1, 2 * w2), ws.temp, ws.temp_cols));
-    }
+    if (pivot)
+        HDBF_TRY(panel_swaps(ctx, A + w1, lda, ipiv + w1, w2, ipiv_add + w1, m - w1, 0, w1, info, ws));
     return HDBF_STATUS_SUCCESS;
 }
 

@@ -890,27 +890,18 @@ hdbf_status getrf_panel(hdbf_context* ctx, int m, int w, double* A, long long ld
         if (held > 0) return getf2_cluster(ctx, m, w, A, lda, ipiv, ipiv_add, info, info_base, pivot);
         return getf2_coop64(ctx, m, w, A, lda, ipiv, ipiv_add, info, info_base, pivot);
     }
-    double* temp = reinterpret_cast<double*>(ws.temp);
     const int w1 = std::max(leaf, w / 2 / leaf * leaf);
     const int w2 = w - w1;
     HDBF_TRY(getrf_panel(ctx, m, w1, A, lda, ipiv, ipiv_add, info, info_base, pivot, ws));
     double* A12 = A + (long long)w1 * lda;
-    if (pivot) {
-        HDBF_TRY(compose_swaps(ctx, ipiv, w1, ipiv_add, m, ws.src, ws.tgt, ws.count, ws.gperm,
-                               info));
-        HDBF_TRY(apply_moves(ctx, A12, lda, w2, ws.src, ws.tgt, ws.count, std::min(m, 2 * w1),
-                             temp, ws.temp_cols));
-    }
+    if (pivot)
+        HDBF_TRY(panel_swaps(ctx, A, lda, ipiv, w1, ipiv_add, m, w1, w2, info, ws));
     HDBF_TRY(trsm_llu(ctx, w1, w2, A, lda, A12, lda));
     HDBF_TRY(dgemm(ctx, 1, false, m - w1, w2, w1, A + w1, lda, A12, lda, A12 + w1, lda));
     HDBF_TRY(getrf_panel(ctx, m - w1, w2, A12 + w1, lda, pivot ? ipiv + w1 : nullptr,
                          ipiv_add + w1, info, info_base + w1, pivot, ws));
-    if (pivot) {
-        HDBF_TRY(compose_swaps(ctx, ipiv + w1, w2, ipiv_add + w1, m - w1, ws.src, ws.tgt,
-                               ws.count, ws.gperm, info));
-        HDBF_TRY(apply_moves(ctx, A + w1, lda, w1, ws.src, ws.tgt, ws.count,
-                             std::min(m - w1, 2 * w2), temp, ws.temp_cols));
-    }
+    if (pivot)
+        HDBF_TRY(panel_swaps(ctx, A + w1, lda, ipiv + w1, w2, ipiv_add + w1, m - w1, 0, w1, info, ws));
     return HDBF_STATUS_SUCCESS;
 }
 

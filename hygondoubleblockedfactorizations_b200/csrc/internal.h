@@ -433,6 +433,14 @@ int configure_cluster_panel(hdbf_context* ctx);
 // (gperm when m ints do not fit in shared memory).
 hdbf_status compose_swaps(hdbf_context* ctx, const int* ipiv, int k, int ipiv_minus, int m,
                           int* src, int* tgt, int* count, int* gperm, int* info);
+// The same swaps, composed and applied in one launch (k <= 512; NOT_SUPPORTED
+// above), to columns [c0, c0 + n0) and [c1, c1 + n1) of A, whose row 0 is the swaps'
+// row 0.  A pivot outside [its row, m) moves nothing, sets info = -1 and the
+// device error.
+hdbf_status swap_rows(hdbf_context* ctx, float* A, long long lda, const int* ipiv, int k, int minus,
+                      int m, int c0, int n0, int c1, int n1, int* info);
+hdbf_status swap_rows(hdbf_context* ctx, double* A, long long lda, const int* ipiv, int k, int minus,
+                      int m, int c0, int n0, int c1, int n1, int* info);
 // A[tgt[i], c] = old A[src[i], c] for c < ncols, i < *count (<= max_moves).
 // Running composition: pos (m ints, row i of the block holds original row
 // pos[i]) is reset to the identity when init is set, then the LAPACK swaps
@@ -523,6 +531,11 @@ struct GetrfWs {
     float* temp = nullptr;  // column-tiled swap buffer
     long long temp_cols = 0;
 };
+// A part's interchanges on columns [c0, c0 + nc) of its rows (drivers.cu).
+hdbf_status panel_swaps(hdbf_context* ctx, float* A, long long lda, const int* ipiv, int k,
+                        int ipiv_add, int m, int c0, int nc, int* info, const GetrfWs& ws);
+hdbf_status panel_swaps(hdbf_context* ctx, double* A, long long lda, const int* ipiv, int k,
+                        int ipiv_add, int m, int c0, int nc, int* info, const GetrfWs& ws);
 // Carve the factorization workspace for order n (reserves it first).
 hdbf_status getrf_workspace(hdbf_context* ctx, int n, GetrfWs* ws);
 hdbf_status getrf_panel(hdbf_context* ctx, int m, int w, float* A, long long lda, int* ipiv,

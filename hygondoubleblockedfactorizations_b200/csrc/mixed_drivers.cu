@@ -383,15 +383,22 @@ hdbf_status getrf_mixed_body(hdbf_context* ctx, int prec, float* A, long long ld
         HDBF_TRY(getrf_panel(ctx, n - p, psz, at(A, lda, p, p), lda, ipiv + p, p, info, p, true,
                              ws));
         // this panel's row interchanges on every other column
-        HDBF_TRY(compose_swaps(ctx, ipiv + p, psz, p, n - p, ws.src, ws.tgt, ws.count, ws.gperm,
-                               info));
-        const int max_moves = std::min(n - p, 2 * psz);
-        if (p > 0)
-            HDBF_TRY(apply_moves(ctx, at(A, lda, p, 0), lda, p, ws.src, ws.tgt, ws.count,
-                                 max_moves, ws.temp, ws.temp_cols));
+        const hdbf_status sw = swap_rows(ctx, at(A, lda, p, 0), lda, ipiv + p, psz, p, n - p, 0, p,
+                                         next, tr, info);
+        if (sw == HDBF_STATUS_NOT_SUPPORTED) {
+            HDBF_TRY(compose_swaps(ctx, ipiv + p, psz, p, n - p, ws.src, ws.tgt, ws.count, ws.gperm,
+                                   info));
+            const int max_moves = std::min(n - p, 2 * psz);
+            if (p > 0)
+                HDBF_TRY(apply_moves(ctx, at(A, lda, p, 0), lda, p, ws.src, ws.tgt, ws.count,
+                                     max_moves, ws.temp, ws.temp_cols));
+            if (tr > 0)
+                HDBF_TRY(apply_moves(ctx, at(A, lda, p, next), lda, tr, ws.src, ws.tgt, ws.count,
+                                     max_moves, ws.temp, ws.temp_cols));
+        } else {
+            HDBF_TRY(sw);
+        }
         if (tr <= 0) continue;
-        HDBF_TRY(apply_moves(ctx, at(A, lda, p, next), lda, tr, ws.src, ws.tgt, ws.count,
-                             max_moves, ws.temp, ws.temp_cols));
         // U12 = L11^{-1} A12 as one tensor-core GEMM: W = L11^{-1} (unit lower)
         // is the FP32 TRSM of the identity.
         float* A12 = at(A, lda, p, next);
