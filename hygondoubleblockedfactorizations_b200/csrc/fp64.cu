@@ -5,11 +5,11 @@
 // type; this file gives them the FP64 overloads of their primitives:
 //
 //   gemm_sub / gemm_sub_tn   C -= op(A) op(B), FP64 FMA: 128x128x8 tiles with
-//                            8x8 outputs per thread for large updates, 64x64x16
-//                            with 4x4 for narrow ones; lower-triangle mode
-//   potf2_small              <= 64 Cholesky leaf, one CTA, LAPACK info
-//   tri_inv64                inverses of the 64x64 diagonal blocks
-//   trsm_rlt / trsm_llu      recursive TRSMs with inverse-apply leaves
+//                            8x8 outputs per thread for large updates, the
+//                            small-update kernel (gemm_small.cu) below, 64x64x16
+//                            tiles for TN; lower-triangle mode
+//   trsm_rlt / trsm_llu      recursive TRSMs on the leaves of trsm_block.cu
+//                            (diagonal tiles and inverses: panel_kernels.cu)
 //   potrf_diag, syrk_lower   recursive diagonal Cholesky, lower SYRK
 //   getrf_panel              recursive LU panel on the grid-wide leaf below
 //   apply_moves              composed row moves, gathered through scratch
@@ -271,6 +271,10 @@ hdbf_status dgemm(hdbf_context* ctx, int mode, bool lower_only, int M, int N, in
     ProfScope prof(ctx, kClsGemm, flops, 8.0 * ((double)M * K + (double)N * K + 2.0 * M * N), M,
                    N, K);
     cudaStream_t s = ctx->stream;
+    if (mode != 2) {
+        const int S = gemm_small_split(ctx, M, N, K);
+        if (S > 0) return gemm_small(ctx, mode == 1, lower_only, S, M, N, K, A, lda, B, ldb, C, ldc);
+    }
     // 128x128 tiles only when they still give two waves of CTAs (one per SM)
     const long long big_tiles = (long long)((M + GBM - 1) / GBM) * ((N + GBN - 1) / GBN);
     if (big_tiles >= 2LL * ctx->sm_count) {
@@ -283,219 +287,17 @@ hdbf_status dgemm(hdbf_context* ctx, int mode, bool lower_only, int M, int N, in
             dgemm_launch<2, false>(s, M, N, K, A, lda, B, ldb, C, ldc);
         }
     } else {
-        if (mode == 0) {
-            if (lower_only) dgemm_launch64<0, true>(s, M, N, K, A, lda, B, ldb, C, ldc);
-            else dgemm_launch64<0, false>(s, M, N, K, A, lda, B, ldb, C, ldc);
-        } else if (mode == 1) {
-            dgemm_launch64<1, false>(s, M, N, K, A, lda, B, ldb, C, ldc);
-        } else {
-            dgemm_launch64<2, false>(s, M, N, K, A, lda, B, ldb, C, ldc);
-        }
+        dgemm_launch64<2, false>(s, M, N, K, A, lda, B, ldb, C, ldc);  // NT, NN: gemm_small
     }
     ctx->launches++;
     return last_cuda(ctx);
 }
 
-// ------------------------------------------------------------- potf2 leaf
-// n <= 64 Cholesky of the lower triangle, one CTA; LAPACK xPOTRF pivot test
-// and info as the FP32 leaf: the first column whose updated diagonal is not
-// > 0 (or is NaN) stops the factorization with its value left in place and
-// info = info_base + j + 1 (first failure wins); a block whose info is
-// already non-zero is left untouched.
-__global__ void __launch_bounds__(256) dpotf2_kernel(int n, double* A, long long lda, int* info,
-                                                     int info_base)
-{
-    __shared__ double S[kL][kL + 1];  // S[c][r] = A(r, c)
-    const int tid = threadIdx.x;
-    if (info && *reinterpret_cast<volatile int*>(info) != 0) return;
-    for (int q = tid; q < kL * kL; q += 256) {
-        const int c = q >> 6, r = q & 63;
-        S[c][r] = (r < n && c < n && r >= c) ? A[(long long)c * lda + r] : 0.0;
-    }
-    __syncthreads();
-    int failed_at = -1;
-    for (int j = 0; j < n; ++j) {
-        const double d = S[j][j];
-        if (!(d > 0.0)) {  // uniform: every thread read the same value
-            failed_at = j;
-            break;
-        }
-        const double sd = sqrt(d);
-        const double rcp = 1.0 / sd;
-        __syncthreads();
-        if (tid == j) S[j][j] = sd;
-        if (tid > j && tid < n) S[j][tid] *= rcp;
-        __syncthreads();
-        const int t = n - j - 1;
-        for (int q = tid; q < t * t; q += 256) {
-            const int c = j + 1 + q / t, r = j + 1 + q % t;
-            if (r >= c) S[c][r] = fma(-S[j][r], S[j][c], S[c][r]);
-        }
-        __syncthreads();
-    }
-    __syncthreads();
-    for (int q = tid; q < kL * kL; q += 256) {
-        const int c = q >> 6, r = q & 63;
-        if (r < n && c < n && r >= c) A[(long long)c * lda + r] = S[c][r];
-    }
-    if (failed_at >= 0 && tid == 0 && info) atomicCAS(info, 0, info_base + failed_at + 1);
-}
-
-// ------------------------------------------------------ triangular leaves
-// Inverses of the 64x64 diagonal blocks of a lower-triangular matrix (unit
-// or non-unit), one CTA per block, thread t solving L_bb x = e_t by forward
-// substitution.  out[b*4096 + c*64 + r] = inv(L_bb)(r, c); a partial last
-// block is padded with the identity.
-__global__ void __launch_bounds__(kL) dtri_inv64_kernel(int n, const double* __restrict__ L,
-                                                        long long ldl, int unit, double* out)
-{
-    __shared__ double Ls[kL][kL + 1];  // Ls[r][c] = L(base + r, base + c)
-    const int base = blockIdx.x * kL;
-    const int nb = min(kL, n - base);
-    const int t = threadIdx.x;
-    for (int idx = t; idx < kL * kL; idx += kL) {
-        const int c = idx / kL, r = idx - c * kL;
-        Ls[r][c] = (r < nb && c < nb && r >= c) ? L[(long long)(base + c) * ldl + base + r] : 0.0;
-    }
-    __syncthreads();
-    double x[kL];
-#pragma unroll
-    for (int i = 0; i < kL; ++i) x[i] = (i == t) ? 1.0 : 0.0;
-#pragma unroll
-    for (int k = 0; k < kL; ++k) {
-        if (k < nb) {
-            if (!unit) x[k] = x[k] / Ls[k][k];
-#pragma unroll
-            for (int i = k + 1; i < kL; ++i) x[i] = fma(-Ls[i][k], x[k], x[i]);
-        }
-    }
-    double* ob = out + (long long)blockIdx.x * kL * kL + (long long)t * kL;
-#pragma unroll
-    for (int i = 0; i < kL; ++i) ob[i] = x[i];
-}
-
-constexpr size_t kApplySmem = sizeof(double) * 2 * kL * (kL + 1);
-
-// B(rows x cols) <- inv * B for rows <= 64: CTA = 64 columns of B, in place.
-__global__ void __launch_bounds__(256) dllu_apply_kernel(int rows, int cols,
-                                                         const double* __restrict__ inv,
-                                                         double* B, long long ldb)
-{
-    extern __shared__ double dsm[];
-    double* Is = dsm;                   // Is[k*65 + r] = inv(r, k)
-    double* Bs = dsm + kL * (kL + 1);   // Bs[k*65 + c] = B(k, c0 + c)
-    const int tid = threadIdx.x;
-    const long long c0 = (long long)blockIdx.x * kL;
-    for (int idx = tid; idx < kL * kL; idx += 256) {
-        const int k = idx >> 6, r = idx & 63;
-        Is[k * (kL + 1) + r] = inv[idx];
-        const int c = idx >> 6, kk = idx & 63;
-        Bs[kk * (kL + 1) + c] = (kk < rows && c0 + c < cols) ? B[(c0 + c) * ldb + kk] : 0.0;
-    }
-    __syncthreads();
-    const int ty = tid >> 4, tx = tid & 15;
-    double acc[4][4] = {};
-    for (int k = 0; k < kL; ++k) {
-        double a[4], b[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = Is[k * (kL + 1) + ty + 16 * i];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) b[j] = Bs[k * (kL + 1) + tx + 16 * j];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const long long c = c0 + tx + 16 * j;
-        if (c >= cols) continue;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int r = ty + 16 * i;
-            if (r < rows) B[c * ldb + r] = acc[i][j];
-        }
-    }
-}
-
-// B(rows x cols) <- B * inv^T for cols <= 64: CTA = 64 rows of B, in place.
-__global__ void __launch_bounds__(256) drlt_apply_kernel(int rows, int cols,
-                                                         const double* __restrict__ inv,
-                                                         double* B, long long ldb)
-{
-    extern __shared__ double dsm[];
-    double* Bs = dsm;                   // Bs[k*65 + r] = B(r0 + r, k)
-    double* Is = dsm + kL * (kL + 1);   // Is[k*65 + c] = inv(c, k)
-    const int tid = threadIdx.x;
-    const long long r0 = (long long)blockIdx.x * kL;
-    for (int idx = tid; idx < kL * kL; idx += 256) {
-        const int k = idx >> 6, x = idx & 63;
-        Is[k * (kL + 1) + x] = inv[idx];
-        Bs[k * (kL + 1) + x] = (k < cols && r0 + x < rows) ? B[(long long)k * ldb + r0 + x] : 0.0;
-    }
-    __syncthreads();
-    const int ty = tid >> 4, tx = tid & 15;
-    double acc[4][4] = {};
-    for (int k = 0; k < kL; ++k) {
-        double a[4], b[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = Bs[k * (kL + 1) + ty + 16 * i];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) b[j] = Is[k * (kL + 1) + tx + 16 * j];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int c = tx + 16 * j;
-        if (c >= cols) continue;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const long long r = r0 + ty + 16 * i;
-            if (r < rows) B[(long long)c * ldb + r] = acc[i][j];
-        }
-    }
-}
-
-hdbf_status dtri_inv(hdbf_context* ctx, int n, const double* L, long long ldl, bool unit,
-                     double* inv)
-{
-    if (n <= 0) return HDBF_STATUS_SUCCESS;
-    const int nb = (n + kL - 1) / kL;
-    ProfScope prof(ctx, kClsTrsmInv, (double)nb * kL * kL * kL / 3.0, 8.0 * 2.0 * nb * kL * kL);
-    dtri_inv64_kernel<<<nb, kL, 0, ctx->stream>>>(n, L, ldl, unit ? 1 : 0, inv);
-    ctx->launches++;
-    return last_cuda(ctx);
-}
-
-hdbf_status dllu_apply(hdbf_context* ctx, int rows, int cols, const double* inv, double* B,
-                       long long ldb)
-{
-    if (rows <= 0 || cols <= 0) return HDBF_STATUS_SUCCESS;
-    ProfScope prof(ctx, kClsTrsmL, (double)rows * rows * cols, 16.0 * (double)rows * cols);
-    const long long grid = ((long long)cols + kL - 1) / kL;
-    dllu_apply_kernel<<<(unsigned)grid, 256, kApplySmem, ctx->stream>>>(rows, cols, inv, B, ldb);
-    ctx->launches++;
-    return last_cuda(ctx);
-}
-
-hdbf_status drlt_apply(hdbf_context* ctx, int rows, int cols, const double* inv, double* B,
-                       long long ldb)
-{
-    if (rows <= 0 || cols <= 0) return HDBF_STATUS_SUCCESS;
-    ProfScope prof(ctx, kClsTrsmR, (double)cols * cols * rows, 16.0 * (double)rows * cols);
-    const long long grid = ((long long)rows + kL - 1) / kL;
-    drlt_apply_kernel<<<(unsigned)grid, 256, kApplySmem, ctx->stream>>>(rows, cols, inv, B, ldb);
-    ctx->launches++;
-    return last_cuda(ctx);
-}
-
+// ------------------------------------------------------------- TRSM recursion
 hdbf_status trsm_rlt_rec64(hdbf_context* ctx, int rows, int cols, const double* L,
                            long long ldl, double* B, long long ldb, const double* inv)
 {
-    if (cols <= kL) return drlt_apply(ctx, rows, cols, inv, B, ldb);
+    if (cols <= llu_block_max_rows()) return rlt_block(ctx, rows, cols, L, ldl, inv, B, ldb);
     const int c1 = split64(cols);
     const int c2 = cols - c1;
     HDBF_TRY(trsm_rlt_rec64(ctx, rows, c1, L, ldl, B, ldb, inv));
@@ -508,7 +310,7 @@ hdbf_status trsm_rlt_rec64(hdbf_context* ctx, int rows, int cols, const double* 
 hdbf_status trsm_llu_rec64(hdbf_context* ctx, int rows, int cols, const double* L,
                            long long ldl, double* B, long long ldb, const double* inv)
 {
-    if (rows <= kL) return dllu_apply(ctx, rows, cols, inv, B, ldb);
+    if (rows <= llu_block_max_rows()) return llu_block(ctx, rows, cols, L, ldl, inv, B, ldb);
     const int r1 = split64(rows);
     const int r2 = rows - r1;
     HDBF_TRY(trsm_llu_rec64(ctx, r1, cols, L, ldl, B, ldb, inv));
@@ -784,10 +586,6 @@ size_t getf2_coop64_scratch_bytes()
 void configure_fp64_kernels(hdbf_context* ctx)
 {
     const size_t cap = ctx->max_smem_optin > 8192 ? ctx->max_smem_optin - 8192 : 40960;
-    cudaFuncSetAttribute(dllu_apply_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)kApplySmem);
-    cudaFuncSetAttribute(drlt_apply_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)kApplySmem);
     cudaFuncSetAttribute(getf2_coop64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)cap);
     cudaGetLastError();
@@ -806,25 +604,21 @@ hdbf_status gemm_sub_tn(hdbf_context* ctx, int M, int N, int K, const double* A,
     return dgemm(ctx, 2, false, M, N, K, A, lda, B, ldb, C, ldc);
 }
 
-hdbf_status potf2_small(hdbf_context* ctx, int n, double* A, long long lda, int* info,
-                        int info_base)
-{
-    if (n <= 0) return HDBF_STATUS_SUCCESS;
-    if (n > kL) return HDBF_STATUS_INVALID_VALUE;
-    ProfScope prof(ctx, kClsPotf2, (double)n * n * n / 3.0, 8.0 * n * n);
-    dpotf2_kernel<<<1, 256, 0, ctx->stream>>>(n, A, lda, info, info_base);
-    ctx->launches++;
-    return last_cuda(ctx);
-}
-
 hdbf_status trsm_rlt(hdbf_context* ctx, int rows, int cols, const double* L, long long ldl,
                      double* B, long long ldb)
 {
     if (rows <= 0 || cols <= 0) return HDBF_STATUS_SUCCESS;
     HDBF_TRY(ensure_ws(ctx, ws_order<double>(cols)));
     double* inv = reinterpret_cast<double*>(ws_inv(ctx));
-    HDBF_TRY(dtri_inv(ctx, cols, L, ldl, false, inv));
+    HDBF_TRY(tri_inv64(ctx, cols, L, ldl, false, inv));
     return trsm_rlt_rec64(ctx, rows, cols, L, ldl, B, ldb, inv);
+}
+
+hdbf_status trsm_rlt_ready(hdbf_context* ctx, int rows, int cols, const double* L, long long ldl,
+                           double* B, long long ldb)
+{
+    if (cols > kL) return trsm_rlt(ctx, rows, cols, L, ldl, B, ldb);
+    return rlt_block(ctx, rows, cols, L, ldl, reinterpret_cast<double*>(ws_inv(ctx)), B, ldb);
 }
 
 hdbf_status trsm_llu(hdbf_context* ctx, int rows, int cols, const double* L, long long ldl,
@@ -833,7 +627,7 @@ hdbf_status trsm_llu(hdbf_context* ctx, int rows, int cols, const double* L, lon
     if (rows <= 0 || cols <= 0) return HDBF_STATUS_SUCCESS;
     HDBF_TRY(ensure_ws(ctx, ws_order<double>(rows)));
     double* inv = reinterpret_cast<double*>(ws_inv(ctx));
-    HDBF_TRY(dtri_inv(ctx, rows, L, ldl, true, inv));
+    HDBF_TRY(tri_inv64(ctx, rows, L, ldl, true, inv));
     return trsm_llu_rec64(ctx, rows, cols, L, ldl, B, ldb, inv);
 }
 
@@ -847,13 +641,15 @@ hdbf_status potrf_diag(hdbf_context* ctx, int n, double* A, long long lda, int* 
                        int info_base)
 {
     if (n <= 0) return HDBF_STATUS_SUCCESS;
-    if (n <= kL) return potf2_small(ctx, n, A, lda, info, info_base);
+    HDBF_TRY(ensure_ws(ctx, ws_order<double>(n)));
+    if (n <= kL)
+        return potf2_small(ctx, n, A, lda, info, info_base, reinterpret_cast<double*>(ws_inv(ctx)));
     const int n1 = split64(n);
     const int n2 = n - n1;
     double* A21 = A + n1;
     double* A22 = A + (long long)n1 * lda + n1;
     HDBF_TRY(potrf_diag(ctx, n1, A, lda, info, info_base));
-    HDBF_TRY(trsm_rlt(ctx, n2, n1, A, lda, A21, lda));
+    HDBF_TRY(trsm_rlt_ready(ctx, n2, n1, A, lda, A21, lda));
     HDBF_TRY(syrk_lower(ctx, n2, n1, A21, lda, A22, lda));
     return potrf_diag(ctx, n2, A22, lda, info, info_base + n1);
 }

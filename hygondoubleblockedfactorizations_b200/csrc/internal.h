@@ -103,7 +103,7 @@ struct hdbf_context {
     // chunk for the parts of one GEMM, as split_kc does (-1: decide per launch).
     int tc_sgemm = 1;
     int tc_plan = -1;
-    int small_plan = -1;  // the same for sgemm_small_split (0: the 128 x 128 kernel)
+    int small_plan = -1;  // the same for gemm_small_split (0: the 128 x 128 kernel)
     unsigned spin_limit = 0; // hdbf_set_wait_limit (0: default)
     // Conditional launches (RunIf): while set, the FP32 GEMM and the
     // diagonal-block kernel run only when *run_if != 0 (read on the device).
@@ -312,13 +312,17 @@ hdbf_status sgemm_sub(hdbf_context* ctx, bool nn, bool lower_only, int M, int N,
 // K split of the FP32 GEMM of shape M x N x K (tri: lower-triangle mode):
 // the number of chunks (1 = no split) and, in *kc, their length.
 int split_count(const hdbf_context* ctx, int M, int N, int K, bool tri, int* kc);
-// Updates below one wave of 128 x 128 tiles (sgemm_small.cu): the CTAs that share
+// Updates below one wave of 128 x 128 tiles (gemm_small.cu): the CTAs that share
 // a tile's K (0: not taken), and the launch.
-int sgemm_small_split(const hdbf_context* ctx, int M, int N, int K);
-hdbf_status sgemm_small(hdbf_context* ctx, bool nn, bool lower, int S, int M, int N, int K,
+int gemm_small_split(const hdbf_context* ctx, int M, int N, int K);
+hdbf_status gemm_small(hdbf_context* ctx, bool nn, bool lower, int S, int M, int N, int K,
                         const float* A, long long lda, const float* B, long long ldb, float* C,
                         long long ldc);
-void configure_sgemm_small(hdbf_context* ctx);
+hdbf_status gemm_small(hdbf_context* ctx, bool nn, bool lower, int S, int M, int N, int K,
+                       const double* A, long long lda, const double* B, long long ldb, double* C,
+                       long long ldc);
+void configure_gemm_small(hdbf_context* ctx);
+void configure_tile_kernels(hdbf_context* ctx);
 // FP32 update on the tensor cores (tc_sgemm.cu): the K chunk for this shape, 0
 // where the FP32 kernel is taken; one chunk of it (a_kc / b_kc: the operand's K
 // is contiguous), whose operand range, in *range, tells the FP32 kernel behind it
@@ -339,7 +343,7 @@ struct SplitPlan {
         c->tc_plan = tc_sgemm_chunk(c, M, N, K, false);
         const int S = split_count(c, M, N, K, false, &kc);
         c->split_kc = S > 1 ? kc : 0;
-        c->small_plan = sgemm_small_split(c, M, N, K);
+        c->small_plan = gemm_small_split(c, M, N, K);
     }
     ~SplitPlan()
     {
@@ -376,10 +380,14 @@ hdbf_status tri_inv64_mode(hdbf_context* ctx, int n, const float* L, long long l
 // forward substitution with the 64x64 inverses in inv, trsm_block.cu).
 hdbf_status llu_block(hdbf_context* ctx, int rows, int cols, const float* L, long long ldl,
                       const float* inv, float* B, long long ldb);
+hdbf_status llu_block(hdbf_context* ctx, int rows, int cols, const double* L, long long ldl,
+                      const double* inv, double* B, long long ldb);
 int llu_block_max_rows();
 // B(rows x cols <= 256) <- B L^{-T}, L lower non-unit, same scheme.
 hdbf_status rlt_block(hdbf_context* ctx, int rows, int cols, const float* L, long long ldl,
                       const float* inv, float* B, long long ldb);
+hdbf_status rlt_block(hdbf_context* ctx, int rows, int cols, const double* L, long long ldl,
+                      const double* inv, double* B, long long ldb);
 void configure_trsm_block_kernels(hdbf_context* ctx);
 // B <- inv * B (trans=false) or inv^T * B (trans=true), rows <= 64.
 hdbf_status llu_apply_t(hdbf_context* ctx, int rows, int cols, const float* inv, float* B,
@@ -556,14 +564,14 @@ hdbf_status gemm_sub(hdbf_context* ctx, bool nn, bool lower_only, int M, int N, 
 hdbf_status gemm_sub_tn(hdbf_context* ctx, int M, int N, int K, const double* A, long long lda,
                         const double* B, long long ldb, double* C, long long ldc);
 hdbf_status potf2_small(hdbf_context* ctx, int n, double* A, long long lda, int* info,
-                        int info_base);
+                        int info_base, double* inv = nullptr);
+hdbf_status tri_inv64(hdbf_context* ctx, int n, const double* L, long long ldl, bool unit,
+                      double* out);
 hdbf_status trsm_rlt(hdbf_context* ctx, int rows, int cols, const double* L, long long ldl,
                      double* B, long long ldb);
-inline hdbf_status trsm_rlt_ready(hdbf_context* ctx, int rows, int cols, const double* L,
-                                  long long ldl, double* B, long long ldb)
-{
-    return trsm_rlt(ctx, rows, cols, L, ldl, B, ldb);
-}
+// After potrf_diag of order <= 64 the inverse is ready; above, it is formed here.
+hdbf_status trsm_rlt_ready(hdbf_context* ctx, int rows, int cols, const double* L, long long ldl,
+                           double* B, long long ldb);
 hdbf_status trsm_llu(hdbf_context* ctx, int rows, int cols, const double* L, long long ldl,
                      double* B, long long ldb);
 hdbf_status syrk_lower(hdbf_context* ctx, int n, int k, const double* A, long long lda,

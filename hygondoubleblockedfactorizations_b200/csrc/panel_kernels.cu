@@ -1,4 +1,4 @@
-// Diagonal-block Cholesky and small triangular-solve kernels (FP32).
+// Diagonal-block Cholesky and small triangular-solve kernels.
 //
 // potf2_small replaces rocsolver_spotrf on the diagonal block
 // (src/potrf/double_blocked_potrf.cpp:34-56, call :334) at the leaf of this
@@ -13,6 +13,10 @@ namespace hdbf {
 namespace {
 
 constexpr int kLeaf = 64;
+constexpr int kTileWords =  // tile, inverse, scratch and reciprocals
+    2 * kLeaf * tile64::kLd + tile64::kScratch + kLeaf;
+template <class T>  // dynamic part
+constexpr size_t kTileSmem = sizeof(T) == 4 ? 0 : sizeof(T) * (size_t)kTileWords;
 
 // Cholesky of an n x n (n <= 64) lower block, one CTA (chol64), and, with inv,
 // the inverse of its factor in tri_inv64's layout, so that the panel solve
@@ -21,13 +25,17 @@ constexpr int kLeaf = 64;
 // diagonal is not > 0 (or is NaN) stops the factorization, its value is left
 // in place, and info = info_base + j + 1 (first failure wins).  A block whose
 // info is already non-zero is left untouched.
-__global__ void __launch_bounds__(tile64::kThreads)
-potf2_kernel(int n, float* A, long long lda, int* info, int info_base, float* inv)
+template <class T>
+__global__ void __launch_bounds__(tile64::kThreads, 1)
+potf2_kernel(int n, T* A, long long lda, int* info, int info_base, T* inv)
 {
-    __shared__ __align__(16) float S[kLeaf * tile64::kLd];
-    __shared__ __align__(16) float W[kLeaf * tile64::kLd];
-    __shared__ __align__(16) float X[tile64::kScratch];
-    __shared__ float rd[kLeaf];
+    // FP32 fits the static limit
+    __shared__ __align__(16) float fixed[sizeof(T) == 4 ? kTileWords : 4];
+    extern __shared__ __align__(16) unsigned char sm_raw[];
+    T* S = sizeof(T) == 4 ? reinterpret_cast<T*>(fixed) : reinterpret_cast<T*>(sm_raw);
+    T* W = S + kLeaf * tile64::kLd;
+    T* X = W + kLeaf * tile64::kLd;
+    T* rd = X + tile64::kScratch;
     __shared__ int s_fail;
     if (info && *reinterpret_cast<volatile int*>(info) != 0) return;
     tile64::load_lower<false>(S, A, lda, n, false);
@@ -47,13 +55,17 @@ potf2_kernel(int n, float* A, long long lda, int* info, int info_base, float* in
 // with the identity.
 // mode 0: lower non-unit, 1: lower unit, 2: upper non-unit (the upper block
 // U is inverted as (U^T)^{-1} and stored transposed).
-__global__ void __launch_bounds__(tile64::kThreads)
-tri_inv64_kernel(int n, const float* __restrict__ L, long long ldl, int mode, float* out)
+template <class T>
+__global__ void __launch_bounds__(tile64::kThreads, 1)
+tri_inv64_kernel(int n, const T* __restrict__ L, long long ldl, int mode, T* out)
 {
-    __shared__ __align__(16) float S[kLeaf * tile64::kLd];
-    __shared__ __align__(16) float W[kLeaf * tile64::kLd];
-    __shared__ __align__(16) float X[tile64::kScratch];
-    __shared__ float rd[kLeaf];
+    // FP32 fits the static limit
+    __shared__ __align__(16) float fixed[sizeof(T) == 4 ? kTileWords : 4];
+    extern __shared__ __align__(16) unsigned char sm_raw[];
+    T* S = sizeof(T) == 4 ? reinterpret_cast<T*>(fixed) : reinterpret_cast<T*>(sm_raw);
+    T* W = S + kLeaf * tile64::kLd;
+    T* X = W + kLeaf * tile64::kLd;
+    T* rd = X + tile64::kScratch;
     const int base = blockIdx.x * kLeaf;
     tile64::load_lower<false>(S, L + (long long)base * ldl + base, ldl, min(kLeaf, n - base),
                               mode == 2);
@@ -106,33 +118,67 @@ __global__ void __launch_bounds__(256) llu_apply_kernel(int rows, int cols,
 
 }  // namespace
 
-hdbf_status potf2_small(hdbf_context* ctx, int n, float* A, long long lda, int* info,
-                        int info_base, float* inv)
+namespace {
+template <class T>
+hdbf_status potf2_t(hdbf_context* ctx, int n, T* A, long long lda, int* info, int info_base, T* inv)
 {
     if (n <= 0) return HDBF_STATUS_SUCCESS;
     if (n > kLeaf) return HDBF_STATUS_INVALID_VALUE;
-    ProfScope prof(ctx, kClsPotf2, (double)n * n * n / 3.0, 8.0 * n * n);
-    potf2_kernel<<<1, tile64::kThreads, 0, ctx->stream>>>(n, A, lda, info, info_base, inv);
+    ProfScope prof(ctx, kClsPotf2, (double)n * n * n / 3.0, 2.0 * sizeof(T) * n * n);
+    potf2_kernel<T><<<1, tile64::kThreads, kTileSmem<T>, ctx->stream>>>(n, A, lda, info, info_base,
+                                                                        inv);
     ctx->launches++;
     return last_cuda(ctx);
+}
+template <class T>
+hdbf_status tri_inv64_t(hdbf_context* ctx, int n, const T* L, long long ldl, int mode, T* out)
+{
+    if (n <= 0) return HDBF_STATUS_SUCCESS;
+    const int blocks = (n + kLeaf - 1) / kLeaf;
+    ProfScope prof(ctx, kClsTrsmInv, (double)blocks * kLeaf * kLeaf * kLeaf / 3.0,
+                   2.0 * sizeof(T) * blocks * kLeaf * kLeaf);
+    tri_inv64_kernel<T><<<blocks, tile64::kThreads, kTileSmem<T>, ctx->stream>>>(n, L, ldl, mode,
+                                                                                 out);
+    ctx->launches++;
+    return last_cuda(ctx);
+}
+}  // namespace
+
+void configure_tile_kernels(hdbf_context*)
+{
+    cudaFuncSetAttribute(potf2_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)kTileSmem<double>);
+    cudaFuncSetAttribute(tri_inv64_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)kTileSmem<double>);
+    cudaGetLastError();
+}
+
+hdbf_status potf2_small(hdbf_context* ctx, int n, float* A, long long lda, int* info,
+                        int info_base, float* inv)
+{
+    return potf2_t(ctx, n, A, lda, info, info_base, inv);
+}
+hdbf_status potf2_small(hdbf_context* ctx, int n, double* A, long long lda, int* info,
+                        int info_base, double* inv)
+{
+    return potf2_t(ctx, n, A, lda, info, info_base, inv);
 }
 
 hdbf_status tri_inv64(hdbf_context* ctx, int n, const float* L, long long ldl, bool unit,
                       float* out)
 {
-    return tri_inv64_mode(ctx, n, L, ldl, unit ? 1 : 0, out);
+    return tri_inv64_t(ctx, n, L, ldl, unit ? 1 : 0, out);
+}
+hdbf_status tri_inv64(hdbf_context* ctx, int n, const double* L, long long ldl, bool unit,
+                      double* out)
+{
+    return tri_inv64_t(ctx, n, L, ldl, unit ? 1 : 0, out);
 }
 
 hdbf_status tri_inv64_mode(hdbf_context* ctx, int n, const float* L, long long ldl, int mode,
                            float* out)
 {
-    if (n <= 0) return HDBF_STATUS_SUCCESS;
-    const int blocks = (n + kLeaf - 1) / kLeaf;
-    ProfScope prof(ctx, kClsTrsmInv, (double)blocks * kLeaf * kLeaf * kLeaf / 3.0,
-                   8.0 * blocks * kLeaf * kLeaf);
-    tri_inv64_kernel<<<blocks, tile64::kThreads, 0, ctx->stream>>>(n, L, ldl, mode, out);
-    ctx->launches++;
-    return last_cuda(ctx);
+    return tri_inv64_t(ctx, n, L, ldl, mode, out);
 }
 
 hdbf_status llu_apply_t(hdbf_context* ctx, int rows, int cols, const float* inv, float* B,

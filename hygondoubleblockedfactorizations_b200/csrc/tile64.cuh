@@ -248,7 +248,8 @@ __device__ __forceinline__ void store_inv(T* dst, const T* W, bool trans)
 // ones on the diagonal), W[c * kLd + r], zero above the diagonal.  X: kScratch
 // entries, rd: 64.  S complete on entry; W complete on return.
 template <class T>
-__device__ void inv64(const T* S, T* W, T* X, T* rd, bool unit)
+__device__ void inv64(const T* __restrict__ S, T* __restrict__ W, T* __restrict__ X,
+                      T* __restrict__ rd, bool unit)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int q = tid; q < kN * kLd; q += kThreads) W[q] = T(0);

@@ -12,8 +12,9 @@
 // register tiles, packed FP32 FMAs); before, each of the ten tile products of a
 // 256-wide block waited for its own loads (57 us at 7500 x 256, now 33; 19 us
 // at 2000 x 64, now 7.5).  The slice width falls when wider slices would not give
-// every SM a CTA.
+// every SM a CTA.  FP32 and FP64.
 #include "internal.h"
+#include "pair.cuh"
 
 namespace hdbf {
 namespace {
@@ -29,38 +30,47 @@ __device__ __forceinline__ uint32_t smem_addr(const void* p)
 {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
-__device__ __forceinline__ void copy16(float* dst, const float* src)
+__device__ __forceinline__ void copy16(void* dst, const void* src)
 {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src)
                  : "memory");
 }
-__device__ __forceinline__ void copy4(float* dst, const float* src, bool have)
+template <class T>
+__device__ __forceinline__ void copy1(T* dst, const T* src, bool have)
 {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_addr(dst)), "l"(src),
-                 "r"(have ? 4 : 0)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(smem_addr(dst)), "l"(src),
+                 "n"(sizeof(T)), "r"(have ? (int)sizeof(T) : 0)
                  : "memory");
 }
 __device__ __forceinline__ void commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-
-// 64 columns of 64 contiguous floats: dst[c * pitch + r] = src[c * ld + r], zero
-// outside rows x cols.
-__device__ __forceinline__ void copy_tile(float* dst, int pitch, const float* src, long long ld,
-                                          int rows, int cols)
+template <class T>
+constexpr int kVec = 16 / (int)sizeof(T);  // elements of a 16-byte copy
+template <class T>
+__device__ __forceinline__ void zero16(T* p)
 {
-    const bool vec = rows == kT && cols == kT && ld % 4 == 0 &&
+    *reinterpret_cast<uint4*>(p) = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// 64 columns of 64 contiguous values: dst[c * 64 + r] = src[c * ld + r], zero
+// outside rows x cols.
+template <class T>
+__device__ __forceinline__ void copy_tile(T* dst, const T* src, long long ld, int rows, int cols)
+{
+    constexpr int V = kVec<T>, PER = kT / V;
+    const bool vec = rows == kT && cols == kT && ld % V == 0 &&
                      (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
     if (vec) {
 #pragma unroll
-        for (int u = 0; u < kTile / 4 / kThr; ++u) {
-            const int q = threadIdx.x + u * kThr, c = q >> 4, r = (q & 15) * 4;
-            copy16(dst + c * pitch + r, src + (long long)c * ld + r);
+        for (int u = 0; u < kT * PER / kThr; ++u) {
+            const int q = threadIdx.x + u * kThr, c = q / PER, r = (q % PER) * V;
+            copy16(dst + c * kT + r, src + (long long)c * ld + r);
         }
     } else {
 #pragma unroll
         for (int u = 0; u < kTile / kThr; ++u) {
             const int q = threadIdx.x + u * kThr, c = q >> 6, r = q & 63;
             const bool have = r < rows && c < cols;
-            copy4(dst + c * pitch + r, have ? src + (long long)c * ld + r : src, have);
+            copy1(dst + c * kT + r, have ? src + (long long)c * ld + r : src, have);
         }
     }
 }
@@ -74,39 +84,71 @@ __device__ __forceinline__ void tile_at(int t, int& i, int& j)
     j = t;
 }
 
-__device__ __forceinline__ unsigned long long pack2(float x, float y)
+// ------------------------------------------------------------------- right
+// acc[c][e] += sign * sum_k x[k * ldx + e] b[k * 64 + c] over 64 of K.
+template <class T, int RP>
+__device__ __forceinline__ void right_product(T acc[4][RP], const T* x, int ldx, const T* b, T sign)
 {
-    unsigned long long v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(x), "f"(y));
-    return v;
-}
-__device__ __forceinline__ float2 unpack2(unsigned long long v)
-{
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a,
-                                     unsigned long long b)
-{
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+    if (RP == 1) {
+#pragma unroll 8
+        for (int k = 0; k < kT; ++k) {
+            T bv[4];
+            Two<T> lo, hi;
+            load_pairs(b + k * kT, lo, hi);
+            lo.get(bv[0], bv[1]);
+            hi.get(bv[2], bv[3]);
+            const T xv = sign * x[k * ldx];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[c][0] = ::fma(xv, bv[c], acc[c][0]);
+        }
+    } else {
+        Two<T> s[4][RP / 2 > 0 ? RP / 2 : 1];
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int h = 0; h < RP / 2; ++h)
+                s[c][h] = Two<T>::make(acc[c][2 * h], acc[c][(2 * h + 1) % RP]);
+#pragma unroll 8
+        for (int k = 0; k < kT; ++k) {
+            T bv[4];
+            Two<T> lo, hi;
+            load_pairs(b + k * kT, lo, hi);
+            lo.get(bv[0], bv[1]);
+            hi.get(bv[2], bv[3]);
+            Two<T> xv[RP / 2 > 0 ? RP / 2 : 1];
+#pragma unroll
+            for (int h = 0; h < RP / 2; ++h)
+                xv[h] = *reinterpret_cast<const Two<T>*>(x + k * ldx + 2 * h);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const T bs = sign * bv[c];
+                const Two<T> bb = Two<T>::make(bs, bs);
+#pragma unroll
+                for (int h = 0; h < RP / 2; ++h) s[c][h].fma(xv[h], bb);
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int h = 0; h < RP / 2; ++h) s[c][h].get(acc[c][2 * h], acc[c][(2 * h + 1) % RP]);
+    }
 }
 
-// ------------------------------------------------------------------- right
 // CTA: 16 RP rows of B, all columns.  X[c * 16 RP + r].  Thread: RP rows
 // (RP * (tid & 15)) x 4 columns (4 * (tid >> 4)) of a 64-column block.
-template <int RP>
+template <class T, int RP>
 __global__ void __launch_bounds__(kThr) rlt_block_kernel(int rows, int cols,
-                                                         const float* __restrict__ L, long long ldl,
-                                                         const float* __restrict__ inv, float* B,
+                                                         const T* __restrict__ L, long long ldl,
+                                                         const T* __restrict__ inv, T* B,
                                                          long long ldb)
 {
     constexpr int RT = 16 * RP;  // rows of the slice
-    extern __shared__ __align__(16) float sm[];
+    extern __shared__ __align__(16) unsigned char sm_raw[];
+    T* sm = reinterpret_cast<T*>(sm_raw);
     const int nb = (cols + kT - 1) / kT, nt = nb * (nb + 1) / 2;
     const int ring = min(nt, kRing);
-    float* tiles = sm;
-    float* X = sm + ring * kTile;
+    T* tiles = sm;
+    T* X = sm + ring * kTile;
     const int tid = threadIdx.x, ty = tid & 15, tx = tid >> 4;
     const long long r0 = (long long)blockIdx.x * RT;
     const int nr = (int)min((long long)RT, (long long)rows - r0);
@@ -114,28 +156,29 @@ __global__ void __launch_bounds__(kThr) rlt_block_kernel(int rows, int cols,
         if (t < nt) {
             int i, j;
             tile_at(t, i, j);
-            float* dst = tiles + (t % ring) * kTile;
-            if (i == j) copy_tile(dst, kT, inv + (long long)i * kTile, kT, kT, kT);
+            T* dst = tiles + (t % ring) * kTile;
+            if (i == j) copy_tile(dst, inv + (long long)i * kTile, kT, kT, kT);
             else  // [k][c] = L(64 i + c, 64 j + k)
-                copy_tile(dst, kT, L + (long long)(j * kT) * ldl + i * kT, ldl,
+                copy_tile(dst, L + (long long)(j * kT) * ldl + i * kT, ldl,
                           min(kT, cols - i * kT), kT);
         }
         commit();
     };
     {
-        const bool vec = nr == RT && ldb % 4 == 0 && (reinterpret_cast<uintptr_t>(B + r0) & 15u) == 0;
+        constexpr int V = kVec<T>;
+        const bool vec = nr == RT && ldb % V == 0 && (reinterpret_cast<uintptr_t>(B + r0) & 15u) == 0;
         const int total = nb * kT * RT;
         if (vec) {
-            for (int q = tid * 4; q < total; q += kThr * 4) {
+            for (int q = tid * V; q < total; q += kThr * V) {
                 const int c = q / RT, r = q % RT;
                 if (c < cols) copy16(X + q, B + (long long)c * ldb + r0 + r);
-                else *reinterpret_cast<float4*>(X + q) = make_float4(0.f, 0.f, 0.f, 0.f);
+                else zero16(X + q);
             }
         } else {
             for (int q = tid; q < total; q += kThr) {
                 const int c = q / RT, r = q % RT;
                 const bool have = r < nr && c < cols;
-                copy4(X + q, have ? B + (long long)c * ldb + r0 + r : B, have);
+                copy1(X + q, have ? B + (long long)c * ldb + r0 + r : B, have);
             }
         }
     }
@@ -143,73 +186,41 @@ __global__ void __launch_bounds__(kThr) rlt_block_kernel(int rows, int cols,
     if (ring > 1) fetch(1); else commit();
     int t = 0;
     for (int i = 0; i < nb; ++i) {
-        unsigned long long acc[4][(RP + 1) / 2];
-        float a1[4];  // RP == 1
+        T acc[4][RP];
         for (int j = 0; j <= i; ++j, ++t) {
             asm volatile("cp.async.wait_group 1;" ::: "memory");
             __syncthreads();  // tile t and X are there; tile t - 1 and X_i's old reads are done
             if (ring > 2) fetch(t + 2); else commit();
             if (j == 0) {
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const float* x = X + (i * kT + tx * 4 + c) * RT + ty * RP;
-                    if (RP == 1) a1[c] = i == 0 ? 0.f : x[0];
+                for (int c = 0; c < 4; ++c)
 #pragma unroll
-                    for (int h = 0; h < RP / 2; ++h)
-                        acc[c][h] = i == 0 ? 0ull : *reinterpret_cast<const unsigned long long*>(x + 2 * h);
-                }
+                    for (int e = 0; e < RP; ++e)
+                        acc[c][e] = i == 0 ? T(0) : X[(i * kT + tx * 4 + c) * RT + ty * RP + e];
             }
-            const float* b = tiles + (t % ring) * kTile + tx * 4;
-            const float* x = X + j * kT * RT + ty * RP;
+            const T* b = tiles + (t % ring) * kTile + tx * 4;
+            const T* x = X + j * kT * RT + ty * RP;
             if (j == i && i > 0) {  // B_i - sum back into X_i, then times D_i
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    float* o = X + (i * kT + tx * 4 + c) * RT + ty * RP;
-                    if (RP == 1) o[0] = a1[c], a1[c] = 0.f;
+                for (int c = 0; c < 4; ++c)
 #pragma unroll
-                    for (int h = 0; h < RP / 2; ++h) {
-                        *reinterpret_cast<unsigned long long*>(o + 2 * h) = acc[c][h];
-                        acc[c][h] = 0ull;
+                    for (int e = 0; e < RP; ++e) {
+                        X[(i * kT + tx * 4 + c) * RT + ty * RP + e] = acc[c][e];
+                        acc[c][e] = T(0);
                     }
-                }
                 __syncthreads();
             }
-            const float sign = j == i ? 1.f : -1.f;
-#pragma unroll 8
-            for (int k = 0; k < kT; ++k) {
-                const float4 bv = *reinterpret_cast<const float4*>(b + k * kT);
-                const float bb[4] = {sign * bv.x, sign * bv.y, sign * bv.z, sign * bv.w};
-                if (RP == 1) {
-                    const float xv = x[k * RT];
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) a1[c] = fmaf(xv, bb[c], a1[c]);
-                }
-#pragma unroll
-                for (int h = 0; h < RP / 2; ++h) {
-                    const unsigned long long xv =
-                        *reinterpret_cast<const unsigned long long*>(x + k * RT + 2 * h);
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) fma2(acc[c][h], xv, pack2(bb[c], bb[c]));
-                }
-            }
+            right_product<T, RP>(acc, x, RT, b, j == i ? T(1) : T(-1));
             if (j == i) {
                 if (i + 1 < nb) __syncthreads();  // X_i is still being read
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     const int col = i * kT + tx * 4 + c;
-                    float v[RP];
-                    if (RP == 1) v[0] = a1[c];
-#pragma unroll
-                    for (int h = 0; h < RP / 2; ++h) {
-                        const float2 p = unpack2(acc[c][h]);
-                        v[2 * h] = p.x;
-                        v[(2 * h + 1) % RP] = p.y;
-                    }
 #pragma unroll
                     for (int e = 0; e < RP; ++e) {
-                        if (i + 1 < nb) X[col * RT + ty * RP + e] = col < cols ? v[e] : 0.f;
+                        if (i + 1 < nb) X[col * RT + ty * RP + e] = col < cols ? acc[c][e] : T(0);
                         if (col < cols && ty * RP + e < nr)
-                            B[(long long)col * ldb + r0 + ty * RP + e] = v[e];
+                            B[(long long)col * ldb + r0 + ty * RP + e] = acc[c][e];
                     }
                 }
             }
@@ -221,18 +232,19 @@ __global__ void __launch_bounds__(kThr) rlt_block_kernel(int rows, int cols,
 // -------------------------------------------------------------------- left
 // CTA: 16 CP columns of B, all rows.  X[n * kLdL + k].  Thread: 4 rows
 // (4 * (tid & 15)) of a 64-row block x CP columns (CP * (tid >> 4)).
-template <int CP>
+template <class T, int CP>
 __global__ void __launch_bounds__(kThr) llu_block_kernel(int rows, int cols,
-                                                         const float* __restrict__ L, long long ldl,
-                                                         const float* __restrict__ inv, float* B,
+                                                         const T* __restrict__ L, long long ldl,
+                                                         const T* __restrict__ inv, T* B,
                                                          long long ldb)
 {
     constexpr int CT = 16 * CP;
-    extern __shared__ __align__(16) float sm[];
+    extern __shared__ __align__(16) unsigned char sm_raw[];
+    T* sm = reinterpret_cast<T*>(sm_raw);
     const int nb = (rows + kT - 1) / kT, nt = nb * (nb + 1) / 2;
     const int ring = min(nt, kRing);
-    float* tiles = sm;
-    float* X = sm + ring * kTile;
+    T* tiles = sm;
+    T* X = sm + ring * kTile;
     const int tid = threadIdx.x, ty = tid & 15, tx = tid >> 4;
     const long long c0 = (long long)blockIdx.x * CT;
     const int nc = (int)min((long long)CT, (long long)cols - c0);
@@ -240,28 +252,29 @@ __global__ void __launch_bounds__(kThr) llu_block_kernel(int rows, int cols,
         if (t < nt) {
             int i, j;
             tile_at(t, i, j);
-            float* dst = tiles + (t % ring) * kTile;
-            if (i == j) copy_tile(dst, kT, inv + (long long)i * kTile, kT, kT, kT);
+            T* dst = tiles + (t % ring) * kTile;
+            if (i == j) copy_tile(dst, inv + (long long)i * kTile, kT, kT, kT);
             else  // [k][m] = L(64 i + m, 64 j + k)
-                copy_tile(dst, kT, L + (long long)(j * kT) * ldl + i * kT, ldl,
+                copy_tile(dst, L + (long long)(j * kT) * ldl + i * kT, ldl,
                           min(kT, rows - i * kT), kT);
         }
         commit();
     };
     {
+        constexpr int V = kVec<T>;
         const int len = nb * kT;
-        const bool vec = rows == len && ldb % 4 == 0 && (reinterpret_cast<uintptr_t>(B) & 15u) == 0;
+        const bool vec = rows == len && ldb % V == 0 && (reinterpret_cast<uintptr_t>(B) & 15u) == 0;
         if (vec) {
-            for (int q = tid * 4; q < CT * len; q += kThr * 4) {
+            for (int q = tid * V; q < CT * len; q += kThr * V) {
                 const int n = q / len, k = q - n * len;
                 if (n < nc) copy16(X + n * kLdL + k, B + (c0 + n) * ldb + k);
-                else *reinterpret_cast<float4*>(X + n * kLdL + k) = make_float4(0.f, 0.f, 0.f, 0.f);
+                else zero16(X + n * kLdL + k);
             }
         } else {
             for (int q = tid; q < CT * len; q += kThr) {
                 const int n = q / len, k = q - n * len;
                 const bool have = n < nc && k < rows;
-                copy4(X + n * kLdL + k, have ? B + (c0 + n) * ldb + k : B, have);
+                copy1(X + n * kLdL + k, have ? B + (c0 + n) * ldb + k : B, have);
             }
         }
     }
@@ -269,7 +282,7 @@ __global__ void __launch_bounds__(kThr) llu_block_kernel(int rows, int cols,
     if (ring > 1) fetch(1); else commit();
     int t = 0;
     for (int i = 0; i < nb; ++i) {
-        unsigned long long acc[CP][2];  // [column][row pair]
+        Two<T> acc[CP][2];  // [column][row pair]
         for (int j = 0; j <= i; ++j, ++t) {
             asm volatile("cp.async.wait_group 1;" ::: "memory");
             __syncthreads();
@@ -277,41 +290,41 @@ __global__ void __launch_bounds__(kThr) llu_block_kernel(int rows, int cols,
             if (j == 0) {
 #pragma unroll
                 for (int c = 0; c < CP; ++c) {
-                    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(
-                        X + (tx * CP + c) * kLdL + i * kT + ty * 4);
-                    acc[c][0] = i == 0 ? 0ull : v.x;
-                    acc[c][1] = i == 0 ? 0ull : v.y;
+                    load_pairs(X + (tx * CP + c) * kLdL + i * kT + ty * 4, acc[c][0], acc[c][1]);
+                    if (i == 0) acc[c][0] = acc[c][1] = Two<T>::zero();
                 }
             }
-            const float* a = tiles + (t % ring) * kTile + ty * 4;
+            const T* a = tiles + (t % ring) * kTile + ty * 4;
             if (j == i && i > 0) {
 #pragma unroll
                 for (int c = 0; c < CP; ++c) {
-                    ulonglong2 v;
-                    v.x = acc[c][0];
-                    v.y = acc[c][1];
-                    *reinterpret_cast<ulonglong2*>(X + (tx * CP + c) * kLdL + i * kT + ty * 4) = v;
-                    acc[c][0] = acc[c][1] = 0ull;
+                    store_pairs(X + (tx * CP + c) * kLdL + i * kT + ty * 4, acc[c][0], acc[c][1]);
+                    acc[c][0] = acc[c][1] = Two<T>::zero();
                 }
                 __syncthreads();
             }
-            const float sign = j == i ? 1.f : -1.f;
-            const float* x = X + tx * CP * kLdL + j * kT;
+            const T sign = j == i ? T(1) : T(-1);
+            const T* x = X + tx * CP * kLdL + j * kT;
 #pragma unroll 4
             for (int k = 0; k < kT; k += 4) {
-                float4 xv[CP];
+                T xv[CP][4];
 #pragma unroll
-                for (int c = 0; c < CP; ++c)
-                    xv[c] = *reinterpret_cast<const float4*>(x + c * kLdL + k);
+                for (int c = 0; c < CP; ++c) {
+                    Two<T> lo, hi;
+                    load_pairs(x + c * kLdL + k, lo, hi);
+                    lo.get(xv[c][0], xv[c][1]);
+                    hi.get(xv[c][2], xv[c][3]);
+                }
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    const ulonglong2 av = *reinterpret_cast<const ulonglong2*>(a + (k + q) * kT);
+                    Two<T> a0, a1;
+                    load_pairs(a + (k + q) * kT, a0, a1);
 #pragma unroll
                     for (int c = 0; c < CP; ++c) {
-                        const float e = sign * (q == 0 ? xv[c].x : q == 1 ? xv[c].y
-                                                       : q == 2 ? xv[c].z : xv[c].w);
-                        fma2(acc[c][0], av.x, pack2(e, e));
-                        fma2(acc[c][1], av.y, pack2(e, e));
+                        const T e = sign * xv[c][q];
+                        const Two<T> ee = Two<T>::make(e, e);
+                        acc[c][0].fma(a0, ee);
+                        acc[c][1].fma(a1, ee);
                     }
                 }
             }
@@ -320,12 +333,13 @@ __global__ void __launch_bounds__(kThr) llu_block_kernel(int rows, int cols,
 #pragma unroll
                 for (int c = 0; c < CP; ++c) {
                     const int n = tx * CP + c;
-                    const float2 p = unpack2(acc[c][0]), q = unpack2(acc[c][1]);
-                    const float v[4] = {p.x, p.y, q.x, q.y};
+                    T v[4];
+                    acc[c][0].get(v[0], v[1]);
+                    acc[c][1].get(v[2], v[3]);
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         const int r = i * kT + ty * 4 + e;
-                        if (i + 1 < nb) X[n * kLdL + r] = r < rows ? v[e] : 0.f;
+                        if (i + 1 < nb) X[n * kLdL + r] = r < rows ? v[e] : T(0);
                         if (r < rows && n < nc) B[(c0 + n) * ldb + r] = v[e];
                     }
                 }
@@ -335,36 +349,79 @@ __global__ void __launch_bounds__(kThr) llu_block_kernel(int rows, int cols,
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-// Dynamic shared memory for nb diagonal blocks; one block needs no more than the
-// default limit, so a launch without a configured handle may take it.
-template <int RP>
+// Dynamic shared memory for nb diagonal blocks; one FP32 block needs no more than
+// the default limit, so a launch without a configured handle may take it.
+template <class T, int RP>
 size_t rlt_smem(int nb)
 {
     const int nt = nb * (nb + 1) / 2;
-    return sizeof(float) * ((size_t)(nt < kRing ? nt : kRing) * kTile + (size_t)nb * kT * 16 * RP);
+    return sizeof(T) * ((size_t)(nt < kRing ? nt : kRing) * kTile + (size_t)nb * kT * 16 * RP);
 }
-template <int CP>
+template <class T, int CP>
 size_t llu_smem(int nb)
 {
     const int nt = nb * (nb + 1) / 2;
-    return sizeof(float) * ((size_t)(nt < kRing ? nt : kRing) * kTile + (size_t)16 * CP * kLdL);
+    return sizeof(T) * ((size_t)(nt < kRing ? nt : kRing) * kTile + (size_t)16 * CP * kLdL);
 }
 
-template <int RP>
-void rlt_launch(hdbf_context* ctx, int rows, int cols, const float* L, long long ldl,
-                const float* inv, float* B, long long ldb)
+template <class T, int RP>
+void rlt_launch(hdbf_context* ctx, int rows, int cols, const T* L, long long ldl, const T* inv, T* B,
+                long long ldb)
 {
     const unsigned grid = (unsigned)(((long long)rows + 16 * RP - 1) / (16 * RP));
-    rlt_block_kernel<RP><<<grid, kThr, rlt_smem<RP>((cols + kT - 1) / kT), ctx->stream>>>(
+    rlt_block_kernel<T, RP><<<grid, kThr, rlt_smem<T, RP>((cols + kT - 1) / kT), ctx->stream>>>(
         rows, cols, L, ldl, inv, B, ldb);
 }
-template <int CP>
-void llu_launch(hdbf_context* ctx, int rows, int cols, const float* L, long long ldl,
-                const float* inv, float* B, long long ldb)
+template <class T, int CP>
+void llu_launch(hdbf_context* ctx, int rows, int cols, const T* L, long long ldl, const T* inv, T* B,
+                long long ldb)
 {
     const unsigned grid = (unsigned)(((long long)cols + 16 * CP - 1) / (16 * CP));
-    llu_block_kernel<CP><<<grid, kThr, llu_smem<CP>((rows + kT - 1) / kT), ctx->stream>>>(
+    llu_block_kernel<T, CP><<<grid, kThr, llu_smem<T, CP>((rows + kT - 1) / kT), ctx->stream>>>(
         rows, cols, L, ldl, inv, B, ldb);
+}
+
+template <class T, int P>
+void configure_one()
+{
+    const int nb = kMaxW / kT;
+    cudaFuncSetAttribute(rlt_block_kernel<T, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)rlt_smem<T, P>(nb));
+    cudaFuncSetAttribute(llu_block_kernel<T, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)llu_smem<T, P>(nb));
+}
+
+template <class T>
+hdbf_status rlt_block_t(hdbf_context* ctx, int rows, int cols, const T* L, long long ldl,
+                        const T* inv, T* B, long long ldb)
+{
+    if (rows <= 0 || cols <= 0) return HDBF_STATUS_SUCCESS;
+    if (cols > kMaxW) return HDBF_STATUS_INVALID_VALUE;
+    ProfScope prof(ctx, kClsTrsmR, (double)cols * cols * rows, 2.0 * sizeof(T) * rows * cols, rows,
+                   cols, (cols + kT - 1) / kT);
+    // 64 rows per CTA when that gives two thirds of the SMs one, else 32, else 16
+    const long long full = 2LL * ctx->sm_count / 3 * 64;
+    if (rows >= full) rlt_launch<T, 4>(ctx, rows, cols, L, ldl, inv, B, ldb);
+    else if (2LL * rows >= full) rlt_launch<T, 2>(ctx, rows, cols, L, ldl, inv, B, ldb);
+    else rlt_launch<T, 1>(ctx, rows, cols, L, ldl, inv, B, ldb);
+    ctx->launches++;
+    return last_cuda(ctx);
+}
+
+template <class T>
+hdbf_status llu_block_t(hdbf_context* ctx, int rows, int cols, const T* L, long long ldl,
+                        const T* inv, T* B, long long ldb)
+{
+    if (rows <= 0 || cols <= 0) return HDBF_STATUS_SUCCESS;
+    if (rows > kMaxW) return HDBF_STATUS_INVALID_VALUE;
+    ProfScope prof(ctx, kClsTrsmL, (double)rows * rows * cols, 2.0 * sizeof(T) * rows * cols, rows,
+                   cols, (rows + kT - 1) / kT);
+    const long long full = 2LL * ctx->sm_count / 3 * 64;  // as rlt_block
+    if (cols >= full) llu_launch<T, 4>(ctx, rows, cols, L, ldl, inv, B, ldb);
+    else if (2LL * cols >= full) llu_launch<T, 2>(ctx, rows, cols, L, ldl, inv, B, ldb);
+    else llu_launch<T, 1>(ctx, rows, cols, L, ldl, inv, B, ldb);
+    ctx->launches++;
+    return last_cuda(ctx);
 }
 
 }  // namespace
@@ -373,19 +430,12 @@ int llu_block_max_rows() { return kMaxW; }
 
 void configure_trsm_block_kernels(hdbf_context*)
 {
-    const int nb = kMaxW / kT;
-    cudaFuncSetAttribute(rlt_block_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)rlt_smem<4>(nb));
-    cudaFuncSetAttribute(rlt_block_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)rlt_smem<2>(nb));
-    cudaFuncSetAttribute(rlt_block_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)rlt_smem<1>(nb));
-    cudaFuncSetAttribute(llu_block_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)llu_smem<4>(nb));
-    cudaFuncSetAttribute(llu_block_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)llu_smem<2>(nb));
-    cudaFuncSetAttribute(llu_block_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)llu_smem<1>(nb));
+    configure_one<float, 4>();
+    configure_one<float, 2>();
+    configure_one<float, 1>();
+    configure_one<double, 4>();
+    configure_one<double, 2>();
+    configure_one<double, 1>();
     cudaGetLastError();
 }
 
@@ -394,17 +444,12 @@ void configure_trsm_block_kernels(hdbf_context*)
 hdbf_status rlt_block(hdbf_context* ctx, int rows, int cols, const float* L, long long ldl,
                       const float* inv, float* B, long long ldb)
 {
-    if (rows <= 0 || cols <= 0) return HDBF_STATUS_SUCCESS;
-    if (cols > kMaxW) return HDBF_STATUS_INVALID_VALUE;
-    ProfScope prof(ctx, kClsTrsmR, (double)cols * cols * rows, 8.0 * (double)rows * cols, rows,
-                   cols, (cols + kT - 1) / kT);
-    // 64 rows per CTA when that gives two thirds of the SMs one, else 32, else 16
-    const long long full = 2LL * ctx->sm_count / 3 * 64;
-    if (rows >= full) rlt_launch<4>(ctx, rows, cols, L, ldl, inv, B, ldb);
-    else if (2LL * rows >= full) rlt_launch<2>(ctx, rows, cols, L, ldl, inv, B, ldb);
-    else rlt_launch<1>(ctx, rows, cols, L, ldl, inv, B, ldb);
-    ctx->launches++;
-    return last_cuda(ctx);
+    return rlt_block_t(ctx, rows, cols, L, ldl, inv, B, ldb);
+}
+hdbf_status rlt_block(hdbf_context* ctx, int rows, int cols, const double* L, long long ldl,
+                      const double* inv, double* B, long long ldb)
+{
+    return rlt_block_t(ctx, rows, cols, L, ldl, inv, B, ldb);
 }
 
 // B(rows x cols) <- L^{-1} B for unit lower L (rows <= 256); inv holds the
@@ -412,16 +457,12 @@ hdbf_status rlt_block(hdbf_context* ctx, int rows, int cols, const float* L, lon
 hdbf_status llu_block(hdbf_context* ctx, int rows, int cols, const float* L, long long ldl,
                       const float* inv, float* B, long long ldb)
 {
-    if (rows <= 0 || cols <= 0) return HDBF_STATUS_SUCCESS;
-    if (rows > kMaxW) return HDBF_STATUS_INVALID_VALUE;
-    ProfScope prof(ctx, kClsTrsmL, (double)rows * rows * cols, 8.0 * (double)rows * cols, rows,
-                   cols, (rows + kT - 1) / kT);
-    const long long full = 2LL * ctx->sm_count / 3 * 64;  // as rlt_block
-    if (cols >= full) llu_launch<4>(ctx, rows, cols, L, ldl, inv, B, ldb);
-    else if (2LL * cols >= full) llu_launch<2>(ctx, rows, cols, L, ldl, inv, B, ldb);
-    else llu_launch<1>(ctx, rows, cols, L, ldl, inv, B, ldb);
-    ctx->launches++;
-    return last_cuda(ctx);
+    return llu_block_t(ctx, rows, cols, L, ldl, inv, B, ldb);
+}
+hdbf_status llu_block(hdbf_context* ctx, int rows, int cols, const double* L, long long ldl,
+                      const double* inv, double* B, long long ldb)
+{
+    return llu_block_t(ctx, rows, cols, L, ldl, inv, B, ldb);
 }
 
 }  // namespace hdbf
