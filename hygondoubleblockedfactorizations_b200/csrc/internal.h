@@ -511,11 +511,12 @@ hdbf_status fill_uniform(hdbf_context* ctx, float* x, size_t count, uint64_t see
 hdbf_status add_damping(cudaStream_t s, float* A, int n, long long lda, float lambda);
 
 // ---------------------------------------------------------------- drivers
-// Cholesky of an n x n (n <= potrf_block_max_n()) diagonal block in one
-// cooperative launch; with W non-null also W = L^{-1} (lower, upper zeroed).
+// Cholesky of an n x n (n <= potrf_block_max_n()) diagonal block on one cluster;
+// with W non-null also W = L^{-1} (lower, upper zeroed), in a second launch.
 hdbf_status potrf_block(hdbf_context* ctx, int n, float* A, long long lda, int* info,
                         int info_base, float* W, long long ldw);
 int potrf_block_max_n();
+void configure_potrf_block(hdbf_context* ctx);
 // Orders up to potrf_block_max_n() also leave the 64x64 diagonal-block
 // inverses of the factor in ws_inv, for a trsm_rlt_ready with the same block.
 hdbf_status potrf_diag(hdbf_context* ctx, int n, float* A, long long lda, int* info,

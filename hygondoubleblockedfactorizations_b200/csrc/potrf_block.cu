@@ -1,27 +1,34 @@
-// Cholesky of a diagonal block of order n <= 1024 in ONE cooperative launch,
-// optionally with the inverse of its factor.
+// Cholesky of a diagonal block of order n <= 1024, optionally with the inverse of
+// its factor.
 //
 // Replaces the reference's rocsolver_spotrf call on the diagonal block
 // (src/potrf/double_blocked_potrf.cpp:34-56, call :334).  The block is cut
-// into 64 x 64 tiles (NT = ceil(n / 64) <= 16) and factored right-looking:
-// for every tile column k the CTAs solve the tiles below the diagonal against
-// the inverse D_k of the factored diagonal tile, then apply the rank-64 update
-// to the trailing tiles; with look-ahead, CTA 0 updates tile (k+1, k+1) first
-// and factors and inverts it (tile64.cuh) while the other CTAs finish the
-// update -- two bounded grid barriers per tile column.  With the
-// inverse requested, W = L^{-1} (lower, the strictly upper tiles zeroed) is
-// formed by recursive doubling over tile blocks: for siblings A and C,
-// W(C,A) = -W(C,C) (L(C,A) W(A,A)), two GEMM phases per level.
-// A recursive factorization of the same block issues ~100 small launches.
+// into 64 x 64 tiles (NT = ceil(n / 64) <= 16) and factored right-looking by one
+// thread-block cluster (potrf_cluster_kernel): CTA 0 owns the chain -- factor and
+// invert tile (k, k) (tile64.cuh), solve tile (k+1, k) against it, update tile
+// (k+1, k+1), all in its shared memory -- and the other CTAs solve the rest of
+// column k, then update the trailing tiles while CTA 0 factors the next diagonal
+// tile.  Tiles travel through L2 (each is read by several CTAs); two barriers per
+// tile column are mbarriers in every CTA's shared memory on which all CTAs arrive
+// remotely.  What bounds it is CTA 0's chain, ~15 us a tile: n = 256 62 us, n =
+// 512 126 us; with a grid-wide barrier twice per tile column and every step through
+// L2 it took 96 and 207 us.
+// With the inverse requested, W = L^{-1} (lower, the strictly upper tiles zeroed)
+// is formed by a second, cooperative launch (tile_inverse_kernel) by recursive
+// doubling over tile blocks: for siblings A and C, W(C,A) = -W(C,C) (L(C,A)
+// W(A,A)), two GEMM phases per level with bounded grid barriers.
 //
 // Pivot test and info follow LAPACK xPOTRF: the first column whose updated
 // diagonal is not > 0 (or is NaN) stops the factorization and info =
 // info_base + column + 1 (first failure wins); a block whose info is already
-// non-zero is left untouched.  Every grid-barrier wait is bounded: on expiry
-// the kernel records a timeout, and later barriers return at once.
+// non-zero is left untouched.  Every wait is bounded by the handle's poll limit:
+// on expiry the kernel records a timeout and the remaining work is skipped; a
+// cluster's CTAs then meet at a hardware barrier, so that none leaves while
+// another may still arrive in its shared memory.
 #include <algorithm>
 
 #include "internal.h"
+#include "pair.cuh"
 #include "tile64.cuh"
 
 namespace hdbf {
@@ -104,148 +111,337 @@ __device__ __forceinline__ void load_pair(float* dA, TileSrc a, float* dB, TileS
     }
 }
 
-// acc[i][j] += sum_k As[k][ty*4+i] * Bs[k][tx*4+j]
+// acc[i][j] += sum_k As[k][r4 + i] * Bs[k][c4 + j]: rows r4 = 4 (tid & 15) in
+// consecutive lanes (whole lines of C), columns c4 = 4 (tid >> 4); packed FMAs.
 __device__ __forceinline__ void tile_mma(float acc[4][4], const float* As, const float* Bs)
 {
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const int r4 = (threadIdx.x & 15) * 4, c4 = (threadIdx.x >> 4) * 4;
+    Two<float> s[2][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        s[0][j] = Two<float>::make(acc[0][j], acc[1][j]);
+        s[1][j] = Two<float>::make(acc[2][j], acc[3][j]);
+    }
 #pragma unroll 8
     for (int k = 0; k < kT; ++k) {
-        const float4 a = *reinterpret_cast<const float4*>(As + k * kLdS + ty * 4);
-        const float4 b = *reinterpret_cast<const float4*>(Bs + k * kLdS + tx * 4);
-        const float av[4] = {a.x, a.y, a.z, a.w};
+        Two<float> a0, a1;
+        load_pairs(As + k * kLdS + r4, a0, a1);
+        const float4 b = *reinterpret_cast<const float4*>(Bs + k * kLdS + c4);
         const float bv[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int j = 0; j < 4; ++j) {
+            const Two<float> bb = Two<float>::make(bv[j], bv[j]);
+            s[0][j].fma(a0, bb);
+            s[1][j].fma(a1, bb);
+        }
+    }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+    for (int j = 0; j < 4; ++j) {
+        s[0][j].get(acc[0][j], acc[1][j]);
+        s[1][j].get(acc[2][j], acc[3][j]);
     }
 }
 
+// ------------------------------------------------------------ cluster kernel
+__device__ __forceinline__ uint32_t smem_addr(const void* p)
+{
+    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+
+// Column-major tile src (leading dimension ld, zero outside rows x cols) into
+// dst[c * kLdS + r], through L2 only: other CTAs write these tiles.  Whole,
+// aligned tiles go by cp.async; the caller commits and waits either way.
+__device__ __forceinline__ void fetch_tile(float* dst, TileSrc t)
+{
+    const bool vec = t.rows == kT && t.cols == kT && t.ld % 4 == 0 &&
+                     (reinterpret_cast<uintptr_t>(t.src) & 15u) == 0;
+    if (vec) {
+#pragma unroll
+        for (int u = 0; u < kT * kT / 4 / kThreads; ++u) {
+            const int q = threadIdx.x + u * kThreads, c = q >> 4, r = (q & 15) * 4;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                             smem_addr(dst + c * kLdS + r)),
+                         "l"(t.src + (long long)c * t.ld + r)
+                         : "memory");
+        }
+    } else {
+        float v[kT * kT / kThreads];
+#pragma unroll
+        for (int u = 0; u < kT * kT / kThreads; ++u) {
+            const int q = threadIdx.x + u * kThreads, c = q >> 6, r = q & 63;
+            v[u] = (r < t.rows && c < t.cols) ? __ldcg(t.src + (long long)c * t.ld + r) : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < kT * kT / kThreads; ++u) {
+            const int q = threadIdx.x + u * kThreads;
+            dst[(q >> 6) * kLdS + (q & 63)] = v[u];
+        }
+    }
+}
+__device__ __forceinline__ void fetch_commit()
+{
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int N>
+__device__ __forceinline__ void fetch_wait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+struct ClusterSmem {
+    float tile[4][kT * kLdS];  // CTA 0: S, W, A(k+1,k), X; others: two pairs of operands
+    float X[tile64::kScratch];
+    float rd[kT];
+    unsigned long long bar[2];
+    int fail_col, stop;
+};
+
+// All CTAs of the cluster arrive on every CTA's barrier; the wait is bounded.
+struct ClusterBarrier {
+    ClusterSmem* sm;
+    int C;
+    unsigned limit;
+    int* err;
+    unsigned phase[2];
+    __device__ void arrive(int b)
+    {
+        __syncthreads();
+        if ((int)threadIdx.x < C)
+            asm volatile(
+                "{\n\t.reg .b32 ra;\n\t"
+                "mapa.shared::cluster.u32 ra, %0, %1;\n\t"
+                "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}" ::"r"(
+                    smem_addr(&sm->bar[b])),
+                "r"((int)threadIdx.x)
+                : "memory");
+    }
+    // false: the wait ran out (uniform over the CTA)
+    __device__ bool wait(int b)
+    {
+        unsigned polls = 0;
+        bool ok = true;
+        for (;;) {
+            uint32_t done;
+            asm volatile(
+                "{\n\t.reg .pred q;\n\t"
+                "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 q, [%1], %2;\n\t"
+                "selp.u32 %0, 1, 0, q;\n\t}"
+                : "=r"(done)
+                : "r"(smem_addr(&sm->bar[b])), "r"(phase[b] & 1u)
+                : "memory");
+            if (done) break;
+            if (++polls > limit) {
+                atomicCAS(err, 0, kErrTimeout);
+                ok = false;
+                break;
+            }
+        }
+        ++phase[b];
+        return __syncthreads_and(ok);
+    }
+};
+
 __global__ void __launch_bounds__(kThreads, 1)
-potrf_block_kernel(int n, float* A, long long lda, int* info, int info_base, float* W,
-                   long long ldw, float* dinv, float* Tsc, unsigned* ctr, int* fail,
-                   int* abort_flag, int* err, const int* run_if)
+potrf_cluster_kernel(int n, float* A, long long lda, int* info, int info_base, float* dinv, int* fail,
+                     int* err, const int* run_if)
+{
+    extern __shared__ __align__(16) unsigned char sm_raw[];
+    ClusterSmem& sm = *reinterpret_cast<ClusterSmem*>(sm_raw);
+    int C, rank;
+    asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(C));
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const int NT = (n + kT - 1) / kT;
+    const int tid = threadIdx.x, r4 = (tid & 15) * 4, c4 = (tid >> 4) * 4;
+    auto ext = [&](int i) { return min(kT, n - i * kT); };
+    auto tile = [&](int i, int j) { return A + (long long)(j * kT) * lda + i * kT; };
+    auto src = [&](int i, int j) { return TileSrc{tile(i, j), lda, ext(i), ext(j)}; };
+    if (tid == 0) {
+        for (int b = 0; b < 2; ++b)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&sm.bar[b])),
+                         "r"(C));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        sm.stop = ((info && *reinterpret_cast<volatile int*>(info) != 0) ||
+                   (run_if && *reinterpret_cast<const volatile int*>(run_if) == 0))
+                      ? 1
+                      : 0;
+    }
+    __syncthreads();
+    const bool skip = sm.stop != 0;  // the same in every CTA: read before any write
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (skip) {
+        if (rank == 0 && tid == 0) *fail = 1;  // no inverse either
+        return;
+    }
+    ClusterBarrier bar{&sm, C, spin_limit_of(err), err, {0u, 0u}};
+    // One CTA needs no barriers: 0 = column k ready (D_k written, step k - 1 applied),
+    // 1 = column k solved.
+    const bool solo = C == 1;
+    float acc[4][4];
+    auto clear = [&]() {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    };
+    auto store_acc = [&](float* T, int rows, int cols) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (r4 + i < rows && c4 + j < cols) T[(long long)(c4 + j) * lda + r4 + i] = acc[i][j];
+    };
+    if (rank == 0) {
+        float *S = sm.tile[0], *W = sm.tile[1], *P = sm.tile[2], *X = sm.tile[3];
+        tile64::load_lower<true>(S, A, lda, ext(0), false);
+        __syncthreads();
+        bool waiting = false;  // arrived on barrier 1, not waited yet
+        for (int k = 0; k < NT; ++k) {
+            const int f = tile64::chol64(S, ext(k), &sm.fail_col);
+            tile64::store_lower(tile(k, k), S, lda, ext(k));
+            if (f >= 0 && tid == 0) {
+                if (info) atomicCAS(info, 0, info_base + k * kT + f + 1);
+                *reinterpret_cast<volatile int*>(fail) = 1;
+            }
+            // also of a failing tile: its columns before the failing one are valid
+            tile64::inv64(S, W, sm.X, sm.rd, false);
+            tile64::store_inv(dinv + (long long)k * kT * kT, W, false);
+            if (!solo) {
+                if (waiting && !bar.wait(1)) break;
+                waiting = false;
+                bar.arrive(0);
+                if (!bar.wait(0)) break;
+            } else {
+                __syncthreads();
+            }
+            if (f >= 0 || k == NT - 1) break;
+            // X = L(k+1, k) = A(k+1, k) D_k^T
+            fetch_tile(P, src(k + 1, k));
+            fetch_commit();
+            float old[4][4];  // tile (k+1, k+1), in flight meanwhile
+            const int e = ext(k + 1);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    old[i][j] = (r4 + i < e && c4 + j <= r4 + i)
+                                    ? __ldcg(tile(k + 1, k + 1) + (long long)(c4 + j) * lda + r4 + i)
+                                    : (r4 + i == c4 + j ? 1.f : 0.f);
+            fetch_wait<0>();
+            __syncthreads();
+            clear();
+            tile_mma(acc, P, W);
+            store_acc(tile(k + 1, k), e, kT);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                *reinterpret_cast<float4*>(X + (c4 + j) * kLdS + r4) =
+                    make_float4(acc[0][j], acc[1][j], acc[2][j], acc[3][j]);
+            if (!solo) {
+                bar.arrive(1);  // its barrier also orders X
+                waiting = true;
+            } else {
+                __syncthreads();
+            }
+            clear();
+            tile_mma(acc, X, X);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) S[(c4 + j) * kLdS + r4 + i] = old[i][j] - acc[i][j];
+            __syncthreads();
+        }
+    } else {
+        const int w = rank - 1, nw = C - 1;
+        bool live = true;
+        for (int k = 0; k < NT && live; ++k) {
+            bar.arrive(0);
+            if (!bar.wait(0)) break;
+            if (tid == 0) sm.stop = *reinterpret_cast<volatile int*>(fail);
+            __syncthreads();
+            if (sm.stop || k == NT - 1) break;
+            for (int i = k + 2 + w; i < NT; i += nw) {  // L(i, k) = A(i, k) D_k^T
+                fetch_tile(sm.tile[0], src(i, k));
+                fetch_tile(sm.tile[1], {dinv + (long long)k * kT * kT, kT, kT, kT});
+                fetch_commit();
+                fetch_wait<0>();
+                __syncthreads();
+                clear();
+                tile_mma(acc, sm.tile[0], sm.tile[1]);
+                store_acc(tile(i, k), ext(i), kT);
+                __syncthreads();
+            }
+            bar.arrive(1);
+            if (!bar.wait(1)) break;
+            // A(i, j) -= L(i, k) L(j, k)^T, pairs in row order after (k+1, k+1); the
+            // next pair's operands load during this one's products
+            const int rem = NT - 1 - k, pairs = rem * (rem + 1) / 2;
+            auto pair_at = [&](int t, int& i, int& j) {
+                i = k + 1;
+                while (t > i - (k + 1)) {
+                    t -= i - k;
+                    ++i;
+                }
+                j = k + 1 + t;
+            };
+            auto fetch_pair = [&](int t, int slot) {
+                if (t < pairs) {
+                    int i, j;
+                    pair_at(t, i, j);
+                    fetch_tile(sm.tile[2 * slot], src(i, k));
+                    if (i != j) fetch_tile(sm.tile[2 * slot + 1], src(j, k));
+                }
+                fetch_commit();
+            };
+            int slot = 0;
+            fetch_pair(1 + w, 0);
+            for (int t = 1 + w; t < pairs; t += nw, slot ^= 1) {
+                int i, j;
+                pair_at(t, i, j);
+                float* T = tile(i, j);
+                const int ei = ext(i), ej = ext(j);
+                float old[4][4];
+#pragma unroll
+                for (int b = 0; b < 4; ++b)
+#pragma unroll
+                    for (int a = 0; a < 4; ++a)
+                        old[a][b] = (r4 + a < ei && c4 + b < ej && (i != j || r4 + a >= c4 + b))
+                                        ? __ldcg(T + (long long)(c4 + b) * lda + r4 + a)
+                                        : 0.f;
+                fetch_pair(t + nw, slot ^ 1);
+                fetch_wait<1>();
+                __syncthreads();
+                clear();
+                tile_mma(acc, sm.tile[2 * slot], sm.tile[2 * slot + (i != j ? 1 : 0)]);
+#pragma unroll
+                for (int b = 0; b < 4; ++b)
+#pragma unroll
+                    for (int a = 0; a < 4; ++a)
+                        if (r4 + a < ei && c4 + b < ej && (i != j || r4 + a >= c4 + b))
+                            T[(long long)(c4 + b) * lda + r4 + a] = old[a][b] - acc[a][b];
+                __syncthreads();
+            }
+            fetch_wait<0>();
+        }
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// ------------------------------------------------------------ inverse kernel
+__global__ void __launch_bounds__(kThreads, 1)
+tile_inverse_kernel(int n, const float* A, long long lda, float* W, long long ldw, const float* dinv,
+                    float* Tsc, unsigned* ctr, const int* fail, int* abort_flag, int* err)
 {
     __shared__ __align__(16) float As[kT * kLdS];
     __shared__ __align__(16) float Bs[kT * kLdS];
-    __shared__ __align__(16) float Xs[tile64::kScratch];
-    __shared__ float rd[kT];
-    __shared__ int s_fail;
-    __shared__ int s_flag;
     const int NT = (n + kT - 1) / kT;
     const int cta = blockIdx.x;
     const unsigned G = gridDim.x;
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    Sync sy{ctr, fail, abort_flag, err, G, 0u, spin_limit_of(err)};
+    const int tid = threadIdx.x, r4 = (tid & 15) * 4, c4 = (tid >> 4) * 4;
+    Sync sy{ctr, const_cast<int*>(fail), abort_flag, err, G, 0u, spin_limit_of(err)};
     auto tile = [&](int i, int j) { return A + (long long)(j * kT) * lda + i * kT; };
     auto ext = [&](int i) { return min(kT, n - i * kT); };
-
-    if (tid == 0)
-        s_flag = ((info && *reinterpret_cast<volatile int*>(info) != 0) ||
-                  (run_if && *reinterpret_cast<const volatile int*>(run_if) == 0))
-                     ? 1
-                     : 0;
-    __syncthreads();
-    const bool skip = s_flag != 0;  // same value in every CTA: read before any write
-    grid_barrier(sy);
-    if (skip) return;
-
-    // Factor and invert diagonal tile k on this CTA.  The inverse is also
-    // formed when the tile fails: the columns before the failing one are valid.
-    auto factor_diag = [&](int k) {
-        tile64::load_lower<true>(As, tile(k, k), lda, ext(k), false);
-        __syncthreads();
-        const int f = tile64::chol64(As, ext(k), &s_fail);
-        tile64::store_lower(tile(k, k), As, lda, ext(k));
-        if (f >= 0 && tid == 0) {
-            if (info) atomicCAS(info, 0, info_base + k * kT + f + 1);
-            atomicExch(fail, 1);
-        }
-        tile64::inv64(As, Bs, Xs, rd, false);
-        tile64::store_inv(dinv + (long long)k * kT * kT, Bs, false);
-        __syncthreads();
-    };
-    // A(i,j) -= L(i,k) L(j,k)^T (lower part only on the diagonal)
-    auto update_tile = [&](int k, int i, int j) {
-        load_pair<false, false>(As, {tile(i, k), lda, ext(i), ext(k)}, Bs,
-                                {tile(j, k), lda, ext(j), ext(k)});
-        __syncthreads();
-        float acc[4][4] = {};
-        tile_mma(acc, As, Bs);
-        float* T = tile(i, j);
-        float old[4][4];  // all loads in flight before the first store
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const int r = ty * 4 + a, c = tx * 4 + b;
-                old[a][b] = (r < ext(i) && c < ext(j) && (i != j || r >= c))
-                                ? __ldcg(T + (long long)c * lda + r)
-                                : 0.f;
-            }
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const int r = ty * 4 + a, c = tx * 4 + b;
-                if (r < ext(i) && c < ext(j) && (i != j || r >= c))
-                    T[(long long)c * lda + r] = old[a][b] - acc[a][b];
-            }
-        __syncthreads();
-    };
-    auto failed = [&]() -> bool {
-        if (tid == 0) s_flag = *reinterpret_cast<volatile int*>(fail) |
-                               *reinterpret_cast<volatile int*>(abort_flag);
-        __syncthreads();
-        return s_flag != 0;
-    };
-
-    // Right-looking over tile columns with look-ahead: during the trailing
-    // update of step k, CTA 0 first updates tile (k+1, k+1) and factors it
-    // while the other CTAs update the remaining tiles.
-    if (cta == 0) factor_diag(0);
-    grid_barrier(sy);
-    bool ok = !failed();
-    for (int k = 0; k < NT - 1 && ok; ++k) {
-        // P2: L(i,k) = A(i,k) D_k^T for i > k
-        for (int i = k + 1 + cta; i < NT; i += G) {
-            load_pair<false, false>(As, {tile(i, k), lda, ext(i), ext(k)}, Bs,
-                                    {dinv + (long long)k * kT * kT, kT, ext(k), ext(k)});
-            __syncthreads();
-            float acc[4][4] = {};
-            tile_mma(acc, As, Bs);
-            float* T = tile(i, k);
-#pragma unroll
-            for (int a = 0; a < 4; ++a)
-#pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    const int r = ty * 4 + a, c = tx * 4 + b;
-                    if (r < ext(i) && c < ext(k)) T[(long long)c * lda + r] = acc[a][b];
-                }
-            __syncthreads();
-        }
-        grid_barrier(sy);
-        // P3 (+ P1 of step k+1 on CTA 0): pairs t >= 1 on CTAs 1.., t = 0 is
-        // tile (k+1, k+1)
-        const int rem = NT - 1 - k;
-        const int pairs = rem * (rem + 1) / 2;
-        if (cta == 0) {
-            update_tile(k, k + 1, k + 1);
-            factor_diag(k + 1);
-        }
-        const int workers = G > 1 ? (int)G - 1 : 1;
-        const int first = G > 1 ? cta - 1 : 0;
-        if (G == 1 || cta > 0) {
-            for (int t = 1 + first; t < pairs; t += workers) {
-                int i = k + 1, left = t;
-                while (left > i - (k + 1)) { left -= i - k; ++i; }
-                update_tile(k, i, k + 1 + left);
-            }
-        }
-        grid_barrier(sy);
-        if (failed()) { ok = false; break; }
-    }
-    if (!ok || !W) return;
+    if (*fail != 0) return;  // written by the launch before: the same for every CTA
 
     // W = L^{-1} by recursive doubling over tile blocks: for sibling blocks
     // A = [b, b+s) and C = [b+s, b+2s) (tiles), W(C,A) = -W(C,C) (L(C,A) W(A,A)),
@@ -293,7 +489,7 @@ potrf_block_kernel(int n, float* A, long long lda, int* info, int info_base, flo
             for (int a = 0; a < 4; ++a)
 #pragma unroll
                 for (int bb = 0; bb < 4; ++bb) {
-                    const int r = ty * 4 + a, c = tx * 4 + bb;
+                    const int r = r4 + a, c = c4 + bb;
                     if (r < ext(ci) && c < ext(aj)) T[(long long)c * ldw + r] = acc[a][bb];
                 }
         }
@@ -317,7 +513,7 @@ potrf_block_kernel(int n, float* A, long long lda, int* info, int info_base, flo
             for (int a = 0; a < 4; ++a)
 #pragma unroll
                 for (int bb = 0; bb < 4; ++bb) {
-                    const int r = ty * 4 + a, c = tx * 4 + bb;
+                    const int r = r4 + a, c = c4 + bb;
                     if (r < ext(ci) && c < ext(aj)) Wp[(long long)c * ldw + r] = -acc[a][bb];
                 }
         }
@@ -338,10 +534,6 @@ hdbf_status potrf_block(hdbf_context* ctx, int n, float* A, long long lda, int* 
     const long long need = W ? ((long long)ldw * n + 255) / 256 : 0;
     HDBF_TRY(ensure_ws(ctx, (int)std::max<long long>(n, std::max<long long>(need, 64))));
     const int NT = (n + kT - 1) / kT;
-    int G = NT * (NT - 1) / 2;
-    if (W && NT * NT > G) G = NT * NT;  // the W set-up pass touches NT^2 tiles
-    if (G > ctx->sm_count) G = ctx->sm_count;
-    if (G < 1) G = 1;
     int* sm = ctx->dev_small + kSmallBlockBar;
     if (cudaMemsetAsync(sm, 0, 3 * sizeof(int), ctx->stream) != cudaSuccess) return last_cuda(ctx);
     unsigned* ctr = reinterpret_cast<unsigned*>(sm);
@@ -349,20 +541,51 @@ hdbf_status potrf_block(hdbf_context* ctx, int n, float* A, long long lda, int* 
     int* abort_flag = sm + 2;
     int* err = ctx->dev_small + kSmallErr;
     float* dinv = ws_inv(ctx);
-    float* Tsc = ws_skinny(ctx);  // n x n scratch (leading dimension ldw) for the inverse
     const double flops = (double)n * n * n / 3.0 + (W ? (double)n * n * n / 3.0 : 0.0);
     ProfScope prof(ctx, kClsPotrfBlock, flops, 8.0 * n * n, n, n, n);
-    const int* run_if = ctx->run_if;
-    void* args[] = {&n, &A, &lda, &info, &info_base, &W, &ldw, &dinv, &Tsc, &ctr, &fail,
-                    &abort_flag, &err, &run_if};
-    const cudaError_t e = cudaLaunchCooperativeKernel((const void*)potrf_block_kernel, dim3(G),
-                                                      dim3(kThreads), args, 0, ctx->stream);
+    // Workers for the pairs of a tile column: none for two tiles (CTA 0 does all
+    // there is), 3 for three, 7 for four, 15 above.
+    int C = NT <= 2 ? 1 : (NT == 3 ? 4 : (NT == 4 ? 8 : 16));
+    while (C > std::max(1, ctx->cluster_max)) C /= 2;
+    if (C == 2) C = 1;
+    if (C == 1 && NT > 2) return HDBF_STATUS_NOT_SUPPORTED;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(C);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = sizeof(ClusterSmem);
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = C;
+    at.val.clusterDim.y = 1;
+    at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, potrf_cluster_kernel, n, A, lda, info, info_base, dinv,
+                                       fail, err, ctx->run_if);
     ctx->launches++;
+    if (e == cudaSuccess && W) {
+        int G = std::min(NT * NT, ctx->sm_count);  // the set-up pass touches NT^2 tiles
+        float* Tsc = ws_skinny(ctx);  // n x n scratch (leading dimension ldw)
+        const float* Ac = A;
+        void* args[] = {&n, &Ac, &lda, &W, &ldw, &dinv, &Tsc, &ctr, &fail, &abort_flag, &err};
+        e = cudaLaunchCooperativeKernel((const void*)tile_inverse_kernel, dim3(G), dim3(kThreads),
+                                        args, 0, ctx->stream);
+        ctx->launches++;
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         return HDBF_STATUS_CUDA_ERROR;
     }
     return HDBF_STATUS_SUCCESS;
+}
+
+void configure_potrf_block(hdbf_context*)
+{
+    cudaFuncSetAttribute(potrf_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)sizeof(ClusterSmem));
+    cudaFuncSetAttribute(potrf_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaGetLastError();
 }
 
 }  // namespace hdbf

@@ -420,6 +420,7 @@ hdbf_status hdbf_create(hdbf_handle* handle)
     configure_tc_sgemm(ctx);
     configure_gemm_small(ctx);
     configure_tile_kernels(ctx);
+    configure_potrf_block(ctx);
     configure_trsm_block_kernels(ctx);
     configure_solve_kernels(ctx);
     configure_batched_kernels(ctx);
