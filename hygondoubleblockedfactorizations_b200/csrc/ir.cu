@@ -38,40 +38,88 @@ __global__ void d2s_kernel(const double* __restrict__ A, long long lda, float* W
 }
 
 // partial[s][c][r] = sum_{j in split s} A(r, j) * X(j, c) for the RHS group
-// blockIdx.z (columns 16 z .. 16 z + 15).
+// blockIdx.z (columns G z .. G z + G - 1).  Bound: A from HBM once (8 n^2 bytes).
+// A thread takes R rows, so that an X value from shared memory serves R FMAs,
+// and has 8 R loads of A in flight (one load at a time left it at 30% of the
+// bandwidth: 1.0 ms at n = 16384, now 0.65).
+template <int R, int G>
 __global__ void __launch_bounds__(kRowsPerCta) resid_partial_kernel(
     const double* __restrict__ A, long long lda, const double* __restrict__ X, long long ldx, int n,
     int nrhs, double* partial)
 {
-    __shared__ double xs[kJChunk][kRhsGroup];
-    const int r = blockIdx.x * kRowsPerCta + threadIdx.x;
+    constexpr int kU = 8;
+    __shared__ __align__(16) double xs[kJChunk][G];
+    const int r0 = blockIdx.x * kRowsPerCta * R + threadIdx.x;
     const int s = blockIdx.y;
-    const int c0 = blockIdx.z * kRhsGroup;
-    const int nc = min(kRhsGroup, nrhs - c0);
+    const int c0 = blockIdx.z * G;
+    const int nc = min(G, nrhs - c0);
     const int per = (n + kSplits - 1) / kSplits;
     const int j0 = s * per, j1 = min(n, j0 + per);
-    double acc[kRhsGroup];
+    double acc[R][G];
 #pragma unroll
-    for (int c = 0; c < kRhsGroup; ++c) acc[c] = 0.0;
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int c = 0; c < G; ++c) acc[i][c] = 0.0;
     for (int jb = j0; jb < j1; jb += kJChunk) {
         const int jn = min(kJChunk, j1 - jb);
         __syncthreads();
-        for (int idx = threadIdx.x; idx < kJChunk * kRhsGroup; idx += kRowsPerCta) {
-            const int jj = idx / kRhsGroup, c = idx % kRhsGroup;
+        for (int idx = threadIdx.x; idx < kJChunk * G; idx += kRowsPerCta) {
+            const int c = idx / kJChunk, jj = idx % kJChunk;
             xs[jj][c] = (jj < jn && c < nc) ? X[(long long)(c0 + c) * ldx + jb + jj] : 0.0;
         }
         __syncthreads();
-        if (r < n) {
-            for (int jj = 0; jj < jn; ++jj) {
-                const double a = A[(long long)(jb + jj) * lda + r];
+        for (int jj = 0; jj < jn; jj += kU) {
+            double a[R][kU];
 #pragma unroll
-                for (int c = 0; c < kRhsGroup; ++c) acc[c] = fma(a, xs[jj][c], acc[c]);
+            for (int u = 0; u < kU; ++u)
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    const int r = r0 + i * kRowsPerCta;
+                    a[i][u] = (r < n && jj + u < jn) ? A[(long long)(jb + jj + u) * lda + r] : 0.0;
+                }
+#pragma unroll
+            for (int u = 0; u < kU; ++u) {
+                if (jj + u >= jn) break;
+#pragma unroll
+                for (int c = 0; c < G; c += 2) {
+                    const double2 x = *reinterpret_cast<const double2*>(&xs[jj + u][c]);
+#pragma unroll
+                    for (int i = 0; i < R; ++i) {
+                        acc[i][c] = fma(a[i][u], x.x, acc[i][c]);
+                        acc[i][c + 1] = fma(a[i][u], x.y, acc[i][c + 1]);
+                    }
+                }
             }
         }
     }
-    if (r < n)
-        for (int c = 0; c < nc; ++c)
-            partial[((long long)s * nrhs + c0 + c) * n + r] = acc[c];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const int r = r0 + i * kRowsPerCta;
+        if (r < n) {
+#pragma unroll
+            for (int c = 0; c < G; ++c)
+                if (c < nc) partial[((long long)s * nrhs + c0 + c) * n + r] = acc[i][c];
+        }
+    }
+}
+
+// Right-hand sides in groups of 16, or of 4 when there are no more; two rows per
+// thread once that still gives every SM a CTA.
+void resid_partial(cudaStream_t s, const double* A, long long lda, const double* X, long long ldx,
+                   int n, int nrhs, double* partial)
+{
+    const int g = nrhs <= 4 ? 4 : kRhsGroup, rows = n >= 4096 ? 2 : 1;
+    const dim3 grid((n + kRowsPerCta * rows - 1) / (kRowsPerCta * rows), kSplits, (nrhs + g - 1) / g);
+    if (g == 4 && rows == 2)
+        resid_partial_kernel<2, 4><<<grid, kRowsPerCta, 0, s>>>(A, lda, X, ldx, n, nrhs, partial);
+    else if (g == 4)
+        resid_partial_kernel<1, 4><<<grid, kRowsPerCta, 0, s>>>(A, lda, X, ldx, n, nrhs, partial);
+    else if (rows == 2)
+        resid_partial_kernel<2, kRhsGroup>
+            <<<grid, kRowsPerCta, 0, s>>>(A, lda, X, ldx, n, nrhs, partial);
+    else
+        resid_partial_kernel<1, kRhsGroup>
+            <<<grid, kRowsPerCta, 0, s>>>(A, lda, X, ldx, n, nrhs, partial);
 }
 
 // R(r, c) = B(r, c) - sum_s partial[s][c][r]
@@ -108,7 +156,13 @@ __global__ void rowabs_partial_kernel(const double* __restrict__ A, long long ld
     const int per = (n + kSplits - 1) / kSplits;
     const int j0 = s * per, j1 = min(n, j0 + per);
     double acc = 0.0;
-    for (int j = j0; j < j1; ++j) acc += fabs(A[(long long)j * lda + r]);
+    for (int j = j0; j < j1; j += 8) {  // eight loads in flight
+        double v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = j + u < j1 ? A[(long long)(j + u) * lda + r] : 0.0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) acc += fabs(v[u]);
+    }
     partial[(long long)s * n + r] = acc;
 }
 
@@ -414,9 +468,8 @@ public:
     hdbf_status matvec(const double* Xv, double* Y)
     {
         cudaStream_t s = ctx_->stream;
-        dim3 g1((n_ + kRowsPerCta - 1) / kRowsPerCta, kSplits, (nrhs_ + kRhsGroup - 1) / kRhsGroup);
         ProfScope prof(ctx_, kClsIr, 2.0 * (double)n_ * n_ * nrhs_, 8.0 * (double)n_ * n_);
-        resid_partial_kernel<<<g1, kRowsPerCta, 0, s>>>(A_, lda_, Xv, n_, n_, nrhs_, b_.part);
+        resid_partial(s, A_, lda_, Xv, n_, n_, nrhs_, b_.part);
         dim3 g2((n_ + 255) / 256, nrhs_);
         matvec_final_kernel<<<g2, 256, 0, s>>>(b_.part, Y, n_, nrhs_);
         ctx_->launches += 2;
@@ -463,9 +516,8 @@ public:
     hdbf_status residual()
     {
         cudaStream_t s = ctx_->stream;
-        dim3 g1((n_ + kRowsPerCta - 1) / kRowsPerCta, kSplits, (nrhs_ + kRhsGroup - 1) / kRhsGroup);
         ProfScope prof(ctx_, kClsIr, 2.0 * (double)n_ * n_ * nrhs_, 8.0 * (double)n_ * n_);
-        resid_partial_kernel<<<g1, kRowsPerCta, 0, s>>>(A_, lda_, X_, ldx_, n_, nrhs_, b_.part);
+        resid_partial(s, A_, lda_, X_, ldx_, n_, nrhs_, b_.part);
         dim3 g2((n_ + 255) / 256, nrhs_);
         resid_final_kernel<<<g2, 256, 0, s>>>(b_.part, B_, ldb_, b_.R, n_, n_, nrhs_);
         ctx_->launches += 2;
