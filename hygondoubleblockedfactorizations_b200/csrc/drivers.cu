@@ -142,22 +142,24 @@ hdbf_status panel_swaps(hdbf_context* ctx, double* A, long long lda, const int* 
 }
 
 // Leaf width for the cluster panel kernel at height m, 0 for the grid-wide one.
-// A cluster holds 64 or more columns up to m = 13300 (FP32): there a column
-// costs 1.7-2.0 us against 4.1-4.5 us.  Taller panels would need leaves of 32
-// or 16 columns (2.4 and 4.6 us a column at m = 16384 and 30000), and the extra
-// merges between them (compose, moves, TRSM, GEMM: ~130 us each) cost more than
-// the grid-wide kernel's 128-column leaf (5-6.5 us a column).
+// The cluster has the cheaper columns while a thread has one row (512 threads a
+// CTA, m <= 8192): 1.3-1.8 us against the grid's 1.9-2.0 us.  Above, its columns
+// cost as much or more (2.4 and 4.6 us at m = 16384 and 30000) and its leaves
+// narrow to 64 columns and fewer, each merge of two (swaps, TRSM, GEMM) ~40 us more.
+// FP32 LU: leaves of 256 bytes up to m = 13300 / up to 8192 / none: n = 8192 25.4 /
+// 25.4 / 25.6 ms, n = 32768 260.3 / 257-259 / 257.4 ms.
 int panel_cluster_leaf(hdbf_context* ctx, int m, int elem)
 {
     if (ctx->panel_mode == 1) return 0;
     const int leaf = getf2_cluster_leaf(ctx, m, elem);
-    return ctx->panel_mode == 2 || leaf * elem >= 256 ? leaf : 0;
+    if (ctx->panel_mode == 2 || leaf * elem >= 512) return leaf;
+    return leaf * elem >= 256 && m <= 512 * ctx->cluster_max ? leaf : 0;
 }
 
 // Recursive (Toledo/Gustavson) LU of an m x w panel.  A leaf is as wide as one
-// cluster can hold at this height, at most the handle's panel-leaf width (32
-// when the cluster kernel is forced); heights beyond a cluster, and the forced
-// grid-wide kernel, take leaves of the panel-leaf width on getf2_coop.  ipiv
+// cluster can hold at this height, or the grid above that and where the grid-wide
+// kernel is forced, at most the handle's panel-leaf width (32 when the cluster
+// kernel is forced).  ipiv
 // receives (local row + 1 + ipiv_add) for the panel's w columns.
 hdbf_status getrf_panel(hdbf_context* ctx, int m, int w, float* A, long long lda, int* ipiv,
                         int ipiv_add, int* info, int info_base, bool pivot, const GetrfWs& ws)
@@ -165,10 +167,12 @@ hdbf_status getrf_panel(hdbf_context* ctx, int m, int w, float* A, long long lda
     if (m <= 0 || w <= 0) return HDBF_STATUS_SUCCESS;
     const int held = panel_cluster_leaf(ctx, m, (int)sizeof(float));
     const int widest = ctx->panel_mode == 2 ? kClusterLeaf : ctx->panel_leaf;
-    const int leaf = held > 0 ? std::min(held, widest) : widest;
+    const int leaf =
+        std::min(held > 0 ? held : getf2_grid_leaf(ctx, m, (int)sizeof(float)), widest);
+    if (leaf < 1) return HDBF_STATUS_NOT_SUPPORTED;
     if (w <= leaf) {
         if (held > 0) return getf2_cluster(ctx, m, w, A, lda, ipiv, ipiv_add, info, info_base, pivot);
-        return getf2_coop(ctx, m, w, A, lda, ipiv, ipiv_add, info, info_base, pivot);
+        return getf2_grid(ctx, m, w, A, lda, ipiv, ipiv_add, info, info_base, pivot);
     }
     const int w1 = split_at(w, leaf);
     const int w2 = w - w1;

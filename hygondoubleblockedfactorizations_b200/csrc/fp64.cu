@@ -11,19 +11,9 @@
 //   trsm_rlt / trsm_llu      recursive TRSMs on the leaves of trsm_block.cu
 //                            (diagonal tiles and inverses: panel_kernels.cu)
 //   potrf_diag, syrk_lower   recursive diagonal Cholesky, lower SYRK
-//   getrf_panel              recursive LU panel on the grid-wide leaf below
+//   getrf_panel              recursive LU panel on the leaves of getf2_cluster.cu
+//                            and getf2_grid.cu
 //   apply_moves              composed row moves, gathered through scratch
-//
-// The panel leaf (getf2_coop64_kernel, <= 64 columns) keeps ~256 rows per
-// CTA in shared memory and runs one global exchange per column: every CTA
-// writes its candidate (|a|, row, the candidate row and, from the owner, the
-// diagonal row) into its slot and publishes a sequence number with a release
-// store; every CTA polls all sequence numbers with acquire loads (bounded),
-// picks the same winner (largest |a|, lowest row on ties -- LAPACK IDAMAX),
-// swaps, scales by the reciprocal pivot (division when |pivot| < DBL_MIN, as
-// xGETF2) and applies the rank-1 update to its own rows.  Sequence numbers
-// are epoch * 256 + column + 1 (epoch = the panel launch counter shared with
-// the FP32 leaf, column < 64), so no launch accepts another launch's slot.
 #include <algorithm>
 #include <cfloat>
 #include <climits>
@@ -319,236 +309,6 @@ hdbf_status trsm_llu_rec64(hdbf_context* ctx, int rows, int cols, const double* 
                           inv + (long long)(r1 / kL) * kL * kL);
 }
 
-// ------------------------------------------------------------ panel leaf
-constexpr int kPThreads = 256;
-constexpr int kPMaxW = 64;
-constexpr int kPMaxGrid = 256;
-// Slot in doubles: [seq (u32) | |a| | row (int) | pad | candidate row | diagonal row]
-constexpr int kPSlot = 4 + 2 * kPMaxW;
-
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p)
-{
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v)
-{
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-__device__ __forceinline__ bool dbetter(double v, int i, double bv, int bi)
-{
-    if (i == INT_MAX) return false;
-    if (bi == INT_MAX) return true;
-    return v > bv || (v == bv && i < bi);
-}
-
-__global__ void __launch_bounds__(kPThreads)
-getf2_coop64_kernel(int m, int w, double* A, long long lda, int rpc, int* ipiv, int ipiv_add,
-                    int* info, int info_base, double* scr, unsigned* epoch_ptr,
-                    unsigned* done_ptr, int* err, int pivot)
-{
-    extern __shared__ double dtile[];  // dtile[c * rpc + r]
-    __shared__ double prow[kPMaxW];
-    __shared__ double orow[kPMaxW];
-    __shared__ double red_v[kPThreads / 32];
-    __shared__ int red_i[kPThreads / 32];
-    __shared__ double cv[kPMaxGrid];
-    __shared__ int ci[kPMaxGrid];
-    __shared__ int s_best_row, s_win_cta, s_abort, s_last;
-
-    const int G = gridDim.x;
-    const int cta = blockIdx.x;
-    const int tid = threadIdx.x;
-    const int lane = tid & 31, warp = tid >> 5;
-    const int r0 = cta * rpc;
-    const int nr = max(0, min(m, r0 + rpc) - r0);
-    const unsigned epoch = *reinterpret_cast<volatile unsigned*>(epoch_ptr);
-    auto slot_of = [&](int par, int q) { return scr + ((long long)par * kPMaxGrid + q) * kPSlot; };
-
-    for (int e = tid; e < nr * w; e += kPThreads) {
-        const int c = e / nr, r = e - c * nr;
-        dtile[c * rpc + r] = A[(long long)c * lda + r0 + r];
-    }
-    if (tid == 0) s_abort = 0;
-    __syncthreads();
-
-    const int steps = min(m, w);
-    for (int j = 0; j < steps; ++j) {
-        const int par = j & 1;
-        const unsigned seq = (epoch << 8) + (unsigned)j + 1u;
-        double* slot = slot_of(par, cta);
-        const int owner = j / rpc;
-
-        // 1. local candidate over owned rows >= j
-        double bv = -1.0;
-        int bi = INT_MAX;
-        if (pivot) {
-            for (int r = tid; r < nr; r += kPThreads) {
-                if (r0 + r >= j) {
-                    const double v = fabs(dtile[j * rpc + r]);
-                    if (bi == INT_MAX || v > bv) { bv = v; bi = r0 + r; }
-                }
-            }
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                const double ov = __shfl_down_sync(0xffffffffu, bv, off);
-                const int oi = __shfl_down_sync(0xffffffffu, bi, off);
-                if (dbetter(ov, oi, bv, bi)) { bv = ov; bi = oi; }
-            }
-            if (lane == 0) { red_v[warp] = bv; red_i[warp] = bi; }
-            __syncthreads();
-            if (tid == 0) {
-                for (int q = 1; q < kPThreads / 32; ++q)
-                    if (dbetter(red_v[q], red_i[q], bv, bi)) { bv = red_v[q]; bi = red_i[q]; }
-                s_best_row = bi;
-                red_v[0] = bv;
-            }
-            __syncthreads();
-        }
-
-        // 2. publish
-        const int my_best = pivot ? s_best_row : INT_MAX;
-        if (tid < w) {
-            if (my_best != INT_MAX) slot[4 + tid] = dtile[tid * rpc + (my_best - r0)];
-            if (cta == owner) slot[4 + kPMaxW + tid] = dtile[tid * rpc + (j - r0)];
-        }
-        if (tid == 0) {
-            slot[1] = pivot ? red_v[0] : -1.0;
-            reinterpret_cast<int*>(slot + 2)[0] = my_best;
-        }
-        __syncthreads();
-        // The release store (after the barrier) orders every thread's slot
-        // writes before the sequence number that other CTAs acquire.
-        if (tid == 0) st_release_u32(reinterpret_cast<unsigned*>(slot), seq);
-
-        // 3. poll every slot (thread q watches CTA q), bounded
-        for (int q = tid; q < G; q += kPThreads) {
-            const double* sq = slot_of(par, q);
-            unsigned polls = 0;
-            while (ld_acquire_u32(reinterpret_cast<const unsigned*>(sq)) != seq) {
-                if (++polls > spin_limit_of(err)) {
-                    atomicCAS(err, 0, kErrTimeout);
-                    s_abort = 1;
-                    break;
-                }
-                if (polls > 256) __nanosleep(32);
-            }
-            cv[q] = __ldcg(sq + 1);
-            ci[q] = __ldcg(reinterpret_cast<const int*>(sq + 2));
-        }
-        __syncthreads();
-        if (s_abort) break;
-
-        // 4. global winner, identical on every CTA
-        if (!pivot) {
-            if (tid == 0) { s_best_row = j; s_win_cta = -1; }
-        } else if (warp == 0) {
-            double gv = -1.0;
-            int gi = INT_MAX, gc = 0;
-            for (int q = lane; q < G; q += 32)
-                if (dbetter(cv[q], ci[q], gv, gi)) { gv = cv[q]; gi = ci[q]; gc = q; }
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                const double ov = __shfl_down_sync(0xffffffffu, gv, off);
-                const int oi = __shfl_down_sync(0xffffffffu, gi, off);
-                const int oc = __shfl_down_sync(0xffffffffu, gc, off);
-                if (dbetter(ov, oi, gv, gi)) { gv = ov; gi = oi; gc = oc; }
-            }
-            if (lane == 0) { s_best_row = gi; s_win_cta = gc; }
-        }
-        __syncthreads();
-        const int p = s_best_row;
-        if (tid < w) {
-            const double* so = slot_of(par, owner);
-            orow[tid] = __ldcg(so + 4 + kPMaxW + tid);
-            if (s_win_cta >= 0) prow[tid] = __ldcg(slot_of(par, s_win_cta) + 4 + tid);
-            else prow[tid] = orow[tid];
-        }
-        if (pivot && cta == 0 && tid == 0) ipiv[j] = p + 1 + ipiv_add;
-        __syncthreads();
-
-        // 5. swap rows j and p (within this column block), scale, rank-1 update
-        if (p != j && tid < w) {
-            if (j >= r0 && j < r0 + nr) dtile[tid * rpc + (j - r0)] = prow[tid];
-            if (p >= r0 && p < r0 + nr) dtile[tid * rpc + (p - r0)] = orow[tid];
-        }
-        __syncthreads();
-        const double piv = prow[j];
-        const bool nz = piv != 0.0;
-        const bool recip = fabs(piv) >= DBL_MIN;
-        const double rcp = 1.0 / piv;
-        if (!nz && cta == 0 && tid == 0 && info) atomicCAS(info, 0, info_base + j + 1);
-        for (int r = tid; r < nr; r += kPThreads) {
-            if (r0 + r > j) {
-                double l = dtile[j * rpc + r];
-                if (nz) {
-                    l = recip ? l * rcp : l / piv;
-                    dtile[j * rpc + r] = l;
-                }
-                for (int c = j + 1; c < w; ++c)
-                    dtile[c * rpc + r] = fma(-l, prow[c], dtile[c * rpc + r]);
-            }
-        }
-        __syncthreads();
-    }
-
-    for (int e = tid; e < nr * w; e += kPThreads) {
-        const int c = e / nr, r = e - c * nr;
-        A[(long long)c * lda + r0 + r] = dtile[c * rpc + r];
-    }
-
-    // Advance the shared launch counter once every CTA is done.
-    __syncthreads();
-    if (tid == 0) {
-        __threadfence();
-        s_last = atomicAdd(done_ptr, 1u) + 1u == (unsigned)G;
-    }
-    __syncthreads();
-    if (s_last && tid == 0) {
-        __threadfence();
-        atomicExch(done_ptr, 0u);
-        atomicAdd(epoch_ptr, 1u);
-    }
-}
-
-hdbf_status getf2_coop64(hdbf_context* ctx, int m, int w, double* A, long long lda, int* ipiv,
-                         int ipiv_add, int* info, int info_base, bool pivot)
-{
-    int piv_flag = pivot ? 1 : 0;
-    if (m <= 0 || w <= 0) return HDBF_STATUS_SUCCESS;
-    if (w > kPMaxW) return HDBF_STATUS_INVALID_VALUE;
-    const size_t smem_cap = ctx->max_smem_optin > 8192 ? ctx->max_smem_optin - 8192 : 40960;
-    const size_t row_bytes = (size_t)w * sizeof(double);
-    const long long fit_rows = (long long)(smem_cap / row_bytes);
-    const int target = ctx->panel_rows > 0 ? ctx->panel_rows : 256;
-    int G = (m + target - 1) / target;
-    if (fit_rows > 0 && (m + fit_rows - 1) / fit_rows > G) G = (int)((m + fit_rows - 1) / fit_rows);
-    if (G > ctx->sm_count) G = ctx->sm_count;
-    if (G > kPMaxGrid) G = kPMaxGrid;
-    if (G < 1) G = 1;
-    int rpc = (m + G - 1) / G;
-    size_t smem = (size_t)rpc * w * sizeof(double);
-    if (smem > smem_cap) return HDBF_STATUS_NOT_SUPPORTED;
-    double* scr = ws_coop64(ctx);
-    unsigned* epoch = reinterpret_cast<unsigned*>(ctx->dev_small + kSmallEpoch);
-    unsigned* done = reinterpret_cast<unsigned*>(ctx->dev_small + kSmallDone);
-    int* err = ctx->dev_small + kSmallErr;
-    ProfScope prof(ctx, kClsPanel, (double)m * w * w - (double)w * w * w / 3.0, 16.0 * m * w);
-    void* args[] = {&m, &w, &A, &lda, &rpc, &ipiv, &ipiv_add, &info, &info_base,
-                    &scr, &epoch, &done, &err, &piv_flag};
-    cudaError_t e = cudaLaunchCooperativeKernel((const void*)getf2_coop64_kernel, dim3(G),
-                                                dim3(kPThreads), args, smem, ctx->stream);
-    ctx->launches++;
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return HDBF_STATUS_CUDA_ERROR;
-    }
-    return HDBF_STATUS_SUCCESS;
-}
-
 // --------------------------------------------------------------- row moves
 // Gather every moved source row of nc columns into scratch, then scatter to
 // the targets (sources and targets are the same row set).
@@ -577,19 +337,6 @@ __global__ void dscatter_rows_kernel(double* A, long long lda, int nc, const int
 }
 
 }  // namespace
-
-size_t getf2_coop64_scratch_bytes()
-{
-    return align_up((size_t)2 * kPMaxGrid * kPSlot * sizeof(double), 256);
-}
-
-void configure_fp64_kernels(hdbf_context* ctx)
-{
-    const size_t cap = ctx->max_smem_optin > 8192 ? ctx->max_smem_optin - 8192 : 40960;
-    cudaFuncSetAttribute(getf2_coop64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)cap);
-    cudaGetLastError();
-}
 
 hdbf_status gemm_sub(hdbf_context* ctx, bool nn, bool lower_only, int M, int N, int K,
                      const double* A, long long lda, const double* B, long long ldb, double* C,
@@ -675,16 +422,17 @@ hdbf_status apply_moves(hdbf_context* ctx, double* A, long long lda, int ncols, 
 }
 
 // Recursive (Toledo/Gustavson) LU of an m x w FP64 panel; leaves as in the FP32
-// panel (64 columns on the grid-wide kernel).
+// panel.
 hdbf_status getrf_panel(hdbf_context* ctx, int m, int w, double* A, long long lda, int* ipiv,
                         int ipiv_add, int* info, int info_base, bool pivot, const GetrfWs& ws)
 {
     if (m <= 0 || w <= 0) return HDBF_STATUS_SUCCESS;
     const int held = panel_cluster_leaf(ctx, m, (int)sizeof(double));
-    const int leaf = held > 0 ? held : kPMaxW;
+    const int leaf = held > 0 ? held : getf2_grid_leaf(ctx, m, (int)sizeof(double));
+    if (leaf < 1) return HDBF_STATUS_NOT_SUPPORTED;
     if (w <= leaf) {
         if (held > 0) return getf2_cluster(ctx, m, w, A, lda, ipiv, ipiv_add, info, info_base, pivot);
-        return getf2_coop64(ctx, m, w, A, lda, ipiv, ipiv_add, info, info_base, pivot);
+        return getf2_grid(ctx, m, w, A, lda, ipiv, ipiv_add, info, info_base, pivot);
     }
     const int w1 = std::max(leaf, w / 2 / leaf * leaf);
     const int w2 = w - w1;

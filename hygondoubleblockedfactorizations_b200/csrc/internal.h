@@ -15,7 +15,7 @@ enum KernelClass {
     kClsPotf2 = 1,    // potf2_kernel
     kClsTrsmR = 2,    // rlt_apply_kernel
     kClsTrsmL = 3,    // llu_apply_kernel
-    kClsPanel = 4,    // getf2_cluster_kernel / getf2_coop_kernel
+    kClsPanel = 4,    // getf2_cluster_kernel / getf2_grid_kernel
     kClsCompose = 5,  // compose_swaps_kernel
     kClsMoves = 6,    // apply_moves kernels
     kClsTrsmInv = 7,  // tri_inv64_kernel
@@ -261,10 +261,9 @@ void* workspace(hdbf_context* ctx, size_t bytes, hdbf_status* st);
 void* mixed_arena(hdbf_context* ctx, size_t bytes, hdbf_status* st);
 
 // Workspace layout for problems of order <= n (byte offsets):
-//   coop  panel-kernel exchange slots (fixed size, offset 0)
+//   panel  panel-kernel exchange slots (fixed size, offset 0)
 //   inv   inverted 64x64 diagonal blocks, ceil(n/64)*4096 floats
 //   perm  running composed row permutation of a GETRF outer block, n ints
-//   coop64  FP64 panel-kernel exchange slots (fixed size)
 //   src, tgt, gperm  composed row moves / permutation scratch, n ints each
 //   temp  column-tiled swap buffer, 64*n floats
 //   skinny  split-K partial sums of the skinny GEMM, 256*n floats
@@ -272,7 +271,7 @@ void* mixed_arena(hdbf_context* ctx, size_t bytes, hdbf_status* st);
 //   words BF16 words of the operands of an FP32 update on the tensor cores, one
 //         half per stream (handle's, look-ahead)
 struct WsLayout {
-    size_t coop, inv, perm, coop64, src, tgt, gperm, temp, skinny, wave, split, words, total;
+    size_t panel, inv, perm, src, tgt, gperm, temp, skinny, wave, split, words, total;
 };
 // Split-K partial sums of under-filled FP32 GEMM launches: two halves of
 // kSplitFloats each, one for the handle's stream and one for its look-ahead
@@ -281,10 +280,9 @@ constexpr size_t kSplitFloats = (size_t)32 << 20;
 WsLayout ws_layout(int n);
 // Guarantee the layout for order n (grows the arena outside stream capture).
 hdbf_status ensure_ws(hdbf_context* ctx, int n);
-float* ws_coop(hdbf_context* ctx);
+void* ws_panel(hdbf_context* ctx);
 float* ws_inv(hdbf_context* ctx);
 int* ws_perm(hdbf_context* ctx);
-double* ws_coop64(hdbf_context* ctx);
 int* ws_src(hdbf_context* ctx);
 int* ws_tgt(hdbf_context* ctx);
 int* ws_gperm(hdbf_context* ctx);
@@ -414,23 +412,27 @@ size_t wave_scratch_bytes(int n);
 void configure_wave_kernels(hdbf_context* ctx);
 void configure_batched_kernels(hdbf_context* ctx);
 
-// Cooperative partially pivoted LU of an m x w panel (w <= 128).  Pivots are
-// written 1-based as (local row + 1 + ipiv_add).
-hdbf_status getf2_coop(hdbf_context* ctx, int m, int w, float* A, long long lda, int* ipiv,
-                       int ipiv_add, int* info, int info_base, bool pivot);
-size_t getf2_coop_scratch_bytes();
-void configure_getrf_kernels(hdbf_context* ctx);
-// Same contract on one thread-block cluster with the block in distributed
-// shared memory (getf2_cluster.cu), FP32 and FP64; NOT_SUPPORTED when w is above
-// getf2_cluster_leaf(m).
+// Partially pivoted LU of an m x w panel leaf, FP32 and FP64.  Pivots are written
+// 1-based as (local row + 1 + ipiv_add).  On one thread-block cluster with the
+// block in distributed shared memory (getf2_cluster.cu), or grid-wide with rows in
+// registers (getf2_grid.cu); NOT_SUPPORTED when w is above getf2_*_leaf(m).
 hdbf_status getf2_cluster(hdbf_context* ctx, int m, int w, float* A, long long lda, int* ipiv,
                           int ipiv_add, int* info, int info_base, bool pivot);
 hdbf_status getf2_cluster(hdbf_context* ctx, int m, int w, double* A, long long lda, int* ipiv,
                           int ipiv_add, int* info, int info_base, bool pivot);
-// Widest leaf one cluster holds at height m for elements of `elem` bytes (0: none).
+hdbf_status getf2_grid(hdbf_context* ctx, int m, int w, float* A, long long lda, int* ipiv,
+                       int ipiv_add, int* info, int info_base, bool pivot);
+hdbf_status getf2_grid(hdbf_context* ctx, int m, int w, double* A, long long lda, int* ipiv,
+                       int ipiv_add, int* info, int info_base, bool pivot);
+// Widest leaf that one cluster, or the grid, holds at height m for elements of
+// `elem` bytes (0: none).
 int getf2_cluster_leaf(hdbf_context* ctx, int m, int elem);
+int getf2_grid_leaf(hdbf_context* ctx, int m, int elem);
+size_t getf2_grid_scratch_bytes();
 // The leaf the panel recursion takes on the cluster kernel (0: the grid-wide one).
 int panel_cluster_leaf(hdbf_context* ctx, int m, int elem);
+void configure_getrf_kernels(hdbf_context* ctx);
+void configure_grid_panel(hdbf_context* ctx);
 int configure_cluster_panel(hdbf_context* ctx);
 
 // Compose LAPACK swaps  row (i) <-> row (ipiv[i]-1-ipiv_minus), i in [0,k),
@@ -584,8 +586,6 @@ hdbf_status apply_moves(hdbf_context* ctx, double* A, long long lda, int ncols, 
                         long long temp_cols);
 hdbf_status getrf_panel(hdbf_context* ctx, int m, int w, double* A, long long lda, int* ipiv,
                         int ipiv_add, int* info, int info_base, bool pivot, const GetrfWs& ws);
-size_t getf2_coop64_scratch_bytes();
-void configure_fp64_kernels(hdbf_context* ctx);
 // Workspace order for a problem of order n in scalar type T: FP64 needs the
 // FP32 layout of twice as many whole 64-row blocks (the inverse-block table
 // holds 4096 doubles per block).

@@ -92,14 +92,12 @@ WsLayout ws_layout(int n)
     if (n < 64) n = 64;
     WsLayout L;
     size_t off = 0;
-    L.coop = off;
-    off += getf2_coop_scratch_bytes();
+    L.panel = off;
+    off += getf2_grid_scratch_bytes();
     L.inv = off;  // whole 64x64 blocks, the last one padded
     off += align_up((size_t)(n + 63) / 64 * 64 * 64 * sizeof(float), 256);
     L.perm = off;
     off += align_up((size_t)n * sizeof(int), 256);
-    L.coop64 = off;
-    off += getf2_coop64_scratch_bytes();
     L.src = off;
     off += align_up((size_t)n * sizeof(int), 256);
     L.tgt = off;
@@ -140,17 +138,13 @@ hdbf_status ensure_ws(hdbf_context* ctx, int n)
     return st;
 }
 
-float* ws_coop(hdbf_context* ctx)
+void* ws_panel(hdbf_context* ctx)
 {
-    return reinterpret_cast<float*>(static_cast<char*>(ctx->ws) + ws_layout(ctx->ws_n).coop);
+    return static_cast<char*>(ctx->ws) + ws_layout(ctx->ws_n).panel;
 }
 float* ws_inv(hdbf_context* ctx)
 {
     return reinterpret_cast<float*>(static_cast<char*>(ctx->ws) + ws_layout(ctx->ws_n).inv);
-}
-double* ws_coop64(hdbf_context* ctx)
-{
-    return reinterpret_cast<double*>(static_cast<char*>(ctx->ws) + ws_layout(ctx->ws_n).coop64);
 }
 
 int* ws_perm(hdbf_context* ctx)
@@ -424,7 +418,7 @@ hdbf_status hdbf_create(hdbf_handle* handle)
     configure_trsm_block_kernels(ctx);
     configure_solve_kernels(ctx);
     configure_batched_kernels(ctx);
-    configure_fp64_kernels(ctx);
+    configure_grid_panel(ctx);
     const int one = 1;  // exchange epoch starts at 1: zeroed slots never match
     cudaMemcpy(ctx->dev_small + kSmallEpoch, &one, sizeof(int), cudaMemcpyHostToDevice);
     cudaDeviceSynchronize();
