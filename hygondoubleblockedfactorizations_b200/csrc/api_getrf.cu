@@ -118,22 +118,23 @@ struct NoSkinny {
     ~NoSkinny() { ctx->no_skinny = false; }
 };
 
-// Double-blocked left-looking LU (src/getrf/double_blocked_getrf.cpp:125-191,
+// Double-blocked LU (src/getrf/double_blocked_getrf.cpp:125-191,
 // src/getrf/getrf_batched_pivot_internal.h:445-624,
-// src/getrf/double_blocked_getrf_npvt.cpp:93-144).
+// src/getrf/double_blocked_getrf_npvt.cpp:93-144): left-looking over outer
+// blocks.  Within a block, after each inner panel its rows of U are completed
+// across the block (GEMM over the block's earlier panels, then a TRSM of the
+// panel's order), and the next panel's columns take one GEMM over all panels of
+// the block so far.  Solving the next panel's columns against all earlier panels
+// instead runs a dependent chain as long as the block so far before every panel:
+// 25.3 against 22.4 ms at n = 8192 (blocks 2048 / 256), 255 against 241 ms at
+// 32768 (8192 / 1024), FP64 17.0 against 14.8 ms at 4096 (2048 / 256).
 //
-// Look-ahead (batched or no pivoting, hdbf_set_lookahead): the outer TRSM of
-// block b+1 runs whole, then its outer GEMM (K = all previous columns) is
-// enqueued on the caller's stream in column chunks of whole inner panels,
-// each followed by an event; the inner-panel chain of block b+1 (panel, row
-// interchanges, inner TRSM + GEMM) runs on the high-priority internal stream
-// and waits only for the chunk it is about to touch, so panel factorizations
-// overlap the rest of the outer GEMM.  The chain joins the caller's stream
-// before the block's outer pivot batch.  Interchanges of a block's panels
-// reach each later inner panel of the block as one composed permutation just
-// before its inner update (instead of one permutation per panel), because
-// the outer GEMM may still be writing those columns; the composition is kept
-// running across the block's panels, and the data movement is the same.
+// Look-ahead (batched or no pivoting, hdbf_set_lookahead): the outer GEMM of a
+// block is enqueued on the caller's stream in two chunks, the first panel's
+// columns and the rest, each followed by an event; the inner-panel chain runs on
+// the high-priority internal stream, where the first panel waits for its own
+// chunk only and so overlaps the rest of the outer GEMM.  The chain joins the
+// caller's stream before the block's outer pivot batch.
 template <class T>
 hdbf_status getrf_db_impl(hdbf_context* ctx, T* A, int lda, int n, int outer_nb,
                           int inner_nb, bool iterative_outer, int trsm_block,
@@ -158,8 +159,7 @@ hdbf_status getrf_db_impl(hdbf_context* ctx, T* A, int lda, int n, int outer_nb,
     if (inner_nb <= 0) inner_nb = outer_nb;
     inner_nb = std::min(inner_nb, outer_nb);
     const bool piv = mode != PivotMode::None;
-    bool la = sizeof(T) == 4 && ctx->lookahead && mode != PivotMode::Immediate && n > outer_nb &&
-              compose_running_fits(ctx, n, inner_nb);
+    bool la = sizeof(T) == 4 && ctx->lookahead && mode != PivotMode::Immediate && n > outer_nb;
     if (la && !ctx->la_stream) {
         // The stream and events are created outside any capture.
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -177,17 +177,10 @@ hdbf_status getrf_db_impl(hdbf_context* ctx, T* A, int lda, int n, int outer_nb,
     if (info) cudaMemsetAsync(info, 0, sizeof(int), ctx->stream);
     const cudaStream_t main_s = ctx->stream;
     int nchunks = 0;  // outer-update chunks of the current block (look-ahead)
-    int chunk_w = 0;  // their width in columns (whole inner panels)
 
     // Inner panels of one outer block [outer, oend).
     auto block_chain = [&](int outer, int oend, bool forked) -> hdbf_status {
-        int waited = 0;
-        auto wait_chunk = [&](int col) {
-            const int c = (col - outer) / chunk_w;
-            while (waited <= c && waited < nchunks)
-                cudaStreamWaitEvent(ctx->stream, ctx->la_ev[waited++], 0);
-        };
-        if (forked) wait_chunk(outer);
+        if (forked) cudaStreamWaitEvent(ctx->stream, ctx->la_ev[0], 0);
         for (int inner = outer; inner < oend; inner += inner_nb) {
             const int isz = std::min(inner_nb, oend - inner);
             const int next = inner + isz;
@@ -196,6 +189,8 @@ hdbf_status getrf_db_impl(hdbf_context* ctx, T* A, int lda, int n, int outer_nb,
                 HDBF_TRY(getrf_panel(ctx, n - inner, isz, at(A, lda, inner, inner), lda,
                                      piv ? ipiv + inner : nullptr, inner, info, inner, piv, ws));
             }
+            if (forked && inner == outer && nchunks > 1)  // the block's other columns
+                cudaStreamWaitEvent(ctx->stream, ctx->la_ev[1], 0);
             if (mode == PivotMode::Immediate) {
                 StageScope sc(ctx, kStPivotProp);
                 const int cb[2] = {0, next};
@@ -205,27 +200,20 @@ hdbf_status getrf_db_impl(hdbf_context* ctx, T* A, int lda, int n, int outer_nb,
             } else if (mode == PivotMode::Batched) {
                 StageScope sc(ctx, kStInnerPivot);
                 const int cb[2] = {outer, next};
-                const int cc[2] = {inner - outer, la ? 0 : oend - next};
+                const int cc[2] = {inner - outer, oend - next};
                 HDBF_TRY(permute_cols(ctx, ws, A, lda, n, inner, ipiv + inner, isz, inner, info,
                                       cb, cc, 2));
             }
             if (next < oend) {  // prepare_next_inner_panel
                 const int nsz = std::min(inner_nb, oend - next);
                 const int hist = next - outer;
-                if (forked) wait_chunk(next);
-                if (la && mode == PivotMode::Batched) {  // the block's interchanges so far
-                    StageScope sc(ctx, kStInnerPivot);
-                    HDBF_TRY(compose_running(ctx, ipiv + outer, inner - outer, hist, outer,
-                                             n - outer, ws_perm(ctx), inner == outer, ws.src,
-                                             ws.tgt, ws.count, info));
-                    HDBF_TRY(apply_moves(ctx, at(A, lda, outer, next), lda, nsz, ws.src, ws.tgt,
-                                         ws.count, std::min(n - outer, 2 * hist),
-                                         ws_temp<T>(ws), ws.temp_cols));
-                }
-                {
+                {  // the panel's rows of U across the block
                     StageScope sc(ctx, kStInnerTrsm);
-                    HDBF_TRY(trsm_llu(ctx, hist, nsz, at(A, lda, outer, outer), lda,
-                                      at(A, lda, outer, next), lda));
+                    HDBF_TRY(gemm_sub(ctx, true, false, isz, oend - next, inner - outer,
+                                      at(A, lda, inner, outer), lda, at(A, lda, outer, next), lda,
+                                      at(A, lda, inner, next), lda));
+                    HDBF_TRY(trsm_llu(ctx, isz, oend - next, at(A, lda, inner, inner), lda,
+                                      at(A, lda, inner, next), lda));
                 }
                 StageScope sc(ctx, kStInnerGemm);
                 HDBF_TRY(gemm_nn_rows(ctx, n - next, nsz, hist, at(A, lda, next, outer), lda,
@@ -273,17 +261,15 @@ hdbf_status getrf_db_impl(hdbf_context* ctx, T* A, int lda, int n, int outer_nb,
                                    iterative_outer, trsm_block));
             StageScope sc(ctx, kStOuterGemm);
             if (la) {
-                const int panels = (nsz + inner_nb - 1) / inner_nb;
-                const int group = (panels + kLaEvents - 2) / (kLaEvents - 1);
-                chunk_w = group * inner_nb;
                 NoSkinny ns(ctx);  // the panel chain may use the split-K scratch
                 SplitPlan sp(ctx, n - next, nsz, next);  // chunks sum as the whole GEMM
-                for (int c0 = 0; c0 < nsz; c0 += chunk_w) {
-                    const int cw = std::min(chunk_w, nsz - c0);
+                for (int c0 = 0; c0 < nsz;) {
+                    const int cw = c0 == 0 ? std::min(inner_nb, nsz) : nsz - c0;
                     HDBF_TRY(gemm_sub(ctx, true, false, n - next, cw, next, at(A, lda, next, 0),
                                        lda, at(A, lda, 0, next + c0), lda,
                                        at(A, lda, next, next + c0), lda));
                     cudaEventRecord(ctx->la_ev[nchunks++], main_s);
+                    c0 += cw;
                 }
             } else {
                 HDBF_TRY(gemm_sub(ctx, true, false, n - next, nsz, next, at(A, lda, next, 0), lda,

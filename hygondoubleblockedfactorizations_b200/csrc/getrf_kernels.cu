@@ -247,70 +247,6 @@ compose_swaps_serial_kernel(const int* __restrict__ ipiv, int k, int ipiv_minus,
     if (tid == 0) *count = base;
 }
 
-// Running composition for the GETRF look-ahead: the block's permutation pos[m]
-// (position -> source row, kept in global memory between launches) is staged
-// in shared memory, the new swaps ipiv[k0..k1) are composed on top of it by
-// the sorted-group method, and every displaced row of the block becomes a
-// move, in increasing target order.
-__global__ void __launch_bounds__(kComposeThreads)
-compose_running_kernel(const int* __restrict__ ipiv, int k0, int k1, int ipiv_minus, int m,
-                       int* pos, int init, int* src, int* tgt, int* count, int* info, int* err)
-{
-    extern __shared__ __align__(16) unsigned char craw[];
-    __shared__ int warp_tot[kComposeThreads / 32];
-    __shared__ int s_bad, s_chunk;
-    const int kk = k1 - k0;
-    const int P = pow2_at_least(kk < 1 ? 1 : kk);
-    int* sp = reinterpret_cast<int*>(craw);
-    unsigned long long* keys =
-        reinterpret_cast<unsigned long long*>(craw + ((size_t)m * sizeof(int) + 15) / 16 * 16);
-    int* bt = reinterpret_cast<int*>(keys + P);
-    int* aux = bt + kk;
-    int* root = aux + kk;
-    int* nv = root + kk;
-    const int tid = threadIdx.x;
-    if (tid == 0) s_bad = 0;
-    __syncthreads();
-    for (int q = tid; q < m; q += kComposeThreads) sp[q] = init ? q : pos[q];
-    for (int t = tid; t < kk; t += kComposeThreads) {
-        const int b = ipiv[k0 + t] - 1 - ipiv_minus;
-        if (b < k0 + t || b >= m) s_bad = 1;
-        bt[t] = b;
-    }
-    __syncthreads();
-    if (s_bad) {
-        if (tid == 0) {
-            *count = 0;
-            if (info) atomicExch(info, -1);
-            atomicCAS(err, 0, kErrBadPivot);
-        }
-        return;
-    }
-    if (kk > 0) {
-        compose_sorted(bt, kk, k0, P, keys, aux, root, nv, [&](int x) { return sp[x]; });
-        // final contents of the targets beyond the swapped rows (aux reused)
-        for (int s = tid; s < kk; s += kComposeThreads) {
-            const unsigned long long key = keys[s];
-            const int b = (int)(key >> 32);
-            const bool last = !(s + 1 < kk && (int)(keys[s + 1] >> 32) == b);
-            aux[s] = (last && b >= k1) ? sp[k0 + root[(int)(key & 0xffffffffu)]] : -1;
-        }
-        __syncthreads();
-        for (int t = tid; t < kk; t += kComposeThreads) {
-            sp[k0 + t] = nv[t];
-            if (aux[t] >= 0) sp[(int)(keys[t] >> 32)] = aux[t];
-        }
-        __syncthreads();
-    }
-    for (int q = tid; q < m; q += kComposeThreads) pos[q] = sp[q];
-    const int base = emit_ordered(m, 0, src, tgt, warp_tot, &s_chunk, [&](int q, int* s, int* t) {
-        *s = sp[q];
-        *t = q;
-        return sp[q] != q;
-    });
-    if (tid == 0) *count = base;
-}
-
 // ------------------------------------------------------------ apply moves
 constexpr int kApplyThreads = 256;
 
@@ -404,8 +340,6 @@ void configure_getrf_kernels(hdbf_context* ctx)
                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap4);
     cudaFuncSetAttribute(apply_moves_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)cap4);
-    cudaFuncSetAttribute(compose_running_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)cap4);
     cudaGetLastError();
 }
 
@@ -429,27 +363,6 @@ hdbf_status compose_swaps(hdbf_context* ctx, const int* ipiv, int k, int ipiv_mi
     ProfScope prof(ctx, kClsCompose, 0.0, 4.0 * k + 8.0 * m);
     compose_swaps_serial_kernel<<<1, kComposeThreads, use_smem ? smem : 0, ctx->stream>>>(
         ipiv, k, ipiv_minus, m, src, tgt, count, gperm, use_smem, info,
-        ctx->dev_small + kSmallErr);
-    ctx->launches++;
-    return last_cuda(ctx);
-}
-
-bool compose_running_fits(hdbf_context* ctx, int m, int kk)
-{
-    const size_t cap = ctx->max_smem_optin > 4096 ? ctx->max_smem_optin - 4096 : 0;
-    return kk >= 0 && kk <= kComposeMaxK && compose_sorted_bytes(m, kk) <= cap;
-}
-
-hdbf_status compose_running(hdbf_context* ctx, const int* ipiv, int k0, int k1, int ipiv_minus,
-                            int m, int* pos, bool init, int* src, int* tgt, int* count, int* info)
-{
-    if (m <= 0) return HDBF_STATUS_SUCCESS;
-    if (k0 < 0 || k1 < k0 || k1 > m || !compose_running_fits(ctx, m, k1 - k0))
-        return HDBF_STATUS_INVALID_VALUE;
-    ProfScope prof(ctx, kClsCompose, 0.0, 12.0 * (k1 - k0) + 12.0 * m);
-    const size_t smem = compose_sorted_bytes(m, k1 - k0);
-    compose_running_kernel<<<1, kComposeThreads, smem, ctx->stream>>>(
-        ipiv, k0, k1, ipiv_minus, m, pos, init ? 1 : 0, src, tgt, count, info,
         ctx->dev_small + kSmallErr);
     ctx->launches++;
     return last_cuda(ctx);

@@ -70,7 +70,7 @@ struct GraphEntry {
 }  // namespace hdbf
 
 namespace hdbf {
-constexpr int kLaEvents = 33;  // 32 outer-update chunks per block + the join
+constexpr int kLaEvents = 3;  // two outer-update chunks per block, the join
 }
 
 struct hdbf_context {
@@ -84,7 +84,7 @@ struct hdbf_context {
     int panel_rows = 256; // target rows per CTA of the grid-wide panel kernel
     // GETRF look-ahead (hdbf_set_lookahead): the panel chain of an outer block
     // runs on a high-priority internal stream while the caller's stream still
-    // applies the outer update chunk by chunk; la_ev[c] marks chunk c done and
+    // applies the outer update in two chunks; la_ev[c] marks chunk c done and
     // la_ev[kLaEvents - 1] joins the panel chain back.
     int lookahead = 1;
     cudaStream_t la_stream = nullptr;
@@ -263,7 +263,6 @@ void* mixed_arena(hdbf_context* ctx, size_t bytes, hdbf_status* st);
 // Workspace layout for problems of order <= n (byte offsets):
 //   panel  panel-kernel exchange slots (fixed size, offset 0)
 //   inv   inverted 64x64 diagonal blocks, ceil(n/64)*4096 floats
-//   perm  running composed row permutation of a GETRF outer block, n ints
 //   src, tgt, gperm  composed row moves / permutation scratch, n ints each
 //   temp  column-tiled swap buffer, 64*n floats
 //   skinny  split-K partial sums of the skinny GEMM, 256*n floats
@@ -271,7 +270,7 @@ void* mixed_arena(hdbf_context* ctx, size_t bytes, hdbf_status* st);
 //   words BF16 words of the operands of an FP32 update on the tensor cores, one
 //         half per stream (handle's, look-ahead)
 struct WsLayout {
-    size_t panel, inv, perm, src, tgt, gperm, temp, skinny, wave, split, words, total;
+    size_t panel, inv, src, tgt, gperm, temp, skinny, wave, split, words, total;
 };
 // Split-K partial sums of under-filled FP32 GEMM launches: two halves of
 // kSplitFloats each, one for the handle's stream and one for its look-ahead
@@ -282,7 +281,6 @@ WsLayout ws_layout(int n);
 hdbf_status ensure_ws(hdbf_context* ctx, int n);
 void* ws_panel(hdbf_context* ctx);
 float* ws_inv(hdbf_context* ctx);
-int* ws_perm(hdbf_context* ctx);
 int* ws_src(hdbf_context* ctx);
 int* ws_tgt(hdbf_context* ctx);
 int* ws_gperm(hdbf_context* ctx);
@@ -452,17 +450,6 @@ hdbf_status swap_rows(hdbf_context* ctx, float* A, long long lda, const int* ipi
 hdbf_status swap_rows(hdbf_context* ctx, double* A, long long lda, const int* ipiv, int k, int minus,
                       int m, int c0, int n0, int c1, int n1, int* info);
 // A[tgt[i], c] = old A[src[i], c] for c < ncols, i < *count (<= max_moves).
-// Running composition: pos (m ints, row i of the block holds original row
-// pos[i]) is reset to the identity when init is set, then the LAPACK swaps
-// ipiv[k0, k1) (1-based, minus ipiv_minus gives rows local to the block) are
-// composed onto it, and every i with pos[i] != i becomes a move (pos[i] -> i),
-// in increasing i.  Fails (count 0, info -1) on a pivot outside [i, m).
-hdbf_status compose_running(hdbf_context* ctx, const int* ipiv, int k0, int k1, int ipiv_minus,
-                            int m, int* pos, bool init, int* src, int* tgt, int* count,
-                            int* info);
-// Whether compose_running takes a block of height m and kk new swaps (its
-// shared memory holds pos[m] and the sorted-group arrays; kk <= 4096).
-bool compose_running_fits(hdbf_context* ctx, int m, int kk);
 hdbf_status apply_moves(hdbf_context* ctx, float* A, long long lda, int ncols,
                         const int* src, const int* tgt, const int* count, int max_moves,
                         float* temp, long long temp_cols);

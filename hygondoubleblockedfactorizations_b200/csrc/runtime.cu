@@ -96,8 +96,6 @@ WsLayout ws_layout(int n)
     off += getf2_grid_scratch_bytes();
     L.inv = off;  // whole 64x64 blocks, the last one padded
     off += align_up((size_t)(n + 63) / 64 * 64 * 64 * sizeof(float), 256);
-    L.perm = off;
-    off += align_up((size_t)n * sizeof(int), 256);
     L.src = off;
     off += align_up((size_t)n * sizeof(int), 256);
     L.tgt = off;
@@ -147,10 +145,6 @@ float* ws_inv(hdbf_context* ctx)
     return reinterpret_cast<float*>(static_cast<char*>(ctx->ws) + ws_layout(ctx->ws_n).inv);
 }
 
-int* ws_perm(hdbf_context* ctx)
-{
-    return reinterpret_cast<int*>(static_cast<char*>(ctx->ws) + ws_layout(ctx->ws_n).perm);
-}
 
 hdbf_status ensure_lookahead(hdbf_context* ctx)
 {
