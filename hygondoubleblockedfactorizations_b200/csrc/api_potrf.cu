@@ -99,6 +99,25 @@ hdbf_status dbtrsm_impl(hdbf_context* ctx, const T* L, long long ldl, T* B,
     return HDBF_STATUS_SUCCESS;
 }
 
+// Order of the last diagonal block that is factored by one launch whatever the
+// block sizes: nothing is below it, so no panel solve has to wait for its parts.
+// The cluster kernel (potrf_block.cu) takes 15-16 us a 64-column tile there, panels
+// of 64 columns 18 us, wider ones more: n = 256 74 -> 66 us, n = 512 157 -> 124 us,
+// n = 2048 (512 / 64) 723 -> 693 us.  Two tiles gain nothing (196 and 199 us at n =
+// 640), nor does a block of 1024 (484 and 491 us at n = 1300).
+constexpr int kTailOrder = 512, kTailAbove = 128;
+template <class T>
+int tail_order(const hdbf_context* ctx)
+{
+    return sizeof(T) == 4 && ctx->cluster_max >= 16 ? kTailOrder : 0;
+}
+// Columns of the next block from `at` on.
+inline int block_width(int n, int at, int width, int tail)
+{
+    const int rest = n - at;
+    return rest > kTailAbove && rest <= tail ? rest : std::min(width, rest);
+}
+
 // src/potrf/double_blocked_potrf.cpp:294-381 with this library's kernels.
 template <class T>
 hdbf_status potrf_db_impl(hdbf_context* ctx, T* A, int lda, int n, int nb, int b, int* info,
@@ -117,11 +136,12 @@ hdbf_status potrf_db_impl(hdbf_context* ctx, T* A, int lda, int n, int nb, int b
                                         use_dbtrsm, syrk_k_tile, m_tile, m_thr, k_thr};
     return run_graph(ctx, key, [&]() -> hdbf_status {
     if (info) cudaMemsetAsync(info, 0, sizeof(int), ctx->stream);
-    for (int outer = 0; outer < n; outer += nb) {
-        const int oend = outer + std::min(nb, n - outer);
-        for (int inner = outer; inner < oend; inner += b) {
-            const int isz = std::min(b, oend - inner);
-            const int ps = inner + isz;
+    const int tail = tail_order<T>(ctx);
+    for (int outer = 0, oend; outer < n; outer = oend) {
+        oend = outer + block_width(n, outer, nb, tail);
+        for (int inner = outer, ps; inner < oend; inner = ps) {
+            const int isz = block_width(oend, inner, b, oend == n ? tail : 0);
+            ps = inner + isz;
             const int rows = n - ps;
             T* Aii = at(A, lda, inner, inner);
             {
@@ -139,7 +159,7 @@ hdbf_status potrf_db_impl(hdbf_context* ctx, T* A, int lda, int n, int nb, int b
             }
             if (ps < oend) {  // update_next_inner_panel (:210-249)
                 StageScope sc(ctx, kStInnerGemm);
-                const int pc = std::min(b, oend - ps);
+                const int pc = block_width(oend, ps, b, oend == n ? tail : 0);
                 const int k = ps - outer;
                 const bool mt = m_tile > 0 && rows > m_thr && k >= k_thr;
                 HDBF_TRY(gemm_nt_rows(ctx, rows, pc, k, at(A, lda, ps, outer), lda,
@@ -149,7 +169,7 @@ hdbf_status potrf_db_impl(hdbf_context* ctx, T* A, int lda, int n, int nb, int b
         }
         if (oend < n) {  // prepare_next_outer_panel (:251-292)
             const int next = oend;
-            const int nsz = std::min(nb, n - next);
+            const int nsz = block_width(n, next, nb, tail);
             const int below = next + nsz;
             const int tk = (syrk_k_tile > 0 && syrk_k_tile < next) ? syrk_k_tile : next;
             if (tk == next) {
@@ -193,8 +213,8 @@ hdbf_status potrf_blocked_rl_impl(hdbf_context* ctx, T* A, int lda, int n, int n
     const std::vector<long long> key = {2 + type_tag<T>(), (long long)A, lda, n, nb, (long long)info};
     return run_graph(ctx, key, [&]() -> hdbf_status {
     if (info) cudaMemsetAsync(info, 0, sizeof(int), ctx->stream);
-    for (int k = 0; k < n; k += nb) {
-        const int psz = std::min(nb, n - k);
+    for (int k = 0, psz; k < n; k += psz) {
+        psz = block_width(n, k, nb, tail_order<T>(ctx));
         const int tr = n - k - psz;
         T* Akk = at(A, lda, k, k);
         HDBF_TRY(potrf_diag(ctx, psz, Akk, lda, info, k));
@@ -265,7 +285,8 @@ hdbf_status rec_potrf_impl(hdbf_context* ctx, T* A, long long lda, int n, int nb
                            int info_base, bool tiled)
 {
     if (n <= 0) return HDBF_STATUS_SUCCESS;
-    if (nb <= 0 || n <= nb) return potrf_diag(ctx, n, A, lda, info, info_base);
+    if (nb <= 0 || n <= std::max(nb, tail_order<T>(ctx)))
+        return potrf_diag(ctx, n, A, lda, info, info_base);
     const int n1 = n / 2;
     const int n2 = n - n1;
     T* A21 = A + n1;
