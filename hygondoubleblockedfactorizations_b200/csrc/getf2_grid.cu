@@ -104,9 +104,9 @@ getf2_grid_kernel(int m, int w, T* A, long long lda, int rpc, int* ipiv, int ipi
     auto slot_of = [&](int par, int q) {
         return slots + ((long long)par * kGridMax + q) * kSlotWords;
     };
-    // One more fruitless poll; true when they ran out.
+    // One more fruitless poll; true when it was the last allowed.
     auto expired = [&](unsigned& polls, int& stop) {
-        if (++polls > limit) {
+        if (++polls >= limit) {
             atomicCAS(err, 0, kErrTimeout);
             stop = 1;
             return true;
