@@ -10,9 +10,10 @@
 // column k, then update the trailing tiles while CTA 0 factors the next diagonal
 // tile.  Tiles travel through L2 (each is read by several CTAs); two barriers per
 // tile column are mbarriers in every CTA's shared memory on which all CTAs arrive
-// remotely.  What bounds it is CTA 0's chain, ~15 us a tile: n = 256 62 us, n =
-// 512 126 us; with a grid-wide barrier twice per tile column and every step through
-// L2 it took 96 and 207 us.
+// remotely.  What bounds it is CTA 0's chain, ~14.5 us a tile (factor 5.9, inverse
+// 2.3, products 3.2, the rest loads, stores and barriers): n = 256 60 us, n = 512
+// 118 us; with a grid-wide barrier twice per tile column and every step through L2
+// it took 96 and 207 us.
 // With the inverse requested, W = L^{-1} (lower, the strictly upper tiles zeroed)
 // is formed by a second, cooperative launch (tile_inverse_kernel) by recursive
 // doubling over tile blocks: for siblings A and C, W(C,A) = -W(C,C) (L(C,A)
@@ -112,8 +113,10 @@ __device__ __forceinline__ void load_pair(float* dA, TileSrc a, float* dB, TileS
 }
 
 // acc[i][j] += sum_k As[k][r4 + i] * Bs[k][c4 + j]: rows r4 = 4 (tid & 15) in
-// consecutive lanes (whole lines of C), columns c4 = 4 (tid >> 4); packed FMAs.
-__device__ __forceinline__ void tile_mma(float acc[4][4], const float* As, const float* Bs)
+// consecutive lanes (whole lines of C), columns c4 = 4 (tid >> 4); packed FMAs.  kmax: a
+// multiple of 8, uniform in a warp.
+__device__ __forceinline__ void tile_mma(float acc[4][4], const float* As, const float* Bs,
+                                         int kmax = kT)
 {
     const int r4 = (threadIdx.x & 15) * 4, c4 = (threadIdx.x >> 4) * 4;
     Two<float> s[2][4];
@@ -123,7 +126,7 @@ __device__ __forceinline__ void tile_mma(float acc[4][4], const float* As, const
         s[1][j] = Two<float>::make(acc[2][j], acc[3][j]);
     }
 #pragma unroll 8
-    for (int k = 0; k < kT; ++k) {
+    for (int k = 0; k < kmax; ++k) {
         Two<float> a0, a1;
         load_pairs(As + k * kLdS + r4, a0, a1);
         const float4 b = *reinterpret_cast<const float4*>(Bs + k * kLdS + c4);
@@ -277,6 +280,7 @@ potrf_cluster_kernel(int n, float* A, long long lda, int* info, int info_base, f
     // One CTA needs no barriers: 0 = column k ready (D_k written, step k - 1 applied),
     // 1 = column k solved.
     const bool solo = C == 1;
+    const int kmax = (tid >> 5) * 8 + 8;  // D_k is lower: this warp's columns end there
     float acc[4][4];
     auto clear = [&]() {
 #pragma unroll
@@ -284,7 +288,15 @@ potrf_cluster_kernel(int n, float* A, long long lda, int* info, int info_base, f
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
     };
+    const bool aligned = lda % 4 == 0 && (reinterpret_cast<uintptr_t>(A) & 15u) == 0;
     auto store_acc = [&](float* T, int rows, int cols) {
+        if (aligned && rows == kT && cols == kT) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                *reinterpret_cast<float4*>(T + (long long)(c4 + j) * lda + r4) =
+                    make_float4(acc[0][j], acc[1][j], acc[2][j], acc[3][j]);
+            return;
+        }
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
@@ -330,7 +342,7 @@ potrf_cluster_kernel(int n, float* A, long long lda, int* info, int info_base, f
             fetch_wait<0>();
             __syncthreads();
             clear();
-            tile_mma(acc, P, W);
+            tile_mma(acc, P, W, kmax);
             store_acc(tile(k + 1, k), e, kT);
 #pragma unroll
             for (int j = 0; j < 4; ++j)
@@ -346,8 +358,9 @@ potrf_cluster_kernel(int n, float* A, long long lda, int* info, int info_base, f
             tile_mma(acc, X, X);
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) S[(c4 + j) * kLdS + r4 + i] = old[i][j] - acc[i][j];
+                *reinterpret_cast<float4*>(S + (c4 + j) * kLdS + r4) =
+                    make_float4(old[0][j] - acc[0][j], old[1][j] - acc[1][j],
+                                old[2][j] - acc[2][j], old[3][j] - acc[3][j]);
             __syncthreads();
         }
     } else {
@@ -366,7 +379,7 @@ potrf_cluster_kernel(int n, float* A, long long lda, int* info, int info_base, f
                 fetch_wait<0>();
                 __syncthreads();
                 clear();
-                tile_mma(acc, sm.tile[0], sm.tile[1]);
+                tile_mma(acc, sm.tile[0], sm.tile[1], kmax);
                 store_acc(tile(i, k), ext(i), kT);
                 __syncthreads();
             }
