@@ -24,6 +24,7 @@ namespace {
 constexpr int kT = 64;      // tile
 constexpr int kKB = 32;     // K per slab
 constexpr int kThr = 256;
+constexpr int kFold = 8;    // slabs per partial sum: FP32 error as small as a K split's
 template <class T>
 constexpr int kStages = sizeof(T) == 4 ? 4 : 3;
 template <class T>
@@ -119,9 +120,10 @@ template <class T, bool NN, bool VEC, bool TRI>
 __global__ void __launch_bounds__(kThr)
 gemm_small_kernel(int M, int N, int K, const T* __restrict__ A, long long lda,
                   const T* __restrict__ B, long long ldb, T* __restrict__ C, long long ldc,
-                  int tiles_m, int kc)
+                  int tiles_m, int kc, const unsigned* range)
 {
     extern __shared__ __align__(16) unsigned char sm_raw[];
+    if (range && !split_range_bad(range)) return;  // done on the tensor cores
     T* sm = reinterpret_cast<T*>(sm_raw);
     constexpr int kSt = kStages<T>;
     int S, split;
@@ -164,6 +166,19 @@ gemm_small_kernel(int M, int N, int K, const T* __restrict__ A, long long lda,
     Two<T> acc[4][2];  // [column][row pair]
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = Two<T>::zero();
+    Two<T> total[4][2];  // FP32: sums of 256 of K each
+#pragma unroll
+    for (int j = 0; j < 4; ++j) total[j][0] = total[j][1] = Two<T>::zero();
+    auto fold = [&]() {
+        const Two<T> one = Two<T>::make(T(1), T(1));
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                total[j][h].fma(acc[j][h], one);
+                acc[j][h] = Two<T>::zero();
+            }
+    };
     for (int s = 0; s < slabs; ++s) {
         asm volatile("cp.async.wait_group %0;" ::"n"(kSt - 2) : "memory");
         __syncthreads();
@@ -193,12 +208,15 @@ gemm_small_kernel(int M, int N, int K, const T* __restrict__ A, long long lda,
                 }
             }
         }
+        if (sizeof(T) == 4 && s % kFold == kFold - 1) fold();
     }
+    if (sizeof(T) == 4) fold();
+    Two<T>(&sums)[4][2] = sizeof(T) == 4 ? total : acc;
     T p[4][4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        acc[j][0].get(p[j][0], p[j][1]);
-        acc[j][1].get(p[j][2], p[j][3]);
+        sums[j][0].get(p[j][0], p[j][1]);
+        sums[j][1].get(p[j][2], p[j][3]);
     }
     if (S == 1) {
 #pragma unroll
@@ -215,7 +233,7 @@ gemm_small_kernel(int M, int N, int K, const T* __restrict__ A, long long lda,
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
 #pragma unroll
-    for (int j = 0; j < 4; ++j) store_pairs(sm + col_of(j) * kLdP + ty * 4, acc[j][0], acc[j][1]);
+    for (int j = 0; j < 4; ++j) store_pairs(sm + col_of(j) * kLdP + ty * 4, sums[j][0], sums[j][1]);
     const int per = kT / S;  // columns of this CTA: 256 threads = 64 rows x 4 columns at a time
     const int row = tid & 63, r = m0 + row;
     T old[8];  // S >= 2: at most 32 columns
@@ -256,7 +274,7 @@ gemm_small_kernel(int M, int N, int K, const T* __restrict__ A, long long lda,
 
 template <class T, bool NN, bool VEC, bool TRI>
 cudaError_t launch(cudaStream_t st, int S, int M, int N, int K, const T* A, long long lda,
-                   const T* B, long long ldb, T* C, long long ldc)
+                   const T* B, long long ldb, T* C, long long ldc, const unsigned* range)
 {
     const int tm = (M + kT - 1) / kT, tn = (N + kT - 1) / kT;
     const int kc = ((K + S - 1) / S + 7) / 8 * 8;
@@ -273,7 +291,7 @@ cudaError_t launch(cudaStream_t st, int S, int M, int N, int K, const T* A, long
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, gemm_small_kernel<T, NN, VEC, TRI>, M, N, K, A, lda, B, ldb, C,
-                              ldc, tm, kc);
+                              ldc, tm, kc, range);
 }
 
 template <class T, bool NN, bool VEC, bool TRI>
@@ -295,21 +313,22 @@ void configure_type()
 
 template <class T>
 hdbf_status gemm_small_t(hdbf_context* ctx, bool nn, bool lower, int S, int M, int N, int K,
-                         const T* A, long long lda, const T* B, long long ldb, T* C, long long ldc)
+                         const T* A, long long lda, const T* B, long long ldb, T* C, long long ldc,
+                         const unsigned* range = nullptr)
 {
     auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     const bool vec = al(A) && al(B) && lda % kVec<T> == 0 && ldb % kVec<T> == 0;
     cudaStream_t s = ctx->stream;
     cudaError_t e;
     if (nn)
-        e = vec ? launch<T, true, true, false>(s, S, M, N, K, A, lda, B, ldb, C, ldc)
-                : launch<T, true, false, false>(s, S, M, N, K, A, lda, B, ldb, C, ldc);
+        e = vec ? launch<T, true, true, false>(s, S, M, N, K, A, lda, B, ldb, C, ldc, range)
+                : launch<T, true, false, false>(s, S, M, N, K, A, lda, B, ldb, C, ldc, range);
     else if (lower)
-        e = vec ? launch<T, false, true, true>(s, S, M, N, K, A, lda, B, ldb, C, ldc)
-                : launch<T, false, false, true>(s, S, M, N, K, A, lda, B, ldb, C, ldc);
+        e = vec ? launch<T, false, true, true>(s, S, M, N, K, A, lda, B, ldb, C, ldc, range)
+                : launch<T, false, false, true>(s, S, M, N, K, A, lda, B, ldb, C, ldc, range);
     else
-        e = vec ? launch<T, false, true, false>(s, S, M, N, K, A, lda, B, ldb, C, ldc)
-                : launch<T, false, false, false>(s, S, M, N, K, A, lda, B, ldb, C, ldc);
+        e = vec ? launch<T, false, true, false>(s, S, M, N, K, A, lda, B, ldb, C, ldc, range)
+                : launch<T, false, false, false>(s, S, M, N, K, A, lda, B, ldb, C, ldc, range);
     ctx->launches++;
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -343,9 +362,9 @@ int gemm_small_split(const hdbf_context* ctx, int M, int N, int K)
 
 hdbf_status gemm_small(hdbf_context* ctx, bool nn, bool lower, int S, int M, int N, int K,
                        const float* A, long long lda, const float* B, long long ldb, float* C,
-                       long long ldc)
+                       long long ldc, const unsigned* range)
 {
-    return gemm_small_t(ctx, nn, lower, S, M, N, K, A, lda, B, ldb, C, ldc);
+    return gemm_small_t(ctx, nn, lower, S, M, N, K, A, lda, B, ldb, C, ldc, range);
 }
 hdbf_status gemm_small(hdbf_context* ctx, bool nn, bool lower, int S, int M, int N, int K,
                        const double* A, long long lda, const double* B, long long ldb, double* C,

@@ -309,11 +309,11 @@ hdbf_status sgemm_sub(hdbf_context* ctx, bool nn, bool lower_only, int M, int N,
 // the number of chunks (1 = no split) and, in *kc, their length.
 int split_count(const hdbf_context* ctx, int M, int N, int K, bool tri, int* kc);
 // Updates below one wave of 128 x 128 tiles (gemm_small.cu): the CTAs that share
-// a tile's K (0: not taken), and the launch.
+// a tile's K (0: not taken), and the launch (range: only if split_range_bad).
 int gemm_small_split(const hdbf_context* ctx, int M, int N, int K);
 hdbf_status gemm_small(hdbf_context* ctx, bool nn, bool lower, int S, int M, int N, int K,
-                        const float* A, long long lda, const float* B, long long ldb, float* C,
-                        long long ldc);
+                       const float* A, long long lda, const float* B, long long ldb, float* C,
+                       long long ldc, const unsigned* range = nullptr);
 hdbf_status gemm_small(hdbf_context* ctx, bool nn, bool lower, int S, int M, int N, int K,
                        const double* A, long long lda, const double* B, long long ldb, double* C,
                        long long ldc);

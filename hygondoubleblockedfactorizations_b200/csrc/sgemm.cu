@@ -404,10 +404,11 @@ hdbf_status sgemm_launch(hdbf_context* ctx, int mode, bool lower_only, int M, in
     if (range) flops = 0.0;  // counted by the tensor-core launch it stands behind
     ProfScope prof(ctx, kClsGemm, flops, 4.0 * ((double)M * K + (double)N * K + 2.0 * M * N), M,
                    N, K);
-    if (!range && !ri && mode != kTN) {
+    if (!ri && mode != kTN) {
         const int small = ctx->small_plan >= 0 ? ctx->small_plan : gemm_small_split(ctx, M, N, K);
         if (small > 0)
-            return gemm_small(ctx, mode == kNN, lower_only, small, M, N, K, A, lda, B, ldb, C, ldc);
+            return gemm_small(ctx, mode == kNN, lower_only, small, M, N, K, A, lda, B, ldb, C, ldc,
+                              range);
     }
     int kc = 0;
     const int S = range ? 1 : split_count(ctx, M, N, K, lower_only, &kc);

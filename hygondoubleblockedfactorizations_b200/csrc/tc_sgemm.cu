@@ -448,7 +448,7 @@ void configure_tc_sgemm(hdbf_context*)
 // faster products save (2048 x 512 x 512: 51 us against 45; 4096 x 512 x 512: 55
 // against 76; 16384 x 512 x 512: 115 against 204; 16384 x 4096 x 4096: 2.85 ms
 // against 10.5, 193 TFLOP/s).  Below 128 columns half of a tile or more is idle.
-// Accuracy draws a second line, in every mode: where few tiles make the FP32
+// Accuracy draws a second line, in every mode: where few tiles make an FP32
 // kernel cut K into five or more partial sums, its rounding errors average out
 // and, on operands of one sign, come out below the truncation here (777 x 640 x
 // 2100 over [0,1): 9.9e-8 against 1.16e-7), so it keeps those shapes.
@@ -459,7 +459,7 @@ int tc_sgemm_chunk(const hdbf_context* ctx, int M, int N, int K, bool tri)
         (M < 256 || N < 128 || K < 128 || (double)M * N * K < 1.0e9))
         return 0;
     int kc_fp32 = 0;
-    if (split_count(ctx, M, N, K, tri, &kc_fp32) > 4) return 0;
+    if (split_count(ctx, M, N, K, tri, &kc_fp32) > 4 || gemm_small_split(ctx, M, N, K) > 4) return 0;
     const long long room = (long long)ws_words_half(ctx) / (6LL * ((long long)M + N));
     const long long kc = std::min<long long>((K + 63) / 64 * 64, room / 64 * 64);
     return kc >= std::min(K, 512) ? (int)kc : 0;
