@@ -15,9 +15,11 @@ value  = whole-job TFLOP/s with inputs resident in HBM (device-timed, CUDA event
          max over ranks; multi-GPU runs are independent replicas, weak scaling).
 e2e    = the same step through the C ABI starting from pinned HOST buffers:
          H2D of each input, factorization, D2H of the factors, pivots and info.
-roofline = the dominant kernel (sgemm_sub_kernel, FP32 SIMT FFMA) from the
-         library's per-launch event profiler over the timed region, against the
-         FP32 SIMT peak (SMs x 128 lanes x 2 flop x max SM clock).
+roofline = the dominant kernel class from the library's per-launch event profiler
+         over the timed region: the FP32 updates on the tensor cores
+         (tc_gemm_kernels: six BF16 products per FP32 product, counted as such
+         against the measured BF16 peak), or else against the FP32 SIMT peak (SMs x
+         128 lanes x 2 flop x max SM clock).
 cpu_baseline = host LAPACK spotrf + sgetrf (SciPy's OpenBLAS, all host threads),
          one step on the bench's own n=32768 inputs; the same leg then checks the
          factors of the last timed step (parity object): CPU FP64 scaled
@@ -977,21 +979,27 @@ def run_ours(args, rank, world):
     if dom:
         name, (nl, tms, fl, by) = dom
         achieved = fl / (tms / 1e3) / 1e12
-        # DRAM bytes per algorithmic flop of sgemm_sub_kernel, measured by ncu
-        # (dram__bytes_read.sum + dram__bytes_write.sum) on the largest launch
-        # of a POTRF n=16384: 852.5 MB over 2.75e11 flop (FMA-pipe count).
-        bytes_per_flop = 852.5e6 / 2.75e11
-        roof = {"bound": "fp32_simt", "kernel": name, "achieved": round(achieved, 3),
-                "peak": round(peak, 2), "unit": "TFLOP/s", "frac": round(achieved / peak, 4),
-                "traffic": round(fl / nl * bytes_per_flop) if name == "sgemm_sub_kernel" else None,
-                "traffic_unit": "bytes per average launch (ncu bytes/flop of a captured "
-                                "n=16384 launch x this launch's algorithmic flops)",
+        tensor = name == "tc_gemm_kernels"
+        peaks = {}
+        try:
+            peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
+        except Exception:
+            pass
+        if tensor:  # each FP32 product is six products of BF16 words
+            executed, peak = 6.0 * achieved, peaks.get("bf16_tflops", 1590.0)
+        else:
+            executed = achieved
+        roof = {"bound": "tensor" if tensor else "fp32_simt", "kernel": name,
+                "achieved": round(executed, 3), "peak": round(peak, 2), "unit": "TFLOP/s",
+                "frac": round(executed / peak, 4), "fp32_tflops": round(achieved, 3), "traffic": None,
                 "algorithmic_flops_per_launch": round(fl / nl),
                 "launches": nl, "avg_launch_ms": round(tms / nl, 4),
                 "share_of_device_time": round(tms / sum(v[1] for v in prof.values()), 4),
-                "peak_source": (f"{sms} SMs x 128 FP32 lanes x 2 flop x {max_mhz:.0f} MHz max SM "
+                "peak_source": (("MEASURED_PEAKS.json bf16_tflops (burst)" if peaks else "fallback")
+                                if tensor else
+                                f"{sms} SMs x 128 FP32 lanes x 2 flop x {max_mhz:.0f} MHz max SM "
                                 "clock (measured-peaks file has no FP32 SIMT figure)")}
-        if clocks and clocks.get("sm_mhz"):
+        if clocks and clocks.get("sm_mhz") and not tensor:
             roof["frac_at_median_clock"] = round(achieved / (peak * clocks["sm_mhz"] / max_mhz), 4)
     kernels = {k: {"launches": v[0], "ms": round(v[1], 3),
                    "tflops": round(v[2] / (v[1] / 1e3) / 1e12, 3) if v[1] > 0 and v[2] > 0 else None,

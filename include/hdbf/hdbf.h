@@ -103,8 +103,10 @@ hdbf_status hdbf_set_graph_mode(hdbf_handle handle, int enabled);
  * On the same leaf both produce identical pivots and factors.  A new handle
  * starts in the mode named by the environment variable HDBF_PANEL_KERNEL (0, 1
  * or 2), else 0.  The panel recursion stops at leaves of 128 columns, or, where
- * one cluster cannot hold that many at the panel's height, at 64; above that
- * height automatic mode takes the grid-wide kernel.  Mode 2 recurses to 32;
+ * one cluster cannot hold that many at the panel's height, at 64; above 8192
+ * rows automatic mode takes the grid-wide kernel, whose leaves narrow to 64 and 32
+ * columns where the panel's rows no longer fit one, or three, to a thread.  Mode 2
+ * recurses to 32;
  * HDBF_PANEL_LEAF (32, 64 or 128) sets a new handle's leaf width, and
  * HDBF_PANEL_ROWS (64..4096, default 256) the rows each CTA of the grid-wide
  * kernel aims to hold. */
@@ -113,12 +115,11 @@ hdbf_status hdbf_set_panel_kernel(hdbf_handle handle, int mode);
 /* Look-ahead in the double-blocked GETRF entry points with batched pivoting
  * or without pivoting (default on; HDBF_LOOKAHEAD=0 turns a new handle's
  * off).  The outer TRSM of the next outer block runs whole; its outer GEMM
- * then runs in column chunks of the inner panel width on the handle's
- * stream, while the inner panels of that block are factored, each as soon as
- * its chunk is updated, on a high-priority internal stream that joins the
- * handle's stream again at the end of the block.  Row interchanges of the
- * block's panels reach each later inner panel, composed, just before its
- * inner update.  Pivots and factors are the same as without look-ahead.
+ * then runs on the handle's stream in two chunks, the first inner panel's
+ * columns and the rest, while the inner panels of that block are factored on a
+ * high-priority internal stream, the first as soon as its chunk is updated; that
+ * stream joins the handle's stream again at the end of the block.  Pivots and
+ * factors are the same as without look-ahead.
  * double_blocked_getrf (immediate pivoting) always runs serially. */
 hdbf_status hdbf_set_lookahead(hdbf_handle handle, int enabled);
 
