@@ -7,6 +7,9 @@
 // A CTA keeps a slice of B (all rows, or all columns) in shared memory and runs
 // the block forward substitution with the inverted diagonal blocks D_i:
 //     X_i = D_i (B_i - sum_{j<i} L_ij X_j)       (and its transpose on the right).
+// Each product L_ij X_j is summed from zero and then subtracted from what is left
+// of B_i: FMAs straight onto B_i would round every term at the size of B_i (five
+// times the error at 256 columns where the off-diagonal part is small).
 // The order of the L and D tiles is known from the start, so they come through
 // a three-deep cp.async ring while earlier ones are multiplied (4 x 4 or smaller
 // register tiles, packed FP32 FMAs); before, each of the ten tile products of a
@@ -85,11 +88,13 @@ __device__ __forceinline__ void tile_at(int t, int& i, int& j)
 }
 
 // ------------------------------------------------------------------- right
-// acc[c][e] += sign * sum_k x[k * ldx + e] b[k * 64 + c] over 64 of K.
+// acc[c][e] = sum_k x[k * ldx + e] b[k * 64 + c] over 64 of K.
 template <class T, int RP>
-__device__ __forceinline__ void right_product(T acc[4][RP], const T* x, int ldx, const T* b, T sign)
+__device__ __forceinline__ void right_product(T acc[4][RP], const T* x, int ldx, const T* b)
 {
     if (RP == 1) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[c][0] = T(0);
 #pragma unroll 8
         for (int k = 0; k < kT; ++k) {
             T bv[4];
@@ -97,7 +102,7 @@ __device__ __forceinline__ void right_product(T acc[4][RP], const T* x, int ldx,
             load_pairs(b + k * kT, lo, hi);
             lo.get(bv[0], bv[1]);
             hi.get(bv[2], bv[3]);
-            const T xv = sign * x[k * ldx];
+            const T xv = x[k * ldx];
 #pragma unroll
             for (int c = 0; c < 4; ++c) acc[c][0] = ::fma(xv, bv[c], acc[c][0]);
         }
@@ -106,8 +111,7 @@ __device__ __forceinline__ void right_product(T acc[4][RP], const T* x, int ldx,
 #pragma unroll
         for (int c = 0; c < 4; ++c)
 #pragma unroll
-            for (int h = 0; h < RP / 2; ++h)
-                s[c][h] = Two<T>::make(acc[c][2 * h], acc[c][(2 * h + 1) % RP]);
+            for (int h = 0; h < RP / 2; ++h) s[c][h] = Two<T>::zero();
 #pragma unroll 8
         for (int k = 0; k < kT; ++k) {
             T bv[4];
@@ -121,8 +125,7 @@ __device__ __forceinline__ void right_product(T acc[4][RP], const T* x, int ldx,
                 xv[h] = *reinterpret_cast<const Two<T>*>(x + k * ldx + 2 * h);
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                const T bs = sign * bv[c];
-                const Two<T> bb = Two<T>::make(bs, bs);
+                const Two<T> bb = Two<T>::make(bv[c], bv[c]);
 #pragma unroll
                 for (int h = 0; h < RP / 2; ++h) s[c][h].fma(xv[h], bb);
             }
@@ -186,17 +189,17 @@ __global__ void __launch_bounds__(kThr) rlt_block_kernel(int rows, int cols,
     if (ring > 1) fetch(1); else commit();
     int t = 0;
     for (int i = 0; i < nb; ++i) {
-        T acc[4][RP];
+        T acc[4][RP], rest[4][RP];  // rest: B_i less the products so far
         for (int j = 0; j <= i; ++j, ++t) {
             asm volatile("cp.async.wait_group 1;" ::: "memory");
             __syncthreads();  // tile t and X are there; tile t - 1 and X_i's old reads are done
             if (ring > 2) fetch(t + 2); else commit();
-            if (j == 0) {
+            if (j == 0 && i > 0) {
 #pragma unroll
                 for (int c = 0; c < 4; ++c)
 #pragma unroll
                     for (int e = 0; e < RP; ++e)
-                        acc[c][e] = i == 0 ? T(0) : X[(i * kT + tx * 4 + c) * RT + ty * RP + e];
+                        rest[c][e] = X[(i * kT + tx * 4 + c) * RT + ty * RP + e];
             }
             const T* b = tiles + (t % ring) * kTile + tx * 4;
             const T* x = X + j * kT * RT + ty * RP;
@@ -204,13 +207,17 @@ __global__ void __launch_bounds__(kThr) rlt_block_kernel(int rows, int cols,
 #pragma unroll
                 for (int c = 0; c < 4; ++c)
 #pragma unroll
-                    for (int e = 0; e < RP; ++e) {
-                        X[(i * kT + tx * 4 + c) * RT + ty * RP + e] = acc[c][e];
-                        acc[c][e] = T(0);
-                    }
+                    for (int e = 0; e < RP; ++e)
+                        X[(i * kT + tx * 4 + c) * RT + ty * RP + e] = rest[c][e];
                 __syncthreads();
             }
-            right_product<T, RP>(acc, x, RT, b, j == i ? T(1) : T(-1));
+            right_product<T, RP>(acc, x, RT, b);
+            if (j < i) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+#pragma unroll
+                    for (int e = 0; e < RP; ++e) rest[c][e] -= acc[c][e];
+            }
             if (j == i) {
                 if (i + 1 < nb) __syncthreads();  // X_i is still being read
 #pragma unroll
@@ -281,29 +288,27 @@ __global__ void __launch_bounds__(kThr) llu_block_kernel(int rows, int cols,
     fetch(0);
     if (ring > 1) fetch(1); else commit();
     int t = 0;
+    const Two<T> minus = Two<T>::make(T(-1), T(-1));
     for (int i = 0; i < nb; ++i) {
-        Two<T> acc[CP][2];  // [column][row pair]
+        Two<T> acc[CP][2], rest[CP][2];  // [column][row pair]; rest as on the right
         for (int j = 0; j <= i; ++j, ++t) {
             asm volatile("cp.async.wait_group 1;" ::: "memory");
             __syncthreads();
             if (ring > 2) fetch(t + 2); else commit();
-            if (j == 0) {
+            if (j == 0 && i > 0) {
 #pragma unroll
-                for (int c = 0; c < CP; ++c) {
-                    load_pairs(X + (tx * CP + c) * kLdL + i * kT + ty * 4, acc[c][0], acc[c][1]);
-                    if (i == 0) acc[c][0] = acc[c][1] = Two<T>::zero();
-                }
+                for (int c = 0; c < CP; ++c)
+                    load_pairs(X + (tx * CP + c) * kLdL + i * kT + ty * 4, rest[c][0], rest[c][1]);
             }
             const T* a = tiles + (t % ring) * kTile + ty * 4;
             if (j == i && i > 0) {
 #pragma unroll
-                for (int c = 0; c < CP; ++c) {
-                    store_pairs(X + (tx * CP + c) * kLdL + i * kT + ty * 4, acc[c][0], acc[c][1]);
-                    acc[c][0] = acc[c][1] = Two<T>::zero();
-                }
+                for (int c = 0; c < CP; ++c)
+                    store_pairs(X + (tx * CP + c) * kLdL + i * kT + ty * 4, rest[c][0], rest[c][1]);
                 __syncthreads();
             }
-            const T sign = j == i ? T(1) : T(-1);
+#pragma unroll
+            for (int c = 0; c < CP; ++c) acc[c][0] = acc[c][1] = Two<T>::zero();
             const T* x = X + tx * CP * kLdL + j * kT;
 #pragma unroll 4
             for (int k = 0; k < kT; k += 4) {
@@ -321,12 +326,17 @@ __global__ void __launch_bounds__(kThr) llu_block_kernel(int rows, int cols,
                     load_pairs(a + (k + q) * kT, a0, a1);
 #pragma unroll
                     for (int c = 0; c < CP; ++c) {
-                        const T e = sign * xv[c][q];
-                        const Two<T> ee = Two<T>::make(e, e);
+                        const Two<T> ee = Two<T>::make(xv[c][q], xv[c][q]);
                         acc[c][0].fma(a0, ee);
                         acc[c][1].fma(a1, ee);
                     }
                 }
+            }
+            if (j < i) {
+#pragma unroll
+                for (int c = 0; c < CP; ++c)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) rest[c][h].fma(acc[c][h], minus);
             }
             if (j == i) {
                 if (i + 1 < nb) __syncthreads();
