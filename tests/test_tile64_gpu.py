@@ -48,3 +48,35 @@ def test_tile_failure(torch_cuda, hd, handle, col, value):
     R = np.tril(L @ L[:k].T - A[:, :k].astype(np.float64))
     bound = 4 * (n + 1) * 2.0 ** -24 * (np.abs(L) @ np.abs(L[:k]).T)
     assert (np.abs(R) <= bound)[~np.isnan(R)].all() and not np.isnan(R[:col]).any()
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("half", [32, 16])
+@pytest.mark.parametrize("diag", [1.0, 1.7])
+def test_inverse_residual(hd, handle, torch_cuda, dtype, half, diag):
+    """Inverse of a 64 x 64 tile whose second diagonal block is ill conditioned while the
+    inverse below it is not: a column solved by substitution has |L W - I| <= (n + 3) u |L|
+    |W| entry by entry (each entry a chain of at most n operations, a reciprocal and a
+    multiplication by it), whatever the condition of the blocks.  With B = I the solve
+    returns the inverse itself."""
+    rng = np.random.default_rng(half)
+    n, unit = 64, 2.0 ** -24 if dtype == np.float32 else 2.0 ** -53
+    L = np.eye(n) * diag
+    for b in range(0, n, 2 * half):
+        L11 = np.tril(rng.uniform(-0.5, 0.5, (half, half)), -1) + diag * np.eye(half)
+        L22 = np.tril(np.full((half, half), -0.5 * diag), -1) + diag * np.eye(half)
+        Y = rng.uniform(-1, 1, (half, half))
+        L[b:b + half, b:b + half] = L11
+        L[b + half:b + 2 * half, b + half:b + 2 * half] = L22
+        L[b + half:b + 2 * half, b:b + half] = -L22 @ Y @ L11
+    L = L.astype(dtype)
+    dL, dB = dev(torch_cuda, L), dev(torch_cuda, np.eye(n, dtype=dtype))
+    name = "trsm_right_lower_transpose" + ("" if dtype == np.float32 else "_double")
+    hd.call(name, handle.ptr, n, n, ptr(dL), n, ptr(dB), n)
+    torch_cuda.cuda.synchronize()
+    handle.check(name)
+    W = host2d(dB, n, n, n).T.astype(np.longdouble)
+    Lw = L.astype(np.longdouble)
+    assert (np.triu(W, 1) == 0).all()
+    bound = (n + 3) * unit * (np.abs(Lw) @ np.abs(W))
+    assert (np.abs(Lw @ W - np.eye(n)) <= bound).all()
