@@ -44,7 +44,7 @@ potf2_kernel(int n, T* A, long long lda, int* info, int info_base, T* inv)
     tile64::store_lower(A, S, lda, n);
     if (fail >= 0 && threadIdx.x == 0 && info) atomicCAS(info, 0, info_base + fail + 1);
     if (inv) {
-        tile64::inv64(S, W, X, rd, false);
+        tile64::inv64<tile64::kReciprocal>(S, W, X, rd);
         tile64::store_inv(inv, W, false);
     }
 }
@@ -70,7 +70,9 @@ tri_inv64_kernel(int n, const T* __restrict__ L, long long ldl, int mode, T* out
     tile64::load_lower<false>(S, L + (long long)base * ldl + base, ldl, min(kLeaf, n - base),
                               mode == 2);
     __syncthreads();
-    tile64::inv64(S, W, X, rd, mode == 1);
+    if (mode == 1) tile64::inv64<tile64::kUnit>(S, W, X, rd);
+    else if (mode == 2) tile64::inv64<tile64::kCorrected>(S, W, X, rd);
+    else tile64::inv64<tile64::kReciprocal>(S, W, X, rd);
     tile64::store_inv(out + (long long)blockIdx.x * kLeaf * kLeaf, W, mode == 2);
 }
 

@@ -316,7 +316,7 @@ potrf_cluster_kernel(int n, float* A, long long lda, int* info, int info_base, f
                 *reinterpret_cast<volatile int*>(fail) = 1;
             }
             // also of a failing tile: its columns before the failing one are valid
-            tile64::inv64(S, W, sm.X, sm.rd, false);
+            tile64::inv64<tile64::kReciprocal>(S, W, sm.X, sm.rd);
             tile64::store_inv(dinv + (long long)k * kT * kT, W, false);
             if (!solo) {
                 if (waiting && !bar.wait(1)) break;

@@ -6,9 +6,9 @@
 // (chol_panel_fast), with look-ahead between the panels.
 // inv64 inverts the four 16 x 16 diagonal blocks (one warp each, a lane per
 // column) and joins them, first 16, then 32: L22 W21 = -L21 W11, the product by all
-// threads and the solve by substitution, so that every column solves its system
-// as backward stably as one long substitution would (the product W21 = -W22 (L21
-// W11) is 0.3 us shorter, but its error grows with the condition of L22).
+// threads and the solve by substitution, so that every column is as accurate as one
+// long substitution would make it (the product W21 = -W22 (L21 W11) is 0.5 us
+// shorter, but its error grows with the condition of L22).
 // One tile in one launch (load, factor, inverse, stores): 9.9 us; 62 us before,
 // with two barriers, an IEEE square root and a division per column of the
 // factor and one thread per column of the inverse, a division per row.
@@ -247,43 +247,81 @@ __device__ __forceinline__ void store_inv(T* dst, const T* W, bool trans)
     }
 }
 
+// How a substitution divides by the diagonal: not at all (unit); by a reciprocal; by a
+// reciprocal and one correction, q += r (x - d q) (Markstein, IBM J. Res. Dev. 34,
+// 1990: the rounded quotient but for rare ties), or, where the diagonal leaves
+// fast_range, by division instead.  Against division everywhere, the plain reciprocal gives
+// the same errors or less in solves with Cholesky factors (right-side TRSM 3 %,
+// POTRS 4 %), but 4-7 % more in U^{-1} and solves with U, which take the correction
+// (0.2 us a tile, in a launch of its own and not on a factorization's chain).
+enum Divide { kUnit, kReciprocal, kCorrected, kPlain };
+
 // x <- inverse of the 16 x 16 lower block D (pitch kLd, 16-byte aligned) times x, in
-// registers; D by broadcast loads of four rows.
-template <class T>
-__device__ __forceinline__ void solve16(T x[16], const T* D, const T* rd)
+// registers; D by broadcast loads of four rows, rd the reciprocals of its diagonal.
+template <Divide HOW, class T>
+__device__ __forceinline__ void substitute16(T x[16], const T* D, const T* rd)
 {
 #pragma unroll
     for (int k = 0; k < 16; ++k) {
         T d[16];
 #pragma unroll
-        for (int g = (k + 1) / 4; g < 4; ++g) {
+        for (int g = (HOW == kCorrected || HOW == kPlain ? k : k + 1) / 4; g < 4; ++g) {
             const Vec4<T> v = *reinterpret_cast<const Vec4<T>*>(D + k * kLd + 4 * g);
 #pragma unroll
             for (int i = 0; i < 4; ++i) d[4 * g + i] = v.x[i];
         }
-        x[k] *= rd[k];
+        if (HOW == kReciprocal) {
+            x[k] *= rd[k];
+        } else if (HOW == kCorrected) {
+            const T q = x[k] * rd[k];
+            x[k] = fma_t(fma_t(-d[k], q, x[k]), rd[k], q);
+        } else if (HOW == kPlain) {
+            x[k] = x[k] / d[k];
+        }
 #pragma unroll
         for (int i = k + 1; i < 16; ++i) x[i] = fma_t(-d[i], x[k], x[i]);
     }
 }
+template <class T>
+__device__ __noinline__ void substitute16_plain(T* x, const T* D)
+{
+    T v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = x[i];
+    substitute16<kPlain>(v, D, D);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) x[i] = v[i];
+}
+template <Divide HOW, class T>
+__device__ __forceinline__ void solve16(T x[16], const T* D, const T* rd, bool fast)
+{
+    if (HOW == kCorrected && !fast) substitute16_plain(x, D);
+    else substitute16<HOW>(x, D, rd);
+}
 
-// W <- inverse of the lower tile in S (upper part of S ignored; unit: implicit
+// W <- inverse of the lower tile in S (upper part of S ignored; HOW kUnit: implicit
 // ones on the diagonal), W[c * kLd + r], zero above the diagonal.  X: kScratch
 // entries, rd: 64.  S complete on entry; W complete on return.
-template <class T>
+template <Divide HOW, class T>
 __device__ void inv64(const T* __restrict__ S, T* __restrict__ W, T* __restrict__ X,
-                      T* __restrict__ rd, bool unit)
+                      T* __restrict__ rd)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int q = tid; q < kN * kLd; q += kThreads) W[q] = T(0);
-    if (tid < kN) rd[tid] = unit ? T(1) : T(1) / S[tid * kLd + tid];
-    __syncthreads();
+    bool fast = true;  // kCorrected: no product of the correction leaves the range
+    if (tid < kN && HOW != kUnit) {
+        const T d = S[tid * kLd + tid];
+        rd[tid] = T(1) / d;
+        fast = fast_range(d < T(0) ? -d : d);
+    }
+    if (HOW == kCorrected) fast = __syncthreads_and(fast);
+    else __syncthreads();
     if (warp < 4 && lane < 16) {
         const int b = warp * 16;
         T x[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) x[i] = i == lane ? T(1) : T(0);
-        solve16(x, S + b * kLd + b, rd + b);
+        solve16<HOW>(x, S + b * kLd + b, rd + b, fast);
 #pragma unroll
         for (int i = 0; i < 16; ++i) W[(b + lane) * kLd + b + i] = x[i];
     }
@@ -308,7 +346,7 @@ __device__ void inv64(const T* __restrict__ S, T* __restrict__ W, T* __restrict_
         T x[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) x[i] = -X[warp * 272 + lane * 17 + i];
-        solve16(x, S + (b + 16) * kLd + b + 16, rd + b + 16);
+        solve16<HOW>(x, S + (b + 16) * kLd + b + 16, rd + b + 16, fast);
 #pragma unroll
         for (int i = 0; i < 16; ++i) W[(b + lane) * kLd + b + 16 + i] = x[i];
     }
@@ -331,14 +369,17 @@ __device__ void inv64(const T* __restrict__ S, T* __restrict__ W, T* __restrict_
         T x[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) x[i] = -X[lane * 33 + i];
-        solve16(x, S + 32 * kLd + 32, rd + 32);
+        solve16<HOW>(x, S + 32 * kLd + 32, rd + 32, fast);
 #pragma unroll
         for (int i = 0; i < 16; ++i) W[lane * kLd + 32 + i] = x[i];
     }
     __syncthreads();
-    {  // their part in the last 16, two rows of one column per thread
+    {  // their part in the last 16, two rows of one column per thread: a sum of its own,
+       // or (kCorrected) the next links of the column's one chain
+        constexpr bool kChain = HOW == kCorrected;
         const int c = tid >> 3, r = (tid & 7) * 2;
-        T t0 = T(0), t1 = T(0);
+        T* x = X + c * 33 + 16 + r;
+        T t0 = kChain ? x[0] : T(0), t1 = kChain ? x[1] : T(0);
 #pragma unroll
         for (int k = 0; k < 16; ++k) {
             const T w = W[c * kLd + 32 + k];
@@ -346,15 +387,15 @@ __device__ void inv64(const T* __restrict__ S, T* __restrict__ W, T* __restrict_
             t0 = fma_t(l[0], w, t0);
             t1 = fma_t(l[1], w, t1);
         }
-        X[c * 33 + 16 + r] += t0;
-        X[c * 33 + 17 + r] += t1;
+        x[0] = kChain ? t0 : x[0] + t0;
+        x[1] = kChain ? t1 : x[1] + t1;
     }
     __syncthreads();
     if (warp == 0) {
         T x[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) x[i] = -X[lane * 33 + 16 + i];
-        solve16(x, S + 48 * kLd + 48, rd + 48);
+        solve16<HOW>(x, S + 48 * kLd + 48, rd + 48, fast);
 #pragma unroll
         for (int i = 0; i < 16; ++i) W[lane * kLd + 48 + i] = x[i];
     }
