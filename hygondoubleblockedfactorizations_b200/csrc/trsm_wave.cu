@@ -9,13 +9,16 @@
 // (three tiles in flight, independent of the solution), and for each
 // dependency j waits on a per-block flag (acquire load, bounded) and folds
 // M_ij x_j into its accumulator.  The chain of the solve runs through the last
-// dependency, i-1 (backward: i+1), so its work is taken out of it: with G =
-// op(inv_i) M_{i,i-1} formed while waiting and z_i = op(inv_i) (b_i - sum over the
-// other j) one step ahead, what follows the arrival of x_{i-1} is one product,
-// x_i = z_i - G x_{i-1}.  x_i is written to a row-major copy that consumers read
-// with 16-byte loads, published with a release store of flag i, and then to B.
-// Per block row, n = 16384, 16 columns: 4.1 us with the reduction and the inverse
-// behind the last arrival, 2.9 now.
+// dependency, i-1 (backward: i+1): everything else -- the other products, their
+// reduction over the threads, b_i less all of that -- is done while waiting for it,
+// its tile and the inverse are in shared memory, and what follows the arrival of
+// x_{i-1} is two products, y_i -= M_{i,i-1} x_{i-1} and x_i = op(inv_i) y_i.  (With
+// G = op(inv_i) M_{i,i-1} formed beforehand one product is left, x_i = op(inv_i) y_i -
+// G x_{i-1}, but the two terms may be large against their difference: backward
+// errors of LU solves came out twice as large.)  x_i is written to a row-major copy
+// that consumers read with 16-byte loads, published with a release store of flag
+// i, and then to B.  Per block row, n = 16384, 16 columns: 4.2 us with the reduction
+// behind the last arrival too, 3.8 now.
 //
 // The effective triangle M is T itself (lower forward or upper backward) or
 // T^T (lower T read transposed, backward); op(inv) is inv or inv^T in the
@@ -83,64 +86,49 @@ __device__ __forceinline__ void load_tile(float* dst, const float* T, long long 
     }
 }
 
-// x[c] += sum_k M(r, k) Xs[k][g CW + c] for a tile in load_tile's orientation.
+// p[e][c] = sum of M(r, k) Xs[k][g CW + c] over the e-th 16 of k, for a tile in
+// load_tile's orientation: four chains of 16 round less than one of 64.
 template <int CW, bool TR>
-__device__ __forceinline__ void tile_times(float x[CW], const float* M, const float* Xs, int xs,
+__device__ __forceinline__ void tile_times(float p[4][CW], const float* M, const float* Xs, int xs,
                                            int r, int g)
 {
-#pragma unroll 4
-    for (int k = 0; k < kB; k += 4) {
-        float a[4];
-        if (TR) {
-            const float4 v = *reinterpret_cast<const float4*>(M + r * kLd + k);
-            a[0] = v.x; a[1] = v.y; a[2] = v.z; a[3] = v.w;
-        } else {
+    constexpr int V = CW % 4 == 0 ? 4 : CW;  // columns per load: 2 or 4
 #pragma unroll
-            for (int e = 0; e < 4; ++e) a[e] = M[(k + e) * kLd + r];
-        }
+    for (int e = 0; e < 4; ++e)
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-#pragma unroll
-            for (int c = 0; c < CW; ++c) x[c] = fmaf(a[e], Xs[(k + e) * xs + g * CW + c], x[c]);
-    }
-}
-
-// M <- I M, both 64 x 64 in load_tile's orientation (I(r, q), M(q, k)): 4 x 4
-// entries per thread.
-template <bool TR>
-__device__ __forceinline__ void premultiply(const float* I, float* M)
-{
-    const int r4 = (threadIdx.x & 15) * 4, k4 = (threadIdx.x >> 4) * 4;
-    float acc[4][4] = {};  // [r][k]
+        for (int c = 0; c < CW; ++c) p[e][c] = 0.f;
 #pragma unroll 2
-    for (int q = 0; q < kB; q += 4) {
-        float4 v[4];  // TR: I(r4 + e, q..); else M(q.., k4 + e)
+    for (int k = 0; k < kB / 4; k += 4) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-            v[e] = *reinterpret_cast<const float4*>(TR ? I + (r4 + e) * kLd + q
-                                                       : M + (k4 + e) * kLd + q);
+        for (int e = 0; e < 4; ++e) {
+            const int k0 = e * (kB / 4) + k;
+            float a[4];
+            if (TR) {
+                const float4 v = *reinterpret_cast<const float4*>(M + r * kLd + k0);
+                a[0] = v.x; a[1] = v.y; a[2] = v.z; a[3] = v.w;
+            } else {
 #pragma unroll
-        for (int s = 0; s < 4; ++s) {
-            const float4 w = *reinterpret_cast<const float4*>(TR ? M + (q + s) * kLd + k4
-                                                                 : I + (q + s) * kLd + r4);
-            const float wv[4] = {w.x, w.y, w.z, w.w};
+                for (int f = 0; f < 4; ++f) a[f] = M[(k0 + f) * kLd + r];
+            }
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float ve = s == 0 ? v[e].x : s == 1 ? v[e].y : s == 2 ? v[e].z : v[e].w;
+            for (int f = 0; f < 4; ++f) {
+                const float* q = Xs + (k0 + f) * xs + g * CW;
 #pragma unroll
-                for (int f = 0; f < 4; ++f) {
-                    if (TR) acc[e][f] = fmaf(ve, wv[f], acc[e][f]);
-                    else acc[f][e] = fmaf(wv[f], ve, acc[f][e]);
+                for (int c = 0; c < CW; c += V) {
+                    float b[V];
+                    if (V == 4) {
+                        const float4 v = *reinterpret_cast<const float4*>(q + c);
+                        b[0] = v.x; b[1] = v.y; b[2 % V] = v.z; b[3 % V] = v.w;
+                    } else {
+                        const float2 v = *reinterpret_cast<const float2*>(q + c);
+                        b[0] = v.x; b[1] = v.y;
+                    }
+#pragma unroll
+                    for (int i = 0; i < V; ++i) p[e][c + i] = fmaf(a[f], b[i], p[e][c + i]);
                 }
             }
         }
     }
-    __syncthreads();
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-        *reinterpret_cast<float4*>(TR ? M + (r4 + e) * kLd + k4 : M + (k4 + e) * kLd + r4) =
-            TR ? make_float4(acc[e][0], acc[e][1], acc[e][2], acc[e][3])
-               : make_float4(acc[0][e], acc[1][e], acc[2][e], acc[3][e]);
 }
 
 template <int NB, bool TR>
@@ -155,8 +143,8 @@ __global__ void __launch_bounds__(kWT, 2) trsv_wave_kernel(int n, int nrhs, cons
     extern __shared__ __align__(16) float smem[];
     float* Mt = smem;                          // kDepth tiles
     float* Is = Mt + kDepth * kB * kLd;        // op(inv_i)
-    float* Gt = Is + kB * kLd;                 // M_{i,i-1}, then op(inv_i) M_{i,i-1}
-    float* Xs = Gt + kB * kLd;                 // x_j (row-major, padded); later y_i
+    float* Gt = Is + kB * kLd;                 // M_{i,i-1}
+    float* Xs = Gt + kB * kLd;                 // x_j (row-major, padded); then y_i
     float* red = Mt;                           // 4 x NB x 64 partial sums (after the tiles)
     __shared__ int s_ticket, s_abort;
 
@@ -227,11 +215,6 @@ __global__ void __launch_bounds__(kWT, 2) trsv_wave_kernel(int n, int nrhs, cons
             const int col = g * CW + c;
             bv[c] = (r < rows && col < nrhs) ? B[(long long)col * ldb + i0 + r] : 0.f;
         }
-        if (m > 0) {  // G
-            cp_wait<kDepth>();
-            __syncthreads();
-            premultiply<TR>(Is, Gt);
-        }
         float acc[NB];
 #pragma unroll
         for (int c = 0; c < NB; ++c) acc[c] = 0.f;
@@ -276,34 +259,36 @@ __global__ void __launch_bounds__(kWT, 2) trsv_wave_kernel(int n, int nrhs, cons
         cp_wait<0>();
         __syncthreads();
 
-        // y_i = b_i - sum over the four k-groups
+        // y_i = b_i - sum over the four k-groups, - M_{i,i-1} x_{i-1}
 #pragma unroll
         for (int c = 0; c < NB; ++c) red[(g * NB + c) * kB + r] = acc[c];
         __syncthreads();
+        float y[CW];
 #pragma unroll
         for (int c = 0; c < CW; ++c) {
             const int col = g * CW + c;
-            float y = bv[c];
+            y[c] = bv[c];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) y -= red[(q * NB + col) * kB + r];
-            Xs[r * XS + col] = (r < rows) ? y : 0.f;
+            for (int q = 0; q < 4; ++q) y[c] -= red[(q * NB + col) * kB + r];
         }
-        __syncthreads();
-        // z_i = op(inv_i) y_i, then x_i = z_i - G x_{i-1}
-        float x[CW];
-#pragma unroll
-        for (int c = 0; c < CW; ++c) x[c] = 0.f;
-        tile_times<CW, TR>(x, Is, Xs, XS, r, g);
         if (m > 0) {
-            __syncthreads();  // y has been read
             if (!take(dep(m - 1))) return;
-            float t[CW];
+            float p[4][CW];
+            tile_times<CW, TR>(p, Gt, Xs, XS, r, g);
 #pragma unroll
-            for (int c = 0; c < CW; ++c) t[c] = 0.f;
-            tile_times<CW, TR>(t, Gt, Xs, XS, r, g);
+            for (int c = 0; c < CW; ++c)
 #pragma unroll
-            for (int c = 0; c < CW; ++c) x[c] -= t[c];
+                for (int e = 0; e < 4; ++e) y[c] -= p[e][c];
+            __syncthreads();  // x_{i-1} has been read
         }
+#pragma unroll
+        for (int c = 0; c < CW; ++c) Xs[r * XS + g * CW + c] = (r < rows) ? y[c] : 0.f;
+        __syncthreads();
+        // x_i = op(inv_i) y_i
+        float x[CW], s[4][CW];
+        tile_times<CW, TR>(s, Is, Xs, XS, r, g);
+#pragma unroll
+        for (int c = 0; c < CW; ++c) x[c] = (s[0][c] + s[1][c]) + (s[2][c] + s[3][c]);
         float* xdst = X + (long long)(i0 + r) * NB + g * CW;
 #pragma unroll
         for (int c = 0; c < CW; ++c) {
