@@ -146,7 +146,7 @@ hdbf_status potrf_db_impl(hdbf_context* ctx, T* A, int lda, int n, int nb, int b
             T* Aii = at(A, lda, inner, inner);
             {
                 StageScope sc(ctx, kStPotrf);
-                HDBF_TRY(potrf_diag(ctx, isz, Aii, lda, info, inner));
+                HDBF_TRY(potrf_diag(ctx, isz, Aii, lda, info, inner, rows <= 0));
             }
             {
                 StageScope sc(ctx, kStTrsm);
@@ -217,7 +217,7 @@ hdbf_status potrf_blocked_rl_impl(hdbf_context* ctx, T* A, int lda, int n, int n
         psz = block_width(n, k, nb, tail_order<T>(ctx));
         const int tr = n - k - psz;
         T* Akk = at(A, lda, k, k);
-        HDBF_TRY(potrf_diag(ctx, psz, Akk, lda, info, k));
+        HDBF_TRY(potrf_diag(ctx, psz, Akk, lda, info, k, tr <= 0));
         if (tr <= 0) continue;
         T* A21 = at(A, lda, k + psz, k);
         HDBF_TRY(trsm_rlt_ready(ctx, tr, psz, Akk, lda, A21, lda));
@@ -286,7 +286,7 @@ hdbf_status rec_potrf_impl(hdbf_context* ctx, T* A, long long lda, int n, int nb
 {
     if (n <= 0) return HDBF_STATUS_SUCCESS;
     if (nb <= 0 || n <= std::max(nb, tail_order<T>(ctx)))
-        return potrf_diag(ctx, n, A, lda, info, info_base);
+        return potrf_diag(ctx, n, A, lda, info, info_base, true);
     const int n1 = n / 2;
     const int n2 = n - n1;
     T* A21 = A + n1;

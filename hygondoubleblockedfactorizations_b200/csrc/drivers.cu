@@ -21,20 +21,22 @@ inline int split_at(int n, int leaf)
 }  // namespace
 
 hdbf_status potrf_diag(hdbf_context* ctx, int n, float* A, long long lda, int* info,
-                       int info_base)
+                       int info_base, bool last)
 {
     if (n <= 0) return HDBF_STATUS_SUCCESS;
     HDBF_TRY(ensure_ws(ctx, n));
-    if (n <= kDiagLeaf) return potf2_small(ctx, n, A, lda, info, info_base, ws_inv(ctx));
-    if (n <= potrf_block_max_n()) return potrf_block(ctx, n, A, lda, info, info_base, nullptr, 0);
+    if (n <= kDiagLeaf)
+        return potf2_small(ctx, n, A, lda, info, info_base, last ? nullptr : ws_inv(ctx));
+    if (n <= potrf_block_max_n())
+        return potrf_block(ctx, n, A, lda, info, info_base, nullptr, 0, last);
     const int n1 = split_at(n, kDiagLeaf);
     const int n2 = n - n1;
     float* A21 = A + n1;
     float* A22 = A + (long long)n1 * lda + n1;
-    HDBF_TRY(potrf_diag(ctx, n1, A, lda, info, info_base));
+    HDBF_TRY(potrf_diag(ctx, n1, A, lda, info, info_base, false));
     HDBF_TRY(trsm_rlt_ready(ctx, n2, n1, A, lda, A21, lda));
     HDBF_TRY(syrk_lower(ctx, n2, n1, A21, lda, A22, lda));
-    return potrf_diag(ctx, n2, A22, lda, info, info_base + n1);
+    return potrf_diag(ctx, n2, A22, lda, info, info_base + n1, last);
 }
 
 namespace {

@@ -385,20 +385,21 @@ hdbf_status syrk_lower(hdbf_context* ctx, int n, int k, const double* A, long lo
 }
 
 hdbf_status potrf_diag(hdbf_context* ctx, int n, double* A, long long lda, int* info,
-                       int info_base)
+                       int info_base, bool last)
 {
     if (n <= 0) return HDBF_STATUS_SUCCESS;
     HDBF_TRY(ensure_ws(ctx, ws_order<double>(n)));
     if (n <= kL)
-        return potf2_small(ctx, n, A, lda, info, info_base, reinterpret_cast<double*>(ws_inv(ctx)));
+        return potf2_small(ctx, n, A, lda, info, info_base,
+                           last ? nullptr : reinterpret_cast<double*>(ws_inv(ctx)));
     const int n1 = split64(n);
     const int n2 = n - n1;
     double* A21 = A + n1;
     double* A22 = A + (long long)n1 * lda + n1;
-    HDBF_TRY(potrf_diag(ctx, n1, A, lda, info, info_base));
+    HDBF_TRY(potrf_diag(ctx, n1, A, lda, info, info_base, false));
     HDBF_TRY(trsm_rlt_ready(ctx, n2, n1, A, lda, A21, lda));
     HDBF_TRY(syrk_lower(ctx, n2, n1, A21, lda, A22, lda));
-    return potrf_diag(ctx, n2, A22, lda, info, info_base + n1);
+    return potrf_diag(ctx, n2, A22, lda, info, info_base + n1, last);
 }
 
 hdbf_status apply_moves(hdbf_context* ctx, double* A, long long lda, int ncols, const int* src,

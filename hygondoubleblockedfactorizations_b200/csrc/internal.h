@@ -503,13 +503,14 @@ hdbf_status add_damping(cudaStream_t s, float* A, int n, long long lda, float la
 // Cholesky of an n x n (n <= potrf_block_max_n()) diagonal block on one cluster;
 // with W non-null also W = L^{-1} (lower, upper zeroed), in a second launch.
 hdbf_status potrf_block(hdbf_context* ctx, int n, float* A, long long lda, int* info,
-                        int info_base, float* W, long long ldw);
+                        int info_base, float* W, long long ldw, bool last = false);
 int potrf_block_max_n();
 void configure_potrf_block(hdbf_context* ctx);
 // Orders up to potrf_block_max_n() also leave the 64x64 diagonal-block
-// inverses of the factor in ws_inv, for a trsm_rlt_ready with the same block.
+// inverses of the factor in ws_inv, for a trsm_rlt_ready with the same block;
+// not the last one with `last` (nothing below the block).
 hdbf_status potrf_diag(hdbf_context* ctx, int n, float* A, long long lda, int* info,
-                       int info_base);
+                       int info_base, bool last);
 hdbf_status trsm_rlt(hdbf_context* ctx, int rows, int cols, const float* L, long long ldl,
                      float* B, long long ldb);
 // trsm_rlt against the block that potrf_diag has just factored on this stream.
@@ -567,7 +568,7 @@ hdbf_status trsm_llu(hdbf_context* ctx, int rows, int cols, const double* L, lon
 hdbf_status syrk_lower(hdbf_context* ctx, int n, int k, const double* A, long long lda,
                        double* C, long long ldc);
 hdbf_status potrf_diag(hdbf_context* ctx, int n, double* A, long long lda, int* info,
-                       int info_base);
+                       int info_base, bool last);
 hdbf_status apply_moves(hdbf_context* ctx, double* A, long long lda, int ncols, const int* src,
                         const int* tgt, const int* count, int max_moves, double* temp,
                         long long temp_cols);

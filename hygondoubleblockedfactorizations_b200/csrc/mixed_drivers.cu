@@ -310,7 +310,7 @@ hdbf_status potrf_mixed_body(hdbf_context* ctx, int prec, float* A, long long ld
             HDBF_TRY(potrf_panel_fallback(ctx, A, lda, A0, n, n, k, psz, flag, info, wb.W, wb.ldw,
                                           fallbacks));
         } else {
-            HDBF_TRY(potrf_diag(ctx, psz, Akk, lda, info, k));
+            HDBF_TRY(potrf_diag(ctx, psz, Akk, lda, info, k, tr <= 0));
         }
         if (tr <= 0) continue;
         float* A21 = at(A, lda, k + psz, k);

@@ -245,8 +245,8 @@ struct ClusterBarrier {
 };
 
 __global__ void __launch_bounds__(kThreads, 1)
-potrf_cluster_kernel(int n, float* A, long long lda, int* info, int info_base, float* dinv, int* fail,
-                     int* err, const int* run_if)
+potrf_cluster_kernel(int n, float* A, long long lda, int* info, int info_base, float* dinv, int last,
+                     int* fail, int* err, const int* run_if)
 {
     extern __shared__ __align__(16) unsigned char sm_raw[];
     ClusterSmem& sm = *reinterpret_cast<ClusterSmem*>(sm_raw);
@@ -316,8 +316,10 @@ potrf_cluster_kernel(int n, float* A, long long lda, int* info, int info_base, f
                 *reinterpret_cast<volatile int*>(fail) = 1;
             }
             // also of a failing tile: its columns before the failing one are valid
-            tile64::inv64<tile64::kReciprocal>(S, W, sm.X, sm.rd);
-            tile64::store_inv(dinv + (long long)k * kT * kT, W, false);
+            if (!last || k < NT - 1) {
+                tile64::inv64<tile64::kReciprocal>(S, W, sm.X, sm.rd);
+                tile64::store_inv(dinv + (long long)k * kT * kT, W, false);
+            }
             if (!solo) {
                 if (waiting && !bar.wait(1)) break;
                 waiting = false;
@@ -539,7 +541,7 @@ tile_inverse_kernel(int n, const float* A, long long lda, float* W, long long ld
 int potrf_block_max_n() { return kT * kMaxNT; }
 
 hdbf_status potrf_block(hdbf_context* ctx, int n, float* A, long long lda, int* info,
-                        int info_base, float* W, long long ldw)
+                        int info_base, float* W, long long ldw, bool last)
 {
     if (n <= 0) return HDBF_STATUS_SUCCESS;
     if (n > kT * kMaxNT || lda < n || (W && ldw < n)) return HDBF_STATUS_INVALID_VALUE;
@@ -575,7 +577,7 @@ hdbf_status potrf_block(hdbf_context* ctx, int n, float* A, long long lda, int* 
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     cudaError_t e = cudaLaunchKernelEx(&cfg, potrf_cluster_kernel, n, A, lda, info, info_base, dinv,
-                                       fail, err, ctx->run_if);
+                                       (int)(last && !W), fail, err, ctx->run_if);
     ctx->launches++;
     if (e == cudaSuccess && W) {
         int G = std::min(NT * NT, ctx->sm_count);  // the set-up pass touches NT^2 tiles
