@@ -24,7 +24,8 @@ constexpr size_t kTileSmem = sizeof(T) == 4 ? 0 : sizeof(T) * (size_t)kTileWords
 // Pivot test and info follow LAPACK xPOTRF: the first column whose updated
 // diagonal is not > 0 (or is NaN) stops the factorization, its value is left
 // in place, and info = info_base + j + 1 (first failure wins).  A block whose
-// info is already non-zero is left untouched.
+// info is already non-zero is left untouched, and inv is then the inverse of the
+// block as it stands, so that the panel solve depends on the matrix alone.
 template <class T>
 __global__ void __launch_bounds__(tile64::kThreads, 1)
 potf2_kernel(int n, T* A, long long lda, int* info, int info_base, T* inv)
@@ -37,12 +38,16 @@ potf2_kernel(int n, T* A, long long lda, int* info, int info_base, T* inv)
     T* X = W + kLeaf * tile64::kLd;
     T* rd = X + tile64::kScratch;
     __shared__ int s_fail;
-    if (info && *reinterpret_cast<volatile int*>(info) != 0) return;
+    // read by every thread before thread 0 may write it behind load_lower's barrier
+    const bool done = info && *reinterpret_cast<volatile int*>(info) != 0;
+    if (done && !inv) return;
     tile64::load_lower<false>(S, A, lda, n, false);
     __syncthreads();
-    const int fail = tile64::chol64(S, n, &s_fail);
-    tile64::store_lower(A, S, lda, n);
-    if (fail >= 0 && threadIdx.x == 0 && info) atomicCAS(info, 0, info_base + fail + 1);
+    if (!done) {
+        const int fail = tile64::chol64(S, n, &s_fail);
+        tile64::store_lower(A, S, lda, n);
+        if (fail >= 0 && threadIdx.x == 0 && info) atomicCAS(info, 0, info_base + fail + 1);
+    }
     if (inv) {
         tile64::inv64<tile64::kReciprocal>(S, W, X, rd);
         tile64::store_inv(inv, W, false);

@@ -22,7 +22,9 @@
 // Pivot test and info follow LAPACK xPOTRF: the first column whose updated
 // diagonal is not > 0 (or is NaN) stops the factorization and info =
 // info_base + column + 1 (first failure wins); a block whose info is already
-// non-zero is left untouched.  Every wait is bounded by the handle's poll limit:
+// non-zero is left untouched.  The inverses of tiles that were not factored are
+// those of the tiles as they stand: what the panel solve makes of the rest of the
+// matrix then depends on the matrix alone.  Every wait is bounded by the handle's poll limit:
 // on expiry the kernel records a timeout and the remaining work is skipped; a
 // cluster's CTAs then meet at a hardware barrier, so that none leaves while
 // another may still arrive in its shared memory.
@@ -263,19 +265,17 @@ potrf_cluster_kernel(int n, float* A, long long lda, int* info, int info_base, f
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&sm.bar[b])),
                          "r"(C));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        sm.stop = ((info && *reinterpret_cast<volatile int*>(info) != 0) ||
-                   (run_if && *reinterpret_cast<const volatile int*>(run_if) == 0))
-                      ? 1
-                      : 0;
+        sm.stop = (run_if && *reinterpret_cast<const volatile int*>(run_if) == 0) ? 2
+                  : (info && *reinterpret_cast<volatile int*>(info) != 0)         ? 1
+                                                                                  : 0;
     }
     __syncthreads();
-    const bool skip = sm.stop != 0;  // the same in every CTA: read before any write
+    const int skip = sm.stop;  // the same in every CTA: read before any write
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    if (skip) {
-        if (rank == 0 && tid == 0) *fail = 1;  // no inverse either
-        return;
-    }
+    if (skip && rank == 0 && tid == 0) *fail = 1;  // no W either
+    if (skip == 2) return;
+    int stands = skip ? 0 : NT;  // first tile that is inverted as it stands
     ClusterBarrier bar{&sm, C, spin_limit_of(err), err, {0u, 0u}};
     // One CTA needs no barriers: 0 = column k ready (D_k written, step k - 1 applied),
     // 1 = column k solved.
@@ -303,7 +303,8 @@ potrf_cluster_kernel(int n, float* A, long long lda, int* info, int info_base, f
             for (int i = 0; i < 4; ++i)
                 if (r4 + i < rows && c4 + j < cols) T[(long long)(c4 + j) * lda + r4 + i] = acc[i][j];
     };
-    if (rank == 0) {
+    if (skip) {
+    } else if (rank == 0) {
         float *S = sm.tile[0], *W = sm.tile[1], *P = sm.tile[2], *X = sm.tile[3];
         tile64::load_lower<true>(S, A, lda, ext(0), false);
         __syncthreads();
@@ -328,6 +329,7 @@ potrf_cluster_kernel(int n, float* A, long long lda, int* info, int info_base, f
             } else {
                 __syncthreads();
             }
+            if (f >= 0) stands = k + 1;
             if (f >= 0 || k == NT - 1) break;
             // X = L(k+1, k) = A(k+1, k) D_k^T
             fetch_tile(P, src(k + 1, k));
@@ -373,6 +375,7 @@ potrf_cluster_kernel(int n, float* A, long long lda, int* info, int info_base, f
             if (!bar.wait(0)) break;
             if (tid == 0) sm.stop = *reinterpret_cast<volatile int*>(fail);
             __syncthreads();
+            if (sm.stop) stands = k + 1;
             if (sm.stop || k == NT - 1) break;
             for (int i = k + 2 + w; i < NT; i += nw) {  // L(i, k) = A(i, k) D_k^T
                 fetch_tile(sm.tile[0], src(i, k));
@@ -437,6 +440,13 @@ potrf_cluster_kernel(int n, float* A, long long lda, int* info, int info_base, f
             }
             fetch_wait<0>();
         }
+    }
+    for (int i = stands + rank; i < NT - last; i += C) {
+        __syncthreads();
+        tile64::load_lower<true>(sm.tile[0], tile(i, i), lda, ext(i), false);
+        __syncthreads();
+        tile64::inv64<tile64::kReciprocal>(sm.tile[0], sm.tile[1], sm.X, sm.rd);
+        tile64::store_inv(dinv + (long long)i * kT * kT, sm.tile[1], false);
     }
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");

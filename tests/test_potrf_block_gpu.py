@@ -54,3 +54,32 @@ def test_block_failure(hd, handle, torch_cuda, n, col):
     assert (np.abs(np.tril(L @ L[:done].T - A[:, :done])) <= bound).all()
     again, info = factor(torch_cuda, hd, handle, spd(n, 3), n)  # the handle goes on
     assert info == 0
+
+
+@pytest.mark.parametrize("n,nb,b,col", [(1000, 512, 256, 100), (700, 1024, 200, 300),
+                                        (1100, 512, 1024, 64), (300, 128, 64, 5)])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_failure_depends_on_the_matrix_alone(hd, torch_cuda, n, nb, b, col, dtype):
+    """What is left behind a failed Cholesky is the same on a new handle and on one that
+    has factored something else in between."""
+    name = "double_blocked_potrf" + ("" if dtype == np.float32 else "_double")
+
+    def run(h, A):
+        d, info = dev(torch_cuda, A.astype(dtype)), info_tensor(torch_cuda)
+        hd.call(name, h.ptr, ptr(d), len(A), len(A), nb, b, ptr(info))
+        torch_cuda.cuda.synchronize()
+        h.check(name)
+        return d.cpu().numpy(), int(info.item())
+
+    bad = spd(n)
+    bad[col, col] = -1.0
+    out = []
+    for other in (None, 3.0 * spd(n, 5), 0.1 * spd(n, 6)):
+        h = hd.Handle(torch_cuda.cuda.current_stream().cuda_stream)
+        if other is not None:
+            assert run(h, other)[1] == 0
+        out.append(run(h, bad))
+        h.close()
+    assert all(info == col + 1 for _, info in out)
+    np.testing.assert_array_equal(out[1][0], out[0][0])
+    np.testing.assert_array_equal(out[2][0], out[0][0])
