@@ -16,6 +16,8 @@
 
 #include <cuda_runtime.h>
 
+#include <cfloat>
+
 namespace hdbf {
 namespace tile64 {
 
@@ -29,17 +31,14 @@ struct alignas(16) Vec4 {
     T x[4];
 };
 
-// 1 / d, and 1 / sqrt(d) with sqrt(d), each to about an ulp: one Newton step
-// on the hardware estimate (and one residual correction of the root).  For d
-// in fast_range, where no intermediate product over- or underflows.
-__device__ __forceinline__ bool fast_range(float d) { return d > 1e-30f && d < 1e30f; }
-__device__ __forceinline__ bool fast_range(double d) { return d > 1e-250 && d < 1e250; }
-__device__ __forceinline__ float fast_rcp(float d)
-{
-    const float r = __fdividef(1.f, d);
-    return fmaf(r, fmaf(-d, r, 1.f), r);
-}
-__device__ __forceinline__ double fast_rcp(double d) { return 1.0 / d; }
+// 1 / sqrt(d) and sqrt(d), each to about an ulp: one Newton step on the hardware
+// estimate, and one residual correction of the root.  For d in fast_range, the normal
+// numbers up to 2^126: no product here overflows, and the one that may underflow, the
+// root's residual below 2^-100, only loses part of the correction.  A matrix may be
+// tiny or huge as a whole, and the careful path costs a tile twice its time (n = 64
+// times 1e32: 24 us, 49 the careful way).
+__device__ __forceinline__ bool fast_range(float d) { return d >= FLT_MIN && d <= 8.5e37f; }
+__device__ __forceinline__ bool fast_range(double d) { return d >= DBL_MIN && d <= 4e307; }
 __device__ __forceinline__ void rsqrt_pair(float d, float& r, float& s)
 {
     r = rsqrtf(d);
@@ -249,8 +248,8 @@ __device__ __forceinline__ void store_inv(T* dst, const T* W, bool trans)
 
 // How a substitution divides by the diagonal: not at all (unit); by a reciprocal; by a
 // reciprocal and one correction, q += r (x - d q) (Markstein, IBM J. Res. Dev. 34,
-// 1990: the rounded quotient but for rare ties), or, where the diagonal leaves
-// fast_range, by division instead.  Against division everywhere, the plain reciprocal gives
+// 1990: the rounded quotient but for rare ties), or, where the diagonal leaves the
+// range in which the residual is exact, by division instead.  Against division everywhere, the plain reciprocal gives
 // the same errors or less in solves with Cholesky factors (right-side TRSM 3 %,
 // POTRS 4 %), but 4-7 % more in U^{-1} and solves with U, which take the correction
 // (0.2 us a tile, in a launch of its own and not on a factorization's chain).
@@ -308,11 +307,11 @@ __device__ void inv64(const T* __restrict__ S, T* __restrict__ W, T* __restrict_
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int q = tid; q < kN * kLd; q += kThreads) W[q] = T(0);
-    bool fast = true;  // kCorrected: no product of the correction leaves the range
+    bool fast = true;
     if (tid < kN && HOW != kUnit) {
         const T d = S[tid * kLd + tid];
         rd[tid] = T(1) / d;
-        fast = fast_range(d < T(0) ? -d : d);
+        fast = d * d > T(1e-36) && d * d < T(1e36);
     }
     if (HOW == kCorrected) fast = __syncthreads_and(fast);
     else __syncthreads();

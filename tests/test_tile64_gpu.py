@@ -80,3 +80,23 @@ def test_inverse_residual(hd, handle, torch_cuda, dtype, half, diag):
     assert (np.triu(W, 1) == 0).all()
     bound = (n + 3) * unit * (np.abs(Lw) @ np.abs(W))
     assert (np.abs(Lw @ W - np.eye(n)) <= bound).all()
+
+
+@pytest.mark.parametrize("n", [8, 64, 200, 700])
+@pytest.mark.parametrize("k", [50, 55, 61])
+def test_scaled_matrix_same_bits(hd, handle, torch_cuda, n, k):
+    """4^k A has the factor 2^k L, bit for bit: every operation scales exactly as long as
+    nothing overflows (and nothing underflows here), whatever path the pivots take."""
+    A = spd(n)
+    assert A.max() * 4.0 ** k < 2.0 ** 125
+
+    def run(M):
+        d, info = dev(torch_cuda, M), info_tensor(torch_cuda)
+        hd.call("double_blocked_potrf", handle.ptr, ptr(d), n, n, 256, 64, ptr(info))
+        torch_cuda.cuda.synchronize()
+        handle.check()
+        assert info.item() == 0
+        return np.tril(host2d(d, n, n, n))
+
+    want = run(A) * np.float32(2.0 ** k)
+    np.testing.assert_array_equal(run(A * np.float32(4.0 ** k)), want)
