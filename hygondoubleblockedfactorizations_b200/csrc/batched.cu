@@ -132,8 +132,10 @@ __device__ __noinline__ int lu_panel_rows(Smem<T, PW>& s, int m, int kb)
             int best = INT_MAX;
 #pragma unroll
             for (int i = 0; i < R; ++i) {
+                // xGETRF's first maximum: a NaN is one on the diagonal (nothing compares
+                // above it; its bits are above an infinity's) and loses elsewhere
                 const float v = fabsf(a[i][0]);
-                const unsigned b = v == v ? __float_as_uint(v) : 0u;  // a NaN loses
+                const unsigned b = v == v || pos[i] == J ? __float_as_uint(v) : 0u;
                 if (pos[i] >= J &&
                     (best == INT_MAX || b > vb || (b == vb && pos[i] < best))) {
                     vb = b;

@@ -93,3 +93,35 @@ def test_failures(hd, handle, torch_cuda, variant):
     L = np.tril(b.matrix(4).cpu().numpy()).astype(np.float64)
     bound = 2 * (48 + 2) * 2.0 ** -24 * (np.abs(L) @ np.abs(L).T)
     assert (np.abs(np.tril(L @ L.T - A[4].astype(np.float64))) <= bound).all()
+
+
+@pytest.mark.parametrize("variant", range(6))
+def test_lu_nan_pivots(hd, handle, torch_cuda, variant):
+    """The first maximum as reference LAPACK's ISAMAX finds it: a NaN on the diagonal is
+    never beaten, a NaN below it never chosen."""
+    where = [(0, 0), (5, 0), (40, 30), (30, 30), (99, 99), (17, 16)]
+    n = 100
+    b = DeviceBatch(torch_cuda, np.ones(len(where), np.int32), np.full(len(where), n, np.int32))
+    A, _ = fill(torch_cuda, b, 7)
+    for i, (r, c) in enumerate(where):
+        # strong entries on the diagonal: without the NaN no row moves
+        A[i] = (np.random.default_rng(i).uniform(-1, 1, (n, n)) + 4 * n * np.eye(n)).astype(
+            np.float32)
+        A[i][r, c] = np.nan
+    b.A.copy_(torch_cuda.from_numpy(np.concatenate([M.ravel(order="F") for M in A])))
+    assert b.run(handle, variant) == 0
+    torch_cuda.cuda.synchronize()
+    for i, (r, c) in enumerate(where):
+        M = A[i].astype(np.float64)
+        piv = []
+        with np.errstate(invalid="ignore"):
+            for j in range(n):
+                p = j
+                for q in range(j + 1, n):
+                    if abs(M[q, j]) > abs(M[p, j]):
+                        p = q
+                piv.append(p)
+                M[[j, p]] = M[[p, j]]
+                M[j + 1:, j] /= M[j, j]
+                M[j + 1:, j + 1:] -= np.outer(M[j + 1:, j], M[j, j + 1:])
+        np.testing.assert_array_equal(b.pivots(i).cpu().numpy() - 1, piv)
