@@ -516,6 +516,39 @@ __device__ __forceinline__ void rhs_update(Smem<T, PW>& s, int k, int kb, int m)
     }
 }
 
+// x / d by d's reciprocal r and one correction (Markstein, IBM J. Res. Dev. 34, 1990:
+// the rounded quotient but for rare ties), where the residual is exact; by division
+// elsewhere.  The plain product x r rounds twice: 2-3 % more error in a solution.
+__device__ __forceinline__ bool plain_quotients(float d) { return d * d > 1e-36f && d * d < 1e36f; }
+template <bool PLAIN>
+__device__ __forceinline__ float quotient(float x, float d, float r)
+{
+    const float q = x * r;
+    return PLAIN ? fmaf(fmaf(-d, q, x), r, q) : x / d;
+}
+// One warp's substitution on x (lane i: row i of kB), d its diagonal, row(q) the factor
+// of x_q in this lane's row; BACK from the last row up.
+template <bool PLAIN, bool BACK, int N, class Row>
+__device__ __forceinline__ float warp_substitute(float x, float d, float r, Row row)
+{
+    const int i = threadIdx.x & 31;
+#pragma unroll
+    for (int s = 0; s < N; ++s) {
+        const int q = BACK ? N - 1 - s : s;
+        const float xq = __shfl_sync(0xffffffffu, quotient<PLAIN>(x, d, r), q);
+        x = (BACK ? i < q : i > q) ? fmaf(-row(q), xq, x) : x;
+    }
+    return quotient<PLAIN>(x, d, r);
+}
+template <bool BACK, int N, class Row>
+__device__ __forceinline__ float warp_solve(float x, float d, Row row)
+{
+    const float r = 1.f / d;
+    if (__all_sync(0xffffffffu, plain_quotients(d)))
+        return warp_substitute<true, BACK, N>(x, d, r, row);
+    return warp_substitute<false, BACK, N>(x, d, r, row);
+}
+
 // x1 <- L11^{-1} x1 on one warp (unit: implicit ones on the diagonal).
 template <int T, int PW>
 __device__ __forceinline__ void rhs_solve(Smem<T, PW>& s, int k, int kb, bool unit)
@@ -524,14 +557,18 @@ __device__ __forceinline__ void rhs_solve(Smem<T, PW>& s, int k, int kb, bool un
     float li[PW];
 #pragma unroll
     for (int q = 0; q < PW; ++q) li[q] = (i < kb && q < i) ? s.P[q * kLdp + i] : 0.f;
-    const float rd = (i < kb && !unit) ? 1.f / s.P[i * kLdp + i] : 1.f;
     float xi = i < kb ? s.x[k + i] : 0.f;
+    if (unit) {
 #pragma unroll
-    for (int q = 0; q < PW; ++q) {
-        const float xq = __shfl_sync(0xffffffffu, xi * rd, q);
-        xi = i > q ? fmaf(-li[q], xq, xi) : xi;
+        for (int q = 0; q < PW; ++q) {
+            const float xq = __shfl_sync(0xffffffffu, xi, q);
+            xi = i > q ? fmaf(-li[q], xq, xi) : xi;
+        }
+    } else {
+        const float d = i < kb ? s.P[i * kLdp + i] : 1.f;
+        xi = warp_solve<false, PW>(xi, d, [&](int q) { return li[q]; });
     }
-    if (i < kb) s.x[k + i] = xi * rd;
+    if (i < kb) s.x[k + i] = xi;
 }
 
 // ------------------------------------------------------------------ LU
@@ -674,14 +711,9 @@ __device__ __forceinline__ void block_back(const float* D, float* x, int kb, con
 #pragma unroll
     for (int q = 0; q < kBk; ++q)
         d[q] = (i < kb && q > i && q < kb) ? (TRANS ? D[q * 33 + i] : D[i * 33 + q]) : 0.f;
-    const float rd = i < kb ? 1.f / D[i * 33 + i] : 1.f;
     float xi = i < kb ? x[i] - (sub ? sub[i] : 0.f) : 0.f;
-#pragma unroll
-    for (int q = kBk - 1; q >= 0; --q) {
-        const float xq = __shfl_sync(0xffffffffu, xi * rd, q);
-        xi = i < q ? fmaf(-d[q], xq, xi) : xi;
-    }
-    if (i < kb) x[i] = xi * rd;
+    xi = warp_solve<true, kBk>(xi, i < kb ? D[i * 33 + i] : 1.f, [&](int q) { return d[q]; });
+    if (i < kb) x[i] = xi;
 }
 
 // x <- U^{-1} x, U the upper triangle of A (non-unit): the block's columns of the

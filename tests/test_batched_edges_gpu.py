@@ -125,3 +125,25 @@ def test_lu_nan_pivots(hd, handle, torch_cuda, variant):
                 M[j + 1:, j] /= M[j, j]
                 M[j + 1:, j + 1:] -= np.outer(M[j + 1:, j], M[j, j + 1:])
         np.testing.assert_array_equal(b.pivots(i).cpu().numpy() - 1, piv)
+
+
+@pytest.mark.parametrize("op", [0, 1])
+@pytest.mark.parametrize("variant", range(6))
+def test_solve_divides(hd, handle, torch_cuda, op, variant):
+    """Diagonal systems over the whole range of exponents, subnormal pivots among them:
+    the solution is the division's, exact here (b = d times a small integer, zero among
+    them; Cholesky: d a power of four)."""
+    n = 70
+    b = DeviceBatch(torch_cuda, np.full(2, op, np.int32), np.full(2, n, np.int32))
+    k = np.arange(n)
+    d = np.float32(2.0) ** np.where(op, -148 + 4 * k, 2 * (-73 + 2 * k)).astype(np.float64)
+    d = d[d < 2.0 ** 120][np.arange(n) % (d < 2.0 ** 120).sum()].astype(np.float32)
+    assert (d > 0).all() and (d < 2.0 ** -126).any()
+    x = (k % 5).astype(np.float32)
+    want = np.concatenate([x, x])
+    b.A.copy_(torch_cuda.from_numpy(np.concatenate([np.diag(d).ravel()] * 2)))
+    b.b.copy_(torch_cuda.from_numpy(np.concatenate([d * x] * 2)))
+    assert b.run(handle, variant) == 0
+    torch_cuda.cuda.synchronize()
+    assert not b.info.cpu().numpy().any()
+    np.testing.assert_array_equal(b.b.cpu().numpy(), want)
