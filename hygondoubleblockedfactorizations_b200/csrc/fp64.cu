@@ -244,6 +244,23 @@ void dgemm_launch64(cudaStream_t s, int M, int N, int K, const double* A, long l
         M, N, K, A, lda, B, ldb, C, ldc, tm);
 }
 
+// The small-update kernel's split (gemm_small.cu), or 0 where 64 x 64 x 16 tiles are
+// faster.  Both have the same tiles and are bound by the FP64 pipe: the small kernel
+// takes 1.17 times as long per step of K (0.075 us), the other 6 us (80 steps) more to
+// start, and only the small one splits K.  4096 x 1024 x 1000: 652 us, 544 in 64 x 64 x
+// 16 tiles; 2048 x 64 x 512: 27 us, 54.  Tall updates of up to three tile columns and
+// one tile per SM are slower in the latter than the steps say (8192 x 64 x 2048: 232
+// us, 187; 1536 x 384 x 2048, as many tiles: 177, 187).
+int small_split64(const hdbf_context* ctx, int M, int N, int K, bool tri)
+{
+    const int S = gemm_small_split(ctx, M, N, K);
+    if (S == 0 || (N <= 192 && tile_count(M, N, 64, false) <= ctx->sm_count)) return S;
+    const long long kc = ((K + S - 1) / S + 7) / 8 * 8;
+    const double small = 1.17 * (double)small_waves(ctx, M, N, tri, S) * kc;
+    const double other = (double)small_waves(ctx, M, N, tri, 1) * K + 80.0;
+    return small < other ? S : 0;
+}
+
 hdbf_status dgemm(hdbf_context* ctx, int mode, bool lower_only, int M, int N, int K,
                   const double* A, long long lda, const double* B, long long ldb, double* C,
                   long long ldc)
@@ -262,7 +279,7 @@ hdbf_status dgemm(hdbf_context* ctx, int mode, bool lower_only, int M, int N, in
                    N, K);
     cudaStream_t s = ctx->stream;
     if (mode != 2) {
-        const int S = gemm_small_split(ctx, M, N, K);
+        const int S = small_split64(ctx, M, N, K, lower_only);
         if (S > 0) return gemm_small(ctx, mode == 1, lower_only, S, M, N, K, A, lda, B, ldb, C, ldc);
     }
     // 128x128 tiles only when they still give two waves of CTAs (one per SM)
@@ -276,8 +293,13 @@ hdbf_status dgemm(hdbf_context* ctx, int mode, bool lower_only, int M, int N, in
         } else {
             dgemm_launch<2, false>(s, M, N, K, A, lda, B, ldb, C, ldc);
         }
+    } else if (mode == 0) {
+        if (lower_only) dgemm_launch64<0, true>(s, M, N, K, A, lda, B, ldb, C, ldc);
+        else dgemm_launch64<0, false>(s, M, N, K, A, lda, B, ldb, C, ldc);
+    } else if (mode == 1) {
+        dgemm_launch64<1, false>(s, M, N, K, A, lda, B, ldb, C, ldc);
     } else {
-        dgemm_launch64<2, false>(s, M, N, K, A, lda, B, ldb, C, ldc);  // NT, NN: gemm_small
+        dgemm_launch64<2, false>(s, M, N, K, A, lda, B, ldb, C, ldc);
     }
     ctx->launches++;
     return last_cuda(ctx);

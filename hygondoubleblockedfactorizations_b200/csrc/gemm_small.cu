@@ -346,8 +346,8 @@ void configure_gemm_small(hdbf_context*)
     cudaGetLastError();
 }
 
-// CTAs that share a tile's K (1, 2, 4 or 8), or 0 where the 128 x 128 kernel is
-// taken: from two CTAs per SM on (one wave of that kernel) its larger tiles win.
+// CTAs that share a tile's K (1, 2, 4 or 8), or 0 above two 128 x 128 tiles per SM,
+// where the larger tiles win for certain; below, the callers compare the two kernels.
 int gemm_small_split(const hdbf_context* ctx, int M, int N, int K)
 {
     if (!ctx->dev_small) return 0;  // no handle behind this context: kernel not configured

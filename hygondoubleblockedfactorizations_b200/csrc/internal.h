@@ -309,8 +309,25 @@ hdbf_status sgemm_sub(hdbf_context* ctx, bool nn, bool lower_only, int M, int N,
 // the number of chunks (1 = no split) and, in *kc, their length.
 int split_count(const hdbf_context* ctx, int M, int N, int K, bool tri, int* kc);
 // Updates below one wave of 128 x 128 tiles (gemm_small.cu): the CTAs that share
-// a tile's K (0: not taken), and the launch (range: only if split_range_bad).
+// a tile's K (0: not taken), the same where an FP32 update takes this kernel
+// (sgemm.cu), and the launch (range: only if split_range_bad).
 int gemm_small_split(const hdbf_context* ctx, int M, int N, int K);
+int sgemm_small(const hdbf_context* ctx, int M, int N, int K, bool tri);
+// Tiles of b x b of an M x N update (tri: on or below the diagonal), and CTAs of
+// one SM, the fullest, when `per` CTAs share each.
+inline long long tile_count(int M, int N, int b, bool tri)
+{
+    const long long tm = (M + b - 1) / b, tn = (N + b - 1) / b;
+    if (!tri) return tm * tn;
+    const long long d = tm < tn ? tm : tn;
+    return d * tm - d * (d - 1) / 2;
+}
+inline long long small_waves(const hdbf_context* ctx, int M, int N, bool tri, int per)
+{
+    const long long sm = ctx->sm_count, all = (tile_count(M, N, 64, false) * per + sm - 1) / sm;
+    const long long own = (tile_count(M, N, 64, tri) * per + sm - 1) / sm;
+    return tri && own < all ? own + 1 : own;  // tiles above the diagonal leave holes
+}
 hdbf_status gemm_small(hdbf_context* ctx, bool nn, bool lower, int S, int M, int N, int K,
                        const float* A, long long lda, const float* B, long long ldb, float* C,
                        long long ldc, const unsigned* range = nullptr);
@@ -337,9 +354,9 @@ struct SplitPlan {
     {
         int kc = 0;
         c->tc_plan = tc_sgemm_chunk(c, M, N, K, false);
+        c->small_plan = sgemm_small(c, M, N, K, false);
         const int S = split_count(c, M, N, K, false, &kc);
         c->split_kc = S > 1 ? kc : 0;
-        c->small_plan = gemm_small_split(c, M, N, K);
     }
     ~SplitPlan()
     {

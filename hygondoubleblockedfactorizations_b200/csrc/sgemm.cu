@@ -361,6 +361,32 @@ int split_count(const hdbf_context* ctx, int M, int N, int K, bool tri, int* kc)
     return (K + *kc - 1) / *kc;
 }
 
+// The small-update kernel's split (gemm_small.cu) where that kernel is the faster one,
+// else 0.  Both costs are counted in steps of K of one 128 x 128 tile (0.095 us) on
+// the fullest SM: a 64 x 64 tile is 0.3 of one, its ring fills in 10 steps; partial
+// sums cost the 128 x 128 kernel a second launch and their traffic, a ragged last
+// tile column its share of a tile, a triangle 150 steps.  Measured over 595 shapes up
+// to 8192 x 2048 x 2048 the choice is 0.1 % behind the better kernel, 12 % at worst
+// (4096 x 192 x 2048); the small kernel for all of them was up to 1.8 times slower
+// (triangle of 1000, K = 2048: 144 us, 79; 2048 x 512 x 2048: 142, 124; 3072 x 1536 x
+// 256: 76, 60), the large one up to 3.3 times (512 x 192 x 256: 41, 13).
+int sgemm_small(const hdbf_context* ctx, int M, int N, int K, bool tri)
+{
+    const int S = gemm_small_split(ctx, M, N, K);
+    if (S == 0) return 0;
+    const double small =
+        0.3 * (double)small_waves(ctx, M, N, tri, S) * (((K + S - 1) / S + 7) / 8 * 8 + 10);
+    int kc = K;
+    const int parts = split_count(ctx, M, N, K, tri, &kc);
+    if (parts < 2) kc = K;
+    const long long sm = ctx->sm_count;
+    double large = (double)((tile_count(M, N, BM, tri) * parts + sm - 1) / sm) * kc *
+                   ((N + BN - 1) / BN * BN) / N;
+    if (parts > 1) large += 30.0 + 1e-5 * (parts + 1) * (double)M * N;
+    if (tri) large += 150.0;
+    return small <= large ? S : 0;
+}
+
 namespace {
 
 hdbf_status sgemm_launch(hdbf_context* ctx, int mode, bool lower_only, int M, int N, int K,
@@ -405,7 +431,8 @@ hdbf_status sgemm_launch(hdbf_context* ctx, int mode, bool lower_only, int M, in
     ProfScope prof(ctx, kClsGemm, flops, 4.0 * ((double)M * K + (double)N * K + 2.0 * M * N), M,
                    N, K);
     if (!ri && mode != kTN) {
-        const int small = ctx->small_plan >= 0 ? ctx->small_plan : gemm_small_split(ctx, M, N, K);
+        const int small =
+            ctx->small_plan >= 0 ? ctx->small_plan : sgemm_small(ctx, M, N, K, lower_only);
         if (small > 0)
             return gemm_small(ctx, mode == kNN, lower_only, small, M, N, K, A, lda, B, ldb, C, ldc,
                               range);
