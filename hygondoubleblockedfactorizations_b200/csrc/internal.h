@@ -458,9 +458,9 @@ int configure_cluster_panel(hdbf_context* ctx);
 // (gperm when m ints do not fit in shared memory).
 hdbf_status compose_swaps(hdbf_context* ctx, const int* ipiv, int k, int ipiv_minus, int m,
                           int* src, int* tgt, int* count, int* gperm, int* info);
-// The same swaps, composed and applied in one launch (k <= 512; NOT_SUPPORTED
-// above), to columns [c0, c0 + n0) and [c1, c1 + n1) of A, whose row 0 is the swaps'
-// row 0.  A pivot outside [its row, m) moves nothing, sets info = -1 and the
+// The same swaps, composed and applied in one launch (NOT_SUPPORTED above 512
+// swaps and where the two launches are faster), to columns [c0, c0 + n0) and
+// [c1, c1 + n1) of A, whose row 0 is the swaps' row 0.  A pivot outside [its row, m) moves nothing, sets info = -1 and the
 // device error.
 hdbf_status swap_rows(hdbf_context* ctx, float* A, long long lda, const int* ipiv, int k, int minus,
                       int m, int c0, int n0, int c1, int n1, int* info);

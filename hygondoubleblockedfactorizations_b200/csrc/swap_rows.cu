@@ -95,8 +95,17 @@ hdbf_status swap_rows_t(hdbf_context* ctx, T* A, long long lda, const int* ipiv,
     n1 = std::max(n1, 0);
     const int n = n0 + n1;
     if (n == 0) return HDBF_STATUS_SUCCESS;
-    // Four CTAs per SM at most: the composition is paid once per CTA.
-    const int passes = std::max(1, (n + kCols * 4 * ctx->sm_count - 1) / (kCols * 4 * ctx->sm_count));
+    // The composition is paid once per CTA, 10 us at 256 swaps and 20 at 512 (four
+    // positions a thread): up to four CTAs per SM, two above 128 swaps, one above 256,
+    // but four again where the moves take longer than that.  384 swaps on 4096 columns:
+    // 63 us with four, 34 with one, 45 composed once and gathered (compose_swaps,
+    // apply_moves); on 8192 columns 95, 99 and 152.
+    const int one = kCols * ctx->sm_count;
+    const int per_sm = k <= 128 || (k > 256 && n > 5 * one) ? 4 : (k <= 256 ? 2 : 1);
+    const int passes = std::max(1, (n + per_sm * one - 1) / (per_sm * one));
+    // FP32 gathers of a few thousand columns: 512 swaps on 3000 columns 36 us here, 32
+    // composed once; on 1500 and on 6000 columns 28 and 66 here, 28 and 73.
+    if (sizeof(T) == 4 && k > 448 && n > one && n <= 4 * one) return HDBF_STATUS_NOT_SUPPORTED;
     const int per = kCols * passes;
     const unsigned grid = (unsigned)((n + per - 1) / per);
     int* err = ctx->dev_small + kSmallErr;
