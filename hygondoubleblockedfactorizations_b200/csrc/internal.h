@@ -183,18 +183,19 @@ __device__ __forceinline__ float pow2f_exact(int k)
     return __uint_as_float((unsigned)(127 + k) << 23);
 }
 
-// Whether an operand pair is outside the range of the three-word BF16 split:
-// range[0], range[1] hold the bits of max |x| of A and of B (0: all zero, or B
-// is part of A).
+// Whether an operand pair is outside the range of the three-word BF16 split
+// (tc_sgemm.cu): range[0], range[1] hold the bits of max |x| of A and of B (0: all
+// zero, or B is part of A).  With exponents a and b the sum of K products, times 2^32, is
+// below 2^(a + b + 2 + 32) K: no overflow for a + b <= 72 and K <= 2^20.  An operand
+// wholly below 2^-90 keeps the FP32 kernel too.
 __device__ __forceinline__ bool split_range_bad(const unsigned* range)
 {
-    bool bad = false;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const unsigned m = __ldcg(range + i);
-        bad = bad || m > (253u << 23) || (m != 0u && m < (37u << 23));  // 2^126, 2^-90
-    }
-    return bad;
+    unsigned ma = __ldcg(range), mb = __ldcg(range + 1);
+    if (mb == 0u) mb = ma;
+    if (ma == 0u) ma = mb;
+    const unsigned a = ma >> 23, b = mb >> 23;  // biased exponents
+    const bool tiny = ma != 0u && (a < 127u - 90u || b < 127u - 90u);
+    return tiny || a > 127u + 110u || b > 127u + 110u || a + b > 2u * 127u + 72u;
 }
 
 // The handle's poll limit, read at kernel start from the small device block

@@ -24,11 +24,14 @@
 // TMEM accumulators alternate per 64 of K; draining one takes a quarter of the
 // time the other takes to fill.
 //
-// Range: the split is exact for |x| >= 2^-110 and finite; below that a value
-// loses bits under 2^-134, which only matters when all of an operand is that
-// small.  The conversion records max |x| of each operand; if it is not finite,
-// above 2^126 or below 2^-90, these kernels leave C alone and the FP32 kernel,
-// launched behind them, does the update (it returns at once otherwise).
+// Range: an FP32 value is a multiple of 2^-149, a BF16 word of 2^-133, so values are
+// split times 2^16 and the sums taken off C times 2^-32: the split is then exact for
+// every value below 2^111, subnormal ones included, row by row and entry by entry, and
+// no result that FP32 can hold comes from a sum below the normal range.  The conversion
+// records max |x| of each operand; where one is not finite, above 2^110 or below
+// 2^-90, or their product so large that a scaled sum might overflow (2^74), these
+// kernels leave C alone and the FP32 kernel, launched behind them, does the update (it
+// returns at once otherwise).
 #include "tc_common.cuh"
 
 #include <cuda_bf16.h>
@@ -46,6 +49,7 @@ constexpr int kTmemCols = 2 * kTN;
 constexpr int kEpiWarps = 8;
 constexpr int kThr = 64 + 32 * kEpiWarps;
 constexpr size_t kSmemBytes = (size_t)kSlots * kSlot + 1024;
+constexpr float kSplitScale = 65536.f, kUnscale = 1.f / (65536.f * 65536.f);
 
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int x,
                                             int y, int z)
@@ -286,7 +290,8 @@ tc_sgemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
                     for (int j = 0; j < 16; ++j) {
                         const int col = n0 + q * 16 + j;
                         if (col < args.N && (!args.lower || row >= col))
-                            args.C[(long long)col * args.ldc + row] = cv[j] - acc[q * 16 + j];
+                            args.C[(long long)col * args.ldc + row] =
+                                fmaf(acc[q * 16 + j], -kUnscale, cv[j]);
                     }
                 }
             }
@@ -306,6 +311,7 @@ struct Words {
 __device__ __forceinline__ Words split3(float x)
 {
     Words o;
+    x *= kSplitScale;
     const __nv_bfloat16 h0 = __float2bfloat16_rn(x);
     const float r1 = x - __bfloat162float(h0);
     const __nv_bfloat16 h1 = __float2bfloat16_rn(r1);
