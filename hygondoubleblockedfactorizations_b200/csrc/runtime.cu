@@ -1,5 +1,5 @@
-#include <algorithm>
 // Handle, stream pool, workspace arena and status plumbing (host C++).
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -21,6 +21,8 @@ static int fitting_order(size_t bytes);
 void* workspace(hdbf_context* ctx, size_t bytes, hdbf_status* st)
 {
     *st = HDBF_STATUS_SUCCESS;
+    // never less than the smallest layout: its regions are used once there is an arena
+    bytes = std::max(bytes, ws_layout(64).total);
     if (bytes <= ctx->ws_bytes && ctx->ws) return ctx->ws;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(ctx->stream, &cs) == cudaSuccess &&

@@ -52,3 +52,32 @@ def test_routes_agree(hd, plain, torch_cuda, dtype, reserve, M, N, K):
     if lower:
         want = np.tril(want) + np.triu(C, 1)
     np.testing.assert_array_equal(host2d(dC, M, M, N), want.astype(dtype))
+
+
+@pytest.mark.parametrize("nbytes", [1, 1 << 20])
+def test_small_reservation(hd, plain, torch_cuda, nbytes):
+    """A reservation below the smallest arena still gives the split-K scratch its room."""
+    M, N, K = 777, 640, 2100
+    plain.reserve(nbytes)
+    rng = np.random.default_rng(1)
+    A, B, C = (rng.integers(-8, 9, s).astype(np.float32) for s in ((M, K), (N, K), (M, N)))
+    free = torch_cuda.cuda.mem_get_info()[0]
+    dA, dB, dC = dev(torch_cuda, A), dev(torch_cuda, B), dev(torch_cuda, C)
+    hd.call("gemm_nt_update", plain.ptr, M, N, K, ptr(dA), M, ptr(dB), N, ptr(dC), M)
+    torch_cuda.cuda.synchronize()
+    plain.check()
+    np.testing.assert_array_equal(host2d(dC, M, M, N), C - A @ B.T)
+    # the arena was whole when the reservation returned: nothing grew afterwards
+    assert free - torch_cuda.cuda.mem_get_info()[0] < 64 << 20
+    assert plain_arena(hd, torch_cuda, nbytes) >= 256 << 20
+
+
+def plain_arena(hd, torch, nbytes):
+    """Device memory that a new handle takes for a reservation."""
+    h = hd.Handle(torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    h.reserve(nbytes)
+    after = torch.cuda.mem_get_info()[0]
+    h.close()
+    return before - after
