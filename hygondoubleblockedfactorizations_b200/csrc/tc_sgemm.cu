@@ -448,6 +448,16 @@ void configure_tc_sgemm(hdbf_context*)
     cudaGetLastError();
 }
 
+// Longest K chunk of an update of this shape: its operands' words are at most those of
+// an update of order max(M, N) + K, the order of the factorization it belongs to
+// (words_bytes, runtime.cu), so the chunk follows from the shape alone.
+static long long shape_chunk(int M, int N, int K)
+{
+    const long long order = (long long)std::max(M, N) + K;
+    return std::max<long long>(
+        64, 2 * order * std::min<long long>(order, 2048) / ((long long)M + N) / 64 * 64);
+}
+
 // K chunk of the split path for an update of this shape: 0 = not taken.  The
 // line is where both take the same time: 2 M N K = 2e9 at tile-sized N, where
 // the conversions, three more launches and a partly filled wave cost what the
@@ -466,9 +476,9 @@ int tc_sgemm_chunk(const hdbf_context* ctx, int M, int N, int K, bool tri)
         return 0;
     int kc_fp32 = 0;
     if (split_count(ctx, M, N, K, tri, &kc_fp32) > 4 || gemm_small_split(ctx, M, N, K) > 4) return 0;
-    const long long room = (long long)ws_words_half(ctx) / (6LL * ((long long)M + N));
-    const long long kc = std::min<long long>((K + 63) / 64 * 64, room / 64 * 64);
-    return kc >= std::min(K, 512) ? (int)kc : 0;
+    const long long kc = std::min<long long>((K + 63) / 64 * 64, shape_chunk(M, N, K));
+    const long long need = 6 * ((long long)M + N) * kc;
+    return need <= (long long)ws_words_half(ctx) ? (int)kc : 0;
 }
 
 hdbf_status tc_sgemm_chunk_run(hdbf_context* ctx, bool a_kc, bool b_kc, bool lower, int M, int N,

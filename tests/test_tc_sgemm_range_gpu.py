@@ -136,3 +136,47 @@ def test_long_k(hd, torch_cuda, handles, M, N, K, lower, low):
     assert (np.abs(got - want) <= bound)[where].all()
     rms = lambda x: float(np.sqrt(np.mean((x - want)[where] ** 2)))
     assert rms(got) <= 1.05 * rms(plain)
+
+
+@pytest.mark.parametrize("M,N,K,lower", [(6000, 6000, 6000, True), (5000, 4000, 6200, False)])
+def test_same_bits_whatever_the_arena(hd, torch_cuda, M, N, K, lower):
+    """How K is cut follows from the shape, not from how far earlier calls grew the
+    handle's arena."""
+    A = uniform((M, K), 7)
+    B = A if lower else uniform((N, K), 8)
+    C = uniform((M, N), 9)
+    out = []
+    h = hd.Handle(torch_cuda.cuda.current_stream().cuda_stream)
+    for order in (max(M, N) + K, 20000):
+        h.reserve(hd.lib().hdbf_workspace_bytes_for(order))
+        out.append(product(torch_cuda, hd, h, A, B, C, lower))
+    h.close()
+    np.testing.assert_array_equal(out[1], out[0])
+
+
+def test_same_factor_whatever_the_handle_did_before(hd, torch_cuda):
+    """An LU whose outer update of K = 6144 is cut in two, before and after the same
+    handle had a larger problem."""
+    n = 12288
+    g = torch_cuda.Generator(device="cuda")
+    g.manual_seed(1)
+    A0 = torch_cuda.rand(n, n, generator=g, device="cuda") * 2 - 1
+    A0[torch_cuda.arange(n), torch_cuda.randperm(n, generator=g, device="cuda")] += 200.0
+    h = hd.Handle(torch_cuda.cuda.current_stream().cuda_stream)
+
+    def factor():
+        A = A0.clone()
+        ipiv = torch_cuda.zeros(n, dtype=torch_cuda.int32, device="cuda")
+        info = torch_cuda.zeros(1, dtype=torch_cuda.int32, device="cuda")
+        hd.call("double_blocked_getrf", h.ptr, ptr(A), n, n, 6144, 512, 0, 0, ptr(ipiv), ptr(info))
+        torch_cuda.cuda.synchronize()
+        h.check()
+        assert info.item() == 0
+        return A, ipiv
+
+    first = factor()
+    h.reserve(hd.lib().hdbf_workspace_bytes_for(32768))
+    again = factor()
+    h.close()
+    assert torch_cuda.equal(first[1], again[1])
+    assert torch_cuda.equal(first[0], again[0])
