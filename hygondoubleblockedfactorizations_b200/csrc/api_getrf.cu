@@ -169,6 +169,7 @@ hdbf_status getrf_db_impl(hdbf_context* ctx, T* A, int lda, int n, int outer_nb,
             la = false;
         }
     }
+    reserve_update_words<T>(ctx, n, la);
     const std::vector<long long> key = {
         10 + (int)mode + type_tag<T>(), (long long)A, lda, n, outer_nb, inner_nb, iterative_outer, trsm_block,
         inner_gemm_m_tile, (long long)ipiv, (long long)info, (long long)ws.src, (long long)ws.tgt,
@@ -295,6 +296,7 @@ hdbf_status getrf_rl_impl(hdbf_context* ctx, T* A, int lda, int n, int nb, int* 
     GetrfWs ws;
     HDBF_TRY(getrf_workspace(ctx, ws_order<T>(n), &ws));
     if (nb <= 0) nb = n;
+    reserve_update_words<T>(ctx, n, false);
     const std::vector<long long> key = {20 + (int)piv + type_tag<T>(), (long long)A, lda, n, nb, (long long)ipiv,
                                         (long long)info};
     return run_graph(ctx, key, [&]() -> hdbf_status {

@@ -129,6 +129,7 @@ hdbf_status potrf_db_impl(hdbf_context* ctx, T* A, int lda, int n, int nb, int b
         return last_cuda(ctx);
     }
     HDBF_TRY(ensure_ws(ctx, ws_order<T>(n)));
+    reserve_update_words<T>(ctx, n, false);
     if (nb <= 0) nb = n;
     if (b <= 0) b = nb;
     b = std::min(b, nb);
@@ -209,6 +210,7 @@ hdbf_status potrf_blocked_rl_impl(hdbf_context* ctx, T* A, int lda, int n, int n
         return last_cuda(ctx);
     }
     HDBF_TRY(ensure_ws(ctx, ws_order<T>(n)));
+    reserve_update_words<T>(ctx, n, false);
     if (nb <= 0) nb = n;
     const std::vector<long long> key = {2 + type_tag<T>(), (long long)A, lda, n, nb, (long long)info};
     return run_graph(ctx, key, [&]() -> hdbf_status {
@@ -307,6 +309,7 @@ hdbf_status rec_potrf_entry(hdbf_context* ctx, T* A, int lda, int n, int nb, int
         return last_cuda(ctx);
     }
     HDBF_TRY(ensure_ws(ctx, ws_order<T>(n)));
+    reserve_update_words<T>(ctx, n, false);
     const std::vector<long long> key = {3 + type_tag<T>(), (long long)A, lda, n, nb, (long long)info, tiled};
     return run_graph(ctx, key, [&]() -> hdbf_status {
         if (info) cudaMemsetAsync(info, 0, sizeof(int), ctx->stream);

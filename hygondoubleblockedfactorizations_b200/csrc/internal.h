@@ -122,6 +122,10 @@ struct hdbf_context {
     int ws_n = 0;  // largest order whose layout fits in ws_bytes
     // Small always-present device block: [0] error word, [1..] barrier words.
     int* dev_small = nullptr;
+    // Operand words of the FP32 updates on the tensor cores, for this handle's stream
+    // and for its look-ahead stream; allocated by the calls that run such updates.
+    void* words[2] = {nullptr, nullptr};
+    size_t words_bytes[2] = {0, 0};
     // Second arena for the mixed-precision path (16-bit shadows, FP64 IR
     // vectors); grown on demand outside stream capture.
     void* mix = nullptr;
@@ -268,10 +272,8 @@ void* mixed_arena(hdbf_context* ctx, size_t bytes, hdbf_status* st);
 //   temp  column-tiled swap buffer, 64*n floats
 //   skinny  split-K partial sums of the skinny GEMM, 256*n floats
 //   wave  wavefront-solve row-major x copy (32 columns) and its flags
-//   words BF16 words of the operands of an FP32 update on the tensor cores, one
-//         half per stream (handle's, look-ahead)
 struct WsLayout {
-    size_t panel, inv, src, tgt, gperm, temp, skinny, wave, split, words, total;
+    size_t panel, inv, src, tgt, gperm, temp, skinny, wave, split, total;
 };
 // Split-K partial sums of under-filled FP32 GEMM launches: two halves of
 // kSplitFloats each, one for the handle's stream and one for its look-ahead
@@ -290,9 +292,24 @@ float* ws_skinny(hdbf_context* ctx);
 // Split-K scratch half for GEMMs enqueued on ctx->stream.
 float* ws_split(hdbf_context* ctx);
 float* ws_wave(hdbf_context* ctx);
-// This stream's half of the words region, and its size in bytes (less the range slots).
-void* ws_words(hdbf_context* ctx);
-size_t ws_words_half(const hdbf_context* ctx);
+// The operand words (256 bytes of range slots first) of updates on ctx->stream: their
+// bytes for a factorization of order n, and their room, grown to `bytes` where no stream
+// capture forbids it.  Without room the FP32 kernels do the update.
+size_t words_bytes(int n);
+bool words_room(hdbf_context* ctx, size_t bytes);
+inline void* ws_words(const hdbf_context* ctx)
+{
+    return ctx->words[ctx->la_stream && ctx->stream == ctx->la_stream ? 1 : 0];
+}
+// Room for the updates of a factorization of order n (FP32 drivers, outside their
+// capture), on the look-ahead stream too, or for one of M x N x K.
+void reserve_words(hdbf_context* ctx, int n, bool lookahead);
+void reserve_words(hdbf_context* ctx, int M, int N, int K);
+template <class T>
+inline void reserve_update_words(hdbf_context* ctx, int n, bool lookahead)
+{
+    if (sizeof(T) == 4) reserve_words(ctx, n, lookahead);
+}
 
 hdbf_status last_cuda(hdbf_context* ctx);
 
@@ -342,6 +359,8 @@ void configure_tile_kernels(hdbf_context* ctx);
 // is contiguous), whose operand range, in *range, tells the FP32 kernel behind it
 // whether it has to do the update (split_range_bad).
 int tc_sgemm_chunk(const hdbf_context* ctx, int M, int N, int K, bool tri);
+// The same, or 0 where there is no room for the operands' words.
+int tc_sgemm_plan(hdbf_context* ctx, int M, int N, int K, bool tri);
 hdbf_status tc_sgemm_chunk_run(hdbf_context* ctx, bool a_kc, bool b_kc, bool lower, int M, int N,
                                int K, const float* A, long long lda, const float* B, long long ldb,
                                float* C, long long ldc, unsigned** range);
@@ -354,7 +373,7 @@ struct SplitPlan {
         : ctx(c), saved(c->split_kc), saved_tc(c->tc_plan), saved_small(c->small_plan)
     {
         int kc = 0;
-        c->tc_plan = tc_sgemm_chunk(c, M, N, K, false);
+        c->tc_plan = tc_sgemm_plan(c, M, N, K, false);
         c->small_plan = sgemm_small(c, M, N, K, false);
         const int S = split_count(c, M, N, K, false, &kc);
         c->split_kc = S > 1 ? kc : 0;

@@ -436,6 +436,7 @@ hdbf_status potrf_mixed(hdbf_context* ctx, int prec, float* A, long long lda, in
     if (b <= 0) b = 512;
     b = std::min(b, n);
     HDBF_TRY(ensure_ws(ctx, n));
+    reserve_words(ctx, n, b, b / 2 + 64);  // a panel's own FP32 updates
     hdbf_status st;
     char* arena = static_cast<char*>(mixed_arena(ctx, mixed_shadow_bytes(n, b, pi.split), &st));
     if (!arena) return st;
@@ -458,6 +459,7 @@ hdbf_status getrf_mixed(hdbf_context* ctx, int prec, float* A, long long lda, in
     if (b <= 0) b = 512;
     b = std::min(b, n);
     HDBF_TRY(ensure_ws(ctx, n));
+    reserve_words(ctx, n, b, b / 2 + 64);  // a panel's own FP32 updates
     hdbf_status st;
     char* arena = static_cast<char*>(mixed_arena(ctx, mixed_shadow_bytes(n, b, pi.split), &st));
     if (!arena) return st;

@@ -82,11 +82,50 @@ void* mixed_arena(hdbf_context* ctx, size_t bytes, hdbf_status* st)
     return ctx->mix;
 }
 
-// Operand words of an update of order n: M + N <= 2 n rows, up to 2048 of K at a
-// time, 6 bytes an element, plus the range slots.
-static size_t words_half(int n)
+// M + N <= 2 n rows, up to 2048 of K at a time, 6 bytes an element, and the range slots.
+size_t words_bytes(int n)
 {
+    if (n < 64) n = 64;
     return align_up((size_t)12 * n * (n < 2048 ? n : 2048), 256) + 256;
+}
+
+static bool grow_words(hdbf_context* ctx, int slot, size_t bytes)
+{
+    if (bytes <= ctx->words_bytes[slot]) return true;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (ctx->capturing || cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess ||
+        cs != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return false;
+    }
+    if (ctx->words[slot]) {
+        graph_cache_clear(ctx);  // cached graphs point into the old words
+        cudaStreamSynchronize(ctx->stream);
+        if (ctx->la_stream) cudaStreamSynchronize(ctx->la_stream);
+        cudaFree(ctx->words[slot]);
+        ctx->words[slot] = nullptr;
+        ctx->words_bytes[slot] = 0;
+    }
+    if (cudaMalloc(&ctx->words[slot], bytes) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->words[slot] = nullptr;
+        return false;
+    }
+    ctx->words_bytes[slot] = bytes;
+    return true;
+}
+
+bool words_room(hdbf_context* ctx, size_t bytes)
+{
+    return grow_words(ctx, ctx->la_stream && ctx->stream == ctx->la_stream ? 1 : 0, bytes);
+}
+
+void reserve_words(hdbf_context* ctx, int n, bool lookahead)
+{
+    // no update of a smaller order reaches the tensor cores: M N K <= 4/27 n^3
+    if (ctx->tc_sgemm == 0 || (ctx->tc_sgemm == 1 && n < 1890)) return;
+    grow_words(ctx, 0, words_bytes(n));
+    if (lookahead) grow_words(ctx, 1, words_bytes(n));
 }
 
 WsLayout ws_layout(int n)
@@ -112,8 +151,6 @@ WsLayout ws_layout(int n)
     off += wave_scratch_bytes(n);
     L.split = off;
     off += align_up(2 * kSplitFloats * sizeof(float), 256);
-    L.words = off;
-    off += 2 * words_half(n);
     L.total = off;
     return L;
 }
@@ -201,13 +238,6 @@ float* ws_split(hdbf_context* ctx)
         reinterpret_cast<float*>(static_cast<char*>(ctx->ws) + ws_layout(ctx->ws_n).split);
     return (ctx->la_stream && ctx->stream == ctx->la_stream) ? base + kSplitFloats : base;
 }
-
-void* ws_words(hdbf_context* ctx)
-{
-    char* base = static_cast<char*>(ctx->ws) + ws_layout(ctx->ws_n).words;
-    return (ctx->la_stream && ctx->stream == ctx->la_stream) ? base + words_half(ctx->ws_n) : base;
-}
-size_t ws_words_half(const hdbf_context* ctx) { return words_half(ctx->ws_n) - 256; }
 
 ProfScope::ProfScope(hdbf_context* ctx, int cls, double flops, double bytes, int m, int n,
                      int k)
@@ -435,6 +465,8 @@ hdbf_status hdbf_destroy(hdbf_handle h)
         cudaStreamDestroy(h->la_stream);
     }
     if (h->ws) cudaFree(h->ws);
+    for (void* w : h->words)
+        if (w) cudaFree(w);
     if (h->dev_small) cudaFree(h->dev_small);
     if (h->mix) cudaFree(h->mix);
     delete h;
@@ -477,14 +509,25 @@ const char* hdbf_status_string(hdbf_status s)
     return "unknown status";
 }
 
-size_t hdbf_workspace_bytes_for(int n) { return ws_layout(n < 1 ? 1 : n).total; }
+static size_t order_bytes(int n) { return ws_layout(n).total + 2 * words_bytes(n); }
+
+size_t hdbf_workspace_bytes_for(int n) { return order_bytes(n < 1 ? 1 : n); }
 
 hdbf_status hdbf_reserve_workspace(hdbf_handle h, size_t bytes)
 {
     if (!h) return HDBF_STATUS_INVALID_HANDLE;
-    hdbf_status st;
-    workspace(h, bytes, &st);
-    return st;
+    int n = 64, top = 1 << 24;  // largest order whose arena and operand words are that much
+    while (n < top) {
+        const int mid = n + (top - n + 1) / 2;
+        if (order_bytes(mid) <= bytes) n = mid; else top = mid - 1;
+    }
+    HDBF_TRY(ensure_ws(h, n));
+    if (grow_words(h, 0, words_bytes(n)) && grow_words(h, 1, words_bytes(n)))
+        return HDBF_STATUS_SUCCESS;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    cudaStreamIsCapturing(h->stream, &cs);
+    return cs != cudaStreamCaptureStatusNone ? HDBF_STATUS_WORKSPACE_TOO_SMALL
+                                             : HDBF_STATUS_ALLOC_FAILED;
 }
 
 hdbf_status hdbf_check_device_errors(hdbf_handle h)

@@ -401,7 +401,7 @@ hdbf_status sgemm_launch(hdbf_context* ctx, int mode, bool lower_only, int M, in
                             C, ldc);
     const int tc = range              ? 0
                    : ctx->tc_plan >= 0 ? ctx->tc_plan
-                                       : tc_sgemm_chunk(ctx, M, N, K, lower_only);
+                                       : tc_sgemm_plan(ctx, M, N, K, lower_only);
     if (tc > 0) {
         const bool a_kc = mode == kTN, b_kc = mode != kNT;  // K contiguous in memory
         for (int k0 = 0; k0 < K; k0 += tc) {

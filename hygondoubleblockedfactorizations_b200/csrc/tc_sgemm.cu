@@ -476,9 +476,20 @@ int tc_sgemm_chunk(const hdbf_context* ctx, int M, int N, int K, bool tri)
         return 0;
     int kc_fp32 = 0;
     if (split_count(ctx, M, N, K, tri, &kc_fp32) > 4 || gemm_small_split(ctx, M, N, K) > 4) return 0;
+    return (int)std::min<long long>((K + 63) / 64 * 64, shape_chunk(M, N, K));
+}
+
+int tc_sgemm_plan(hdbf_context* ctx, int M, int N, int K, bool tri)
+{
+    const int kc = tc_sgemm_chunk(ctx, M, N, K, tri);
+    return kc > 0 && words_room(ctx, 256 + 6 * ((size_t)M + N) * kc) ? kc : 0;
+}
+
+void reserve_words(hdbf_context* ctx, int M, int N, int K)
+{
+    if (ctx->tc_sgemm == 0 || (ctx->tc_sgemm == 1 && (double)M * N * K < 1.0e9)) return;
     const long long kc = std::min<long long>((K + 63) / 64 * 64, shape_chunk(M, N, K));
-    const long long need = 6 * ((long long)M + N) * kc;
-    return need <= (long long)ws_words_half(ctx) ? (int)kc : 0;
+    words_room(ctx, 256 + 6 * ((size_t)M + N) * kc);
 }
 
 hdbf_status tc_sgemm_chunk_run(hdbf_context* ctx, bool a_kc, bool b_kc, bool lower, int M, int N,

@@ -55,7 +55,11 @@ const char* hdbf_status_string(hdbf_status status);
 /* Grow the handle's device workspace to at least `bytes` now, so that later
  * calls made under CUDA stream capture do not need to allocate. */
 hdbf_status hdbf_reserve_workspace(hdbf_handle handle, size_t bytes);
-/* Workspace the factorization routines need for order n (bytes). */
+/* Workspace an FP32 factorization of order n needs (bytes): the arena, and the
+ * operand words of its tensor-core updates.  Calls grow either on demand outside
+ * stream capture; FP64 and mixed-precision calls never take the operand words of
+ * their order (most of this at large n).  Where those have no room, in a caller's
+ * capture or on a full device, the FP32 kernels do the updates. */
 size_t hdbf_workspace_bytes_for(int n);
 
 /* Synchronise the handle's stream, then read and clear the device-side error

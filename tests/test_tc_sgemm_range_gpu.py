@@ -147,7 +147,7 @@ def test_same_bits_whatever_the_arena(hd, torch_cuda, M, N, K, lower):
     C = uniform((M, N), 9)
     out = []
     h = hd.Handle(torch_cuda.cuda.current_stream().cuda_stream)
-    for order in (max(M, N) + K, 20000):
+    for order in (64, max(M, N) + K, 20000):
         h.reserve(hd.lib().hdbf_workspace_bytes_for(order))
         out.append(product(torch_cuda, hd, h, A, B, C, lower))
     h.close()
