@@ -640,6 +640,7 @@ hdbf_status run_graph(hdbf_context* ctx, std::vector<long long> key, Body&& body
 {
     if (!graph_can_capture(ctx)) return body();
     key.push_back(ctx->profiling ? 1 : 0);
+    key.push_back(ctx->tc_sgemm);
     if (GraphEntry* e = graph_find(ctx, key)) return graph_launch(ctx, e);
     cudaStream_t saved = nullptr;
     const size_t mark = ctx->prof.size();

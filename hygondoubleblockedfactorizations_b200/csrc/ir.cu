@@ -394,6 +394,14 @@ IrBlocks ir_blocks(bool spd, int prec, int n)
     return IrBlocks{nb, nb};
 }
 
+// HDBF_PREC_FP32 names the arithmetic: FP32 operands on the SIMT kernels.
+struct NoTensorUpdates {
+    hdbf_context* ctx;
+    int saved;
+    explicit NoTensorUpdates(hdbf_context* c) : ctx(c), saved(c->tc_sgemm) { ctx->tc_sgemm = 0; }
+    ~NoTensorUpdates() { ctx->tc_sgemm = saved; }
+};
+
 class IrSolver {
 public:
     IrSolver(hdbf_context* ctx, bool spd, const double* A, long long lda, int n, int nrhs,
@@ -410,6 +418,7 @@ public:
         HDBF_TRY(last_cuda(ctx_));
         const IrBlocks blk = ir_blocks(spd_, prec, n_);
         if (prec == HDBF_PREC_FP32) {
+            NoTensorUpdates simt(ctx_);
             if (spd_)
                 double_blocked_potrf_kblocked_syrk(ctx_, b_.W, n_, n_, blk.outer, blk.inner, 0,
                                                    b_.info);

@@ -19,7 +19,7 @@ extern "C" {
 #endif
 
 typedef enum hdbf_precision {
-    HDBF_PREC_FP32 = 0,   /* FP32 updates */
+    HDBF_PREC_FP32 = 0,   /* FP32 SIMT updates (no tensor cores) */
     HDBF_PREC_BF16 = 1,   /* one BF16 product per update */
     HDBF_PREC_FP16 = 2,   /* one FP16 product per update (power-of-two operand scaling) */
     HDBF_PREC_BF16X3 = 3, /* operands split hi+lo in BF16: hi*hi + hi*lo + lo*hi */

@@ -180,3 +180,29 @@ def test_same_factor_whatever_the_handle_did_before(hd, torch_cuda):
     h.close()
     assert torch_cuda.equal(first[1], again[1])
     assert torch_cuda.equal(first[0], again[0])
+
+
+@pytest.mark.parametrize("kind", ["posv", "gesv"])
+def test_prec_fp32_is_simt(hd, torch_cuda, kind):
+    """HDBF_PREC_FP32 is documented as FP32 SIMT updates, whatever the handle's own FP32
+    factorizations use (the same orders on it do run on the tensor cores)."""
+    import ctypes
+
+    torch, n = torch_cuda, 4096
+    h = hd.Handle(torch.cuda.current_stream().cuda_stream)
+    A = torch.full((n, n), 0.5 / n, dtype=torch.float64, device="cuda")
+    A.diagonal().fill_(1.0)
+    B = torch.ones(1, n, dtype=torch.float64, device="cuda")
+    X, out = torch.zeros_like(B), hd.IrInfo()
+    h.profile_begin()
+    st = hd.call("hdbf_d%s_mixed_auto" % kind, h.ptr, hd.PREC["fp32"], A.data_ptr(), n, n, 1,
+                 B.data_ptr(), n, X.data_ptr(), n, 1e-13, 30, ctypes.byref(out))
+    ran = h.profile_end()
+    assert st == 0 and out.converged and out.final_precision == hd.PREC["fp32"]
+    assert ran["sgemm_sub_kernel"][0] > 0
+    assert ran.get("tc_gemm_kernels", (0,))[0] == 0
+    A32, info = A.float(), torch.zeros(1, dtype=torch.int32, device="cuda")
+    h.profile_begin()
+    hd.call("double_blocked_potrf", h.ptr, ptr(A32), n, n, 2048, 256, ptr(info))
+    assert h.profile_end()["tc_gemm_kernels"][0] > 0
+    h.close()
