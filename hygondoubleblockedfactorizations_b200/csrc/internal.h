@@ -357,7 +357,8 @@ void configure_tile_kernels(hdbf_context* ctx);
 // FP32 update on the tensor cores (tc_sgemm.cu): the K chunk for this shape, 0
 // where the FP32 kernel is taken; one chunk of it (a_kc / b_kc: the operand's K
 // is contiguous), whose operand range, in *range, tells the FP32 kernel behind it
-// whether it has to do the update (split_range_bad).
+// whether it has to do the update (split_range_bad).  NOT_SUPPORTED, with nothing
+// launched, where the operands' tensor maps cannot be encoded.
 int tc_sgemm_chunk(const hdbf_context* ctx, int M, int N, int K, bool tri);
 // The same, or 0 where there is no room for the operands' words.
 int tc_sgemm_plan(hdbf_context* ctx, int M, int N, int K, bool tri);

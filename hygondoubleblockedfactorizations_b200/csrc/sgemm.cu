@@ -409,9 +409,16 @@ hdbf_status sgemm_launch(hdbf_context* ctx, int mode, bool lower_only, int M, in
             const float* Ak = a_kc ? A + k0 : A + (long long)k0 * lda;
             const float* Bk = b_kc ? B + k0 : B + (long long)k0 * ldb;
             unsigned* r = nullptr;
-            HDBF_TRY(tc_sgemm_chunk_run(ctx, a_kc, b_kc, lower_only, M, N, kk, Ak, lda, Bk, ldb, C,
-                                        ldc, &r));
-            HDBF_TRY(sgemm_launch(ctx, mode, lower_only, M, N, kk, Ak, lda, Bk, ldb, C, ldc, r));
+            const hdbf_status st = tc_sgemm_chunk_run(ctx, a_kc, b_kc, lower_only, M, N, kk, Ak, lda,
+                                                      Bk, ldb, C, ldc, &r);
+            if (st != HDBF_STATUS_SUCCESS && st != HDBF_STATUS_NOT_SUPPORTED) return st;
+            // the kernel behind, or, where no tensor map could be had, the update itself
+            const int plan = ctx->tc_plan;
+            ctx->tc_plan = 0;
+            const hdbf_status behind =
+                sgemm_launch(ctx, mode, lower_only, M, N, kk, Ak, lda, Bk, ldb, C, ldc, r);
+            ctx->tc_plan = plan;
+            HDBF_TRY(behind);
         }
         return HDBF_STATUS_SUCCESS;
     }

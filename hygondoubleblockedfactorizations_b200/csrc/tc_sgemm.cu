@@ -500,18 +500,18 @@ hdbf_status tc_sgemm_chunk_run(hdbf_context* ctx, bool a_kc, bool b_kc, bool low
     unsigned* slots = reinterpret_cast<unsigned*>(base);
     unsigned short* wa = reinterpret_cast<unsigned short*>(base + 256);
     const int ldk = (K + 7) / 8 * 8;
-    *range = slots;
-    if (cudaMemsetAsync(slots, 0, 2 * sizeof(unsigned), ctx->stream) != cudaSuccess)
-        return last_cuda(ctx);
-    HDBF_TRY(split_operand(ctx, a_kc, M, K, A, lda, wa, ldk, slots));
     // C -= A A^T: B is the head of A
     const bool same = !a_kc && !b_kc && A == B && lda == ldb && N <= M;
     unsigned short* wb = same ? wa : wa + 3 * (size_t)M * ldk;
     const int b_rows = same ? M : N;
-    if (!same) HDBF_TRY(split_operand(ctx, b_kc, N, K, B, ldb, wb, ldk, slots + 1));
-    CUtensorMap ma, mb;
+    CUtensorMap ma, mb;  // before the first launch: without them nothing has happened
     if (!word_map(&ma, wa, ldk, M, K, kTM) || !word_map(&mb, wb, ldk, b_rows, K, kTN))
         return HDBF_STATUS_NOT_SUPPORTED;
+    *range = slots;
+    if (cudaMemsetAsync(slots, 0, 2 * sizeof(unsigned), ctx->stream) != cudaSuccess)
+        return last_cuda(ctx);
+    HDBF_TRY(split_operand(ctx, a_kc, M, K, A, lda, wa, ldk, slots));
+    if (!same) HDBF_TRY(split_operand(ctx, b_kc, N, K, B, ldb, wb, ldk, slots + 1));
     X6Args a;
     a.M = M;
     a.N = N;
