@@ -33,7 +33,7 @@
 // applies the rank-NB update to its own rows, in column order: the result is
 // bit-identical to column-by-column elimination (getf2_grid.cu).
 // Measured per column, against the grid-wide kernel's 1.9-2.0 us: 1.3 us at m =
-// 1001, 1.5 at 4096, 1.8 at 8192, 2.1 at 16384 (FP32).  The rest is issue and
+// 1001, 1.5 at 4096, 1.8 at 8192, 2.4 at 16384 (FP32).  The rest is issue and
 // fixed latencies: ~300 dependent instructions per warp and column.
 // Waits on an mbarrier are bounded by the handle's poll limit; an expired wait
 // records a timeout and the CTA runs on without waiting or arriving (a second

@@ -9,25 +9,26 @@
 #include "hdbf/hdbf.h"
 
 namespace hdbf {
-// Kernel classes for the per-launch event profiler (hdbf_profile_*).
+// Kernel classes for the per-launch event profiler (hdbf_profile_*).  The names that
+// callers see (hdbf_profile_class_name) stay as they were first given.
 enum KernelClass {
-    kClsGemm = 0,     // sgemm_sub_kernel (GEMM / SYRK trailing updates)
+    kClsGemm = 0,     // sgemm_sub_kernel, gemm_small_kernel and the FP64 GEMMs
     kClsPotf2 = 1,    // potf2_kernel
-    kClsTrsmR = 2,    // rlt_apply_kernel
-    kClsTrsmL = 3,    // llu_apply_kernel
+    kClsTrsmR = 2,    // rlt_block_kernel ("rlt_apply_kernel")
+    kClsTrsmL = 3,    // llu_block_kernel, llu_apply_kernel ("llu_apply_kernel")
     kClsPanel = 4,    // getf2_cluster_kernel / getf2_grid_kernel
-    kClsCompose = 5,  // compose_swaps_kernel
-    kClsMoves = 6,    // apply_moves kernels
+    kClsCompose = 5,  // compose_swaps_kernel, ipiv_to_perm's kernels
+    kClsMoves = 6,    // swap_rows_kernel, apply_moves kernels
     kClsTrsmInv = 7,  // tri_inv64_kernel
-    kClsTcGemm = 8,   // tc_gemm_persistent_kernel / tc_gemm_sub_kernel (tcgen05 updates)
-    kClsConvert = 9,  // FP32 -> 16-bit shadow conversions
+    kClsTcGemm = 8,   // tc_gemm_persistent_kernel / tc_gemm_sub_kernel / tc_sgemm_kernel
+    kClsConvert = 9,  // FP32 -> 16-bit shadow and word conversions
     kClsIr = 10,      // FP64 residual / update / norm kernels
     kClsOther = 11,
     kClsWave = 12,     // trsv_wave_kernel (wavefront triangular solves)
     kClsSkinny = 13,   // skinny_kernel (updates with N <= 32)
     kClsBatched = 14,  // batched_factor_solve_kernel
     kClsSelector = 15, // selector MLP kernels
-    kClsPotrfBlock = 16, // potrf_block_kernel (cooperative diagonal-block Cholesky)
+    kClsPotrfBlock = 16, // potrf_cluster_kernel, tile_inverse_kernel ("potrf_block_kernel")
     kNumClasses = 17
 };
 // Algorithm stages of the double-blocked drivers for the per-stage profile

@@ -98,8 +98,9 @@ static bool grow_words(hdbf_context* ctx, int slot, size_t bytes)
         cudaGetLastError();
         return false;
     }
+    // Cached graphs point into the old words, or do without any.
+    graph_cache_clear(ctx);
     if (ctx->words[slot]) {
-        graph_cache_clear(ctx);  // cached graphs point into the old words
         cudaStreamSynchronize(ctx->stream);
         if (ctx->la_stream) cudaStreamSynchronize(ctx->la_stream);
         cudaFree(ctx->words[slot]);
