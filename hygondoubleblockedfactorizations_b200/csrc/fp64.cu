@@ -250,14 +250,16 @@ void dgemm_launch64(cudaStream_t s, int M, int N, int K, const double* A, long l
 // start, and only the small one splits K.  4096 x 1024 x 1000: 652 us, 544 in 64 x 64 x
 // 16 tiles; 2048 x 64 x 512: 27 us, 54.  Tall updates of up to three tile columns and
 // one tile per SM are slower in the latter than the steps say (8192 x 64 x 2048: 232
-// us, 187; 1536 x 384 x 2048, as many tiles: 177, 187).
-int small_split64(const hdbf_context* ctx, int M, int N, int K, bool tri)
+// us, 187; 1536 x 384 x 2048, as many tiles: 177, 187).  Without 16-byte accesses (!vec)
+// the small kernel takes 1.25 times as long a step, the other 60 steps more a tile
+// (2048 x 2048 x 128 with odd leading dimensions: 109 us, 162).
+int small_split64(const hdbf_context* ctx, int M, int N, int K, bool tri, bool vec)
 {
     const int S = gemm_small_split(ctx, M, N, K);
     if (S == 0 || (N <= 192 && tile_count(M, N, 64, false) <= ctx->sm_count)) return S;
     const long long kc = ((K + S - 1) / S + 7) / 8 * 8;
-    const double small = 1.17 * (double)small_waves(ctx, M, N, tri, S) * kc;
-    const double other = (double)small_waves(ctx, M, N, tri, 1) * K + 80.0;
+    const double small = (vec ? 1.17 : 1.25) * (double)small_waves(ctx, M, N, tri, S) * kc;
+    const double other = (double)small_waves(ctx, M, N, tri, 1) * (vec ? K : K + 60) + 80.0;
     return small < other ? S : 0;
 }
 
@@ -279,7 +281,9 @@ hdbf_status dgemm(hdbf_context* ctx, int mode, bool lower_only, int M, int N, in
                    N, K);
     cudaStream_t s = ctx->stream;
     if (mode != 2) {
-        const int S = small_split64(ctx, M, N, K, lower_only);
+        auto even = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+        const bool vec = even(A) && even(B) && lda % 2 == 0 && ldb % 2 == 0;
+        const int S = small_split64(ctx, M, N, K, lower_only, vec);
         if (S > 0) return gemm_small(ctx, mode == 1, lower_only, S, M, N, K, A, lda, B, ldb, C, ldc);
     }
     // 128x128 tiles only when they still give two waves of CTAs (one per SM)

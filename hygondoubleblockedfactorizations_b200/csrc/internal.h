@@ -331,7 +331,7 @@ int split_count(const hdbf_context* ctx, int M, int N, int K, bool tri, int* kc)
 // a tile's K (0: not taken), the same where an FP32 update takes this kernel
 // (sgemm.cu), and the launch (range: only if split_range_bad).
 int gemm_small_split(const hdbf_context* ctx, int M, int N, int K);
-int sgemm_small(const hdbf_context* ctx, int M, int N, int K, bool tri);
+int sgemm_small(const hdbf_context* ctx, int M, int N, int K, bool tri, bool vec);
 // Tiles of b x b of an M x N update (tri: on or below the diagonal), and CTAs of
 // one SM, the fullest, when `per` CTAs share each.
 inline long long tile_count(int M, int N, int b, bool tri)
@@ -376,7 +376,7 @@ struct SplitPlan {
     {
         int kc = 0;
         c->tc_plan = tc_sgemm_plan(c, M, N, K, false);
-        c->small_plan = sgemm_small(c, M, N, K, false);
+        c->small_plan = sgemm_small(c, M, N, K, false, true);
         const int S = split_count(c, M, N, K, false, &kc);
         c->split_kc = S > 1 ? kc : 0;
     }

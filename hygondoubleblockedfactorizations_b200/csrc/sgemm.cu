@@ -369,20 +369,24 @@ int split_count(const hdbf_context* ctx, int M, int N, int K, bool tri, int* kc)
 // to 8192 x 2048 x 2048 the choice is 0.1 % behind the better kernel, 12 % at worst
 // (4096 x 192 x 2048); the small kernel for all of them was up to 1.8 times slower
 // (triangle of 1000, K = 2048: 144 us, 79; 2048 x 512 x 2048: 142, 124; 3072 x 1536 x
-// 256: 76, 60), the large one up to 3.3 times (512 x 192 x 256: 41, 13).
-int sgemm_small(const hdbf_context* ctx, int M, int N, int K, bool tri)
+// 256: 76, 60), the large one up to 3.3 times (512 x 192 x 256: 41, 13).  Operands that
+// no 16-byte access fits (!vec) cost the small kernel 0.12 more a step and the large
+// one, unless it splits K, 400 steps a tile for its scattered C (4096 x 512 x 64 with
+// odd leading dimensions: 21 us, 54; 2001 x 2001 x 1024: 314, 271).
+int sgemm_small(const hdbf_context* ctx, int M, int N, int K, bool tri, bool vec)
 {
     const int S = gemm_small_split(ctx, M, N, K);
     if (S == 0) return 0;
-    const double small =
-        0.3 * (double)small_waves(ctx, M, N, tri, S) * (((K + S - 1) / S + 7) / 8 * 8 + 10);
+    const double small = (vec ? 0.3 : 0.42) * (double)small_waves(ctx, M, N, tri, S) *
+                         (((K + S - 1) / S + 7) / 8 * 8 + 10);
     int kc = K;
     const int parts = split_count(ctx, M, N, K, tri, &kc);
     if (parts < 2) kc = K;
     const long long sm = ctx->sm_count;
-    double large = (double)((tile_count(M, N, BM, tri) * parts + sm - 1) / sm) * kc *
-                   ((N + BN - 1) / BN * BN) / N;
+    const double waves = (double)((tile_count(M, N, BM, tri) * parts + sm - 1) / sm);
+    double large = waves * kc * ((N + BN - 1) / BN * BN) / N;
     if (parts > 1) large += 30.0 + 1e-5 * (parts + 1) * (double)M * N;
+    else if (!vec) large += 400.0 * waves;
     if (tri) large += 150.0;
     return small <= large ? S : 0;
 }
@@ -439,7 +443,7 @@ hdbf_status sgemm_launch(hdbf_context* ctx, int mode, bool lower_only, int M, in
                    N, K);
     if (!ri && mode != kTN) {
         const int small =
-            ctx->small_plan >= 0 ? ctx->small_plan : sgemm_small(ctx, M, N, K, lower_only);
+            ctx->small_plan >= 0 ? ctx->small_plan : sgemm_small(ctx, M, N, K, lower_only, vec);
         if (small > 0)
             return gemm_small(ctx, mode == kNN, lower_only, small, M, N, K, A, lda, B, ldb, C, ldc,
                               range);
