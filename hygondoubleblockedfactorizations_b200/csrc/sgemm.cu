@@ -365,14 +365,16 @@ int split_count(const hdbf_context* ctx, int M, int N, int K, bool tri, int* kc)
 // else 0.  Both costs are counted in steps of K of one 128 x 128 tile (0.095 us) on
 // the fullest SM: a 64 x 64 tile is 0.3 of one, its ring fills in 10 steps; partial
 // sums cost the 128 x 128 kernel a second launch and their traffic, a ragged last
-// tile column its share of a tile, a triangle 150 steps.  Measured over 595 shapes up
-// to 8192 x 2048 x 2048 the choice is 0.1 % behind the better kernel, 12 % at worst
-// (4096 x 192 x 2048); the small kernel for all of them was up to 1.8 times slower
-// (triangle of 1000, K = 2048: 144 us, 79; 2048 x 512 x 2048: 142, 124; 3072 x 1536 x
-// 256: 76, 60), the large one up to 3.3 times (512 x 192 x 256: 41, 13).  Operands that
-// no 16-byte access fits (!vec) cost the small kernel 0.12 more a step and the large
-// one, unless it splits K, 400 steps a tile for its scattered C (4096 x 512 x 64 with
-// odd leading dimensions: 21 us, 54; 2001 x 2001 x 1024: 314, 271).
+// tile column its share of a tile, a triangle 150 steps.  Operands that no 16-byte
+// access fits (!vec) cost the small kernel 0.12 more a step and the large one, unless
+// it splits K, 400 steps a tile for its scattered C.  The small kernel for all of them
+// was up to 1.8 times slower (triangle of 1000, K = 2048: 144 us, 79; 768 x 384 x 2048:
+// 60, 42; 3072 x 1536 x 256: 76, 60), the large one up to 3.3 times (512 x 192 x 256: 41,
+// 13; 4096 x 512 x 64 with odd leading dimensions: 54, 21).
+// The small kernel folds its sums every 256 of K.  A much longer chain in the large one
+// has larger errors (2048 x 300 x 4096 over [0,1), chains of 683: 1.7e-7 against
+// 8.5e-8), so above 352 (2048 in six) the small one keeps the update, although it may
+// take up to a third longer (3072 x 1536 x 2048: 516 us, 390).
 int sgemm_small(const hdbf_context* ctx, int M, int N, int K, bool tri, bool vec)
 {
     const int S = gemm_small_split(ctx, M, N, K);
@@ -382,6 +384,7 @@ int sgemm_small(const hdbf_context* ctx, int M, int N, int K, bool tri, bool vec
     int kc = K;
     const int parts = split_count(ctx, M, N, K, tri, &kc);
     if (parts < 2) kc = K;
+    if (kc > 352) return S;
     const long long sm = ctx->sm_count;
     const double waves = (double)((tile_count(M, N, BM, tri) * parts + sm - 1) / sm);
     double large = waves * kc * ((N + BN - 1) / BN * BN) / N;
