@@ -17,13 +17,14 @@
 // G x_{i-1}, but the two terms may be large against their difference: backward
 // errors of LU solves came out twice as large.)  x_i is written to a row-major copy
 // that consumers read with 16-byte loads, published with a release store of flag
-// i, and then to B.  Per block row, n = 16384, 16 columns: 4.2 us with the reduction
-// behind the last arrival too, 3.8 now.
+// i, and then to B.  Per block row, n = 16384, 4 columns: 4.2 us with the reduction
+// behind the last arrival too, 3.3 now.
 //
 // The effective triangle M is T itself (lower forward or upper backward) or
 // T^T (lower T read transposed, backward); op(inv) is inv or inv^T in the
 // same orientation, so one template flag covers both.
 #include "internal.h"
+#include "pair.cuh"
 
 namespace hdbf {
 namespace {
@@ -86,46 +87,62 @@ __device__ __forceinline__ void load_tile(float* dst, const float* T, long long 
     }
 }
 
-// p[e][c] = sum of M(r, k) Xs[k][g CW + c] over the e-th 16 of k, for a tile in
-// load_tile's orientation: four chains of 16 round less than one of 64.
-template <int CW, bool TR>
-__device__ __forceinline__ void tile_times(float p[4][CW], const float* M, const float* Xs, int xs,
-                                           int r, int g)
+// red[(e * NB + c) * 64 + r] = sum of M(r, k) Xs[k][c] over the e-th 16 of k, for a tile
+// in load_tile's orientation: four chains of 16 round less than one of 64.  A thread
+// takes four rows and a quarter of the columns of one of the sums, so that shared
+// memory is read a quarter as often as with a row per thread.
+template <int NB, bool TR>
+__device__ __forceinline__ void tile_times(float* red, const float* M, const float* Xs)
 {
-    constexpr int V = CW % 4 == 0 ? 4 : CW;  // columns per load: 2 or 4
+    constexpr int XS = NB + 4, CB = NB / 4;
+    const int e = threadIdx.x >> 6, q = threadIdx.x & 15, c0 = ((threadIdx.x >> 4) & 3) * CB;
+    Two<float> acc[4][CB / 2];  // [row][column pair]
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int c = 0; c < CW; ++c) p[e][c] = 0.f;
-#pragma unroll 2
+        for (int h = 0; h < CB / 2; ++h) acc[i][h] = Two<float>::zero();
+#pragma unroll
     for (int k = 0; k < kB / 4; k += 4) {
+        const int k0 = e * (kB / 4) + k;
+        float4 m[4];  // TR: rows q + 16 i at k0 .. k0 + 3; else k0 + f at rows 4 q .. 4 q + 3
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int k0 = e * (kB / 4) + k;
-            float a[4];
-            if (TR) {
-                const float4 v = *reinterpret_cast<const float4*>(M + r * kLd + k0);
-                a[0] = v.x; a[1] = v.y; a[2] = v.z; a[3] = v.w;
-            } else {
+        for (int f = 0; f < 4; ++f)
+            m[f] = *reinterpret_cast<const float4*>(TR ? M + (q + 16 * f) * kLd + k0
+                                                       : M + (k0 + f) * kLd + 4 * q);
 #pragma unroll
-                for (int f = 0; f < 4; ++f) a[f] = M[(k0 + f) * kLd + r];
+        for (int f = 0; f < 4; ++f) {
+            Two<float> x[CB / 2];
+            const float* p = Xs + (k0 + f) * XS + c0;
+#pragma unroll
+            for (int h = 0; h < CB / 2; h += 2) {
+                if (CB >= 4) load_pairs(p + 2 * h, x[h], x[(h + 1) % (CB / 2)]);
+                else x[h] = *reinterpret_cast<const Two<float>*>(p + 2 * h);
             }
 #pragma unroll
-            for (int f = 0; f < 4; ++f) {
-                const float* q = Xs + (k0 + f) * xs + g * CW;
+            for (int i = 0; i < 4; ++i) {
+                const float4 v = m[TR ? i : f];
+                const int w = TR ? f : i;
+                const float a = w == 0 ? v.x : w == 1 ? v.y : w == 2 ? v.z : v.w;
+                const Two<float> aa = Two<float>::make(a, a);
 #pragma unroll
-                for (int c = 0; c < CW; c += V) {
-                    float b[V];
-                    if (V == 4) {
-                        const float4 v = *reinterpret_cast<const float4*>(q + c);
-                        b[0] = v.x; b[1] = v.y; b[2 % V] = v.z; b[3 % V] = v.w;
-                    } else {
-                        const float2 v = *reinterpret_cast<const float2*>(q + c);
-                        b[0] = v.x; b[1] = v.y;
-                    }
+                for (int h = 0; h < CB / 2; ++h) acc[i][h].fma(aa, x[h]);
+            }
+        }
+    }
+    float* out = red + (e * NB + c0) * kB;
 #pragma unroll
-                    for (int i = 0; i < V; ++i) p[e][c + i] = fmaf(a[f], b[i], p[e][c + i]);
-                }
+    for (int h = 0; h < CB / 2; ++h) {
+        float v[2][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[i][h].get(v[0][i], v[1][i]);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            if (!TR) {
+                *reinterpret_cast<float4*>(out + (2 * h + c) * kB + 4 * q) =
+                    make_float4(v[c][0], v[c][1], v[c][2], v[c][3]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) out[(2 * h + c) * kB + q + 16 * i] = v[c][i];
             }
         }
     }
@@ -273,22 +290,25 @@ __global__ void __launch_bounds__(kWT, 2) trsv_wave_kernel(int n, int nrhs, cons
         }
         if (m > 0) {
             if (!take(dep(m - 1))) return;
-            float p[4][CW];
-            tile_times<CW, TR>(p, Gt, Xs, XS, r, g);
+            tile_times<NB, TR>(red, Gt, Xs);
+            __syncthreads();
 #pragma unroll
             for (int c = 0; c < CW; ++c)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) y[c] -= p[e][c];
-            __syncthreads();  // x_{i-1} has been read
+                for (int e = 0; e < 4; ++e) y[c] -= red[(e * NB + g * CW + c) * kB + r];
         }
 #pragma unroll
         for (int c = 0; c < CW; ++c) Xs[r * XS + g * CW + c] = (r < rows) ? y[c] : 0.f;
         __syncthreads();
         // x_i = op(inv_i) y_i
-        float x[CW], s[4][CW];
-        tile_times<CW, TR>(s, Is, Xs, XS, r, g);
+        tile_times<NB, TR>(red, Is, Xs);
+        __syncthreads();
+        float x[CW];
 #pragma unroll
-        for (int c = 0; c < CW; ++c) x[c] = (s[0][c] + s[1][c]) + (s[2][c] + s[3][c]);
+        for (int c = 0; c < CW; ++c) {
+            const float* s = red + (g * CW + c) * kB + r;
+            x[c] = (s[0] + s[NB * kB]) + (s[2 * NB * kB] + s[3 * NB * kB]);
+        }
         float* xdst = X + (long long)(i0 + r) * NB + g * CW;
 #pragma unroll
         for (int c = 0; c < CW; ++c) {
