@@ -102,8 +102,8 @@ hdbf_status dbtrsm_impl(hdbf_context* ctx, const T* L, long long ldl, T* B,
 // Order of the last diagonal block that is factored by one launch whatever the
 // block sizes: nothing is below it, so no panel solve has to wait for its parts.
 // The cluster kernel (potrf_block.cu) takes 15-16 us a 64-column tile there, panels
-// of 64 columns 18 us, wider ones more: n = 256 74 -> 66 us, n = 512 157 -> 124 us,
-// n = 2048 (512 / 64) 723 -> 693 us.  Two tiles gain nothing (196 and 199 us at n =
+// of 64 columns 18 us, wider ones more: n = 256 74 -> 62 us, n = 512 157 -> 125 us,
+// n = 2048 (512 / 64) 723 -> 705 us.  Two tiles gain nothing (196 and 199 us at n =
 // 640), nor does a block of 1024 (484 and 491 us at n = 1300).
 constexpr int kTailOrder = 512, kTailAbove = 128;
 template <class T>

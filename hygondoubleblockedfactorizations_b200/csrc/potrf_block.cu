@@ -10,9 +10,9 @@
 // column k, then update the trailing tiles while CTA 0 factors the next diagonal
 // tile.  Tiles travel through L2 (each is read by several CTAs); two barriers per
 // tile column are mbarriers in every CTA's shared memory on which all CTAs arrive
-// remotely.  What bounds it is CTA 0's chain, ~14.5 us a tile (factor 5.9, inverse
-// 2.3, products 3.2, the rest loads, stores and barriers): n = 256 60 us, n = 512
-// 118 us; with a grid-wide barrier twice per tile column and every step through L2
+// remotely.  What bounds it is CTA 0's chain, ~15 us a tile (factor 5.9, inverse
+// 2.8, products 3.2, the rest loads, stores and barriers): n = 256 57 us, n = 512
+// 120 us; with a grid-wide barrier twice per tile column and every step through L2
 // it took 96 and 207 us.
 // With the inverse requested, W = L^{-1} (lower, the strictly upper tiles zeroed)
 // is formed by a second, cooperative launch (tile_inverse_kernel) by recursive

@@ -9,7 +9,7 @@
 // threads and the solve by substitution, so that every column is as accurate as one
 // long substitution would make it (the product W21 = -W22 (L21 W11) is 0.5 us
 // shorter, but its error grows with the condition of L22).
-// One tile in one launch (load, factor, inverse, stores): 9.9 us; 62 us before,
+// One tile in one launch (load, factor, inverse, stores): 10.4 us; 62 us before,
 // with two barriers, an IEEE square root and a division per column of the
 // factor and one thread per column of the inverse, a division per row.
 #pragma once
